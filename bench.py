@@ -818,7 +818,7 @@ def bench_knn(dev, steps=5):
     nq, nt = 50000, 200000
     ops = 2.0 * nq * nt * 256  # +-1 dot products: one multiply and one add per bit per pair
     pk, pk_src = peaks()
-    fp8_peak = 2.0 * pk.get("bf16_tflops", 1900.0)  # dense FP8 issues at twice the bf16 rate
+    fp4_peak = 4.0 * pk.get("bf16_tflops", 1900.0)  # dense FP4 (K = 64) issues at four times the bf16 rate
     out = {"metric": "query x train pairs/s (brute-force k=2 Hamming kNN, 50,000 x 200,000)", "unit": "pairs/s"}
     for name, q, t in (("uniform", syn.random_descriptors(nq, 1), syn.random_descriptors(nt, 2)),
                        ("clustered", syn.clustered_descriptors(nq, 2000, 0.1, 3),
@@ -859,11 +859,11 @@ def bench_knn(dev, steps=5):
                      "tensor_cores_equal_popc": bool(same),
                      "e2e": {"value": nq * nt / e2e_s, "unit": "pairs/s", "h2d_bytes_per_step": 32 * (nq + nt),
                              "d2h_bytes_per_step": 16 * nq},
-                     "roofline": {"bound": "tensor", "kernel": "k_knn_tc (expansion + merge included in the time)",
-                                  "achieved": achieved, "peak": fp8_peak, "unit": "TFLOP/s",
-                                  "frac": achieved / fp8_peak,
-                                  "ops_per_step": ops, "peak_source": f"2 x bf16 burst ({pk_src}); dense FP8",
-                                  "ncu_tensor_pipe_active": "69.4 % (profiles/knn_tc_50kx200k.md)"}}
+                     "roofline": {"bound": "tensor", "kernel": "k_knn_tc (expansion + last choice included in the time)",
+                                  "achieved": achieved, "peak": fp4_peak, "unit": "TFLOP/s",
+                                  "frac": achieved / fp4_peak,
+                                  "ops_per_step": ops, "peak_source": f"4 x bf16 burst ({pk_src}); dense FP4",
+                                  "ncu_tensor_pipe_active": "70 % (profiles/knn_tc_50kx200k.md)"}}
         if name == "uniform":
             out["value"] = nq * nt / (tc_ms / 1e3)
             out["e2e"] = out[name]["e2e"]

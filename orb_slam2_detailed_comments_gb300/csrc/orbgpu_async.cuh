@@ -11,6 +11,7 @@
 namespace orbgpu {
 
 #define ORBGPU_SPIN_LIMIT (1u << 26)
+#define ORBGPU_POLL_NS 1000000u       // how long one poll may sleep: waiting warps leave the issue slots to the others
 #define ORBGPU_WAIT_NS 1000000000ull  // one second
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -40,13 +41,13 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
         uint32_t done;
         asm volatile(
             "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
             "selp.u32 %0, 1, 0, p;\n\t}"
             : "=r"(done)
-            : "r"(a), "r"(parity)
+            : "r"(a), "r"(parity), "r"(ORBGPU_POLL_NS)
             : "memory");
         if (done) return true;
-        if ((i & 31) == 31) {
+        if ((i & 7) == 7) {
             const uint64_t t = global_ns();
             if (t0 == 0) t0 = t;
             else if (t - t0 > ORBGPU_WAIT_NS) return false;

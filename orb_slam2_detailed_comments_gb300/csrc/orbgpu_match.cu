@@ -1014,6 +1014,24 @@ bool frame_ok(const orbgpu_frame* f) {
 
 }  // namespace
 
+// The matcher's scratch, grown to 'bytes', and its 64 page-locked bytes, for
+// the kNN (every call on a matcher is complete when it returns, so the
+// scratch is free between calls).
+int orbgpu_matcher_scratch_internal(orbgpu_matcher* m, size_t bytes, void** scratch, int** pinned) {
+    const int rc = ensure_scratch(m, bytes);
+    *scratch = m->scratch;
+    *pinned = m->h_pinned;
+    return rc;
+}
+// Gives back a scratch that one very large call grew beyond what a matcher
+// keeps between calls.
+void orbgpu_matcher_trim_internal(orbgpu_matcher* m) {
+    if (m->scratch_bytes <= (size_t)512 << 20) return;
+    cudaFree(m->scratch);
+    m->scratch = nullptr;
+    m->scratch_bytes = 0;
+}
+
 extern "C" int orbgpu_matcher_create(float nnratio, int check_orientation, void* stream, orbgpu_matcher** out) {
     if (!out) return ORBGPU_ERR_BAD_ARG;
     int dev;

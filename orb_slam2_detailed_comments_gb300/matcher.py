@@ -339,7 +339,7 @@ class ORBmatcher:
         """Brute-force k=2 over DescriptorDistance (device tensors) -> (idx1, d1, idx2, d2),
         plus the ratio test's accept mask (uint8) when 'ratio' is given.
 
-        algo 0: popcount kernel; 1: tensor cores (+-1 FP8 dot products); -1:
+        algo 0: popcount kernel; 1: tensor cores (+-1 FP4 dot products); -1:
         automatic (tuned crossover).  All give the same (distance, lower index
         first) results."""
         import torch

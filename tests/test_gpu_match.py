@@ -238,6 +238,31 @@ def test_knn_tensor_cores_oracle(torch, oracle, nq, nt):
         assert np.array_equal(a.cpu().numpy(), b), name
 
 
+# tile edges: query pairs of 256 rows, train tiles of 160 and groups of 32,
+# popcount tiles of 256 rows and shares of 32; several runs of one query pair
+@pytest.mark.parametrize("nq,nt", [(1, 31), (31, 32), (33, 33), (128, 159), (129, 160), (255, 161), (256, 255),
+                                   (257, 257), (513, 319), (40, 49999), (700, 25601)])
+def test_knn_tile_edges(torch, oracle, nq, nt):
+    """Both kernels at the edges of their tiles, with many equal distances
+    (bytes of two bits), from rows that start at an odd address for the
+    tensor-core path (which reads any address)."""
+    from orb_slam2_detailed_comments_gb300 import ORBmatcher
+    from orb_slam2_detailed_comments_gb300 import synthetic as syn
+    q, t = syn.random_descriptors(nq, 15) & 3, syn.random_descriptors(nt, 16) & 3
+    ref = oracle.knn2(q, t)
+    m = ORBmatcher()
+
+    def device(a, shift):
+        buf = torch.empty(a.size + shift, dtype=torch.uint8, device="cuda")
+        buf[shift:] = torch.from_numpy(a.reshape(-1)).cuda()
+        return buf[shift:].view(-1, 32)
+    for algo, shift in ((0, 0), (1, 0), (1, 3), (1, 4)):
+        dq, dt = device(q, shift), device(t, shift)
+        torch.cuda.synchronize()
+        for a, b, name in zip(m.knn2(dq, dt, algo=algo), ref, ("idx1", "d1", "idx2", "d2")):
+            assert np.array_equal(a.cpu().numpy(), b), (algo, shift, name)
+
+
 def test_knn_tensor_cores_golden_and_ties(torch, golden):
     """Golden vectors, then clustered descriptors (many equal distances) against
     the popcount kernel at a size with many slices."""
