@@ -16,6 +16,7 @@
 #include <cstring>
 #include <vector>
 
+#include "orbgpu_grid.cuh"
 #include "orbgpu_host.h"
 #include "orbgpu_stereo.cuh"
 
@@ -583,9 +584,10 @@ extern "C" void* orbgpu_batch_stream(const orbgpu_batch* b) { return b ? (void*)
 
 // ---------------------------------------------------------------- batched SearchByProjection
 // SearchByProjection(Frame&, vector<MapPoint*>, th) (src/ORBmatcher.cc:72-183)
-// for every frame of the last batch at once: grid build, candidate listing
-// (warp per map point, fixed-capacity slots) and the in-order resolution
-// (one warp per frame), five launches for the whole batch.
+// for every frame of the last batch at once, five launches: the grids' cell
+// starts (a block per frame) and records, the candidate lists (8 lanes per
+// map point, fixed-capacity rows), each list's best, and the in-order
+// resolution (a block per frame).
 namespace orbgpu {
 
 struct BatchFrameInfo {
@@ -594,145 +596,80 @@ struct BatchFrameInfo {
     float scale[16];
 };
 
-__global__ void k_bgrid_count(const orbgpu_keypoint* kps, const int* counts, int cap, const BatchFrameInfo* info,
-                              int* key_cell, int* cell_count) {
+// Every frame's cell starts (and the cells' fill positions); clears the call's
+// status words.
+__global__ void __launch_bounds__(1024) k_bgrid_starts(const orbgpu_keypoint* kps, const int* counts, int cap,
+                                                       const BatchFrameInfo* info, int* cell_start, int* cursor,
+                                                       int* status) {
+    __shared__ int s_cell[ORBGPU_GRID_CELLS];
+    const int f = blockIdx.x;
+    if (f == 0 && threadIdx.x < 4) status[threadIdx.x] = 0;
+    grid_starts_block(kps + (size_t)f * cap, min(counts[f], cap), 0.0f, 0.0f, info[f].invW, info[f].invH, s_cell,
+                      cell_start + (size_t)f * (ORBGPU_GRID_CELLS + 1));
+    for (int c = threadIdx.x; c < ORBGPU_GRID_CELLS; c += 1024) cursor[(size_t)f * ORBGPU_GRID_CELLS + c] = s_cell[c];
+}
+
+__global__ void __launch_bounds__(256) k_bgrid_fill(const orbgpu_keypoint* kps, const int* counts, int cap,
+                                                    const BatchFrameInfo* info, int* cursor, GridRec* recs) {
     const int f = blockIdx.y;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= min(counts[f], cap)) return;
     const orbgpu_keypoint kp = kps[(size_t)f * cap + i];
-    const int px = (int)roundf(__fmul_rn(__fsub_rn(kp.x, 0.0f), info[f].invW));
-    const int py = (int)roundf(__fmul_rn(__fsub_rn(kp.y, 0.0f), info[f].invH));
-    int c = -1;
-    if (px >= 0 && px < ORBGPU_GRID_COLS && py >= 0 && py < ORBGPU_GRID_ROWS) c = px * ORBGPU_GRID_ROWS + py;
-    key_cell[(size_t)f * cap + i] = c;
-    if (c >= 0) atomicAdd(&cell_count[f * (ORBGPU_GRID_COLS * ORBGPU_GRID_ROWS) + c], 1);
+    const int c = pos_in_grid(kp, 0.0f, 0.0f, info[f].invW, info[f].invH);
+    if (c >= 0) recs[(size_t)f * cap + atomicAdd(&cursor[(size_t)f * ORBGPU_GRID_CELLS + c], 1)] = grid_rec(kp, c, i);
 }
 
-__global__ void k_bgrid_scan(const int* cell_count, int* cell_start, int* cursor) {
-    __shared__ int s_scan[32];
-    const int ncell = ORBGPU_GRID_COLS * ORBGPU_GRID_ROWS;
-    const int f = blockIdx.x;
-    const int* cc = cell_count + (size_t)f * ncell;
-    int* cs = cell_start + (size_t)f * (ncell + 1);
-    int* cu = cursor + (size_t)f * ncell;
-    int base = 0;
-    for (int b0 = 0; b0 < ncell; b0 += blockDim.x) {
-        const int c = b0 + threadIdx.x;
-        const int v = c < ncell ? cc[c] : 0;
-        int tot;
-        const int ex = block_exclusive_scan(v, s_scan, &tot);
-        if (c < ncell) {
-            cs[c] = base + ex;
-            cu[c] = base + ex;
-        }
-        base += tot;
-    }
-    if (threadIdx.x == 0) cs[ncell] = base;
-}
-
-__global__ void k_bgrid_fill(const int* counts, int cap, const int* key_cell, int* cursor, int* cell_keys) {
-    const int f = blockIdx.y;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= min(counts[f], cap)) return;
-    const int c = key_cell[(size_t)f * cap + i];
-    if (c >= 0) cell_keys[(size_t)f * cap + atomicAdd(&cursor[f * (ORBGPU_GRID_COLS * ORBGPU_GRID_ROWS) + c], 1)] = i;
+__device__ __forceinline__ ProjFrame batch_frame(int f, int cap, const BatchFrameInfo* info, const int* cell_start,
+                                                 const GridRec* recs, const uint8_t* desc) {
+    ProjFrame F;
+    F.cell_start = cell_start + (size_t)f * (ORBGPU_GRID_CELLS + 1);
+    F.recs = recs + (size_t)f * cap;
+    F.desc = desc + (size_t)f * cap * 32;
+    F.uright = nullptr;
+    F.minX = F.minY = 0.0f;
+    F.invW = info[f].invW;
+    F.invH = info[f].invH;
+    F.scale = info[f].scale;
+    return F;
 }
 
 // BPROJ_SEG lanes per map point (32 / BPROJ_SEG map points per warp): a
-// window covers about a dozen grid cells and a handful of keypoints.
-#define BPROJ_SEG 16
-__global__ void k_bproj_candidates(const orbgpu_keypoint* kps, const uint8_t* desc, int cap, const BatchFrameInfo* info,
-                                   const int* cell_start, const int* cell_keys, const int* key_cell,
-                                   const orbgpu_mappoint* mps,
-                                   const uint8_t* mp_desc, const int* mp_off, float th, float nnratio, int slot_cap,
-                                   uint64_t* slots, int* slot_count, int* status) {
-    // A candidate with nnratio * dist > TH_HIGH (nnratio <= 1) can neither be
-    // accepted (dist > TH_HIGH) nor make an accepted best fail the ratio test
-    // (best <= TH_HIGH < nnratio * dist), so the lists leave it out.
+// window of the 64-frame step covers half a dozen grid columns with 13 to 73
+// keypoints, 2 to 7 of them in the disc and its levels.  Bound by the latency
+// of its chain of loads (map point, cell starts, record, descriptor): 0.080 ms
+// for 192,000 map points with 8 lanes, 0.089 with 16, 0.111 with 16 and the
+// keypoints read through the cells' key lists.
+#define BPROJ_SEG 8
+template <typename Key>
+__global__ void k_bproj_candidates(const uint8_t* desc, int cap, const BatchFrameInfo* info, const int* cell_start,
+                                   const GridRec* recs, const orbgpu_mappoint* mps, const uint8_t* mp_desc,
+                                   const int* mp_off, float th, float nnratio, int slot_cap, Key* slots,
+                                   int* slot_count, int* status) {
     constexpr int W = BPROJ_SEG;
-    const bool drop_far = nnratio <= 1.0f;
     const int f = blockIdx.y;
-    const int lane = threadIdx.x & 31, sl = lane & (W - 1), sbase = lane & ~(W - 1);
-    const unsigned smask = (W == 32 ? 0xffffffffu : ((1u << W) - 1)) << sbase;
+    const int lane = threadIdx.x & 31;
     const int local = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * (32 / W) + lane / W;
     const int imp = mp_off[f] + local;
     const bool have = imp < mp_off[f + 1];
     if (__all_sync(0xffffffffu, !have)) return;
-    const BatchFrameInfo& I = info[f];
-    const orbgpu_keypoint* K = kps + (size_t)f * cap;
-    const uint8_t* D = desc + (size_t)f * cap * 32;
-    const int* cs = cell_start + (size_t)f * (ORBGPU_GRID_COLS * ORBGPU_GRID_ROWS + 1);
-    const int* ck = cell_keys + (size_t)f * cap;
-    const int* kc = key_cell + (size_t)f * cap;
     orbgpu_mappoint mp{};
     if (have) mp = mps[imp];
-    bool active = have && mp.track_in_view && !mp.bad && mp.track_scale_level >= 0 && mp.track_scale_level < 16;
-    int x0 = 0, x1 = -1, y0 = 0, y1 = -1, level = 0;
-    float x = 0.f, y = 0.f, rr = 0.f;
-    if (active) {
-        level = mp.track_scale_level;
-        float r = mp.view_cos > 0.998f ? 2.5f : 4.0f;
-        if (th != 1.0f) r = __fmul_rn(r, th);
-        const float radius = __fmul_rn(r, I.scale[level]);
-        x = mp.proj_x;
-        y = mp.proj_y;
-        x0 = max(0, (int)floorf(__fmul_rn(__fsub_rn(__fsub_rn(x, 0.0f), radius), I.invW)));
-        x1 = min(ORBGPU_GRID_COLS - 1, (int)ceilf(__fmul_rn(__fadd_rn(__fsub_rn(x, 0.0f), radius), I.invW)));
-        y0 = max(0, (int)floorf(__fmul_rn(__fsub_rn(__fsub_rn(y, 0.0f), radius), I.invH)));
-        y1 = min(ORBGPU_GRID_ROWS - 1, (int)ceilf(__fmul_rn(__fadd_rn(__fsub_rn(y, 0.0f), radius), I.invH)));
-        active = x0 < ORBGPU_GRID_COLS && x1 >= 0 && y0 < ORBGPU_GRID_ROWS && y1 >= 0 && x0 <= x1 && y0 <= y1;
-        rr = __fmul_rn(radius, radius);
-    }
-    uint4 dm0 = make_uint4(0, 0, 0, 0), dm1 = dm0;  // the map point's descriptor
-    if (active) {
-        const uint4* dp = reinterpret_cast<const uint4*>(mp_desc + (size_t)imp * 32);
-        dm0 = dp[0];
-        dm1 = dp[1];
-    }
-    int total = 0;
-    seg_window_cols<W>(cs, ck, ORBGPU_GRID_ROWS, active, x0, x1, y0, y1, [&](int idx, bool valid) {
-        bool ok = false;
-        int dist = 256, c = 0;
-        if (valid) {
-            c = kc[idx];
-            const orbgpu_keypoint kp = K[idx];
-            ok = kp.octave >= level - 1 && kp.octave <= level;
-            if (ok) {
-                const float dx = __fsub_rn(kp.x, x), dy = __fsub_rn(kp.y, y);
-                ok = __fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)) < rr;
-            }
-            if (ok) {
-                const uint4* kd = reinterpret_cast<const uint4*>(D + (size_t)idx * 32);
-                dist = hamming256(dm0, dm1, kd[0], kd[1]);
-                ok = !(drop_far && __fmul_rn(nnratio, (float)dist) > (float)ORBGPU_TH_HIGH);
-            }
-        }
-        const unsigned msk = __ballot_sync(0xffffffffu, ok) & smask;
-        if (ok) {
-            const int pos = total + __popc(msk & ((1u << lane) - 1));
-            if (pos < slot_cap)
-                slots[(size_t)imp * slot_cap + pos] =
-                    ((uint64_t)(uint32_t)dist << 40) | ((uint64_t)(uint32_t)c << 20) | (uint64_t)(uint32_t)idx;
-        }
-        total += __popc(msk);
-    });
-    if (have && sl == 0) {
+    const int total = proj_candidates<W, Key>(batch_frame(f, cap, info, cell_start, recs, desc), mp, have,
+                                              mp_desc + (size_t)imp * 32, th, nnratio, slots + (size_t)imp * slot_cap,
+                                              slot_cap);
+    if (have && (lane & (W - 1)) == 0) {
         slot_count[imp] = total;
         if (total > slot_cap) atomicMax(status, total);
     }
 }
 
-// Parallel resolution by fixed-point rounds.  In the reference a map point
-// sees a keypoint as claimed iff an earlier map point of the same call took
-// it.  Round r evaluates every map point against the claims made by the
-// results of round r-1 (claim owner = smallest map point index that took the
-// keypoint); once a round changes no result, every map point's result is
-// consistent with the results of the map points before it, which by
-// induction over the map point order is the sequential result.  Three claim
+// The fixed-point rounds of proj_resolve_block in global memory, one launch
+// each, for frames that do not fit in shared memory (64-bit keys: any number
+// of keypoints).  Three claim
 // arrays rotate: read (round r-1's claims), write (round r's), and the one
 // cleared for round r+1.  A frame that has not converged after the last
 // round is replayed serially by k_bproj_resolve.
-#define BPROJ_ROUNDS 12
+#define BPROJ_ROUNDS 13
 #define BPROJ_NONE 0x7f7f7f7f
 
 __global__ void k_bproj_round(const orbgpu_keypoint* kps, int cap, const int* counts, const int* mp_off,
@@ -795,203 +732,35 @@ __global__ void k_bproj_round(const orbgpu_keypoint* kps, int cap, const int* co
     }
 }
 
-// The same fixed-point resolution with one block per frame and the whole
-// frame in shared memory: the map points' candidate keys (32 bits: distance,
-// GetFeaturesInArea cell, keypoint index -- the lexicographic order of the
-// 64-bit keys, all distinct), the keypoints' octaves, the results and two
-// claim arrays.  A map point's result is the best and second-best of its
-// candidates not claimed by an earlier map point in the previous round, i.e.
-// the first two such in key order: each thread keeps the four smallest keys
-// of its map points in registers and reads the whole list only when fewer
-// than two of them are unclaimed.  Rounds repeat until one changes nothing
-// (at most M + 1 rounds: round r fixes the first r + 1 map points).  Used
-// when every frame's candidates fit (smem_bytes of dynamic shared memory);
-// the global-memory rounds above handle the rest.
-#define BPROJ_MPT 4  // map points per thread with register top-4 lists (1024 threads: M <= 4096)
+// The PROJ_TOP smallest keys of every map point's list, on the whole device: in
+// the resolution's one block per frame the rows' latency was most of its time.
+__global__ void __launch_bounds__(256) k_bproj_top(int total_mp, int slot_cap, const uint32_t* slots,
+                                                   const int* slot_count, uint4* tops) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= total_mp) return;
+    const int cnt = min(slot_count[i], slot_cap);
+    uint32_t t[PROJ_TOP];
+    top_load(slots + (size_t)i * slot_cap, cnt, t);
+    if (cnt > 0) tops[2 * (size_t)i] = make_uint4(t[0], t[1], t[2], t[3]);
+    if (cnt > 4) tops[2 * (size_t)i + 1] = make_uint4(t[4], t[5], t[6], t[7]);
+}
+
+// The resolution with one block per frame (proj_resolve_block).
 __global__ void __launch_bounds__(1024)
     k_bproj_resolve_smem(const orbgpu_keypoint* kps, int cap, const int* counts, const int* mp_off, int slot_cap,
-                         const uint64_t* slots, const int* slot_count, float nnratio, int smem_bytes,
+                         const uint32_t* slots, const int* slot_count, const uint4* tops, float nnratio,
                          int* match_out, int* nmatches, int* status) {
     extern __shared__ __align__(16) int s_dyn[];
-    __shared__ int s_scan[32];
-    __shared__ int s_flag[3];
     const int f = blockIdx.x;
-    const int tid = threadIdx.x, nt = blockDim.x;
-    const int mp0 = mp_off[f], M = mp_off[f + 1] - mp0;
-    const int n = min(counts[f], cap);
-    constexpr int NONE = 0x7fffffff;
-    constexpr uint32_t NOKEY = 0xFFFFFFFFu;
-    int* s_start = s_dyn;  // M + 1: candidate list of map point i
-    int base = 0;
-    for (int i0 = 0; i0 < M; i0 += nt) {
-        const int i = i0 + tid;
-        const int v = i < M ? min(slot_count[mp0 + i], slot_cap) : 0;
-        int tot;
-        const int ex = block_exclusive_scan(v, s_scan, &tot);
-        if (i < M) s_start[i] = base + ex;
-        base += tot;
-    }
-    if (4L * (2 * M + 1 + 2 * cap + base) + cap + 16 > smem_bytes) {  // the frame's candidates do not fit
-        if (tid == 0) atomicOr(status + 2, 1);
-        return;
-    }
-    int* s_res = s_start + (M + 1);                          // M
-    int* cr = s_res + M;                                     // cap: claims of the previous round
-    int* cw = cr + cap;                                      // cap: claims of this round
-    uint32_t* s_key = reinterpret_cast<uint32_t*>(cw + cap);  // base
-    uint8_t* s_oct = reinterpret_cast<uint8_t*>(s_key + base);  // cap
-    if (tid == 0) s_start[M] = base;
-    if (tid < 3) s_flag[tid] = 0;
-    for (int k = tid; k < cap; k += nt) {
-        cr[k] = NONE;
-        cw[k] = NONE;
-    }
-    for (int k = tid; k < n; k += nt) s_oct[k] = (uint8_t)kps[(size_t)f * cap + k].octave;
-    __syncthreads();
-    // keys, one thread per map point (independent loads); the four smallest of
-    // the thread's first BPROJ_MPT map points kept in registers
-    uint32_t top[BPROJ_MPT][4];
-    int tcnt[BPROJ_MPT];
-#pragma unroll
-    for (int q = 0; q < BPROJ_MPT; q++) {
-        tcnt[q] = 0;
-#pragma unroll
-        for (int j = 0; j < 4; j++) top[q][j] = NOKEY;
-    }
-    for (int i = tid, q = 0; i < M; i += nt, q++) {
-        const int s0 = s_start[i], cnt = s_start[i + 1] - s0;
-        const uint64_t* S = slots + (size_t)(mp0 + i) * slot_cap;
-        uint32_t t0 = NOKEY, t1 = NOKEY, t2 = NOKEY, t3 = NOKEY;
-        for (int b = 0; b < cnt; b++) {
-            const uint64_t key = S[b];
-            const uint32_t dist = (uint32_t)(key >> 40), cell = (uint32_t)(key >> 20) & 0xFFFFFu,
-                           idx = (uint32_t)key & 0xFFFFFu;
-            const uint32_t k32 = dist >= 256 ? NOKEY : (dist << 24) | (cell << 12) | idx;
-            s_key[s0 + b] = k32;
-            // insertion into the sorted four
-            if (k32 < t3) {
-                if (k32 < t2) {
-                    t3 = t2;
-                    if (k32 < t1) {
-                        t2 = t1;
-                        if (k32 < t0) {
-                            t1 = t0;
-                            t0 = k32;
-                        } else {
-                            t1 = k32;
-                        }
-                    } else {
-                        t2 = k32;
-                    }
-                } else {
-                    t3 = k32;
-                }
-            }
-        }
-#pragma unroll
-        for (int qq = 0; qq < BPROJ_MPT; qq++)
-            if (qq == q) {
-                top[qq][0] = t0;
-                top[qq][1] = t1;
-                top[qq][2] = t2;
-                top[qq][3] = t3;
-                tcnt[qq] = cnt;
-            }
-        s_res[i] = -2;
-    }
-    // map point i's result from claims cr: the first two candidates in key
-    // order that no earlier map point claimed
-    auto decide = [&](int i, uint32_t best, uint32_t second) -> int {
-        if (best == NOKEY) return -1;
-        const int bestDist = (int)(best >> 24);
-        const int bestIdx = (int)(best & 0xFFFu);
-        const int bestLevel = s_oct[bestIdx];
-        const int bestDist2 = second == NOKEY ? 256 : (int)(second >> 24);
-        const int bestLevel2 = second == NOKEY ? -1 : s_oct[second & 0xFFFu];
-        if (bestDist <= ORBGPU_TH_HIGH && !(bestLevel == bestLevel2 && (float)bestDist > __fmul_rn(nnratio, (float)bestDist2)))
-            return bestIdx;
-        return -1;
-    };
-    auto full_scan = [&](int i, uint32_t& best, uint32_t& second) {
-        best = NOKEY;
-        second = NOKEY;
-        for (int e = s_start[i]; e < s_start[i + 1]; e++) {
-            const uint32_t key = s_key[e];
-            if (key == NOKEY || cr[key & 0xFFFu] < i) continue;
-            if (key < best) {
-                second = best;
-                best = key;
-            } else if (key < second) {
-                second = key;
-            }
-        }
-    };
-    bool converged = M == 0;
-    int rounds_run = 0;
-    for (int round = 0; round <= M + 1 && !converged; round++) {
-        rounds_run = round + 1;
-        if (tid == 0) s_flag[(round + 1) % 3] = 0;
-        __syncthreads();
-#pragma unroll
-        for (int q = 0; q < BPROJ_MPT; q++) {
-            const int i = tid + q * nt;
-            if (i >= M) continue;
-            uint32_t best = NOKEY, second = NOKEY;
-            int found = 0;
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const uint32_t key = top[q][j];
-                if (found < 2 && key != NOKEY && !(cr[key & 0xFFFu] < i)) {
-                    if (found == 0) best = key;
-                    else second = key;
-                    found++;
-                }
-            }
-            if (found < 2 && tcnt[q] > 4) full_scan(i, best, second);
-            const int r = decide(i, best, second);
-            if (r != s_res[i]) {
-                s_res[i] = r;
-                s_flag[round % 3] = 1;
-            }
-            if (r >= 0) atomicMin(&cw[r], i);
-        }
-        for (int i = tid + BPROJ_MPT * nt; i < M; i += nt) {
-            uint32_t best, second;
-            full_scan(i, best, second);
-            const int r = decide(i, best, second);
-            if (r != s_res[i]) {
-                s_res[i] = r;
-                s_flag[round % 3] = 1;
-            }
-            if (r >= 0) atomicMin(&cw[r], i);
-        }
-        __syncthreads();
-        converged = s_flag[round % 3] == 0;
-        // this round's claims are read by the next; the array read now is cleared for writing
-        int* t = cr;
-        cr = cw;
-        cw = t;
-        if (!converged)
-            for (int k = tid; k < cap; k += nt) cw[k] = NONE;
-    }
-    if (tid == 0) {
-        if (!converged) atomicOr(status + 2, 2);
-        atomicMax(status + 3, rounds_run);
-    }
+    const int mp0 = mp_off[f], n = min(counts[f], cap);
     int* Mo = match_out + (size_t)f * cap;
-    for (int k = tid; k < cap; k += nt) Mo[k] = k < n ? -1 : -3;
-    __syncthreads();
-    int nm = 0;
-    for (int i = tid; i < M; i += nt) {
-        const int r = s_res[i];
-        if (r >= 0) {
-            Mo[r] = i;
-            nm++;
-        }
+    const int rounds = proj_resolve_block(kps + (size_t)f * cap, n, mp_off[f + 1] - mp0, slots + (size_t)mp0 * slot_cap,
+                                          slot_cap, slot_count + mp0, tops + 2 * (size_t)mp0, nnratio, nullptr, s_dyn, Mo, nmatches + f);
+    for (int k = n + threadIdx.x; k < cap; k += blockDim.x) Mo[k] = -3;
+    if (threadIdx.x == 0) {
+        if (rounds == 0) atomicOr(status + 2, 2);
+        atomicMax(status + 3, rounds);
     }
-    int tot;
-    block_exclusive_scan(nm, s_scan, &tot);
-    if (tid == 0) nmatches[f] = tot;
 }
 
 // Writes match_out / nmatches from the converged results; frames that did
@@ -1075,8 +844,6 @@ struct orbgpu_batch_proj {
     size_t bytes = 0;
     int slot_cap = 64;
     int* h_pinned = nullptr;
-    int* h_cands = nullptr;  // per-frame candidate totals (pinned)
-    int h_cands_cap = 0;
     int last_serial_frames = 0;
     int last_launches = 0;
     int last_rounds = 0;  // fixed-point rounds of the slowest frame (shared-memory resolution)
@@ -1119,15 +886,22 @@ extern "C" int orbgpu_batch_search_by_projection(orbgpu_batch* b, const orbgpu_k
     orbgpu_batch_proj& P = g_bproj;
     if (!P.h_pinned) ORBGPU_CUDA_TRY(cudaMallocHost(&P.h_pinned, 64));
     cudaStream_t st = b->stream;
+    // every frame in shared memory when it fits (one launch), else the
+    // global-memory fixed-point rounds and the result write-out (serial replay
+    // for any frame that did not converge)
+    const bool smem = P.mode == 0 && cap < ORBGPU_KEY32_MAX_N && proj_resolve_smem(cap, max_mp) <= 224 * 1024;
+    const size_t key_bytes = smem ? sizeof(uint32_t) : sizeof(uint64_t);
     for (int attempt = 0; attempt < 3; attempt++) {
-        const size_t need = sizeof(BatchFrameInfo) * nf + sizeof(int) * ((size_t)nf * ncell * 2 + (size_t)nf * (ncell + 1) +
-                                                                      (size_t)nf * cap * 5 + (nf + 1) + 2 * total_mp +
-                                                                      BPROJ_ROUNDS * nf + nf + 16) +
-                            sizeof(uint64_t) * (size_t)std::max(1, total_mp) * P.slot_cap + 8 * 256;
+        const size_t need = sizeof(BatchFrameInfo) * nf + sizeof(GridRec) * (size_t)nf * cap +
+                            2 * sizeof(uint4) * (size_t)std::max(1, total_mp) +
+                            sizeof(int) * ((size_t)nf * (2 * ncell + 1) + (size_t)nf * cap * 3 + (nf + 1) + 2 * total_mp +
+                                           BPROJ_ROUNDS * nf + nf + 16) +
+                            key_bytes * (size_t)std::max(1, total_mp) * P.slot_cap + 16 * 256;
         if (need > P.bytes) {
             ORBGPU_CUDA_TRY(cudaStreamSynchronize(st));
             if (P.scratch) cudaFree(P.scratch);
             P.scratch = nullptr;
+            P.bytes = 0;
             ORBGPU_CUDA_TRY(dev_malloc(&P.scratch, need));
             P.bytes = need;
             P.last_upload.clear();
@@ -1141,14 +915,13 @@ extern "C" int orbgpu_batch_search_by_projection(orbgpu_batch* b, const orbgpu_k
         };
         BatchFrameInfo* info = (BatchFrameInfo*)take(sizeof(BatchFrameInfo) * nf);
         int* d_off = (int*)take(sizeof(int) * (nf + 1));  // uploaded with info in one copy
-        int* cell_count = (int*)take(sizeof(int) * (size_t)nf * ncell);
-        int* cursor = (int*)take(sizeof(int) * (size_t)nf * ncell);
         int* cell_start = (int*)take(sizeof(int) * (size_t)nf * (ncell + 1));
-        int* key_cell = (int*)take(sizeof(int) * (size_t)nf * cap);
-        int* cell_keys = (int*)take(sizeof(int) * (size_t)nf * cap);
+        int* cursor = (int*)take(sizeof(int) * (size_t)nf * ncell);
+        GridRec* recs = (GridRec*)take(sizeof(GridRec) * (size_t)nf * cap);
+        uint4* tops = (uint4*)take(2 * sizeof(uint4) * (size_t)std::max(1, total_mp));
         int* slot_count = (int*)take(sizeof(int) * std::max(1, total_mp));
         int* status = (int*)take(sizeof(int) * 4);
-        uint64_t* slots = (uint64_t*)take(sizeof(uint64_t) * (size_t)std::max(1, total_mp) * P.slot_cap);
+        void* slots = take(key_bytes * (size_t)std::max(1, total_mp) * P.slot_cap);
         int* claims3 = (int*)take(sizeof(int) * (size_t)3 * nf * cap);
         int* res = (int*)take(sizeof(int) * std::max(1, total_mp));
         int* changed = (int*)take(sizeof(int) * BPROJ_ROUNDS * nf);
@@ -1180,32 +953,21 @@ extern "C" int orbgpu_batch_search_by_projection(orbgpu_batch* b, const orbgpu_k
                 P.last_upload.swap(up);
             }
         }
-        ORBGPU_CUDA_TRY(cudaMemsetAsync(cell_count, 0, sizeof(int) * (size_t)nf * ncell, st));
-        ORBGPU_CUDA_TRY(cudaMemsetAsync(status, 0, sizeof(int) * 4, st));
-        dim3 gk((cap + 255) / 256, nf);
-        k_bgrid_count<<<gk, 256, 0, st>>>(kps, counts, cap, info, key_cell, cell_count);
-        k_bgrid_scan<<<nf, 1024, 0, st>>>(cell_count, cell_start, cursor);
-        k_bgrid_fill<<<gk, 256, 0, st>>>(counts, cap, key_cell, cursor, cell_keys);
+        k_bgrid_starts<<<nf, 1024, 0, st>>>(kps, counts, cap, info, cell_start, cursor, status);
+        k_bgrid_fill<<<dim3((cap + 255) / 256, nf), 256, 0, st>>>(kps, counts, cap, info, cursor, recs);
         const int wpb = 8;
         const int mp_per_block = wpb * (32 / BPROJ_SEG);
         dim3 gc((std::max(1, max_mp) + mp_per_block - 1) / mp_per_block, nf);
-        k_bproj_candidates<<<gc, 32 * wpb, 0, st>>>(kps, desc, cap, info, cell_start, cell_keys, key_cell, mappoints,
-                                                   mp_descriptors, d_off, th, nnratio, P.slot_cap, slots, slot_count,
-                                                   status);
-        // every frame in shared memory when it fits (one launch, sized for up
-        // to t_cap candidates per frame; the kernel reports a frame above it),
-        // else the global-memory fixed-point rounds and the result write-out
-        // (serial replay for any frame that did not converge)
-        // s_start, s_res, two claim arrays (ints), octaves and dirty flags
-        // (bytes), then 4 bytes per candidate (6 with the keypoint index):
-        // the kernel lays its frame out once it knows the frame's candidates
-        const size_t fixed = sizeof(int) * ((size_t)2 * max_mp + 1 + 2 * (size_t)cap) + (size_t)cap + (size_t)max_mp + 64;
-        const size_t smem_max = 226 * 1024;  // below the 227 KiB per-block limit with the static part
-        if (P.mode == 0 && cap < 4096 && fixed + 4 * 1024 <= smem_max) {
-            const size_t smem = smem_max;
+        if (smem) {
+            k_bproj_candidates<uint32_t><<<gc, 32 * wpb, 0, st>>>(desc, cap, info, cell_start, recs, mappoints, mp_descriptors,
+                                                                 d_off, th, nnratio, P.slot_cap, (uint32_t*)slots,
+                                                                 slot_count, status);
+            k_bproj_top<<<(std::max(1, total_mp) + 255) / 256, 256, 0, st>>>(total_mp, P.slot_cap, (const uint32_t*)slots,
+                                                                            slot_count, tops);
             ORBGPU_CUDA_TRY(allow_max_dynamic_smem(k_bproj_resolve_smem));
-            k_bproj_resolve_smem<<<nf, 1024, smem, st>>>(kps, cap, counts, d_off, P.slot_cap, slots, slot_count, nnratio,
-                                                         (int)smem, match_out, nmatches, status);
+            k_bproj_resolve_smem<<<nf, 1024, proj_resolve_smem(cap, max_mp), st>>>(
+                kps, cap, counts, d_off, P.slot_cap, (const uint32_t*)slots, slot_count, tops, nnratio,
+                match_out, nmatches, status);
             ORBGPU_CUDA_TRY(cudaGetLastError());
             ORBGPU_CUDA_TRY(cudaMemcpyAsync(P.h_pinned, status, sizeof(int) * 4, cudaMemcpyDeviceToHost, st));
             ORBGPU_CUDA_TRY(cudaStreamSynchronize(st));
@@ -1214,23 +976,25 @@ extern "C" int orbgpu_batch_search_by_projection(orbgpu_batch* b, const orbgpu_k
                 continue;
             }
             P.last_serial_frames = 0;
-            P.last_launches = 4 + 1;
+            P.last_launches = 5;
             P.last_rounds = P.h_pinned[3];
-            if (P.h_pinned[2] & 2) {
+            if (P.h_pinned[2]) {
                 orbgpu_set_last_error("batched projection: shared-memory resolution failed", __FILE__, __LINE__);
                 return ORBGPU_ERR_CUDA;
             }
-            if (!(P.h_pinned[2] & 1)) return ORBGPU_OK;
-            // a frame above t_cap: the global-memory rounds below
-        } else {
-            ORBGPU_CUDA_TRY(cudaMemcpyAsync(P.h_pinned, status, sizeof(int), cudaMemcpyDeviceToHost, st));
-            ORBGPU_CUDA_TRY(cudaStreamSynchronize(st));
-            if (P.h_pinned[0] > P.slot_cap) {
-                P.slot_cap = ((P.h_pinned[0] + 63) / 64) * 64;
-                continue;
-            }
+            return ORBGPU_OK;
         }
-        P.last_launches = 4 + BPROJ_ROUNDS + 1;
+        k_bproj_candidates<uint64_t><<<gc, 32 * wpb, 0, st>>>(desc, cap, info, cell_start, recs, mappoints, mp_descriptors,
+                                                             d_off, th, nnratio, P.slot_cap, (uint64_t*)slots, slot_count,
+                                                             status);
+        ORBGPU_CUDA_TRY(cudaGetLastError());
+        ORBGPU_CUDA_TRY(cudaMemcpyAsync(P.h_pinned, status, sizeof(int), cudaMemcpyDeviceToHost, st));
+        ORBGPU_CUDA_TRY(cudaStreamSynchronize(st));
+        if (P.h_pinned[0] > P.slot_cap) {
+            P.slot_cap = ((P.h_pinned[0] + 63) / 64) * 64;
+            continue;
+        }
+        P.last_launches = 3 + BPROJ_ROUNDS + 1;
         const int warps = std::max((std::max(1, max_mp) + wpb - 1) / wpb * wpb, ((cap + 31) / 32 + wpb - 1) / wpb * wpb);
         P.h_pinned[1] = warps;
         ORBGPU_CUDA_TRY(cudaMemcpyAsync(nwarp, &P.h_pinned[1], sizeof(int), cudaMemcpyHostToDevice, st));
@@ -1239,9 +1003,9 @@ extern "C" int orbgpu_batch_search_by_projection(orbgpu_batch* b, const orbgpu_k
         ORBGPU_CUDA_TRY(cudaMemsetAsync(changed, 0, sizeof(int) * BPROJ_ROUNDS * nf, st));
         dim3 gr(warps / wpb, nf);
         for (int r = 0; r < BPROJ_ROUNDS; r++)
-            k_bproj_round<<<gr, 32 * wpb, 0, st>>>(kps, cap, counts, d_off, P.slot_cap, slots, slot_count, nnratio, r,
+            k_bproj_round<<<gr, 32 * wpb, 0, st>>>(kps, cap, counts, d_off, P.slot_cap, (const uint64_t*)slots, slot_count, nnratio, r,
                                                   claims3, res, changed, nwarp);
-        k_bproj_finish<<<nf, 32, 0, st>>>(kps, cap, counts, d_off, P.slot_cap, slots, slot_count, nnratio, changed, res,
+        k_bproj_finish<<<nf, 32, 0, st>>>(kps, cap, counts, d_off, P.slot_cap, (const uint64_t*)slots, slot_count, nnratio, changed, res,
                                          match_out, nmatches, status);
         ORBGPU_CUDA_TRY(cudaGetLastError());
         ORBGPU_CUDA_TRY(cudaMemcpyAsync(P.h_pinned + 2, status + 1, sizeof(int), cudaMemcpyDeviceToHost, st));
@@ -1281,177 +1045,193 @@ __device__ __forceinline__ float bpose_row(const float* row, float X0, float X1,
     return __fadd_rn(__double2float_rn(s), row[3]);
 }
 
-__global__ void k_bpf_candidates(const orbgpu_keypoint* kps, const uint8_t* desc, int cap, const BatchFrameInfo* info,
-                                 const int* cell_start, const int* cell_keys, const int* key_cell,
-                                 const BatchMotion* motions,
-                                 const orbgpu_keypoint* last_kps, const orbgpu_frame_mappoint* last_mps,
-                                 const uint8_t* last_desc, const int* last_off, float th, int slot_cap,
-                                 uint32_t* slots, int* slot_count, int* status, int* frame_cands) {
-    const int ncell = ORBGPU_GRID_COLS * ORBGPU_GRID_ROWS;
+// Every frame's grid, in one launch; clears the call's status words.
+__global__ void __launch_bounds__(1024) k_bgrid_build(const orbgpu_keypoint* kps, const int* counts, int cap,
+                                                      const BatchFrameInfo* info, int* cell_start, GridRec* recs,
+                                                      int* status) {
+    const int f = blockIdx.x;
+    if (f == 0 && threadIdx.x < 4) status[threadIdx.x] = 0;
+    grid_build_block(kps + (size_t)f * cap, min(counts[f], cap), 0.0f, 0.0f, info[f].invW, info[f].invH,
+                     cell_start + (size_t)f * (ORBGPU_GRID_CELLS + 1), recs + (size_t)f * cap);
+}
+
+// BPF_PER map points per warp: the first BPF_PER lanes project one each (the
+// double products go to a pipe of two lanes a cycle, where a warp computing
+// one map point on all its lanes took the pipe for most of the kernel), then
+// 16 lanes walk each window, two at a time.
+#define BPF_SEG 16
+#define BPF_PER 4
+__global__ void k_bpf_candidates(const uint8_t* desc, int cap, const BatchFrameInfo* info, const int* cell_start,
+                                 const GridRec* recs, const BatchMotion* motions, const orbgpu_keypoint* last_kps,
+                                 const orbgpu_frame_mappoint* last_mps, const uint8_t* last_desc, const int* last_off,
+                                 float th, int slot_cap, uint32_t* slots, int* slot_count, int* status) {
+    constexpr int W = BPF_SEG;
     const int f = blockIdx.y;
     const int lane = threadIdx.x & 31;
-    const int local = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    const int i = last_off[f] + local;
-    if (i >= last_off[f + 1]) return;
-    const orbgpu_frame_mappoint mp = last_mps[i];
+    const int first = last_off[f] + (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * BPF_PER;
+    const int end = last_off[f + 1];
+    if (first >= end) return;
     const BatchMotion& mo = motions[f];
-    const BatchFrameInfo& I = info[f];
-    const orbgpu_keypoint* K = kps + (size_t)f * cap;
-    const uint8_t* D = desc + (size_t)f * cap * 32;
-    const int* cs = cell_start + (size_t)f * (ncell + 1);
-    const int* ck = cell_keys + (size_t)f * cap;
-    const int* kc = key_cell + (size_t)f * cap;
-    const int oct = last_kps[i].octave;
-    int total = 0;
-    bool live = (mp.flags & ORBGPU_MP_PRESENT) && !(mp.flags & ORBGPU_MP_OUTLIER) && oct >= 0 && oct < 16;
+    const ProjFrame F = batch_frame(f, cap, info, cell_start, recs, desc);
     float u = 0.f, v = 0.f;
-    if (live) {
-        const float xc = bpose_row(mo.T, mp.x, mp.y, mp.z);
-        const float yc = bpose_row(mo.T + 4, mp.x, mp.y, mp.z);
-        const float zc = bpose_row(mo.T + 8, mp.x, mp.y, mp.z);
-        const float invzc = __double2float_rn(__ddiv_rn(1.0, (double)zc));
-        u = __fadd_rn(__fmul_rn(__fmul_rn(mo.fx, xc), invzc), mo.cx);
-        v = __fadd_rn(__fmul_rn(__fmul_rn(mo.fy, yc), invzc), mo.cy);
-        live = !(invzc < 0.f) && isfinite(u) && isfinite(v) && !(u < 0.0f || u > mo.maxX) && !(v < 0.0f || v > mo.maxY);
+    int oct = -1;  // -1: no window
+    if (lane < BPF_PER && first + lane < end) {
+        const orbgpu_frame_mappoint mp = last_mps[first + lane];
+        const int o = last_kps[first + lane].octave;
+        if ((mp.flags & ORBGPU_MP_PRESENT) && !(mp.flags & ORBGPU_MP_OUTLIER) && o >= 0 && o < 16) {
+            const float xc = bpose_row(mo.T, mp.x, mp.y, mp.z);
+            const float yc = bpose_row(mo.T + 4, mp.x, mp.y, mp.z);
+            const float zc = bpose_row(mo.T + 8, mp.x, mp.y, mp.z);
+            const float invzc = __double2float_rn(__ddiv_rn(1.0, (double)zc));
+            u = __fadd_rn(__fmul_rn(__fmul_rn(mo.fx, xc), invzc), mo.cx);
+            v = __fadd_rn(__fmul_rn(__fmul_rn(mo.fy, yc), invzc), mo.cy);
+            if (!(invzc < 0.f) && isfinite(u) && isfinite(v) && !(u < 0.0f || u > mo.maxX) && !(v < 0.0f || v > mo.maxY))
+                oct = o;
+        }
     }
-    if (live) {
-        const float radius = __fmul_rn(th, I.scale[oct]);
-        int minL, maxL;
-        if (mo.level_mode == 1) {
-            minL = oct;
-            maxL = -1;
-        } else if (mo.level_mode == 2) {
-            minL = 0;
-            maxL = oct;
-        } else {
-            minL = oct - 1;
-            maxL = oct + 1;
+    const int sbase = lane & ~(W - 1);
+    const unsigned smask = ((1u << W) - 1) << sbase;
+#pragma unroll 1
+    for (int p = 0; p < BPF_PER; p += 32 / W) {
+        const int src = p + lane / W, i = first + src;
+        const float uu = __shfl_sync(0xffffffffu, u, src), vv = __shfl_sync(0xffffffffu, v, src);
+        const int o = __shfl_sync(0xffffffffu, oct, src);
+        bool active = o >= 0;
+        int minL = 0, maxL = -1, x0 = 0, x1 = -1, y0 = 0, y1 = -1;
+        float rr = 0.f;
+        uint4 dm0 = make_uint4(0, 0, 0, 0), dm1 = dm0;
+        if (active) {
+            const float radius = __fmul_rn(th, F.scale[o]);
+            if (mo.level_mode == 1) {
+                minL = o;
+                maxL = -1;
+            } else if (mo.level_mode == 2) {
+                minL = 0;
+                maxL = o;
+            } else {
+                minL = o - 1;
+                maxL = o + 1;
+            }
+            x0 = max(0, (int)floorf(__fmul_rn(__fsub_rn(__fsub_rn(uu, 0.0f), radius), F.invW)));
+            x1 = min(ORBGPU_GRID_COLS - 1, (int)ceilf(__fmul_rn(__fadd_rn(__fsub_rn(uu, 0.0f), radius), F.invW)));
+            y0 = max(0, (int)floorf(__fmul_rn(__fsub_rn(__fsub_rn(vv, 0.0f), radius), F.invH)));
+            y1 = min(ORBGPU_GRID_ROWS - 1, (int)ceilf(__fmul_rn(__fadd_rn(__fsub_rn(vv, 0.0f), radius), F.invH)));
+            active = x0 < ORBGPU_GRID_COLS && x1 >= 0 && y0 < ORBGPU_GRID_ROWS && y1 >= 0 && x0 <= x1 && y0 <= y1;
+            rr = __fmul_rn(radius, radius);
+            const uint4* dp = reinterpret_cast<const uint4*>(last_desc + (size_t)i * 32);
+            dm0 = dp[0];
+            dm1 = dp[1];
         }
         const bool check = (minL > 0) || (maxL >= 0);  // GetFeaturesInArea's level test (src/Frame.cc:628)
-        const int x0 = max(0, (int)floorf(__fmul_rn(__fsub_rn(__fsub_rn(u, 0.0f), radius), I.invW)));
-        const int x1 = min(ORBGPU_GRID_COLS - 1, (int)ceilf(__fmul_rn(__fadd_rn(__fsub_rn(u, 0.0f), radius), I.invW)));
-        const int y0 = max(0, (int)floorf(__fmul_rn(__fsub_rn(__fsub_rn(v, 0.0f), radius), I.invH)));
-        const int y1 = min(ORBGPU_GRID_ROWS - 1, (int)ceilf(__fmul_rn(__fadd_rn(__fsub_rn(v, 0.0f), radius), I.invH)));
-        if (x0 < ORBGPU_GRID_COLS && x1 >= 0 && y0 < ORBGPU_GRID_ROWS && y1 >= 0) {
-            const uint8_t* dmp = last_desc + (size_t)i * 32;
-            const float rr = __fmul_rn(radius, radius);
-            warp_window_keys(cs, ck, kc, ORBGPU_GRID_ROWS, x0, x1, y0, y1, [&](int idx, int c, bool valid) {
-                bool ok = false;
-                int dist = 256;
-                if (valid) {
-                    const orbgpu_keypoint kp = K[idx];
-                    ok = !(check && (kp.octave < minL || (maxL >= 0 && kp.octave > maxL)));
-                    if (ok) {
-                        const float dx = __fsub_rn(kp.x, u), dy = __fsub_rn(kp.y, v);
-                        ok = __fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)) < rr;
-                    }
-                    if (ok) {
-                        dist = hamming256_ptr(dmp, D + (size_t)idx * 32);
-                        ok = dist <= ORBGPU_TH_HIGH;
-                    }
-                }
-                const unsigned msk = __ballot_sync(0xffffffffu, ok);
-                if (ok) {
-                    const int pos = total + __popc(msk & ((1u << lane) - 1));
-                    if (pos < slot_cap)
-                        slots[(size_t)i * slot_cap + pos] = ((uint32_t)dist << 24) | ((uint32_t)c << 12) | (uint32_t)idx;
-                }
-                total += __popc(msk);
-            });
+        int total = 0;
+        seg_window_recs<W>(F.cell_start, F.recs, active, x0, x1, y0, y1, [&](const GridRec& rec, bool valid) {
+            const int oc = rec.octave();
+            bool ok = valid && !(check && (oc < minL || (maxL >= 0 && oc > maxL))) && in_disc(rec, uu, vv, rr);
+            int dist = 256;
+            if (ok) {
+                const uint4* kd = reinterpret_cast<const uint4*>(F.desc + (size_t)rec.idx * 32);
+                dist = hamming256(dm0, dm1, kd[0], kd[1]);
+                ok = dist <= ORBGPU_TH_HIGH;
+            }
+            const unsigned msk = __ballot_sync(0xffffffffu, ok) & smask;
+            if (ok) {
+                const int pos = total + __popc(msk & ((1u << lane) - 1));
+                if (pos < slot_cap) slots[(size_t)i * slot_cap + pos] = make_key<uint32_t>(dist, rec.cell(), (int)rec.idx);
+            }
+            total += __popc(msk);
+        });
+        if (i < end && lane == sbase) {
+            slot_count[i] = total;
+            if (total > slot_cap) atomicMax(status, total);
         }
-    }
-    if (lane == 0) {
-        slot_count[i] = total;
-        if (total > slot_cap) atomicMax(status, total);
-        if (total > 0) atomicAdd(&frame_cands[f], min(total, slot_cap));
     }
 }
 
-// One block per frame.  Shared memory: list starts (M + 1), results (M),
-// two claim arrays (cap), observed flags and histogram bins (M bytes each),
-// and the keys when t_cap > 0 (else they are read from the global slots).
+// One block per frame: the fixed point of the in-order assignment (as
+// proj_resolve_block, but the first unclaimed candidate is the answer and an
+// owner without observations blocks nothing), the owners, the rotation
+// histogram, the three maxima and the resets.  Each thread keeps the four
+// smallest keys of its first PROJ_MPT map points in registers and reads the
+// row in global memory again only when all four are claimed.  Shared memory:
+// results (M), two claim arrays (cap), observed flags and bins (M bytes each).
+__host__ __device__ inline size_t bpf_resolve_smem(int cap, int M) { return 4 * ((size_t)M + 2 * (size_t)cap) + 2 * (size_t)M + 16; }
 __global__ void __launch_bounds__(1024)
     k_bpf_resolve(const orbgpu_keypoint* kps, int cap, const int* counts, const orbgpu_keypoint* last_kps,
                   const orbgpu_frame_mappoint* last_mps, const int* last_off, int slot_cap, const uint32_t* slots,
-                  const int* slot_count, int check_ori, int t_cap, int* match_out, int* nmatches, int* status) {
+                  const int* slot_count, int check_ori, int* match_out, int* nmatches, int* status) {
     extern __shared__ __align__(16) int s_dyn[];
     __shared__ int s_scan[32];
     __shared__ int s_flag[3];
     __shared__ int hist[ORBGPU_HISTO_LENGTH];
     __shared__ int s_ind[3];
     const int f = blockIdx.x;
-    const int tid = threadIdx.x;
+    const int tid = threadIdx.x, nt = blockDim.x;
     const int mp0 = last_off[f], M = last_off[f + 1] - mp0;
     const int n = min(counts[f], cap);
-    int* s_start = s_dyn;               // M + 1
-    int* s_res = s_start + (M + 1);     // M
-    int* cr = s_res + M;                // cap
-    int* cw = cr + cap;                 // cap
-    uint32_t* s_key = reinterpret_cast<uint32_t*>(cw + cap);            // t_cap
-    uint8_t* s_obs = reinterpret_cast<uint8_t*>(s_key + t_cap);         // M
-    uint8_t* s_bin = s_obs + M;                                         // M
-    int base = 0;
-    for (int i0 = 0; i0 < M; i0 += blockDim.x) {
-        const int i = i0 + tid;
-        const int v = i < M ? min(slot_count[mp0 + i], slot_cap) : 0;
-        int tot;
-        const int ex = block_exclusive_scan(v, s_scan, &tot);
-        if (i < M) s_start[i] = base + ex;
-        base += tot;
-    }
-    const bool in_smem = t_cap > 0;
-    if (in_smem && base > t_cap) {
-        if (tid == 0) atomicOr(status + 2, 1);
-        return;
-    }
-    if (tid == 0) s_start[M] = base;
+    int* s_res = s_dyn;     // M
+    int* cr = s_res + M;    // cap
+    int* cw = cr + cap;     // cap
+    uint8_t* s_obs = reinterpret_cast<uint8_t*>(cw + cap);  // M
+    uint8_t* s_bin = s_obs + M;                             // M
     if (tid < 3) s_flag[tid] = 0;
     if (tid < ORBGPU_HISTO_LENGTH) hist[tid] = 0;
-    __syncthreads();
-    if (in_smem)  // every candidate entry by one thread: the slot loads are independent
-        for (int t = tid; t < base; t += blockDim.x) {
-            int lo = 0, hi = M - 1;  // last i with s_start[i] <= t
-            while (lo < hi) {
-                const int mid = (lo + hi + 1) >> 1;
-                if (s_start[mid] <= t) lo = mid;
-                else hi = mid - 1;
-            }
-            s_key[t] = slots[(size_t)(mp0 + lo) * slot_cap + (t - s_start[lo])];
-        }
-    for (int i = tid; i < M; i += blockDim.x) {
+    uint32_t top[PROJ_MPT][4];
+    int cnt[PROJ_MPT];
+#pragma unroll
+    for (int q = 0; q < PROJ_MPT; q++) {
+        const int i = tid + q * nt;
+        cnt[q] = i < M ? min(slot_count[mp0 + i], slot_cap) : 0;
+    }
+#pragma unroll
+    for (int q = 0; q < PROJ_MPT; q++) top_load(slots + (size_t)(mp0 + tid + q * nt) * slot_cap, cnt[q], top[q]);
+    for (int i = tid; i < M; i += nt) {
         s_res[i] = -2;
         s_obs[i] = (last_mps[mp0 + i].flags & ORBGPU_MP_OBSERVED) ? 1 : 0;
     }
-    for (int k = tid; k < cap; k += blockDim.x) {
-        cr[k] = 0x7fffffff;
-        cw[k] = 0x7fffffff;
+    for (int k = tid; k < cap; k += nt) {
+        cr[k] = PROJ_FREE;
+        cw[k] = PROJ_FREE;
     }
+    auto full_scan = [&](int i, int c) {
+        uint32_t best = PROJ_NOKEY;
+        row_visit(slots + (size_t)(mp0 + i) * slot_cap, c, [&](uint32_t key) {
+            if (key < best && !(cr[key & 0xFFFu] < i)) best = key;
+        });
+        return best;
+    };
     bool converged = M == 0;
     for (int round = 0; round <= M + 1 && !converged; round++) {
         if (tid == 0) s_flag[(round + 1) % 3] = 0;
         __syncthreads();
-        for (int i = tid; i < M; i += blockDim.x) {
-            const int cnt = s_start[i + 1] - s_start[i];
-            const uint32_t* L = in_smem ? s_key + s_start[i] : slots + (size_t)(mp0 + i) * slot_cap;
-            uint32_t best = 0xFFFFFFFFu;
-            for (int e = 0; e < cnt; e++) {
-                const uint32_t key = L[e];
-                if (!(cr[key & 0xFFFu] < i) && key < best) best = key;
-            }
-            const int r = best == 0xFFFFFFFFu ? -1 : (int)(best & 0xFFFu);
+        auto settle = [&](int i, uint32_t best) {
+            const int r = best == PROJ_NOKEY ? -1 : (int)(best & 0xFFFu);
             if (r != s_res[i]) {
                 s_res[i] = r;
                 s_flag[round % 3] = 1;
             }
             if (r >= 0 && s_obs[i]) atomicMin(&cw[r], i);
+        };
+#pragma unroll
+        for (int q = 0; q < PROJ_MPT; q++) {
+            const int i = tid + q * nt;
+            if (i >= M) continue;
+            uint32_t best = PROJ_NOKEY;
+#pragma unroll
+            for (int j = 3; j >= 0; j--) {
+                const uint32_t key = top[q][j];
+                if (key != PROJ_NOKEY && !(cr[key & 0xFFFu] < i)) best = key;
+            }
+            if (best == PROJ_NOKEY && cnt[q] > 4) best = full_scan(i, cnt[q]);
+            settle(i, best);
         }
+        for (int i = tid + PROJ_MPT * nt; i < M; i += nt) settle(i, full_scan(i, min(slot_count[mp0 + i], slot_cap)));
         __syncthreads();
         converged = s_flag[round % 3] == 0;
         int* t = cr;
         cr = cw;
         cw = t;
         if (!converged)
-            for (int k = tid; k < cap; k += blockDim.x) cw[k] = 0x7fffffff;
+            for (int k = tid; k < cap; k += nt) cw[k] = PROJ_FREE;
     }
     if (!converged && tid == 0) atomicOr(status + 2, 2);
     // owners (the last map point that assigned each keypoint), rotation histogram
@@ -1555,12 +1335,6 @@ extern "C" int orbgpu_batch_search_by_projection_frame(orbgpu_batch* b, const or
     orbgpu_batch_proj& P = g_bproj;
     P.last_upload.clear();  // this search reuses the scratch the projection search caches its uploads in
     if (!P.h_pinned) ORBGPU_CUDA_TRY(cudaMallocHost(&P.h_pinned, 64));
-    if (P.h_cands_cap < nf) {
-        if (P.h_cands) cudaFreeHost(P.h_cands);
-        P.h_cands = nullptr;
-        ORBGPU_CUDA_TRY(cudaMallocHost(&P.h_cands, sizeof(int) * nf));
-        P.h_cands_cap = nf;
-    }
     std::vector<BatchMotion> hm(nf);
     std::vector<BatchFrameInfo> hi(nf);
     for (int f = 0; f < nf; f++) {
@@ -1581,15 +1355,24 @@ extern "C" int orbgpu_batch_search_by_projection_frame(orbgpu_batch* b, const or
         for (int l = 0; l < 16; l++) hi[f].scale[l] = b->frame_scale[(size_t)f * 16 + l];
     }
     cudaStream_t st = b->stream;
+    const size_t smem = bpf_resolve_smem(cap, max_mp);
+    if (sizeof(int) * ((size_t)2 * max_mp + 1 + 2 * (size_t)cap) + 2 * (size_t)max_mp + 64 > 200 * 1024) {
+        orbgpu_set_last_error("batched frame search: a frame's map points exceed shared memory", __FILE__, __LINE__);
+        return ORBGPU_ERR_CAPACITY;
+    }
     for (int attempt = 0; attempt < 3; attempt++) {
-        const size_t need = sizeof(BatchFrameInfo) * nf + sizeof(BatchMotion) * nf +
-                            sizeof(int) * ((size_t)nf * ncell * 2 + (size_t)nf * (ncell + 1) + (size_t)nf * cap * 2 +
-                                           (nf + 1) + (size_t)std::max(1, total_mp) + nf + 16) +
+        // frame info, motions and offsets, back to back: one upload
+        auto up16 = [](size_t n) { return (n + 255) & ~(size_t)255; };
+        const size_t info_b = up16(sizeof(BatchFrameInfo) * nf), mot_b = up16(sizeof(BatchMotion) * nf),
+                     off_b = sizeof(int) * (nf + 1), up_b = info_b + mot_b + off_b;
+        const size_t need = up16(up_b) + sizeof(GridRec) * (size_t)nf * cap +
+                            sizeof(int) * ((size_t)nf * (ncell + 1) + (size_t)std::max(1, total_mp) + 16) +
                             sizeof(uint32_t) * (size_t)std::max(1, total_mp) * P.slot_cap + 16 * 256;
         if (need > P.bytes) {
             ORBGPU_CUDA_TRY(cudaStreamSynchronize(st));
             if (P.scratch) cudaFree(P.scratch);
             P.scratch = nullptr;
+            P.bytes = 0;
             ORBGPU_CUDA_TRY(dev_malloc(&P.scratch, need));
             P.bytes = need;
         }
@@ -1600,64 +1383,46 @@ extern "C" int orbgpu_batch_search_by_projection_frame(orbgpu_batch* b, const or
             off += n;
             return p;
         };
-        BatchFrameInfo* info = (BatchFrameInfo*)take(sizeof(BatchFrameInfo) * nf);
-        BatchMotion* mot = (BatchMotion*)take(sizeof(BatchMotion) * nf);
-        int* cell_count = (int*)take(sizeof(int) * (size_t)nf * ncell);
-        int* cursor = (int*)take(sizeof(int) * (size_t)nf * ncell);
+        uint8_t* up = take(up_b);
+        BatchFrameInfo* info = (BatchFrameInfo*)up;
+        BatchMotion* mot = (BatchMotion*)(up + info_b);
+        int* d_off = (int*)(up + info_b + mot_b);
         int* cell_start = (int*)take(sizeof(int) * (size_t)nf * (ncell + 1));
-        int* key_cell = (int*)take(sizeof(int) * (size_t)nf * cap);
-        int* cell_keys = (int*)take(sizeof(int) * (size_t)nf * cap);
-        int* d_off = (int*)take(sizeof(int) * (nf + 1));
+        GridRec* recs = (GridRec*)take(sizeof(GridRec) * (size_t)nf * cap);
         int* slot_count = (int*)take(sizeof(int) * std::max(1, total_mp));
         int* status = (int*)take(sizeof(int) * 4);
-        int* frame_cands = (int*)take(sizeof(int) * nf);
         uint32_t* slots = (uint32_t*)take(sizeof(uint32_t) * (size_t)std::max(1, total_mp) * P.slot_cap);
-        ORBGPU_CUDA_TRY(cudaMemcpyAsync(info, hi.data(), sizeof(BatchFrameInfo) * nf, cudaMemcpyHostToDevice, st));
-        ORBGPU_CUDA_TRY(cudaMemcpyAsync(mot, hm.data(), sizeof(BatchMotion) * nf, cudaMemcpyHostToDevice, st));
-        ORBGPU_CUDA_TRY(cudaMemcpyAsync(d_off, last_offsets, sizeof(int) * (nf + 1), cudaMemcpyHostToDevice, st));
-        ORBGPU_CUDA_TRY(cudaMemsetAsync(cell_count, 0, sizeof(int) * (size_t)nf * ncell, st));
-        ORBGPU_CUDA_TRY(cudaMemsetAsync(status, 0, sizeof(int) * 4, st));
-        ORBGPU_CUDA_TRY(cudaMemsetAsync(frame_cands, 0, sizeof(int) * nf, st));
-        dim3 gk((cap + 255) / 256, nf);
-        k_bgrid_count<<<gk, 256, 0, st>>>(kps, counts, cap, info, key_cell, cell_count);
-        k_bgrid_scan<<<nf, 1024, 0, st>>>(cell_count, cell_start, cursor);
-        k_bgrid_fill<<<gk, 256, 0, st>>>(counts, cap, key_cell, cursor, cell_keys);
-        const int wpb = 8;
-        if (max_mp > 0) {
-            dim3 gc((max_mp + wpb - 1) / wpb, nf);
-            k_bpf_candidates<<<gc, 32 * wpb, 0, st>>>(kps, desc, cap, info, cell_start, cell_keys, key_cell, mot, last_kps,
-                                                      last_mps, last_desc, d_off, th, P.slot_cap, slots, slot_count,
-                                                      status, frame_cands);
+        if (P.h_stage_cap < up_b) {
+            if (P.h_stage) cudaFreeHost(P.h_stage);
+            P.h_stage = nullptr;
+            P.h_stage_cap = 0;
+            ORBGPU_CUDA_TRY(cudaMallocHost(&P.h_stage, up_b));
+            P.h_stage_cap = up_b;
         }
+        // the previous call's copy has completed (every call ends synchronised)
+        std::memcpy(P.h_stage, hi.data(), sizeof(BatchFrameInfo) * nf);
+        std::memcpy(P.h_stage + info_b, hm.data(), sizeof(BatchMotion) * nf);
+        std::memcpy(P.h_stage + info_b + mot_b, last_offsets, off_b);
+        ORBGPU_CUDA_TRY(cudaMemcpyAsync(up, P.h_stage, up_b, cudaMemcpyHostToDevice, st));
+        k_bgrid_build<<<nf, 1024, 0, st>>>(kps, counts, cap, info, cell_start, recs, status);
+        const int wpb = 4;
+        if (max_mp > 0) {
+            dim3 gc((max_mp + wpb * BPF_PER - 1) / (wpb * BPF_PER), nf);
+            k_bpf_candidates<<<gc, 32 * wpb, 0, st>>>(desc, cap, info, cell_start, recs, mot, last_kps, last_mps, last_desc,
+                                                      d_off, th, P.slot_cap, slots, slot_count, status);
+        }
+        ORBGPU_CUDA_TRY(allow_max_dynamic_smem(k_bpf_resolve));
+        k_bpf_resolve<<<nf, 1024, smem, st>>>(kps, cap, counts, last_kps, last_mps, d_off, P.slot_cap, slots, slot_count,
+                                               check_ori, match_out, nmatches, status);
         ORBGPU_CUDA_TRY(cudaGetLastError());
-        ORBGPU_CUDA_TRY(cudaMemcpyAsync(P.h_pinned, status, sizeof(int), cudaMemcpyDeviceToHost, st));
-        ORBGPU_CUDA_TRY(cudaMemcpyAsync(P.h_cands, frame_cands, sizeof(int) * nf, cudaMemcpyDeviceToHost, st));
+        ORBGPU_CUDA_TRY(cudaMemcpyAsync(P.h_pinned, status, sizeof(int) * 4, cudaMemcpyDeviceToHost, st));
         ORBGPU_CUDA_TRY(cudaStreamSynchronize(st));
         if (P.h_pinned[0] > P.slot_cap) {  // a window held more candidates than the slots: widen and redo
             P.slot_cap = ((P.h_pinned[0] + 63) / 64) * 64;
             continue;
         }
-        int t_max = 0;
-        for (int f = 0; f < nf; f++) t_max = std::max(t_max, P.h_cands[f]);
-        const size_t fixed = sizeof(int) * ((size_t)2 * max_mp + 1 + 2 * (size_t)cap) + 2 * (size_t)max_mp + 64;
-        size_t smem = fixed + sizeof(uint32_t) * (size_t)t_max;
-        int t_cap = std::max(1, t_max);
-        if (smem > 200 * 1024) {  // keys stay in global memory
-            smem = fixed;
-            t_cap = 0;
-        }
-        if (smem > 200 * 1024) {
-            orbgpu_set_last_error("batched frame search: a frame's map points exceed shared memory", __FILE__, __LINE__);
-            return ORBGPU_ERR_CAPACITY;
-        }
-        ORBGPU_CUDA_TRY(allow_max_dynamic_smem(k_bpf_resolve));
-        k_bpf_resolve<<<nf, 1024, smem, st>>>(kps, cap, counts, last_kps, last_mps, d_off, P.slot_cap, slots, slot_count,
-                                               check_ori, t_cap, match_out, nmatches, status);
-        ORBGPU_CUDA_TRY(cudaGetLastError());
-        ORBGPU_CUDA_TRY(cudaMemcpyAsync(P.h_pinned + 2, status + 1, sizeof(int) * 2, cudaMemcpyDeviceToHost, st));
-        ORBGPU_CUDA_TRY(cudaStreamSynchronize(st));
-        P.last_launches = 5;
-        if (P.h_pinned[3] != 0) {
+        P.last_launches = 3;
+        if (P.h_pinned[2] != 0) {
             orbgpu_set_last_error("batched frame search: resolution failed", __FILE__, __LINE__);
             return ORBGPU_ERR_CUDA;
         }

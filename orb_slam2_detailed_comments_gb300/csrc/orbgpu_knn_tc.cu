@@ -300,9 +300,9 @@ __global__ void __launch_bounds__(128) k_tc_probe(const uint8_t* qa, const uint8
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 256;" ::"r"(tmem));
 }
 
-// mbar_wait by every lane of the warp, with one outcome.
+// mbar_wait_sleep by every lane of the warp, with one outcome.
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity) {
-    return __all_sync(0xffffffffu, mbar_wait(bar, parity));
+    return __all_sync(0xffffffffu, mbar_wait_sleep(bar, parity));
 }
 
 // ---------------------------------------------------------------- kNN kernel

@@ -238,6 +238,71 @@ def test_knn_tensor_cores_oracle(torch, oracle, nq, nt):
         assert np.array_equal(a.cpu().numpy(), b), name
 
 
+def random_frame(n, w, h, seed, entropy):
+    """n keypoints anywhere (a few outside the grid) with descriptors of 'entropy' random bits a byte."""
+    from orb_slam2_detailed_comments_gb300._lib import KEYPOINT_DTYPE
+    rng = np.random.default_rng(seed)
+    k = np.zeros(n, KEYPOINT_DTYPE)
+    k["x"], k["y"] = rng.uniform(-2, w + 2, n), rng.uniform(-2, h + 2, n)
+    k["octave"], k["angle"], k["class_id"] = rng.choice([0, 0, 0, 1, 2, 7], n), rng.uniform(0, 360, n), -1
+    return k, rng.integers(0, 256, (n, 32), dtype=np.uint8) & np.uint8((1 << entropy) - 1)
+
+
+# keypoints around the 32-bit keys' and the one-block grid's limits, map points
+# around a block's threads and its registers, windows of more candidates than a row
+@pytest.mark.parametrize("n,m,w,h,th,nnratio,entropy", [
+    (1, 1, 320, 240, 1.0, 0.8, 2), (100, 1025, 320, 240, 6.0, 0.8, 1), (2000, 4097, 640, 480, 2.0, 0.9, 1),
+    (4095, 3000, 1280, 720, 3.0, 0.6, 2), (4096, 3000, 1280, 720, 3.0, 0.6, 2), (8193, 500, 640, 480, 1.0, 0.8, 2),
+    (3000, 700, 320, 240, 8.0, 0.9, 1), (1500, 2000, 640, 480, 4.0, 1.3, 1)])
+def test_projection_search_limits(torch, oracle, n, m, w, h, th, nnratio, entropy):
+    """SearchByProjection(Frame, MapPoints): the one-block resolution and the
+    global-memory rounds, with many conflicts and keypoints claimed before."""
+    from oracle import pyoracle
+    from orb_slam2_detailed_comments_gb300 import FrameView, ORBmatcher
+    from orb_slam2_detailed_comments_gb300._lib import MAPPOINT_DTYPE
+    k, d = random_frame(n, w, h, 31 + n, entropy)
+    rng = np.random.default_rng(m)
+    src = rng.integers(0, n, m)
+    mps = np.zeros(m, MAPPOINT_DTYPE)
+    mps["proj_x"], mps["proj_y"] = k["x"][src] + rng.normal(0, 3, m), k["y"][src] + rng.normal(0, 3, m)
+    mps["view_cos"], mps["proj_xr"] = rng.choice([1.0, 0.5], m), -1
+    mps["track_scale_level"] = np.minimum(k["octave"][src] + rng.integers(0, 2, m), 7)
+    mps["track_in_view"], mps["bad"] = rng.random(m) < 0.95, rng.random(m) < 0.05
+    mpd = d[src] ^ (rng.integers(0, 256, (m, 32), dtype=np.uint8) & rng.integers(0, 256, (m, 32), dtype=np.uint8)
+                    & np.uint8((1 << entropy) - 1))
+    claimed = (rng.random(n) < 0.1).astype(np.uint8)
+    s, _ = pyoracle.scale_tables(8, 1.2)
+    ref = oracle.search_by_projection(k.view(pyoracle.KP_DTYPE), d, w, h, mps.view(pyoracle.MP_DTYPE), mpd, th=th,
+                                      nnratio=nnratio, claimed=claimed)
+    nm, match = ORBmatcher(nnratio, True).SearchByProjection(FrameView(k, d, w, h, s), mps, mpd, th, claimed)
+    assert nm == ref[0] and np.array_equal(match, ref[1])
+
+
+@pytest.mark.parametrize("n1,n2,window,nnratio,entropy", [
+    (1, 1, 10, 0.9, 2), (300, 33, 60, 0.9, 1), (2049, 1500, 40, 0.9, 1), (3000, 3000, 30, 0.6, 2),
+    (9000, 8200, 20, 0.9, 1), (1200, 1200, 100, 1.2, 1)])
+def test_initialization_search_limits(torch, oracle, n1, n2, window, nnratio, entropy):
+    """SearchForInitialization with many keypoints taking one another's
+    matches, up to frames past the shared-memory arrays."""
+    from oracle import pyoracle
+    from orb_slam2_detailed_comments_gb300 import FrameView, ORBmatcher
+    w, h = 640, 480
+    k2, d2 = random_frame(n2, w, h, 5 + n2, entropy)
+    rng = np.random.default_rng(n1)
+    src = rng.integers(0, n2, n1)
+    k1, d1 = k2[src].copy(), d2[src] ^ (rng.integers(0, 256, (n1, 32), dtype=np.uint8) & np.uint8(1)
+                                        & rng.integers(0, 256, (n1, 32), dtype=np.uint8))
+    k1["x"] += rng.normal(0, 4, n1).astype(np.float32)
+    k1["angle"] = (k1["angle"] + rng.choice([5.0, 5.0, 120.0], n1).astype(np.float32)) % np.float32(360)
+    prev = np.ascontiguousarray(np.stack([k1["x"], k1["y"]], 1))
+    s, _ = pyoracle.scale_tables(8, 1.2)
+    ref = oracle.search_for_initialization(k1.view(pyoracle.KP_DTYPE), d1, k2.view(pyoracle.KP_DTYPE), d2, w, h,
+                                           prev_xy=prev, window=window, nnratio=nnratio, check_ori=True)
+    nm, m12, prev_out = ORBmatcher(nnratio, True).SearchForInitialization(FrameView(k1, d1, w, h, s),
+                                                                        FrameView(k2, d2, w, h, s), prev, window)
+    assert nm == ref[0] and np.array_equal(m12, ref[1]) and np.array_equal(prev_out, ref[2])
+
+
 # tile edges: query pairs of 256 rows, train tiles of 160 and groups of 32,
 # popcount tiles of 256 rows and shares of 32; several runs of one query pair
 @pytest.mark.parametrize("nq,nt", [(1, 31), (31, 32), (33, 33), (128, 159), (129, 160), (255, 161), (256, 255),
