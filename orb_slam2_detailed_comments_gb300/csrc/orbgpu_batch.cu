@@ -119,6 +119,7 @@ struct orbgpu_batch {
     size_t descs_cap = 0;
     int ndesc = 0;
     int max_kept = 0, sort_cap = 0;
+    long features = 0;  // the budgets of all levels with cells
     ImageSrc* d_src = nullptr;
     ImageSrc* h_src = nullptr;  // pinned
     bool pending = false;       // an asynchronous extraction whose status has not been read
@@ -400,8 +401,10 @@ static int plan_batch(orbgpu_batch* b, int nframes, const int* widths, const int
     ORBGPU_CUDA_TRY(cudaMemcpyAsync(b->d_prefix, pre.data(), sizeof(int) * pre.size(), cudaMemcpyHostToDevice, st));
     b->max_kept = 0;
     b->sort_cap = 1;
+    b->features = 0;
     for (int f = 0; f < nframes; f++)
         for (auto& L : b->cur[f]->geom) {
+            if (L.ncells > 0) b->features += L.nfeat + 1;
             b->max_kept = std::max(b->max_kept, L.node_cap);
             while (b->sort_cap < L.node_cap) b->sort_cap <<= 1;
         }
@@ -458,7 +461,7 @@ static void enqueue_pipeline(orbgpu_batch* b, orbgpu_keypoint* kps, uint8_t* des
     mark(3);
     launch_distribute(b->d_descs, b->ndesc, b->sort_cap, b->max_kept, b->d_status, st);
     mark(4);
-    launch_describe(b->d_descs, b->ndesc, b->max_kept, kps, desc, b->d_status, st);
+    launch_describe(b->d_descs, b->ndesc, b->features, kps, desc, b->d_status, st);
     mark(5);
     // gather, strip per level, resize per level >= 1, FAST cells,
     // DistributeOctTree, describe

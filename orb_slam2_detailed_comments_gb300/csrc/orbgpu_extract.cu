@@ -550,6 +550,7 @@ struct SizePlan {
     int rows = 22;  // strip rows of the resize / blur launches
     int fast_first = 0, fast_count = 0;
     int max_kept = 0, sort_cap = 0;
+    long features = 0;  // the budgets of all levels with cells
     uint64_t last_use = 0;
     int gen = -1;  // tuning generation of the work lists
 };
@@ -657,6 +658,7 @@ static int build_plan(orbgpu_extractor* ex, int w, int h, SizePlan** out) {
     P->max_kept = 0;
     P->sort_cap = 1;
     for (auto& L : g) {
+        if (L.ncells > 0) P->features += L.nfeat + 1;
         P->max_kept = std::max(P->max_kept, L.node_cap);
         while (P->sort_cap < L.node_cap) P->sort_cap <<= 1;
     }
@@ -865,7 +867,7 @@ extern "C" int orbgpu_extract(orbgpu_extractor* ex, const uint8_t* image, int wi
     launch_fast(ex->d_descs, RangeMap{P.d_items + P.fast_first, nl, 0, 1}, P.fast_count, ex->d_status, mwc, mhc, mbox,
                 st);
     launch_distribute(ex->d_descs, nl, P.sort_cap, P.max_kept, ex->d_status, st);
-    launch_describe(ex->d_descs, nl, P.max_kept, okps, odesc, ex->d_status, st);
+    launch_describe(ex->d_descs, nl, P.features, okps, odesc, ex->d_status, st);
     ORBGPU_CUDA_TRY(cudaGetLastError());
     ORBGPU_CUDA_TRY(cudaMemcpyAsync(ex->h_pinned, ex->d_status, sizeof(int), cudaMemcpyDeviceToHost, st));
     ORBGPU_CUDA_TRY(cudaMemcpyAsync(ex->h_pinned + 4, hd[0].frame_total, sizeof(int), cudaMemcpyDeviceToHost, st));

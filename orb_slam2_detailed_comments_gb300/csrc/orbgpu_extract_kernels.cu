@@ -1240,10 +1240,11 @@ __device__ __forceinline__ float lookup_exception(const uint32_t* keys, const fl
 
 // Orientation and descriptor of the kept keypoints, up to 32 keypoints per
 // warp task (one per lane) and no block-level synchronisation after the
-// prologue.  A task holds TS = 8, 16 or 32 keypoints: the smallest size whose
-// tasks fit in one pass of the grid's warps (every block computes the same
-// keypoint total), so a small launch spreads its keypoints over more warps
-// instead of queueing 64 staging rounds on a few ('task' > 0 fixes TS).
+// prologue.  A task holds TS <= 32 keypoints: the least that lets one pass of
+// the grid's warps take all of them (every block computes the same keypoint
+// total), so a small launch spreads its keypoints over more warps instead of
+// queueing staging rounds on a few, and a large one leaves no warp without a
+// task ('task' > 0 fixes TS).
 // The task's patches are staged in shared memory by tensor copies in rounds
 // of R keypoints through D buffers of the warp, each with its mbarrier; D
 // rounds are in flight while one is computed:
@@ -1318,10 +1319,11 @@ __global__ void __launch_bounds__(32 * WPB) k_describe(const LevelDesc* descs, i
         for (int v = 0; v <= ORBGPU_HALF_PATCH; v++)
             if (c_umax[v] >= au) vmax = v;
     uint32_t par = 0;  // bit b: the phase parity buffer b waits for next
-    const long grid_warps = (long)gridDim.x * WPB;
-    const int TS = task ? task : total <= 8 * grid_warps ? 8 : total <= 16 * grid_warps ? 16 : 32;
+    const int grid_warps = gridDim.x * WPB;
+    const int TS = task ? task : min(32, max(1, (total + grid_warps - 1) / grid_warps));
     const int ntasks = (total + TS - 1) / TS;
-    for (int t = blockIdx.x * WPB + warp; t < ntasks; t += gridDim.x * WPB) {
+    // consecutive tasks on different blocks: the last, partial pass is spread over the SMs
+    for (int t = warp * gridDim.x + blockIdx.x; t < ntasks; t += grid_warps) {
         // this lane's keypoint: level, position, output row, validity
         const int g = t * TS + lane;
         int e = 0, x = 0, y = 0, score = 0, o = 0;
@@ -1632,23 +1634,25 @@ void launch_distribute(const LevelDesc* descs, int ndescs, int sort_cap, int nod
     allow_max_dynamic_smem(k_distribute);
     if (ndescs > 0) k_distribute<<<ndescs, 512, smem, st>>>(descs, status, sort_cap, node_smem_cap, key_smem_cap);
 }
-void launch_describe(const LevelDesc* descs, int ndescs, int max_kept, orbgpu_keypoint* kps, uint8_t* desc, int* status,
+void launch_describe(const LevelDesc* descs, int ndescs, long features, orbgpu_keypoint* kps, uint8_t* desc, int* status,
                      cudaStream_t st) {
-    if (ndescs <= 0 || max_kept <= 0) return;
+    if (ndescs <= 0) return;
     const int nsm = nsm_of_current_device();
     const int R = tunables().describe_group, D = R * tunables().describe_depth > 8 ? 2 : tunables().describe_depth;
     // D buffers of R box slots per warp, 24 slots (60 KiB) per block: three
-    // blocks per SM.  max_kept (the node capacity) overestimates a level's
-    // keypoints about twice; a grid of 32-keypoint tasks' worth of warps, or
-    // for a launch that would not fill the SMs that way, 8-keypoint tasks'
-    // worth on up to one block per SM (the kernel picks the task size from
-    // the grid and the keypoint count); warps stride over the tasks
+    // blocks per SM.  A launch short of keypoints is bound by one warp's
+    // staging rounds, a long one by its tasks' double-precision passes (one per
+    // task, whatever its lanes): up to 8 keypoints per warp of the full device
+    // it takes as many blocks as keypoints give warps (one 640x480 frame 32 ->
+    // 19 us against 8 keypoints a task, five frames 43 -> 29), beyond that the
+    // blocks per SM that hold them in tasks of at most 32 (96,000 keypoints: 94
+    // us with two, 117 with three; 128,000: 136 with three, 159 with two)
     const int wpb = 24 / (R * D);
     const size_t smem = (size_t)D * R * wpb * DESC_SLOT + 128 + sizeof(int) * (ndescs + 1);
-    const long est = (long)ndescs * max_kept / 2;
-    long want = (est + 32 * wpb - 1) / (32 * wpb);
-    if (want < nsm) want = std::min((long)nsm, (est + 8 * wpb - 1) / (8 * wpb));
-    const int blocks = (int)std::max(1L, std::min(want, (long)nsm * 3));
+    const long full = (long)nsm * wpb;  // warps of one block per SM
+    const long blocks_l = features <= 8 * 3 * full ? std::min((features + wpb - 1) / wpb, 3L * nsm)
+                                                   : nsm * std::min(3L, (features + 32 * full - 1) / (32 * full));
+    const int blocks = (int)std::max(1L, blocks_l);
     auto run = [&](auto kernel) {
         allow_max_dynamic_smem(kernel);
         kernel<<<blocks, 32 * wpb, smem, st>>>(descs, ndescs, tunables().describe_task, kps, desc, status);

@@ -189,7 +189,8 @@ int strip_rows(long level0_pixels);
 // node capacity (its arrays go to shared memory when they fit).
 void launch_distribute(const LevelDesc* descs, int ndescs, int sort_cap, int node_cap, int* status,
                        cudaStream_t st);
-void launch_describe(const LevelDesc* descs, int ndescs, int max_kept, orbgpu_keypoint* kps, uint8_t* desc, int* status,
+// features: about how many keypoints the launch describes (the levels' budgets).
+void launch_describe(const LevelDesc* descs, int ndescs, long features, orbgpu_keypoint* kps, uint8_t* desc, int* status,
                      cudaStream_t st);
 
 }  // namespace orbgpu
