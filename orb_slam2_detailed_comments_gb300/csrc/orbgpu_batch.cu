@@ -123,7 +123,13 @@ struct orbgpu_batch {
     ImageSrc* d_src = nullptr;
     ImageSrc* h_src = nullptr;  // pinned
     bool pending = false;       // an asynchronous extraction whose status has not been read
+    // status (4 ints), k_pyramid's ticket (at 4) and the levels' counters (from
+    // 8): cleared before every extraction
     int* d_status = nullptr;
+    size_t status_cap = 0, status_ints = 8;
+    bool fused = false;  // all resizes and strips in one launch (k_pyramid)
+    PyramidPlan pyramid;
+    int pyr_off = 0;
     int* d_totals = nullptr;  // per frame
     int* h_pinned = nullptr;
     cudaGraphExec_t graph = nullptr;
@@ -179,7 +185,8 @@ extern "C" int orbgpu_batch_create(int max_frames, int max_width, int max_height
         }
         b->own_stream = true;
     }
-    if (cudaMalloc(&b->d_status, sizeof(int) * 4) != cudaSuccess ||
+    b->status_cap = 8;
+    if (cudaMalloc(&b->d_status, sizeof(int) * 8) != cudaSuccess ||
         cudaMalloc(&b->d_totals, sizeof(int) * max_frames) != cudaSuccess ||
         cudaMallocHost(&b->h_pinned, sizeof(int) * (8 + max_frames)) != cudaSuccess ||
         cudaMalloc(&b->d_src, sizeof(ImageSrc) * max_frames) != cudaSuccess ||
@@ -349,6 +356,23 @@ static int plan_batch(orbgpu_batch* b, int nframes, const int* widths, const int
         ORBGPU_CUDA_TRY(dev_malloc(&b->d_descs, sizeof(LevelDesc) * b->max_frames * nlevels));
         b->descs_cap = (size_t)b->max_frames * nlevels;
     }
+    // the levels' band counters follow the status and the ticket
+    size_t status_ints = 8;
+    std::vector<size_t> done_off(ndesc);
+    for (int f = 0; f < nframes; f++)
+        for (int l = 0; l < nlevels; l++) {
+            done_off[(size_t)f * nlevels + l] = status_ints;
+            status_ints += (b->cur[f]->geom[l].h + PYRAMID_BAND - 1) / PYRAMID_BAND;
+        }
+    if (status_ints > b->status_cap) {
+        ORBGPU_CUDA_TRY(cudaStreamSynchronize(st));
+        destroy_graph(b);
+        cudaFree(b->d_status);
+        b->d_status = nullptr;
+        b->status_cap = 0;
+        ORBGPU_CUDA_TRY(dev_malloc(&b->d_status, sizeof(int) * status_ints));
+        b->status_cap = status_ints;
+    }
     std::vector<LevelDesc> hd(ndesc);
     b->frame_scale.assign((size_t)nframes * 16, 1.0f);
     for (int f = 0; f < nframes; f++) {
@@ -357,6 +381,7 @@ static int plan_batch(orbgpu_batch* b, int nframes, const int* widths, const int
                    f * per_frame_cap, per_frame_cap, &hd[(size_t)f * nlevels]);
         for (int l = 0; l < nlevels; l++) {
             hd[(size_t)f * nlevels + l].frame_total = b->d_totals + f;
+            hd[(size_t)f * nlevels + l].done = b->d_status + done_off[(size_t)f * nlevels + l];
             b->frame_scale[(size_t)f * 16 + l] = P->tables.scale[l];
         }
     }
@@ -390,11 +415,22 @@ static int plan_batch(orbgpu_batch* b, int nframes, const int* widths, const int
         }
     pre.push_back(acc);
     b->fast_count = acc;
+    std::vector<int> lw, lh;
+    for (int f = 0; f < nframes; f++)
+        for (const LevelGeom& L : b->cur[f]->geom) {
+            lw.push_back(L.w);
+            lh.push_back(L.h);
+        }
+    b->fused = plan_pyramid(b->rows, nframes, nlevels, lw, lh, b->pyramid);
+    b->status_ints = b->fused ? status_ints : 8;
+    b->pyr_off = (int)pre.size();
+    pre.insert(pre.end(), b->pyramid.prefix.begin(), b->pyramid.prefix.end());
     if (pre.size() > b->prefix_cap) {
         ORBGPU_CUDA_TRY(cudaStreamSynchronize(st));
         if (b->d_prefix) cudaFree(b->d_prefix);
         b->d_prefix = nullptr;
-        const size_t cap = (size_t)(b->max_frames + 1) * nlevels + (size_t)b->max_frames * nlevels + 1;
+        const size_t cap = (size_t)(b->max_frames + 1) * nlevels + (size_t)b->max_frames * nlevels + 1 +
+                           (size_t)(2 * nlevels - 1) * b->max_frames;
         ORBGPU_CUDA_TRY(dev_malloc(&b->d_prefix, sizeof(int) * std::max(cap, pre.size())));
         b->prefix_cap = std::max(cap, pre.size());
     }
@@ -434,19 +470,24 @@ static void enqueue_pipeline(orbgpu_batch* b, orbgpu_keypoint* kps, uint8_t* des
     mark(0);
     k_gather_images<<<g, 256, 0, st>>>(b->d_src, b->nframes);
     mark(1);
-    // levels 1.. are resized in a chain on the side stream while the strips
-    // of the levels already resized run on the batch's stream
-    cudaEventRecord(b->ev_fork, st);
-    cudaStreamWaitEvent(b->side, b->ev_fork, 0);
-    for (int l = 1; l < b->nlevels; l++) {
-        launch_level_resize(b->d_descs, RangeMap{b->d_prefix + b->rb_off[l], b->nframes, l, b->nlevels},
-                            b->rb_count[l], b->rows, b->side);
-        cudaEventRecord(b->ev_level[l], b->side);
-    }
-    for (int l = 0; l < b->nlevels; l++) {
-        if (l > 0) cudaStreamWaitEvent(st, b->ev_level[l], 0);
-        launch_level_strip(b->d_descs, RangeMap{b->d_prefix + b->rb_off[l], b->nframes, l, b->nlevels},
-                           b->rb_count[l], b->rows, st);
+    if (b->fused) {
+        launch_pyramid(b->d_descs, b->pyramid, b->d_prefix + b->pyr_off, b->nframes, b->nlevels, b->d_status + 4,
+                       b->d_status, st);
+    } else {
+        // levels 1.. are resized in a chain on the side stream while the strips
+        // of the levels already resized run on the batch's stream
+        cudaEventRecord(b->ev_fork, st);
+        cudaStreamWaitEvent(b->side, b->ev_fork, 0);
+        for (int l = 1; l < b->nlevels; l++) {
+            launch_level_resize(b->d_descs, RangeMap{b->d_prefix + b->rb_off[l], b->nframes, l, b->nlevels},
+                                b->rb_count[l], b->rows, b->side);
+            cudaEventRecord(b->ev_level[l], b->side);
+        }
+        for (int l = 0; l < b->nlevels; l++) {
+            if (l > 0) cudaStreamWaitEvent(st, b->ev_level[l], 0);
+            launch_level_strip(b->d_descs, RangeMap{b->d_prefix + b->rb_off[l], b->nframes, l, b->nlevels},
+                               b->rb_count[l], b->rows, st);
+        }
     }
     mark(2);
     int mwc = 1, mhc = 1, mbox = 0;
@@ -463,9 +504,9 @@ static void enqueue_pipeline(orbgpu_batch* b, orbgpu_keypoint* kps, uint8_t* des
     mark(4);
     launch_describe(b->d_descs, b->ndesc, b->features, kps, desc, b->d_status, st);
     mark(5);
-    // gather, strip per level, resize per level >= 1, FAST cells,
-    // DistributeOctTree, describe
-    b->launches_per_run = 1 + 2 * b->nlevels - 1 + 3;
+    // gather, strip per level and resize per level >= 1 (or the pyramid), FAST
+    // cells, DistributeOctTree, describe
+    b->launches_per_run = 1 + (b->fused ? 1 : 2 * b->nlevels - 1) + 3;
 }
 
 // The device status of the last extraction (copied to h_pinned[0] at its end)
@@ -524,7 +565,7 @@ static int batch_extract(orbgpu_batch* b, int nframes, const uint8_t* const* ima
                        b->arena + (size_t)f * b->slot_bytes + b->cur[f]->layout.lv[0].pyr, L0.pitch};
     }
     ORBGPU_CUDA_TRY(cudaMemcpyAsync(b->d_src, b->h_src, sizeof(ImageSrc) * nframes, cudaMemcpyHostToDevice, st));
-    ORBGPU_CUDA_TRY(cudaMemsetAsync(b->d_status, 0, sizeof(int) * 4, st));
+    ORBGPU_CUDA_TRY(cudaMemsetAsync(b->d_status, 0, sizeof(int) * b->status_ints, st));
     const bool graph_ok = b->graph && b->graph_sig == b->sig && b->graph_kps == keypoints && b->graph_desc == descriptors;
     if (graph_ok) {
         ORBGPU_CUDA_TRY(cudaGraphLaunch(b->graph, st));

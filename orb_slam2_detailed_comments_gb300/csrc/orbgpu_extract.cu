@@ -549,6 +549,14 @@ struct SizePlan {
     std::vector<int> rb_first, rb_count;
     int rows = 22;  // strip rows of the resize / blur launches
     int fast_first = 0, fast_count = 0;
+    // small images: all resizes and strips in one launch (k_pyramid)
+    bool fused = false;
+    PyramidPlan pyramid;
+    // the call's status (4 ints), k_pyramid's ticket (at 4) and the levels'
+    // counters (from 8): cleared before every call
+    int* d_sync = nullptr;
+    size_t sync_bytes = 0;
+    std::vector<int> done_off;
     int max_kept = 0, sort_cap = 0;
     long features = 0;  // the budgets of all levels with cells
     uint64_t last_use = 0;
@@ -573,7 +581,6 @@ struct orbgpu_extractor {
     // current geometry (mirrors cur)
     int cur_w = -1, cur_h = -1;
     LevelDesc* d_descs = nullptr;
-    int* d_status = nullptr;
     // output staging
     orbgpu_keypoint* d_kps = nullptr;
     uint8_t* d_desc = nullptr;
@@ -585,6 +592,7 @@ static void free_plan(SizePlan* p) {
     if (!p) return;
     cudaFree(p->arena);
     cudaFree(p->d_items);
+    cudaFree(p->d_sync);
     delete p;
 }
 
@@ -650,7 +658,17 @@ static int build_plan(orbgpu_extractor* ex, int w, int h, SizePlan** out) {
     }
     pre.push_back(acc);
     P->fast_count = acc;
-    if (dev_malloc(&P->d_items, pre.size() * sizeof(int)) != cudaSuccess ||
+    std::vector<int> lw, lh;
+    int sync_ints = 8;
+    for (const LevelGeom& L : g) {
+        lw.push_back(L.w);
+        lh.push_back(L.h);
+        P->done_off.push_back(sync_ints);
+        sync_ints += (L.h + PYRAMID_BAND - 1) / PYRAMID_BAND;
+    }
+    P->fused = plan_pyramid(P->rows, 1, (int)g.size(), lw, lh, P->pyramid);
+    P->sync_bytes = sizeof(int) * sync_ints;
+    if (dev_malloc(&P->d_sync, P->sync_bytes) != cudaSuccess || dev_malloc(&P->d_items, pre.size() * sizeof(int)) != cudaSuccess ||
         cudaMemcpy(P->d_items, pre.data(), pre.size() * sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess) {
         free_plan(P);
         return ORBGPU_ERR_OOM;
@@ -759,9 +777,8 @@ extern "C" int orbgpu_extractor_create(int nfeatures, float scale_factor, int nl
         return ORBGPU_ERR_CUDA;
     }
     cudaError_t e1 = cudaMalloc(&ex->d_descs, sizeof(LevelDesc) * ORBGPU_MAX_LEVELS);
-    cudaError_t e2 = cudaMalloc(&ex->d_status, sizeof(int) * 4);
     cudaError_t e3 = cudaMallocHost(&ex->h_pinned, sizeof(int) * 32);
-    if (e1 != cudaSuccess || e2 != cudaSuccess || e3 != cudaSuccess) {
+    if (e1 != cudaSuccess || e3 != cudaSuccess) {
         orbgpu_set_last_error("device allocation failed", __FILE__, __LINE__);
         orbgpu_extractor_destroy(ex);
         return ORBGPU_ERR_OOM;
@@ -793,7 +810,6 @@ extern "C" int orbgpu_extractor_destroy(orbgpu_extractor* ex) {
     for (SizePlan* p : ex->plans) free_plan(p);
     ex->plans.clear();
     cudaFree(ex->d_descs);
-    cudaFree(ex->d_status);
     cudaFree(ex->d_kps);
     cudaFree(ex->d_desc);
     cudaFreeHost(ex->h_pinned);
@@ -838,25 +854,31 @@ extern "C" int orbgpu_extract(orbgpu_extractor* ex, const uint8_t* image, int wi
     }
     LevelDesc hd[ORBGPU_MAX_LEVELS];
     fill_descs(g, ex->tables, P.layout, P.arena, 0, ex->ini_th, ex->min_th, 0, capacity, hd);
+    for (int l = 0; l < nl; l++) hd[l].done = P.d_sync + P.done_off[l];
+    int* const d_status = P.d_sync;
     cudaStream_t st = ex->stream;
     ORBGPU_CUDA_TRY(cudaMemcpyAsync(ex->d_descs, hd, sizeof(LevelDesc) * nl, cudaMemcpyHostToDevice, st));
-    ORBGPU_CUDA_TRY(cudaMemsetAsync(ex->d_status, 0, sizeof(int) * 4, st));
+    ORBGPU_CUDA_TRY(cudaMemsetAsync(P.d_sync, 0, P.sync_bytes, st));
     // level 0 = the image
     ORBGPU_CUDA_TRY(cudaMemcpy2DAsync(hd[0].dst, hd[0].pitch, image, step, width, height,
                                       image_mem == ORBGPU_MEM_DEVICE ? cudaMemcpyDeviceToDevice
                                                                      : cudaMemcpyHostToDevice,
                                       st));
-    // levels 1.. resized in a chain on the side stream while the strips of
-    // the levels already resized run on the extractor's stream
-    ORBGPU_CUDA_TRY(cudaEventRecord(ex->ev_fork, st));
-    ORBGPU_CUDA_TRY(cudaStreamWaitEvent(ex->side, ex->ev_fork, 0));
-    for (int l = 1; l < nl; l++) {
-        launch_level_resize(ex->d_descs, RangeMap{P.d_items + P.rb_first[l], 1, l, 0}, P.rb_count[l], P.rows, ex->side);
-        ORBGPU_CUDA_TRY(cudaEventRecord(ex->ev_level[l], ex->side));
-    }
-    for (int l = 0; l < nl; l++) {
-        if (l > 0) ORBGPU_CUDA_TRY(cudaStreamWaitEvent(st, ex->ev_level[l], 0));
-        launch_level_strip(ex->d_descs, RangeMap{P.d_items + P.rb_first[l], 1, l, 0}, P.rb_count[l], P.rows, st);
+    if (P.fused) {
+        launch_pyramid(ex->d_descs, P.pyramid, nullptr, 1, nl, d_status + 4, d_status, st);
+    } else {
+        // levels 1.. resized in a chain on the side stream while the strips of
+        // the levels already resized run on the extractor's stream
+        ORBGPU_CUDA_TRY(cudaEventRecord(ex->ev_fork, st));
+        ORBGPU_CUDA_TRY(cudaStreamWaitEvent(ex->side, ex->ev_fork, 0));
+        for (int l = 1; l < nl; l++) {
+            launch_level_resize(ex->d_descs, RangeMap{P.d_items + P.rb_first[l], 1, l, 0}, P.rb_count[l], P.rows, ex->side);
+            ORBGPU_CUDA_TRY(cudaEventRecord(ex->ev_level[l], ex->side));
+        }
+        for (int l = 0; l < nl; l++) {
+            if (l > 0) ORBGPU_CUDA_TRY(cudaStreamWaitEvent(st, ex->ev_level[l], 0));
+            launch_level_strip(ex->d_descs, RangeMap{P.d_items + P.rb_first[l], 1, l, 0}, P.rb_count[l], P.rows, st);
+        }
     }
     int mwc = 1, mhc = 1, mbox = 0;
     for (const LevelGeom& L : g) {
@@ -864,12 +886,12 @@ extern "C" int orbgpu_extract(orbgpu_extractor* ex, const uint8_t* image, int wi
         mhc = std::max(mhc, L.hCell);
         if (L.ncells > 0) mbox = std::max(mbox, fast_cell_box_w(L.wCell) * (L.hCell + 6));
     }
-    launch_fast(ex->d_descs, RangeMap{P.d_items + P.fast_first, nl, 0, 1}, P.fast_count, ex->d_status, mwc, mhc, mbox,
+    launch_fast(ex->d_descs, RangeMap{P.d_items + P.fast_first, nl, 0, 1}, P.fast_count, d_status, mwc, mhc, mbox,
                 st);
-    launch_distribute(ex->d_descs, nl, P.sort_cap, P.max_kept, ex->d_status, st);
-    launch_describe(ex->d_descs, nl, P.features, okps, odesc, ex->d_status, st);
+    launch_distribute(ex->d_descs, nl, P.sort_cap, P.max_kept, d_status, st);
+    launch_describe(ex->d_descs, nl, P.features, okps, odesc, d_status, st);
     ORBGPU_CUDA_TRY(cudaGetLastError());
-    ORBGPU_CUDA_TRY(cudaMemcpyAsync(ex->h_pinned, ex->d_status, sizeof(int), cudaMemcpyDeviceToHost, st));
+    ORBGPU_CUDA_TRY(cudaMemcpyAsync(ex->h_pinned, d_status, sizeof(int), cudaMemcpyDeviceToHost, st));
     ORBGPU_CUDA_TRY(cudaMemcpyAsync(ex->h_pinned + 4, hd[0].frame_total, sizeof(int), cudaMemcpyDeviceToHost, st));
     ORBGPU_CUDA_TRY(cudaStreamSynchronize(st));
     const int status = ex->h_pinned[0];

@@ -156,7 +156,7 @@ __host__ __device__ __forceinline__ int arc_strength(const uint8_t* roi, int rw,
 // Both kernels tile a level in strips of 120 columns x TH rows, RS_WPB strips
 // (one warp each) per block, so they share one block count per level.
 #define RS_COLS 120       // level columns per strip
-#define RS_WPB 2          // strips (warps) per block
+#define RS_WPB RS_BLOCK_TILES  // strips (warps) per block
 #define RS_CAND (30 * 28) // FAST candidates of one 7-row block at most
 
 // Level l (l >= 1) from level l-1: cv::resize INTER_LINEAR in 11-bit fixed
@@ -168,21 +168,17 @@ __host__ __device__ __forceinline__ int arc_strength(const uint8_t* roi, int rw,
 // summing to 2047..2049 (checked when the tables are built), so the
 // vertical sum 4 (h0 b0 + h1 b1) + 2^23 stays below 2^32 and its byte 3 is
 // (h0 b0 + h1 b1 + 2^21) >> 22.
-template <int TH>
-__global__ void __launch_bounds__(32 * RS_WPB) k_level_resize(const LevelDesc* descs, RangeMap rm) {
-    __shared__ int4 s_rows[RS_WPB][TH + 1];  // output row i: source rows r0, r1, 4 b0 | 4 b1 << 16
-    WorkItem it;
-    map_item(rm, blockIdx.x, it.desc, it.index);
-    const LevelDesc& d = descs[it.desc];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+// One tile by one warp; rows: TH + 1 entries of shared memory (output row i:
+// source rows r0, r1, 4 b0 | 4 b1 << 16).  ready() is called once the tables
+// are loaded, before the first source row is: false ends the tile.
+template <int TH, typename Ready>
+__device__ __forceinline__ bool resize_tile(const LevelDesc& d, int tile, int4* rows, Ready ready) {
+    const int lane = threadIdx.x & 31;
     const int w = d.w, h = d.h;
     const int tiles_x = (w + RS_COLS - 1) / RS_COLS;
-    const int tile = it.index * RS_WPB + warp;
-    if (tile >= tiles_x * ((h + TH - 1) / TH)) return;
     const int x0 = (tile % tiles_x) * RS_COLS, y0 = (tile / tiles_x) * TH;
     const int X = x0 + 4 * lane;
     const bool writer = lane < RS_COLS / 4 && X < w;
-    int4* rows = s_rows[warp];
     for (int i = lane; i <= TH; i += 32) {
         const int y = min(y0 + i, h - 1);
         const int sy = d.yofs[y];
@@ -235,6 +231,7 @@ __global__ void __launch_bounds__(32 * RS_WPB) k_level_resize(const LevelDesc* d
         }
     };
 
+    if (!ready()) return false;
     const int nrows = min(TH, h - y0);
     // source words of output rows i (set i & 1) and i + 1, loaded two rows ahead
     uint32_t pw[2][6];
@@ -279,6 +276,21 @@ __global__ void __launch_bounds__(32 * RS_WPB) k_level_resize(const LevelDesc* d
         row_step(i, pw[0]);
         if (i + 1 < nrows) row_step(i + 1, pw[1]);
     }
+    return true;
+}
+
+__device__ __forceinline__ int level_tiles(const LevelDesc& d, int th) {
+    return ((d.w + RS_COLS - 1) / RS_COLS) * ((d.h + th - 1) / th);
+}
+
+template <int TH>
+__global__ void __launch_bounds__(32 * RS_WPB) k_level_resize(const LevelDesc* descs, RangeMap rm) {
+    __shared__ int4 s_rows[RS_WPB][TH + 1];
+    WorkItem it;
+    map_item(rm, blockIdx.x, it.desc, it.index);
+    const LevelDesc& d = descs[it.desc];
+    const int tile = it.index * RS_WPB + (threadIdx.x >> 5);
+    if (tile < level_tiles(d, TH)) resize_tile<TH>(d, tile, s_rows[threadIdx.x >> 5], []() { return true; });
 }
 
 // The 7x7 Gaussian (8-bit fixed point, REFLECT_101) of every pixel of level l
@@ -324,20 +336,14 @@ __device__ __forceinline__ uint32_t rs_compass(uint32_t c, uint32_t p0, uint32_t
     return (((b0 | b8) & (b4 | b12)) | ((d0 | d8) & (d4 | d12))) & 0x80008000u;
 }
 
+// One strip by one warp.
 template <int TH>
-__global__ void __launch_bounds__(32 * RS_WPB, 12) k_level_strip(const LevelDesc* descs, RangeMap rm) {
+__device__ __forceinline__ void strip_tile(const LevelDesc& d, int tile, StripShared<TH>& S) {
     static_assert((TH + 6) % 7 == 0, "TH + 6 rows must be whole blocks of 7");
     constexpr int NB = (TH + 6) / 7;
-    __shared__ __align__(16) StripShared<TH> sh_all[RS_WPB];
-    WorkItem it;
-    map_item(rm, blockIdx.x, it.desc, it.index);
-    const LevelDesc& d = descs[it.desc];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31;
     const int w = d.w, h = d.h, pitch = d.pitch;
     const int tiles_x = (w + RS_COLS - 1) / RS_COLS;
-    const int tile = it.index * RS_WPB + warp;
-    if (tile >= tiles_x * ((h + TH - 1) / TH)) return;
-    StripShared<TH>& S = sh_all[warp];
     const int x0 = (tile % tiles_x) * RS_COLS, y0 = (tile / tiles_x) * TH;
     const int X = x0 - 4 + 4 * lane;
     const bool writer = lane >= 1 && lane <= 30 && X < w;
@@ -438,6 +444,114 @@ __global__ void __launch_bounds__(32 * RS_WPB, 12) k_level_strip(const LevelDesc
             }
         }
     }
+}
+
+template <int TH>
+__global__ void __launch_bounds__(32 * RS_WPB, 12) k_level_strip(const LevelDesc* descs, RangeMap rm) {
+    __shared__ __align__(16) StripShared<TH> sh_all[RS_WPB];
+    WorkItem it;
+    map_item(rm, blockIdx.x, it.desc, it.index);
+    const LevelDesc& d = descs[it.desc];
+    const int tile = it.index * RS_WPB + (threadIdx.x >> 5);
+    if (tile < level_tiles(d, TH)) strip_tile<TH>(d, tile, sh_all[threadIdx.x >> 5]);
+}
+
+// All resizes and strips of a small launch (a frame, a few frames) in one
+// kernel: seven resizes that wait for one another take seven launches
+// otherwise, most of a frame's time.  A block takes the next ticket (in ticket
+// order: resizes of level 1, 2, strips of level 0, resizes of level 3, strips
+// of level 1, ...), whose two tiles wait for the row bands they read --
+// d.done[band] counts the tiles of a band of RT rows that are written -- and
+// count themselves in theirs.  A ticket waits only for lower tickets, and every
+// lower ticket is held by a block that is running or done, so the waits end
+// whatever order the device starts the blocks in; they are bounded all the same
+// (status bit 128).
+//
+// Bound by the chain of levels: per level the poll that sees the band, the
+// tile (two rows of loads in flight: 7,000 cycles for 8 rows) and the fence
+// before its count (1,500).  So the resizes' tiles are RT = 2 rows, or 4 where
+// the tiles are so many that their fixed cost counts; the strips are TH = 8.
+struct PyrEntry {
+    int level;
+    bool resize;
+};
+// stage of a launch of n levels -> its level and kind (2 n - 1 stages)
+__host__ __device__ inline PyrEntry pyr_entry(int stage, int n) {
+    // R1, R2, S0, R3, S1, ..., R(n-1), S(n-3), S(n-2), S(n-1); one level: S0
+    if (n == 1) return {0, false};
+    if (stage == 0) return {1, true};
+    const int k = stage - 1;  // R2, S0, R3, S1, ...
+    if (k / 2 + 2 < n) return k & 1 ? PyrEntry{k / 2, false} : PyrEntry{k / 2 + 2, true};
+    return {stage - (n - 1), false};  // the last two strips
+}
+
+// Waits until the bands [b0, b1] of d are written.
+__device__ __forceinline__ bool bands_ready(const LevelDesc& d, int b0, int b1) {
+    const int lane = threadIdx.x & 31;
+    const int need = (d.w + RS_COLS - 1) / RS_COLS;
+    bool ok = true;
+    for (int b = b0 + lane; b <= b1 && ok; b += 32) {
+        const int* p = d.done + b;
+        uint64_t t0 = 0;
+        for (uint32_t i = 0; i < ORBGPU_SPIN_LIMIT; i++) {
+            int v;
+            asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+            ok = v >= need;
+            if (ok) break;
+            __nanosleep(100);  // the waiting warps leave the issue slots and L2 to the ones at work
+            if ((i & 63) == 63) {
+                const uint64_t t = global_ns();
+                if (t0 == 0) t0 = t;
+                else if (t - t0 > ORBGPU_WAIT_NS) break;
+            }
+        }
+    }
+    return __all_sync(0xffffffffu, ok);
+}
+
+// first[s]: the first block of stage s; prefix: the first block of every
+// (stage, frame), stage-major, relative to its stage.
+template <int TH, int RT>
+__global__ void __launch_bounds__(32 * RS_WPB, 12)
+    k_pyramid(const LevelDesc* descs, const __grid_constant__ PyramidStages stages, const int* prefix, int nframes,
+              int nlevels, int* ticket, int* status) {
+    union Shared {
+        int4 rows[RT + 1];
+        StripShared<TH> strip;
+    };
+    __shared__ __align__(16) Shared sh[RS_WPB];
+    __shared__ int s_ticket;
+    if (threadIdx.x == 0) s_ticket = atomicAdd(ticket, 1);
+    __syncthreads();
+    int stage = 0;
+    while (stage + 1 < 2 * nlevels - 1 && stages.first[stage + 1] <= s_ticket) stage++;
+    WorkItem it{0, s_ticket - stages.first[stage]};
+    if (nframes > 1) map_item(RangeMap{prefix + (size_t)stage * nframes, nframes, 0, 1}, it.index, it.desc, it.index);
+    const PyrEntry e = pyr_entry(stage, nlevels);
+    const LevelDesc& d = descs[it.desc * nlevels + e.level];
+    const int warp = threadIdx.x >> 5;
+    const int tile = it.index * RS_WPB + warp;
+    if (tile >= level_tiles(d, e.resize ? RT : TH)) return;
+    const int tiles_x = (d.w + RS_COLS - 1) / RS_COLS;
+    bool ok;
+    if (e.resize) {
+        const int band = tile / tiles_x, last = min(RT, d.h - band * RT) - 1;
+        ok = resize_tile<RT>(d, tile, sh[warp].rows, [&]() {
+            // the source rows of the tile's first and last row
+            return e.level == 1 || bands_ready((&d)[-1], sh[warp].rows[0].x / RT, sh[warp].rows[last].y / RT);
+        });
+        __syncwarp();
+        if (ok && (threadIdx.x & 31) == 0) {
+            __threadfence();  // the tile's rows before its count
+            atomicAdd(d.done + band, 1);
+        }
+    } else {
+        // three rows of halo on each side, reflected inside the level
+        const int y0 = tile / tiles_x * TH, y1 = min(y0 + TH, d.h) - 1;
+        ok = e.level == 0 || bands_ready(d, max(y0 - 3, 0) / RT, min(y1 + 3, d.h - 1) / RT);
+        if (ok) strip_tile<TH>(d, tile, sh[warp].strip);
+    }
+    if (!ok && (threadIdx.x & 31) == 0) atomicOr(status, 128);
 }
 
 #define FAST_MAX_ROI 72
@@ -1557,6 +1671,46 @@ void launch_level_strip(const LevelDesc* descs, RangeMap rm, int nitems, int row
         case 64: launch_strip_only<64>(descs, rm, nitems, st); break;
         default: launch_strip_only<36>(descs, rm, nitems, st); break;
     }
+}
+
+// Whether a launch of strips of 'rows' rows is short enough for k_pyramid, and
+// with which tiles.  Measured on frames of 752x480 (the resizes and strips, in
+// microseconds; one launch per level, tiles of 4 rows, of 2 rows):
+// 1 frame 63, 35, 29; 2 66, 37, 31; 4 68, 39, 41; 8 78, 57, 66; 12 87, 78, 96;
+// 16 99, 100, 124; 24 121, 148, 187.  The whole extraction, whose other kernels
+// then start later or earlier, crosses at the same place (12 frames 247 -> 239,
+// 16 269 -> 273).  One such frame has 1,339 strips and 5,000 tiles at 2 rows.
+bool plan_pyramid(int rows, int nframes, int nlevels, const std::vector<int>& w, const std::vector<int>& h, PyramidPlan& P) {
+    P = PyramidPlan{};
+    if (rows != 8) return false;
+    auto tiles = [&](size_t i, int th) { return (long)((w[i] + RS_COLS - 1) / RS_COLS) * ((h[i] + th - 1) / th); };
+    long strips = 0, resizes2 = 0;
+    for (int f = 0; f < nframes; f++)
+        for (int l = 0; l < nlevels; l++) {
+            strips += tiles((size_t)f * nlevels + l, 8);
+            if (l > 0) resizes2 += tiles((size_t)f * nlevels + l, 2);
+        }
+    const long resident = 24L * nsm_of_current_device();  // warps: 12 blocks per SM
+    if (strips > 5 * resident) return false;
+    P.rt = 2 * (strips + resizes2) <= 7 * resident ? 2 : 4;
+    int acc = 0;
+    for (int stage = 0; stage < 2 * nlevels - 1; stage++) {
+        const PyrEntry e = pyr_entry(stage, nlevels);
+        P.stages.first[stage] = acc;
+        int in_stage = 0;
+        for (int f = 0; f < nframes; f++) {
+            P.prefix.push_back(in_stage);
+            in_stage += (int)((tiles((size_t)f * nlevels + e.level, e.resize ? P.rt : 8) + RS_WPB - 1) / RS_WPB);
+        }
+        acc += in_stage;
+    }
+    P.blocks = acc;
+    return true;
+}
+void launch_pyramid(const LevelDesc* descs, const PyramidPlan& P, const int* prefix, int nframes, int nlevels, int* ticket,
+                    int* status, cudaStream_t st) {
+    if (P.rt == 2) k_pyramid<8, 2><<<P.blocks, 32 * RS_WPB, 0, st>>>(descs, P.stages, prefix, nframes, nlevels, ticket, status);
+    else k_pyramid<8, 4><<<P.blocks, 32 * RS_WPB, 0, st>>>(descs, P.stages, prefix, nframes, nlevels, ticket, status);
 }
 
 // Blocks of k_level_resize / k_level_strip for a w x h level (RS_WPB strips

@@ -10,6 +10,8 @@
 //                        detection region (a candidate bit map): one warp per
 //                        120-column strip, rows walked with a 7-row register
 //                        window.
+//   k_pyramid            both for every level of a frame or a few, in one
+//                        launch.
 //   k_fast_cells         one 30-px cell at a time per warp (persistent, in
 //                        chunks of 1 or 2 cells): the cell's ROI staged in
 //                        shared memory by a tensor copy, the segment test and
@@ -20,10 +22,12 @@
 //   k_distribute         one (frame, level) per block: DistributeOctTree as a
 //                        sequence of parallel split steps over node creation
 //                        numbers, its arrays in shared memory when they fit.
-//   k_describe           8, 16 or 32 keypoints per warp task, their patches
+//   k_describe           1 to 32 keypoints per warp task, their patches
 //                        staged in shared memory by tensor copies in rounds
 //                        of 1 to 4: IC_Angle, fastAtan2, rBRIEF.
 #pragma once
+
+#include <vector>
 
 #include "orbgpu_common.cuh"
 
@@ -55,6 +59,7 @@ struct LevelDesc {
     const short* xalpha;  // 2 weights per output column
     const int* yofs;      // source row per output row (unclamped)
     const short* ybeta;   // 2 weights per output row
+    int* done;            // per band of rows: tiles of this level written so far (k_pyramid)
     // FAST cells
     int nCols, nRows, wCell, hCell;
     int maxBorderX, maxBorderY;
@@ -184,6 +189,26 @@ inline int fast_cell_box_w(int wcell) { return (15 + wcell + 6 + 15) & ~15; }
 void launch_fast(const LevelDesc* descs, RangeMap rm, int ncells, int* status, int max_wcell, int max_hcell,
                  int max_box_bytes, cudaStream_t st);
 int resize_blur_tiles(int w, int h, int rows);
+#define RS_BLOCK_TILES 2  // tiles (warps) of a resize / strip block
+// The resizes and strips of a small launch in one kernel (k_pyramid): the
+// first block of each of its 2 nlevels - 1 stages, the first block of every
+// (stage, frame) relative to its stage, and the rows of the resizes' tiles.
+struct PyramidStages {
+    int first[2 * ORBGPU_MAX_LEVELS];
+};
+struct PyramidPlan {
+    PyramidStages stages{};
+    std::vector<int> prefix;
+    int blocks = 0, rt = 4;
+};
+#define PYRAMID_BAND 2  // the levels' counters are sized for bands of this many rows
+// Whether a launch of strips of 'rows' rows takes it, and its plan; w and h:
+// the levels' sizes, frame-major.
+bool plan_pyramid(int rows, int nframes, int nlevels, const std::vector<int>& w, const std::vector<int>& h, PyramidPlan& P);
+// prefix: P.prefix on the device; the ticket and the levels' 'done' counters
+// are zero beforehand.
+void launch_pyramid(const LevelDesc* descs, const PyramidPlan& P, const int* prefix, int nframes, int nlevels, int* ticket,
+                    int* status, cudaStream_t st);
 int strip_rows(long level0_pixels);
 // DistributeOctTree of every (frame, level); node_cap: the largest level's
 // node capacity (its arrays go to shared memory when they fit).

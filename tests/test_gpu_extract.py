@@ -249,3 +249,51 @@ def test_batch_parameters_vs_oracle(torch, oracle, scale, nlevels, ini, mn):
         assert c[f] == len(ref.keypoints), f"frame {f}"
         assert_kps_equal(k[f, :c[f]], ref.keypoints, f"frame {f}")
         assert np.array_equal(d[f, :c[f]], ref.descriptors)
+
+
+# One launch for all resizes and strips: one level (strips only), two and three
+# (the stages' order at its ends), eight; widths and heights around the tiles'
+# 120 columns and 2, 4 and 8 rows; a source span of many bands.
+@pytest.mark.parametrize("w,h,scale,nlevels", [(121, 81, 1.2, 1), (120, 96, 1.2, 2), (241, 83, 1.1, 3),
+                                               (359, 203, 1.2, 8), (640, 473, 3.0, 3)])
+def test_pyramid_launches(torch, oracle, w, h, scale, nlevels):
+    from orb_slam2_detailed_comments_gb300 import ORBextractor, autotune
+    from orb_slam2_detailed_comments_gb300._lib import KEYPOINT_DTYPE
+    from orb_slam2_detailed_comments_gb300 import synthetic as syn
+    from orb_slam2_detailed_comments_gb300.batch import BatchExtractor
+    imgs = [syn.scene(w, h, 60), syn.scene(w + 3, h + 1, 61), syn.scene(w + 640, h + 480, 62),
+            syn.scene(w + 900, h + 481, 63)]
+    refs = [oracle.extract(i, nfeatures=400, scale_factor=scale, nlevels=nlevels) for i in imgs]
+
+    def check():
+        for img, ref in zip(imgs, refs):
+            ex = ORBextractor(400, scale, nlevels, 20, 7)
+            kps, desc = ex(img)
+            for l, (a, b) in enumerate(zip(ex.pyramid_numpy(), ref.pyramid)):
+                assert np.array_equal(a, b), f"{img.shape} level {l}"
+            for l, (a, b) in enumerate(zip(ex.pyramid_numpy(blurred=True), ref.pyramid)):
+                bb = np.zeros_like(b)
+                oracle.lib.orc_blur_level(b.ctypes.data_as(pyoracle.C.c_void_p), b.shape[1], b.shape[0],
+                                          bb.ctypes.data_as(pyoracle.C.c_void_p))
+                assert np.array_equal(a, bb), f"{img.shape} blurred level {l}"
+            assert_kps_equal(kps, ref.keypoints, f"{img.shape}")
+            assert np.array_equal(desc, ref.descriptors)
+        for n in (1, 2, 4):
+            b = BatchExtractor(n, w + 900, h + 481, 400, scale_factor=scale, nlevels=nlevels)
+            cap = b.per_frame_capacity
+            for _ in range(2):  # the second call replays the graph
+                k, d, c = b.extract([torch.from_numpy(i).cuda() for i in imgs[:n]], [400] * n)
+                k = k.cpu().numpy().view(KEYPOINT_DTYPE).reshape(n, cap)
+                d = d.cpu().numpy().reshape(n, cap, 32)
+                for f, ref in enumerate(refs[:n]):
+                    m = int(c[f])
+                    assert_kps_equal(k[f, :m], ref.keypoints, f"frame {f} of {n}")
+                    assert np.array_equal(d[f, :m], ref.descriptors)
+
+    check()
+    before = autotune.current()
+    try:
+        autotune.set_param("strip_rows_small", 0)  # one launch per level
+        check()
+    finally:
+        autotune.apply({k: v for k, v in before.items() if k != "knn_tc_min_pairs"})
