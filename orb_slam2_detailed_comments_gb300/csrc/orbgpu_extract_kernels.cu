@@ -1721,15 +1721,18 @@ int resize_blur_tiles(int w, int h, int rows) {
 }
 // Strip rows of a launch whose level 0 holds 'px' pixels: the tuned value,
 // or (unless the policy is off) 8 when the tuned strips of level 0 would not
-// fill the device's resident warps one and a half times over (a warp walks
-// its strip's rows one after the other, so a short launch is bound by that
-// walk, not by the work).
+// fill the device's resident warps twice over (a warp walks its strip's rows
+// one after the other, so a short launch is bound by that walk, not by the
+// work).  Resizes and strips in microseconds at 8, 22, 36, 64 rows (strips of
+// 22 rows per resident warp): 32 frames of mixed sizes (1.7) 184, 196, 184,
+// 184; 64 of 752x480 (2.4) 258, 243, 257, 257; 64 mixed (3.4) 326, 294, 321,
+// 326; 128 of 1241x376 (6.2) 567, 464, 483, 526.
 int strip_rows(long px) {
     const int th = tunables().resize_rows;
     if (tunables().strip_rows_small == 0 || th <= 8) return th;
     const long strips = px / ((long)RS_COLS * th);
     const long resident = (long)nsm_of_current_device() * 12 * RS_WPB;  // k_level_strip: 12 blocks per SM
-    return 2 * strips < 3 * resident ? 8 : th;
+    return strips < 2 * resident ? 8 : th;
 }
 void launch_fast(const LevelDesc* descs, RangeMap rm, int ncells, int* status, int max_wcell, int max_hcell,
                  int max_box_bytes, cudaStream_t st) {

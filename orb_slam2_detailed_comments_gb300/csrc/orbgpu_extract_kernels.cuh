@@ -121,7 +121,7 @@ struct LevelDesc {
 // Changing one bumps the generation, so cached frame plans and captured
 // graphs are rebuilt.
 struct Tunables {
-    int resize_rows = 36;
+    int resize_rows = 22;
     int fast_cells_per_block = 4;
     int describe_group = 1;
     int describe_depth = 2;
