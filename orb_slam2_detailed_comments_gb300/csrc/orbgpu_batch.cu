@@ -118,7 +118,7 @@ struct orbgpu_batch {
     LevelDesc* d_descs = nullptr;
     size_t descs_cap = 0;
     int ndesc = 0;
-    int max_kept = 0, sort_cap = 0;
+    int max_kept = 0;
     long features = 0;  // the budgets of all levels with cells
     ImageSrc* d_src = nullptr;
     ImageSrc* h_src = nullptr;  // pinned
@@ -436,13 +436,11 @@ static int plan_batch(orbgpu_batch* b, int nframes, const int* widths, const int
     }
     ORBGPU_CUDA_TRY(cudaMemcpyAsync(b->d_prefix, pre.data(), sizeof(int) * pre.size(), cudaMemcpyHostToDevice, st));
     b->max_kept = 0;
-    b->sort_cap = 1;
     b->features = 0;
     for (int f = 0; f < nframes; f++)
         for (auto& L : b->cur[f]->geom) {
             if (L.ncells > 0) b->features += L.nfeat + 1;
             b->max_kept = std::max(b->max_kept, L.node_cap);
-            while (b->sort_cap < L.node_cap) b->sort_cap <<= 1;
         }
     b->nframes = nframes;
     b->ndesc = ndesc;
@@ -500,7 +498,7 @@ static void enqueue_pipeline(orbgpu_batch* b, orbgpu_keypoint* kps, uint8_t* des
     launch_fast(b->d_descs, RangeMap{b->d_prefix + b->fast_off, b->ndesc, 0, 1}, b->fast_count, b->d_status, mwc, mhc,
                 mbox, st);
     mark(3);
-    launch_distribute(b->d_descs, b->ndesc, b->sort_cap, b->max_kept, b->d_status, st);
+    launch_distribute(b->d_descs, b->nframes, b->nlevels, b->max_kept, b->d_status, st);
     mark(4);
     launch_describe(b->d_descs, b->ndesc, b->features, kps, desc, b->d_status, st);
     mark(5);

@@ -276,15 +276,8 @@ size_t FrameLayout::plan(const std::vector<LevelGeom>& g, size_t base) {
         o.cell_count = take(sizeof(int) * std::max(1, L.ncells));
         o.cand = take(sizeof(uint32_t) * std::max(1, L.cand_cap));
         o.node_of = take(sizeof(int) * std::max(1, L.cand_cap));
-        o.quad = take(std::max(1, L.cand_cap));
-        o.nodes_a = take(sizeof(DNode) * L.node_cap);
-        o.nodes_b = take(sizeof(DNode) * L.node_cap);
-        o.cnt4 = take(sizeof(int4) * L.node_cap);
-        o.childpos = take(sizeof(int4) * L.node_cap);
-        o.aux0 = take(sizeof(int) * L.node_cap);
-        o.aux1 = take(sizeof(int) * L.node_cap);
-        o.aux2 = take(sizeof(int) * L.node_cap);
-        o.best = take(sizeof(uint32_t) * L.node_cap);
+        o.nodes = take(dist_node_bytes(L.node_cap));
+        o.sort = take(sizeof(unsigned long long) * dist_sort_cap(L.node_cap));
         o.kept = take(sizeof(uint32_t) * L.node_cap);
     }
     level_counts = take(sizeof(int) * 16);
@@ -337,15 +330,8 @@ void fill_descs(const std::vector<LevelGeom>& g, const ExtractorTables& t, const
         d.node_cap = L.node_cap;
         d.cand = (uint32_t*)(arena + o.cand);
         d.node_of = (int*)(arena + o.node_of);
-        d.quad = arena + o.quad;
-        d.nodes_a = arena + o.nodes_a;
-        d.nodes_b = arena + o.nodes_b;
-        d.cnt4 = (int4*)(arena + o.cnt4);
-        d.childpos = (int4*)(arena + o.childpos);
-        d.aux0 = (int*)(arena + o.aux0);
-        d.aux1 = (int*)(arena + o.aux1);
-        d.aux2 = (int*)(arena + o.aux2);
-        d.best = (uint32_t*)(arena + o.best);
+        d.nodes = arena + o.nodes;
+        d.sort = (unsigned long long*)(arena + o.sort);
         d.kept = (uint32_t*)(arena + o.kept);
         d.level_counts = (int*)(arena + lay.level_counts);
         d.kept_count = d.level_counts + l;
@@ -557,7 +543,7 @@ struct SizePlan {
     int* d_sync = nullptr;
     size_t sync_bytes = 0;
     std::vector<int> done_off;
-    int max_kept = 0, sort_cap = 0;
+    int max_kept = 0;
     long features = 0;  // the budgets of all levels with cells
     uint64_t last_use = 0;
     int gen = -1;  // tuning generation of the work lists
@@ -674,11 +660,9 @@ static int build_plan(orbgpu_extractor* ex, int w, int h, SizePlan** out) {
         return ORBGPU_ERR_OOM;
     }
     P->max_kept = 0;
-    P->sort_cap = 1;
     for (auto& L : g) {
         if (L.ncells > 0) P->features += L.nfeat + 1;
         P->max_kept = std::max(P->max_kept, L.node_cap);
-        while (P->sort_cap < L.node_cap) P->sort_cap <<= 1;
     }
     P->w = w;
     P->h = h;
@@ -888,7 +872,7 @@ extern "C" int orbgpu_extract(orbgpu_extractor* ex, const uint8_t* image, int wi
     }
     launch_fast(ex->d_descs, RangeMap{P.d_items + P.fast_first, nl, 0, 1}, P.fast_count, d_status, mwc, mhc, mbox,
                 st);
-    launch_distribute(ex->d_descs, nl, P.sort_cap, P.max_kept, d_status, st);
+    launch_distribute(ex->d_descs, 1, nl, P.max_kept, d_status, st);
     launch_describe(ex->d_descs, nl, P.features, okps, odesc, d_status, st);
     ORBGPU_CUDA_TRY(cudaGetLastError());
     ORBGPU_CUDA_TRY(cudaMemcpyAsync(ex->h_pinned, d_status, sizeof(int), cudaMemcpyDeviceToHost, st));

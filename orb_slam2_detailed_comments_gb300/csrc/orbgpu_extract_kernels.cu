@@ -948,390 +948,437 @@ __global__ void k_fast_strength_map(const uint8_t* img, int pitch, int w, int h,
 // split step therefore rebuilds the list as: the children created in this
 // step in reverse creation order, followed by the nodes that were not split,
 // in their previous order.  Node arrays are indexed by list position.
+//
+// One (frame, level) per 512-thread block.  A step is one pass of the keys --
+// each follows its node to its new list position, takes its quadrant there and
+// counts itself -- and one pass of the nodes, four lanes each, which places the
+// children by ballots and one block-wide sum and leaves, in the place of a
+// node's four counts, the list positions of its four quadrants.  Bound by
+// latency: of 31,000 cycles for a level of 1,747 keys (16 us; the launch's
+// other levels are shorter) the candidates' loads take 8,000, a pass of the
+// nodes 2,500, of the keys 1,600 (six shared-memory operations each), the
+// final phase's order and cut 3,400.  Keys in registers were no faster (the
+// registers spilled at three blocks per SM), one instead of four lanes' worth of
+// serial code per node took three times as long.
+// Every node with several keys was created by the last step, so the reference's
+// order of the final phase (most keys first, then latest created) is (keys
+// descending, list position ascending), and a node's place in it is the number
+// of nodes before it: counted up to DIST_T nodes (1,900 cycles for the 128 of a
+// usual level, 6,200 by the bitonic sort that longer lists take).
+// One 1280x720 frame 34.5 -> 22.4 us, 64 frames 73.6 -> 39.1 us.
+#define DIST_T 512
+__device__ __forceinline__ int dist_first() { return (threadIdx.x & 31) * (DIST_T / 32) + (threadIdx.x >> 5); }
+// Dynamic shared memory: the sort keys of the final phase, then the node arrays
+// and the keys' arrays as far as the launch's budget holds them.
+extern __shared__ __align__(16) unsigned long long s_dist[];
 
-__device__ __forceinline__ int quadrant_of(uint32_t p, const DNode& n) {
-    const float x = (float)((int)(p & 0xFFF) - (ORBGPU_EDGE_THRESHOLD - 3));
-    const float y = (float)((int)((p >> 12) & 0xFFF) - (ORBGPU_EDGE_THRESHOLD - 3));
-    const int halfX = (int)ceilf(__fdiv_rn((float)(n.x1 - n.x0), 2.f));
-    const int halfY = (int)ceilf(__fdiv_rn((float)(n.y1 - n.y0), 2.f));
-    const int xm = n.x0 + halfX, ym = n.y0 + halfY;
-    if (x < (float)xm) return y < (float)ym ? 0 : 2;
-    return y < (float)ym ? 1 : 3;
-}
-
-__device__ __forceinline__ DNode child_rect(const DNode& n, int q) {
-    const int halfX = (int)ceilf(__fdiv_rn((float)(n.x1 - n.x0), 2.f));
-    const int halfY = (int)ceilf(__fdiv_rn((float)(n.y1 - n.y0), 2.f));
-    const int xm = n.x0 + halfX, ym = n.y0 + halfY;
-    DNode c;
-    c.x0 = (int16_t)((q & 1) ? xm : n.x0);
-    c.x1 = (int16_t)((q & 1) ? n.x1 : xm);
-    c.y0 = (int16_t)((q & 2) ? ym : n.y0);
-    c.y1 = (int16_t)((q & 2) ? n.y1 : ym);
-    return c;
-}
-
-// The working arrays of one level's DistributeOctTree: the keys (candidate,
-// node, quadrant) and the nodes (two node lists, quadrant counts, child
-// positions, three scratch ints, best key), each in shared memory when the
-// launch's budget holds it, else in the level's global buffers.
+// The working arrays of one level: the node arrays of nc nodes (two lists) in
+// one block of memory and the keys' candidate and node * 4 + quadrant.  SM: all
+// in shared memory at these offsets (32-bit addresses); else by pointer.
+template <bool SM>
 struct DistArrays {
-    uint32_t* cand;
-    int* node_of;
-    uint8_t* quad;
-    DNode *a, *b;
-    int4 *cnt4, *childpos;
-    int *aux0, *aux1, *aux2;
-    uint32_t* best;
+    uint8_t *sort_mem, *nodes, *cand_mem, *at_mem;
+    int nodes_off, cand_off, at_off, nc;
+    template <typename T>
+    __device__ __forceinline__ T* at_(uint8_t* p, int off) const {
+        return SM ? (T*)((uint8_t*)s_dist + off) : (T*)p;
+    }
+    template <typename T>
+    __device__ __forceinline__ T* node_array(int bytes_before) const {
+        return SM ? (T*)((uint8_t*)s_dist + nodes_off + bytes_before * nc) : (T*)(nodes + (size_t)bytes_before * nc);
+    }
+    // the nodes of several keys: keys << 32 | ~position
+    __device__ __forceinline__ unsigned long long* sort() const { return at_<unsigned long long>(sort_mem, 0); }
+    // keys per quadrant, then the quadrants' positions in the next list
+    __device__ __forceinline__ int4* cnt(int list) const { return node_array<int4>(16 * list); }
+    // x0 | x1 << 16, y0 | y1 << 16; only nodes that can be split
+    __device__ __forceinline__ int2* rect(int list) const { return node_array<int2>(32 + 8 * list); }
+    // the split lines xm | ym << 16 in candidate coordinates; 0: a node of one key
+    __device__ __forceinline__ uint32_t* mid(int list) const { return node_array<uint32_t>(48 + 4 * list); }
+    // final phase: place among the candidates; node | children << 16 by place; creation base
+    __device__ __forceinline__ int* place() const { return node_array<int>(56); }
+    __device__ __forceinline__ uint32_t* order() const { return node_array<uint32_t>(60); }
+    __device__ __forceinline__ int* created() const { return node_array<int>(64); }
+    // key k's place in cand() and at(): lanes 16 keys apart (dist_first) take
+    // different banks
+    static __device__ __forceinline__ int at_key(int k) { return SM ? k + (k >> 4) : k; }
+    __device__ __forceinline__ uint32_t* cand() const { return at_<uint32_t>(cand_mem, cand_off); }
+    __device__ __forceinline__ int* at() const { return at_<int>(at_mem, at_off); }
 };
-#define DIST_KEY_BYTES 9  // per key: cand, node_of, quad
-// Shared-memory offsets of the node arrays for nc nodes: a and b, then
-// (16-byte aligned) cnt4 and childpos, then aux0-2 and best; the total is a
-// multiple of 16.
-__host__ __device__ inline size_t dist_nodes_ab(size_t nc) { return (2 * nc * sizeof(DNode) + 15) & ~(size_t)15; }
-__host__ __device__ inline size_t dist_node_bytes(size_t nc) {
-    return (dist_nodes_ab(nc) + 2 * nc * sizeof(int4) + 4 * nc * sizeof(int) + 15) & ~(size_t)15;
+
+__device__ __forceinline__ int2 dist_mid(int2 r) {
+    const int x0 = (int16_t)r.x, x1 = r.x >> 16, y0 = (int16_t)r.y, y1 = r.y >> 16;
+    return {x0 + ((x1 - x0 + 1) >> 1), y0 + ((y1 - y0 + 1) >> 1)};  // ceil of half the extent
+}
+__device__ __forceinline__ uint32_t dist_mid_word(int2 m) {
+    constexpr int o = ORBGPU_EDGE_THRESHOLD - 3;
+    return (uint32_t)(m.x + o) | (uint32_t)(m.y + o) << 16;
+}
+__device__ __forceinline__ int dist_quadrant(uint32_t p, uint32_t mid) {
+    return (int)((p & 0xFFF) >= (mid & 0xFFFF)) + 2 * (int)(((p >> 12) & 0xFFF) >= (mid >> 16));
+}
+// Block-wide sums of one value per warp, and the sums of the warps before;
+// one barrier.  Consecutive calls take the two halves of part in turn.
+struct DistSums {
+    int4 before, total;
+};
+__device__ __forceinline__ DistSums dist_sums(int4 warp_value, int4 (*part)[DIST_T / 32], int& half) {
+    constexpr unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    if (lane == 0) part[half][wid] = warp_value;
+    __syncthreads();
+    const int4 v = lane < DIST_T / 32 ? part[half][lane] : make_int4(0, 0, 0, 0);
+    const int m = lane < wid ? -1 : 0;
+    half ^= 1;
+    return {make_int4(__reduce_add_sync(FULL, v.x & m), __reduce_add_sync(FULL, v.y & m), __reduce_add_sync(FULL, v.z & m),
+                      0),
+            make_int4(__reduce_add_sync(FULL, v.x), __reduce_add_sync(FULL, v.y), __reduce_add_sync(FULL, v.z),
+                      __reduce_add_sync(FULL, v.w))};
 }
 
-// Applies one split step.  split_rank[n] >= 0 is node n's rank in creation
-// order (nsplit nodes split), -1 for nodes kept.  order[rank] = node.
-// Returns (through smem) the new alive count and the number of children with
-// more than one key.
-__device__ void split_step(const LevelDesc& d, const DistArrays& m, DNode*& A, DNode*& B, int& alive, int K,
-                           int nsplit, int& next_id, int& n_big, int* s_scan, int* s_vars) {
-    int* split_rank = m.aux0;
-    int* order = m.aux1;
-    int* base = m.aux2;
-    // 1. quadrant counts for keys of split nodes
-    for (int n = threadIdx.x; n < alive; n += blockDim.x) m.cnt4[n] = make_int4(0, 0, 0, 0);
-    __syncthreads();
-    for (int k = threadIdx.x; k < K; k += blockDim.x) {
-        const int n = m.node_of[k];
-        if (split_rank[n] < 0) continue;
-        const int q = quadrant_of(m.cand[k], A[n]);
-        m.quad[k] = (uint8_t)q;
-        atomicAdd(&((int*)&m.cnt4[n])[q], 1);
+// The keys follow their nodes to the new list (buffer nx of the nodes; the old
+// one holds the positions) and count in their quadrants.  Neighbouring lanes
+// take keys apart, so that they seldom count in the same node.
+template <bool SM>
+__device__ __forceinline__ void dist_count(const DistArrays<SM>& m, int cur, int K) {
+    const int nx = cur ^ 1;
+    const int* pos = (const int*)m.cnt(cur);
+    int* cnt = (int*)m.cnt(nx);
+    const uint32_t *mid = m.mid(nx), *cand = m.cand();
+    int* at = m.at();
+#pragma unroll 2
+    for (int k = dist_first(); k < K; k += DIST_T) {
+        const int i = m.at_key(k), n = pos[at[i]];
+        const uint32_t w = mid[n];
+        const int q = dist_quadrant(cand[i], w) & (w ? 3 : 0);
+        at[i] = 4 * n + q;
+        if (w) atomicAdd(&cnt[4 * n + q], 1);
+    }
+}
+// Per node the key with the largest response, first in key order.
+template <bool SM>
+__device__ __forceinline__ void dist_best(const DistArrays<SM>& m, int cur, int K, uint32_t* kept) {
+    const int* pos = (const int*)m.cnt(cur);
+    uint32_t* best = (uint32_t*)m.cnt(cur ^ 1);
+    const uint32_t* cand = m.cand();
+    int* at = m.at();
+    auto rank = [&](uint32_t p, int k) { return ((p >> 24) << 20) | (uint32_t)(0xFFFFF - k); };
+#pragma unroll 2
+    for (int k = dist_first(); k < K; k += DIST_T) {
+        const int i = m.at_key(k), n = pos[at[i]];
+        at[i] = n;
+        atomicMax(&best[n], rank(cand[i], k));
     }
     __syncthreads();
-    // 2. children per split node, in creation order -> creation base
-    int E = 0;
-    const int U_count = alive - nsplit;
-    for (int b0 = 0; b0 < nsplit; b0 += blockDim.x) {
-        const int rk = b0 + threadIdx.x;
-        int c = 0;
-        if (rk < nsplit) {
-            const int4 q = m.cnt4[order[rk]];
-            c = (q.x > 0) + (q.y > 0) + (q.z > 0) + (q.w > 0);
+#pragma unroll 2
+    for (int k = dist_first(); k < K; k += DIST_T) {
+        const int i = m.at_key(k), n = at[i];
+        const uint32_t p = cand[i];
+        if (best[n] == rank(p, k)) kept[n] = p;
+    }
+}
+
+// Places of the nv sort keys in descending order -> m.order() (node | children
+// << 16).  m.place() is zero beforehand; a barrier at the end.
+template <bool SM>
+__device__ __forceinline__ void dist_order(const DistArrays<SM>& m, int nv, const int4* cnt) {
+    auto place = [&](int rank, unsigned long long key) {
+        const int n = (int)(0xFFFFFFFFu - (uint32_t)key);
+        const int4 q = cnt[n];
+        m.order()[rank] = (uint32_t)n | (uint32_t)((q.x > 0) + (q.y > 0) + (q.z > 0) + (q.w > 0)) << 16;
+    };
+    if (nv <= DIST_T) {
+        // each node's place as the sum of 'parts' threads' counts
+        int shift = 5;
+        while ((1 << shift) < nv) shift++;
+        const int parts = DIST_T >> shift, part = threadIdx.x >> shift, j = threadIdx.x & ((1 << shift) - 1);
+        const int chunk = (nv + parts - 1) / parts, lo = part * chunk, hi = min(nv, lo + chunk);
+        if (j < nv && lo < hi) {
+            const unsigned long long key = m.sort()[j];
+            int before = 0;
+#pragma unroll 8
+            for (int i = lo; i < hi; i++) before += m.sort()[i] > key;
+            atomicAdd(&m.place()[j], before);
         }
-        int tot;
-        const int ex = block_exclusive_scan(c, s_scan, &tot);
-        if (rk < nsplit) base[rk] = E + ex;
-        E += tot;
-    }
-    __syncthreads();
-    if (E + U_count > d.node_cap) {  // node arrays too small: report and stop
-        if (threadIdx.x == 0) s_vars[15] = 1;
         __syncthreads();
-        n_big = 0;
-        return;
+        if (threadIdx.x < nv) place(m.place()[threadIdx.x], m.sort()[threadIdx.x]);
+    } else {
+        int np2 = 1;
+        while (np2 < nv) np2 <<= 1;
+        for (int k = nv + threadIdx.x; k < np2; k += DIST_T) m.sort()[k] = 0ull;
+        __syncthreads();
+        for (int size = 2; size <= np2; size <<= 1)
+            for (int stride = size >> 1; stride > 0; stride >>= 1) {
+                for (int t = threadIdx.x; t < np2 / 2; t += DIST_T) {
+                    const int lo = 2 * t - (t & (stride - 1));
+                    const int hi = lo + stride;
+                    const bool desc = ((lo & size) == 0);
+                    const unsigned long long a = m.sort()[lo], b = m.sort()[hi];
+                    if ((a < b) == desc) {
+                        m.sort()[lo] = b;
+                        m.sort()[hi] = a;
+                    }
+                }
+                __syncthreads();
+            }
+        for (int j = threadIdx.x; j < nv; j += DIST_T) place(j, m.sort()[j]);
     }
-    // 3. unsplit nodes keep their order after the E children
-    int U = 0;
-    for (int b0 = 0; b0 < alive; b0 += blockDim.x) {
-        const int n = b0 + threadIdx.x;
-        const int u = (n < alive && split_rank[n] < 0) ? 1 : 0;
-        int tot;
-        const int ex = block_exclusive_scan(u, s_scan, &tot);
-        if (u) {
-            B[E + U + ex] = A[n];
-            m.childpos[n] = make_int4(E + U + ex, 0, 0, 0);
-        }
-        U += tot;
-    }
-    // 4. children
-    int big = 0;
-    for (int rk = threadIdx.x; rk < nsplit; rk += blockDim.x) {
-        const int n = order[rk];
-        const int4 q4 = m.cnt4[n];
-        const int cq[4] = {q4.x, q4.y, q4.z, q4.w};
-        int pos4[4] = {-1, -1, -1, -1};
-        int r = 0;
-        for (int q = 0; q < 4; q++) {
-            if (cq[q] == 0) continue;
-            const int e = base[rk] + r++;
-            const int pos = E - 1 - e;
-            DNode c = child_rect(A[n], q);
-            c.cnt = cq[q];
-            c.id = next_id + e;
-            c.flags = cq[q] == 1 ? 1 : 0;
-            B[pos] = c;
-            pos4[q] = pos;
-            big += cq[q] > 1;
-        }
-        m.childpos[n] = make_int4(pos4[0], pos4[1], pos4[2], pos4[3]);
-    }
-    __syncthreads();
-    // 5. keys follow their nodes
-    for (int k = threadIdx.x; k < K; k += blockDim.x) {
-        const int n = m.node_of[k];
-        const int4 cp = m.childpos[n];
-        if (split_rank[n] < 0) m.node_of[k] = cp.x;
-        else {
-            const int q = m.quad[k];
-            m.node_of[k] = q == 0 ? cp.x : (q == 1 ? cp.y : (q == 2 ? cp.z : cp.w));
-        }
-    }
-    // block sum of 'big'
-    int tot_big;
-    block_exclusive_scan(big, s_scan, &tot_big);
-    DNode* t = A;
-    A = B;
-    B = t;
-    next_id += E;
-    alive = E + U;
-    n_big = tot_big;
     __syncthreads();
 }
 
-__global__ void __launch_bounds__(512) k_distribute(const LevelDesc* descs, int* status, int sort_cap,
-                                                     int node_smem_cap, int key_smem_cap) {
-    const LevelDesc& d = descs[blockIdx.x];
-    __shared__ int s_scan[32];
-    __shared__ int s_vars[16];
-    __shared__ int s_root_cnt[64];
-    __shared__ int s_root_pos[64];
-    // dynamic: the final phase's sort keys (sort_cap), then node arrays for
-    // node_smem_cap nodes (if > 0), then key arrays for key_smem_cap keys
-    extern __shared__ __align__(16) unsigned long long s_sort[];
-    uint8_t* sp = reinterpret_cast<uint8_t*>(s_sort + sort_cap);
-    DistArrays m;
-    if (node_smem_cap >= d.node_cap) {
-        const size_t nc = (size_t)node_smem_cap;
-        m.a = reinterpret_cast<DNode*>(sp);
-        m.b = m.a + nc;
-        m.cnt4 = reinterpret_cast<int4*>(sp + dist_nodes_ab(nc));
-        m.childpos = m.cnt4 + nc;
-        m.aux0 = reinterpret_cast<int*>(m.childpos + nc);
-        m.aux1 = m.aux0 + nc;
-        m.aux2 = m.aux1 + nc;
-        m.best = reinterpret_cast<uint32_t*>(m.aux2 + nc);
-    } else {
-        m.a = (DNode*)d.nodes_a;
-        m.b = (DNode*)d.nodes_b;
-        m.cnt4 = d.cnt4;
-        m.childpos = d.childpos;
-        m.aux0 = d.aux0;
-        m.aux1 = d.aux1;
-        m.aux2 = d.aux2;
-        m.best = d.best;
+template <bool SM>
+__device__ __forceinline__ void distribute_level(const LevelDesc& d, const DistArrays<SM>& m, int K, int* status) {
+    __shared__ int4 s_part[2][DIST_T / 32];
+    __shared__ int s_children;
+    constexpr unsigned FULL = 0xffffffffu;
+    const int t = threadIdx.x, lane = t & 31, wid = t >> 5, N = d.nfeat, node_cap = d.node_cap;
+    const unsigned lt = (1u << lane) - 1, node_bits = 0xFu << (lane & ~3);
+    int half = 0, cur = 0;  // the list's buffers
+    int alive = d.nIni;     // nodes of the list, the empty initial nodes included
+    int nv = 0;             // ... that hold several keys
+    bool first = true, final_phase = false;
+    for (int guard = 0;; guard++) {
+        const int nx = cur ^ 1;
+        int* cnt = (int*)m.cnt(cur);
+        int E = 0;
+        if (final_phase) {
+            // split the largest nodes first, ties broken by later creation
+            // first, until N is reached (src/ORBextractor.cc:908-991)
+            for (int n = t; n < alive; n += DIST_T) m.created()[n] = -1;
+            if (t == 0) s_children = -1;
+            dist_order(m, nv, m.cnt(cur));
+            // a warp takes consecutive rows of 32 candidates; children - 1 is
+            // 0..3, summed by two ballots
+            const int per = (nv + DIST_T - 1) / DIST_T, r0 = wid * per;
+            int grown = 0;
+            for (int r = r0; r < r0 + per; r++) {
+                const int j = 32 * r + lane, g = j < nv ? (int)(m.order()[j] >> 16) - 1 : 0;
+                grown += __popc(__ballot_sync(FULL, g & 1)) + 2 * __popc(__ballot_sync(FULL, g & 2));
+            }
+            const DistSums S = dist_sums(make_int4(grown, 0, 0, 0), s_part, half);
+            int at = S.before.x;
+            for (int r = r0; r < r0 + per; r++) {
+                const int j = 32 * r + lane, a = j < nv ? (int)m.order()[j] : 1 << 16, g = (a >> 16) - 1;
+                const unsigned b0 = __ballot_sync(FULL, g & 1), b1 = __ballot_sync(FULL, g & 2);
+                const int ex = at + __popc(b0 & lt) + 2 * __popc(b1 & lt);
+                at += __popc(b0) + 2 * __popc(b1);
+                if (j < nv && alive + ex < N) {
+                    m.created()[a & 0xFFFF] = ex + j;
+                    if (alive + ex + g >= N) s_children = ex + g + j + 1;  // the last candidate to split
+                }
+            }
+            __syncthreads();
+            E = s_children < 0 ? S.total.x + nv : s_children;
+        }
+        // The nodes, four lanes (quadrants) each, a warp taking consecutive
+        // rows of eight nodes: which lanes hold a child, a child of several
+        // keys; which first lanes hold a node that is kept.
+        struct Row {
+            unsigned child, big, keep;
+            int n, keys, base;  // base: creation base in the final phase
+            bool split;
+        };
+        auto row_of = [&](int r) {
+            Row R;
+            R.n = 8 * r + (lane >> 2);
+            const bool in = R.n < alive;
+            R.keys = in ? cnt[4 * R.n + (lane & 3)] : 0;
+            const bool counted = in && m.mid(cur)[R.n] != 0;
+            const unsigned some = __ballot_sync(FULL, R.keys > 0) & node_bits;
+            const unsigned several = __ballot_sync(FULL, R.keys > 1);
+            R.base = final_phase && in ? m.created()[R.n] : -1;
+            R.split = final_phase ? R.base >= 0 : counted && ((several & node_bits) || __popc(some) > 1);
+            R.child = __ballot_sync(FULL, R.split && R.keys > 0);
+            R.big = __ballot_sync(FULL, R.split && R.keys > 1);
+            // one key; or the final phase ends with this step
+            R.keep = __ballot_sync(FULL, in && !R.split && (!counted || some) && (lane & 3) == 0);
+            return R;
+        };
+        const int per = ((alive + 7) / 8 + DIST_T / 32 - 1) / (DIST_T / 32), r0 = wid * per;
+        int4 sum = make_int4(0, 0, 0, 0);
+        for (int r = r0; r < r0 + per; r++) {
+            const Row R = row_of(r);
+            sum.x += __popc(R.child);
+            sum.y += __popc(R.keep);
+            sum.z += __popc(R.big);
+            // initial nodes that hold keys
+            sum.w += __popc(R.keep | (__ballot_sync(FULL, R.split) & 0x11111111u));
+        }
+        const DistSums S = dist_sums(sum, s_part, half);
+        if (!final_phase) E = S.total.x;
+        const int kept = S.total.y;
+        if (E + kept > node_cap) {  // node arrays too small: report and stop
+            if (t == 0) {
+                atomicOr(status, 32);
+                *d.kept_count = 0;
+            }
+            return;
+        }
+        int child = S.before.x, keep = S.before.y, big = S.before.z;
+        for (int r = r0; r < r0 + per; r++) {
+            const Row R = row_of(r);
+            int p;
+            bool place;
+            uint32_t mid = 0;
+            if (R.split) {
+                const int created = final_phase ? R.base + __popc(R.child & node_bits & lt) : child + __popc(R.child & lt);
+                p = E - 1 - created;
+                place = R.keys > 0;
+                if (R.keys > 1) {
+                    const int2 rc = m.rect(cur)[R.n], xy = dist_mid(rc);
+                    int2 c;
+                    c.x = (lane & 1) ? (xy.x & 0xFFFF) | (rc.x & 0xFFFF0000) : (rc.x & 0xFFFF) | xy.x << 16;
+                    c.y = (lane & 2) ? (xy.y & 0xFFFF) | (rc.y & 0xFFFF0000) : (rc.y & 0xFFFF) | xy.y << 16;
+                    m.rect(nx)[p] = c;
+                    mid = dist_mid_word(dist_mid(c));
+                    m.sort()[big + __popc(R.big & lt)] = (unsigned long long)R.keys << 32 | (0xFFFFFFFFu - (uint32_t)p);
+                }
+            } else {
+                p = E + keep + __popc(R.keep & ((1u << (lane & ~3)) - 1));
+                place = R.keep >> lane & 1;
+            }
+            if (place) {
+                m.mid(nx)[p] = mid;
+                m.cnt(nx)[p] = make_int4(0, 0, 0, 0);
+                m.place()[p] = 0;
+            }
+            if (R.n < alive) cnt[4 * R.n + (lane & 3)] = p;
+            child += __popc(R.child);
+            keep += __popc(R.keep);
+            big += __popc(R.big);
+        }
+        const int prev = first ? S.total.w : alive;
+        alive = E + kept;
+        nv = S.total.z;
+        __syncthreads();
+        // full passes: src/ORBextractor.cc:759-904
+        bool done = alive >= N || alive == prev;
+        if (final_phase) done = done || nv == 0;
+        else if (!done) final_phase = alive + nv * 3 > N;
+        if (guard == 127 && !done) {
+            if (t == 0) atomicOr(status, 8);
+            done = true;
+        }
+        first = false;
+        if (done) {
+            dist_best(m, cur, K, d.kept);
+            if (t == 0) *d.kept_count = alive;
+            return;
+        }
+        dist_count(m, cur, K);
+        __syncthreads();
+        cur = nx;
     }
-    sp += dist_node_bytes((size_t)node_smem_cap);
-    const int ncells = d.nCols * d.nRows;
+}
+
+template <bool SM>
+__device__ __forceinline__ void distribute(const LevelDesc& d, const DistArrays<SM>& m, int K, int first_slot, int* status) {
+    __shared__ int s_root[64];
+    const int nIni = d.nIni, ncells = d.nCols * d.nRows, cell_cap = d.cell_cap;
+    const int Wd = d.maxBorderX - (ORBGPU_EDGE_THRESHOLD - 3), Hd = d.maxBorderY - (ORBGPU_EDGE_THRESHOLD - 3);
+    const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
+    const uint32_t* slots = d.slots;
+    const int* cell_count = d.cell_count;
     // 1. candidates in the reference's emission order: cell rows, cell
-    //    columns, then the detector's row-major order inside each cell (the
-    //    count first: it decides where the key arrays live)
-    int K = 0;
-    for (int b0 = 0; b0 < ncells; b0 += blockDim.x) {
-        const int c = b0 + threadIdx.x;
-        int tot;
-        block_exclusive_scan(c < ncells ? d.cell_count[c] : 0, s_scan, &tot);
-        K += tot;
+    //    columns, then the detector's row-major order inside each cell.  A
+    //    warp notes the slot of every key of its rows of 32 cells, so that
+    //    each key is one load.
+    const int per = (ncells + DIST_T - 1) / DIST_T, r0 = wid * per;
+    int* at = m.at();
+    for (int r = r0; r < r0 + per; r++) {
+        const int c = 32 * r + lane, n = c < ncells ? __ldg(cell_count + c) : 0;
+        int x = n;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        for (int k = 0; k < n; k++) at[m.at_key(first_slot + x - n + k)] = c * cell_cap + k;
+        first_slot += __shfl_sync(0xffffffffu, x, 31);
     }
-    if (K <= key_smem_cap) {
-        m.cand = reinterpret_cast<uint32_t*>(sp);
-        m.node_of = reinterpret_cast<int*>(m.cand + key_smem_cap);
-        m.quad = reinterpret_cast<uint8_t*>(m.node_of + key_smem_cap);
-    } else {
-        m.cand = d.cand;
-        m.node_of = d.node_of;
-        m.quad = d.quad;
-    }
-    K = 0;
-    for (int b0 = 0; b0 < ncells; b0 += blockDim.x) {
-        const int c = b0 + threadIdx.x;
-        const int cnt = c < ncells ? d.cell_count[c] : 0;
-        int tot;
-        const int ex = block_exclusive_scan(cnt, s_scan, &tot);
-        for (int k = 0; k < cnt; k++) m.cand[K + ex + k] = d.slots[(size_t)c * d.cell_cap + k];
-        K += tot;
+    // 2. the initial nodes; s_root[r]: the first column of node r by the
+    //    reference's rounded division (src/ORBextractor.cc:722)
+    const int minB = ORBGPU_EDGE_THRESHOLD - 3;
+    const float hX = __fdiv_rn((float)Wd, (float)nIni);
+    for (int r = t; r < nIni; r += DIST_T) {
+        const int2 rc = {((int)__fmul_rn(hX, (float)r) & 0xFFFF) | (int)__fmul_rn(hX, (float)(r + 1)) << 16, Hd << 16};
+        m.rect(0)[r] = rc;
+        m.mid(0)[r] = dist_mid_word(dist_mid(rc));
+        m.cnt(0)[r] = make_int4(0, 0, 0, 0);
+        int x = max((int)__fmul_rn(hX, (float)r) - 1, 0);  // the quotient is monotone in the column
+        while ((int)__fdiv_rn((float)x, hX) < r) x++;
+        s_root[r] = x + minB;
     }
     __syncthreads();
+    uint32_t* cand = m.cand();
+    for (int k0 = t; k0 < K; k0 += 4 * DIST_T) {
+        uint32_t p[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) p[i] = k0 + i * DIST_T < K ? __ldg(slots + at[m.at_key(k0 + i * DIST_T)]) : 0;
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+            if (k0 + i * DIST_T < K) cand[m.at_key(k0 + i * DIST_T)] = p[i];
+    }
+    __syncthreads();
+    // every key counts in one of a few places: the warp's sums first, a byte
+    // per quadrant
+    for (int k0 = dist_first() - lane * (DIST_T / 32); k0 < K; k0 += 4 * DIST_T) {
+        int a[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int k = k0 + lane * (DIST_T / 32) + i * DIST_T;
+            a[i] = -1;
+            if (k >= K) continue;
+            const uint32_t p = cand[m.at_key(k)];
+            int r = 0;
+            while (r + 1 < nIni && (int)(p & 0xFFF) >= s_root[r + 1]) r++;
+            at[m.at_key(k)] = a[i] = 4 * r + dist_quadrant(p, m.mid(0)[r]);
+        }
+        for (int r = 0; r < nIni; r++) {
+            unsigned w = 0;
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+                if (a[i] >> 2 == r) w += 1u << (8 * (a[i] & 3));
+            w = __reduce_add_sync(0xffffffffu, w);
+            if (lane < 4) atomicAdd((int*)m.cnt(0) + 4 * r + lane, (int)(w >> (8 * lane) & 255u));
+        }
+    }
+    __syncthreads();
+    distribute_level(d, m, K, status);
+}
+
+// descs: frame-major; the blocks take the levels in order, so that the long
+// first levels of a batch do not start last.
+__global__ void __launch_bounds__(DIST_T, 3) k_distribute(const LevelDesc* descs, int nframes, int nlevels, int* status,
+                                                           int sort_cap, int node_smem_cap, int key_smem_cap) {
+    const LevelDesc& d = descs[(blockIdx.x % nframes) * nlevels + blockIdx.x / nframes];
+    __shared__ int4 s_part[2][DIST_T / 32];
+    const int ncells = d.nCols * d.nRows, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int* cell_count = d.cell_count;
+    const int per = (ncells + DIST_T - 1) / DIST_T, r0 = wid * per;
+    int sum = 0;
+#pragma unroll 4
+    for (int r = r0; r < r0 + per; r++) sum += 32 * r + lane < ncells ? __ldg(cell_count + 32 * r + lane) : 0;
+    sum = __reduce_add_sync(0xffffffffu, sum);
+    int half = 0;
+    const DistSums S = dist_sums(make_int4(sum, 0, 0, 0), s_part, half);
+    const int K = S.total.x;
     if (K == 0 || d.nIni <= 0) {
         if (threadIdx.x == 0) *d.kept_count = 0;
         return;
     }
-    DNode* A = m.a;
-    DNode* B = m.b;
-    const int minB = ORBGPU_EDGE_THRESHOLD - 3;
-    const int Wd = d.maxBorderX - minB, Hd = d.maxBorderY - minB;
-    const int nIni = d.nIni;
-    const float hX = __fdiv_rn((float)Wd, (float)nIni);
-    // 2. initial nodes
-    if (threadIdx.x < 64) s_root_cnt[threadIdx.x] = 0;
-    __syncthreads();
-    for (int k = threadIdx.x; k < K; k += blockDim.x) {
-        const float x = (float)((int)(m.cand[k] & 0xFFF) - minB);
-        int r = (int)__fdiv_rn(x, hX);
-        if (r >= nIni) { atomicOr(status, 4); r = nIni - 1; }
-        m.node_of[k] = r;
-        atomicAdd(&s_root_cnt[r], 1);
+    const int nodes_off = sort_cap * (int)sizeof(unsigned long long);
+    const int cand_off = nodes_off + (int)dist_node_bytes(node_smem_cap), at_off = cand_off + 4 * (key_smem_cap + (key_smem_cap >> 4));
+    uint8_t* const base = (uint8_t*)s_dist;
+    const bool nodes_fit = node_smem_cap >= d.node_cap, keys_fit = K <= key_smem_cap;
+    if (nodes_fit && keys_fit) {
+        distribute(d, DistArrays<true>{nullptr, nullptr, nullptr, nullptr, nodes_off, cand_off, at_off, node_smem_cap}, K, S.before.x,
+                   status);
+    } else {
+        distribute(d, DistArrays<false>{sort_cap > 0 ? base : (uint8_t*)d.sort, nodes_fit ? base + nodes_off : d.nodes, keys_fit ? base + cand_off : (uint8_t*)d.cand,
+                                        keys_fit ? base + at_off : (uint8_t*)d.node_of, 0, 0, 0, nodes_fit ? node_smem_cap : d.node_cap},
+                   K, S.before.x, status);
     }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int a = 0;
-        for (int r = 0; r < nIni; r++) {
-            s_root_pos[r] = -1;
-            if (s_root_cnt[r] == 0) continue;
-            DNode n;
-            n.x0 = (int16_t)(int)__fmul_rn(hX, (float)r);
-            n.x1 = (int16_t)(int)__fmul_rn(hX, (float)(r + 1));
-            n.y0 = 0;
-            n.y1 = (int16_t)Hd;
-            n.cnt = s_root_cnt[r];
-            n.id = r;
-            n.flags = 2 | (s_root_cnt[r] == 1 ? 1 : 0);
-            A[a] = n;
-            s_root_pos[r] = a++;
-        }
-        s_vars[0] = a;
-    }
-    __syncthreads();
-    for (int k = threadIdx.x; k < K; k += blockDim.x) m.node_of[k] = s_root_pos[m.node_of[k]];
-    if (threadIdx.x == 0) s_vars[15] = 0;
-    int alive = s_vars[0];
-    int next_id = nIni;
-    const int N = d.nfeat;
-    __syncthreads();
-    // 3. full passes (src/ORBextractor.cc:759-904)
-    bool final_phase = false;
-    for (int guard = 0; guard < 64; guard++) {
-        const int prev = alive;
-        // every node without bNoMore splits, in list order
-        int nsplit = 0;
-        for (int b0 = 0; b0 < alive; b0 += blockDim.x) {
-            const int n = b0 + threadIdx.x;
-            const int s = (n < alive && !(A[n].flags & 1)) ? 1 : 0;
-            int tot;
-            const int ex = block_exclusive_scan(s, s_scan, &tot);
-            if (n < alive) {
-                m.aux0[n] = s ? nsplit + ex : -1;
-                if (s) m.aux1[nsplit + ex] = n;
-            }
-            nsplit += tot;
-        }
-        __syncthreads();
-        int n_big = 0;
-        split_step(d, m, A, B, alive, K, nsplit, next_id, n_big, s_scan, s_vars);
-        if (s_vars[15]) break;
-        if (alive >= N || alive == prev) break;
-        if (alive + n_big * 3 > N) { final_phase = true; break; }
-        if (guard == 63) atomicOr(status, 8);
-    }
-    // 4. final phase (src/ORBextractor.cc:908-991): split the largest nodes
-    //    first, ties broken by later creation first, until N is reached.
-    if (final_phase) {
-        for (int guard = 0; guard < 64; guard++) {
-            const int prev = alive;
-            // nodes with more than one key (all created by the last step)
-            int nv = 0;
-            for (int b0 = 0; b0 < alive; b0 += blockDim.x) {
-                const int n = b0 + threadIdx.x;
-                const int s = (n < alive && A[n].cnt > 1) ? 1 : 0;
-                int tot;
-                const int ex = block_exclusive_scan(s, s_scan, &tot);
-                if (s) s_sort[nv + ex] = ((unsigned long long)A[n].cnt << 40) | ((unsigned long long)A[n].id << 16) | (unsigned long long)n;
-                nv += tot;
-            }
-            __syncthreads();
-            if (nv == 0) break;
-            int np2 = 1;
-            while (np2 < nv) np2 <<= 1;
-            for (int k = nv + threadIdx.x; k < np2; k += blockDim.x) s_sort[k] = 0ull;
-            __syncthreads();
-            // bitonic sort, descending
-            for (int size = 2; size <= np2; size <<= 1)
-                for (int stride = size >> 1; stride > 0; stride >>= 1) {
-                    for (int t = threadIdx.x; t < np2 / 2; t += blockDim.x) {
-                        const int lo = 2 * t - (t & (stride - 1));
-                        const int hi = lo + stride;
-                        const bool desc = ((lo & size) == 0);
-                        const unsigned long long a = s_sort[lo], b = s_sort[hi];
-                        if ((a < b) == desc) {
-                            s_sort[lo] = b;
-                            s_sort[hi] = a;
-                        }
-                    }
-                    __syncthreads();
-                }
-            // children count of each candidate node -> how many to split
-            for (int n = threadIdx.x; n < alive; n += blockDim.x) m.cnt4[n] = make_int4(0, 0, 0, 0);
-            for (int n = threadIdx.x; n < alive; n += blockDim.x) m.aux0[n] = -1;
-            __syncthreads();
-            for (int j = threadIdx.x; j < nv; j += blockDim.x) m.aux0[(int)(s_sort[j] & 0xFFFF)] = j;
-            __syncthreads();
-            for (int k = threadIdx.x; k < K; k += blockDim.x) {
-                const int n = m.node_of[k];
-                if (m.aux0[n] < 0) continue;
-                const int q = quadrant_of(m.cand[k], A[n]);
-                atomicAdd(&((int*)&m.cnt4[n])[q], 1);
-            }
-            __syncthreads();
-            // prefix of (children - 1) in processing order; first j reaching N
-            int acc = 0;
-            int J = nv - 1;
-            if (threadIdx.x == 0) s_vars[1] = nv - 1;
-            __syncthreads();
-            for (int b0 = 0; b0 < nv; b0 += blockDim.x) {
-                const int j = b0 + threadIdx.x;
-                int g = 0;
-                if (j < nv) {
-                    const int4 q = m.cnt4[(int)(s_sort[j] & 0xFFFF)];
-                    g = (q.x > 0) + (q.y > 0) + (q.z > 0) + (q.w > 0) - 1;
-                }
-                int tot;
-                const int ex = block_exclusive_scan(g, s_scan, &tot);
-                if (j < nv && alive + acc + ex + g >= N) atomicMin(&s_vars[1], j);
-                acc += tot;
-            }
-            __syncthreads();
-            J = s_vars[1];
-            const int nsplit = J + 1;
-            for (int n = threadIdx.x; n < alive; n += blockDim.x) m.aux0[n] = -1;
-            __syncthreads();
-            for (int j = threadIdx.x; j < nsplit; j += blockDim.x) {
-                const int n = (int)(s_sort[j] & 0xFFFF);
-                m.aux0[n] = j;
-                m.aux1[j] = n;
-            }
-            __syncthreads();
-            int n_big = 0;
-            split_step(d, m, A, B, alive, K, nsplit, next_id, n_big, s_scan, s_vars);
-            if (s_vars[15]) break;
-            if (alive >= N || alive == prev) break;
-            if (guard == 63) atomicOr(status, 8);
-        }
-    }
-    if (s_vars[15]) {
-        if (threadIdx.x == 0) {
-            atomicOr(status, 32);
-            *d.kept_count = 0;
-        }
-        return;
-    }
-    // 5. per node the key with the largest response, first in key order
-    for (int n = threadIdx.x; n < alive; n += blockDim.x) m.best[n] = 0u;
-    __syncthreads();
-    for (int k = threadIdx.x; k < K; k += blockDim.x) {
-        const uint32_t p = m.cand[k];
-        const uint32_t key = ((p >> 24) << 20) | (uint32_t)(0xFFFFF - k);
-        atomicMax(&m.best[m.node_of[k]], key);
-    }
-    __syncthreads();
-    for (int n = threadIdx.x; n < alive; n += blockDim.x) {
-        const int k = 0xFFFFF - (int)(m.best[n] & 0xFFFFF);
-        d.kept[n] = m.cand[k];
-    }
-    if (threadIdx.x == 0) *d.kept_count = alive;
 }
 
 // ---------------------------------------------------------------- describe
@@ -1773,23 +1820,28 @@ void launch_fast(const LevelDesc* descs, RangeMap rm, int ncells, int* status, i
         default: run(k_fast_cells<4>); break;
     }
 }
-void launch_distribute(const LevelDesc* descs, int ndescs, int sort_cap, int node_cap, int* status,
-                       cudaStream_t st) {
+void launch_distribute(const LevelDesc* descs, int nframes, int nlevels, int node_cap, int* status, cudaStream_t st) {
     // a 72 KiB budget per block (three 512-thread blocks per SM): the sort
-    // keys, the node arrays of the launch's largest level if they fit, and
-    // the keys of as many candidates as the rest holds (a level with more
+    // keys, the node arrays of the launch's largest level, as far as they fit,
+    // and the keys of as many candidates as the rest holds (a level with more
     // keeps them in global memory)
-    const size_t budget = 72 * 1024, sort_b = (size_t)sort_cap * sizeof(unsigned long long);
-    size_t node_b = dist_node_bytes((size_t)node_cap);
+    const size_t budget = 72 * 1024;
+    int sort_cap = (int)dist_sort_cap(node_cap);
+    size_t sort_b = (size_t)sort_cap * sizeof(unsigned long long), node_b = dist_node_bytes((size_t)node_cap);
     int node_smem_cap = node_cap;
     if (sort_b + node_b + 16 * 1024 > budget) {
         node_b = 0;
         node_smem_cap = 0;
     }
-    const int key_smem_cap = (int)(((budget > sort_b + node_b ? budget - sort_b - node_b : 0) / DIST_KEY_BYTES) & ~15);
-    const size_t smem = std::max(budget, sort_b);
+    if (sort_b > budget) {
+        sort_b = 0;
+        sort_cap = 0;
+    }
+    const int key_smem_cap = (int)((budget - sort_b - node_b) / (2 * sizeof(int)) * 16 / 17 & ~(size_t)15);
     allow_max_dynamic_smem(k_distribute);
-    if (ndescs > 0) k_distribute<<<ndescs, 512, smem, st>>>(descs, status, sort_cap, node_smem_cap, key_smem_cap);
+    if (nframes > 0)
+        k_distribute<<<nframes * nlevels, DIST_T, budget, st>>>(descs, nframes, nlevels, status, sort_cap, node_smem_cap,
+                                                                key_smem_cap);
 }
 void launch_describe(const LevelDesc* descs, int ndescs, long features, orbgpu_keypoint* kps, uint8_t* desc, int* status,
                      cudaStream_t st) {

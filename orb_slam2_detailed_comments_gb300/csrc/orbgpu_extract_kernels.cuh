@@ -83,15 +83,8 @@ struct LevelDesc {
     int node_cap;
     uint32_t* cand;   // cand_cap
     int* node_of;     // cand_cap
-    uint8_t* quad;    // cand_cap
-    void* nodes_a;    // node_cap DNode
-    void* nodes_b;    // node_cap DNode
-    int4* cnt4;       // node_cap
-    int4* childpos;   // node_cap
-    int* aux0;        // node_cap (split rank / order)
-    int* aux1;        // node_cap
-    int* aux2;        // node_cap
-    uint32_t* best;   // node_cap
+    uint8_t* nodes;   // DistributeOctTree's node arrays, dist_node_bytes(node_cap)
+    unsigned long long* sort;  // its sort keys, dist_sort_cap(node_cap)
     uint32_t* kept;   // node_cap: distributed keypoints, packed like slots
     int* kept_count;  // one int
     // describe
@@ -134,13 +127,6 @@ struct Tunables {
 };
 const Tunables& tunables();
 int tune_generation();
-
-struct DNode {
-    int16_t x0, x1, y0, y1;
-    int32_t cnt;
-    int32_t id;
-    int32_t flags;  // 1 = bNoMore, 2 = initial node
-};
 
 // One tile of k_level_resize_blur / one cell of k_fast_cells.
 struct WorkItem {
@@ -210,10 +196,15 @@ bool plan_pyramid(int rows, int nframes, int nlevels, const std::vector<int>& w,
 void launch_pyramid(const LevelDesc* descs, const PyramidPlan& P, const int* prefix, int nframes, int nlevels, int* ticket,
                     int* status, cudaStream_t st);
 int strip_rows(long level0_pixels);
+__host__ __device__ inline size_t dist_node_bytes(size_t nc) { return 68 * nc; }  // nc nodes, 16-byte aligned
+inline size_t dist_sort_cap(size_t nc) {
+    size_t n = 1;
+    while (n < nc) n <<= 1;
+    return n;
+}
 // DistributeOctTree of every (frame, level); node_cap: the largest level's
-// node capacity (its arrays go to shared memory when they fit).
-void launch_distribute(const LevelDesc* descs, int ndescs, int sort_cap, int node_cap, int* status,
-                       cudaStream_t st);
+// node capacity (its arrays and the sort keys go to shared memory when they fit).
+void launch_distribute(const LevelDesc* descs, int nframes, int nlevels, int node_cap, int* status, cudaStream_t st);
 // features: about how many keypoints the launch describes (the levels' budgets).
 void launch_describe(const LevelDesc* descs, int ndescs, long features, orbgpu_keypoint* kps, uint8_t* desc, int* status,
                      cudaStream_t st);

@@ -33,8 +33,8 @@ struct LevelGeom {
 };
 
 struct LevelOffsets {
-    size_t pyr, blur, xofs, xalpha, yofs, ybeta, cbits, slots, cell_count, cand, node_of, quad, nodes_a,
-        nodes_b, cnt4, childpos, aux0, aux1, aux2, best, kept;
+    size_t pyr, blur, xofs, xalpha, yofs, ybeta, cbits, slots, cell_count, cand, node_of, nodes, sort,
+        kept;
 };
 
 // Byte offsets of one frame's buffers inside a device arena.

@@ -297,3 +297,24 @@ def test_pyramid_launches(torch, oracle, w, h, scale, nlevels):
         check()
     finally:
         autotune.apply({k: v for k, v in before.items() if k != "knn_tc_min_pairs"})
+
+
+# DistributeOctTree: one key, lists of a few and of thousands of nodes (counted
+# and sorted places in the final phase, node and key arrays in shared and in
+# global memory), one and many initial nodes, more cells than threads.
+@pytest.mark.parametrize("w,h,nf,nlevels,noise", [(640, 480, 1, 8, 0), (640, 480, 12, 1, 0), (1280, 720, 2600, 1, 0),
+                                                  (1280, 720, 9000, 3, 1), (1600, 120, 700, 2, 1), (300, 260, 400, 2, 1),
+                                                  (2000, 1100, 3000, 4, 1), (640, 480, 20000, 1, 1)])
+def test_distribute_limits(torch, oracle, w, h, nf, nlevels, noise):
+    from orb_slam2_detailed_comments_gb300 import ORBextractor
+    from orb_slam2_detailed_comments_gb300 import synthetic as syn
+    img = syn.scene(w, h, 70)
+    if noise:
+        rng = np.random.default_rng(71)
+        img = rng.integers(0, 256, (h, w), dtype=np.uint8)
+        img[:, : w // 3] = syn.scene(w, h, 72)[:, : w // 3]
+    ex = ORBextractor(nf, 1.2, nlevels, 20, 7)
+    kps, desc = ex(img)
+    ref = oracle.extract(img, nfeatures=nf, nlevels=nlevels, want_pyramid=False)
+    assert_kps_equal(kps, ref.keypoints, f"{w}x{h} {nf}")
+    assert np.array_equal(desc, ref.descriptors)
