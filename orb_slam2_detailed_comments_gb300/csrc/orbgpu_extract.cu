@@ -538,13 +538,13 @@ struct SizePlan {
     // small images: all resizes and strips in one launch (k_pyramid)
     bool fused = false;
     PyramidPlan pyramid;
-    // the call's status (4 ints), k_pyramid's ticket (at 4) and the levels'
-    // counters (from 8): cleared before every call
-    int* d_sync = nullptr;
+    // the call's status (at 0), keypoint total (1), k_pyramid's ticket (4) and
+    // the levels' counters (from 8): cleared before every call
     size_t sync_bytes = 0;
     std::vector<int> done_off;
     int max_kept = 0;
     long features = 0;  // the budgets of all levels with cells
+    int max_total = 0;  // keypoints at most
     uint64_t last_use = 0;
     int gen = -1;  // tuning generation of the work lists
 };
@@ -566,19 +566,21 @@ struct orbgpu_extractor {
     uint64_t use_clock = 0;
     // current geometry (mirrors cur)
     int cur_w = -1, cur_h = -1;
-    LevelDesc* d_descs = nullptr;
-    // output staging
-    orbgpu_keypoint* d_kps = nullptr;
-    uint8_t* d_desc = nullptr;
-    int out_cap = 0;
-    int* h_pinned = nullptr;  // status + counts
+    // The call's small data, in one block on each side, so that a call is one
+    // copy up, one down and one synchronisation besides the image: the level
+    // descriptors, then (from IO_SYNC) the plan's sync words, then the outputs
+    // for the host.  Page-locked: what is copied up (the sync words stay zero),
+    // then what was copied down (from h_down), then the image (h_image).
+    uint8_t *d_io = nullptr, *h_io = nullptr, *h_down = nullptr, *h_image = nullptr;
+    size_t sync_cap = 0, out_cap = 0, image_cap = 0;  // bytes
 };
+static constexpr size_t IO_SYNC = (sizeof(LevelDesc) * ORBGPU_MAX_LEVELS + 255) & ~(size_t)255;
+static size_t align256(size_t n) { return (n + 255) & ~(size_t)255; }
 
 static void free_plan(SizePlan* p) {
     if (!p) return;
     cudaFree(p->arena);
     cudaFree(p->d_items);
-    cudaFree(p->d_sync);
     delete p;
 }
 
@@ -653,15 +655,18 @@ static int build_plan(orbgpu_extractor* ex, int w, int h, SizePlan** out) {
         sync_ints += (L.h + PYRAMID_BAND - 1) / PYRAMID_BAND;
     }
     P->fused = plan_pyramid(P->rows, 1, (int)g.size(), lw, lh, P->pyramid);
-    P->sync_bytes = sizeof(int) * sync_ints;
-    if (dev_malloc(&P->d_sync, P->sync_bytes) != cudaSuccess || dev_malloc(&P->d_items, pre.size() * sizeof(int)) != cudaSuccess ||
+    P->sync_bytes = sizeof(int) * (P->fused ? sync_ints : 8);
+    if (dev_malloc(&P->d_items, pre.size() * sizeof(int)) != cudaSuccess ||
         cudaMemcpy(P->d_items, pre.data(), pre.size() * sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess) {
         free_plan(P);
         return ORBGPU_ERR_OOM;
     }
     P->max_kept = 0;
     for (auto& L : g) {
-        if (L.ncells > 0) P->features += L.nfeat + 1;
+        if (L.ncells > 0) {
+            P->features += L.nfeat + 1;
+            P->max_total += L.node_cap;
+        }
         P->max_kept = std::max(P->max_kept, L.node_cap);
     }
     P->w = w;
@@ -708,15 +713,55 @@ static int setup_geometry(orbgpu_extractor* ex, int w, int h) {
     return ORBGPU_OK;
 }
 
-static int ensure_out(orbgpu_extractor* ex, int cap) {
-    if (cap <= ex->out_cap) return ORBGPU_OK;
-    if (ex->d_kps) cudaFree(ex->d_kps);
-    if (ex->d_desc) cudaFree(ex->d_desc);
-    ex->d_kps = nullptr;
-    ex->d_desc = nullptr;
-    ORBGPU_CUDA_TRY(cudaMalloc(&ex->d_kps, sizeof(orbgpu_keypoint) * (size_t)cap));
-    ORBGPU_CUDA_TRY(cudaMalloc(&ex->d_desc, 32 * (size_t)cap));
-    ex->out_cap = cap;
+static size_t host_out_bytes(int n) { return align256(sizeof(orbgpu_keypoint) * n) + 32 * (size_t)n; }
+// Grows the call's blocks to a plan's sync words, 'out' bytes of outputs and
+// an image of 'image' bytes.  No call is in flight.
+static int ensure_io(orbgpu_extractor* ex, size_t sync, size_t out, size_t image) {
+    if (sync <= ex->sync_cap && out <= ex->out_cap && image <= ex->image_cap) return ORBGPU_OK;
+    sync = std::max(align256(sync), ex->sync_cap);
+    out = std::max(align256(out), ex->out_cap);
+    image = std::max(align256(image), ex->image_cap);
+    cudaFree(ex->d_io);
+    cudaFreeHost(ex->h_io);
+    ex->d_io = ex->h_io = nullptr;
+    ex->sync_cap = ex->out_cap = ex->image_cap = 0;
+    ORBGPU_CUDA_TRY(dev_malloc(&ex->d_io, IO_SYNC + sync + out));
+    ORBGPU_CUDA_TRY(cudaMallocHost(&ex->h_io, IO_SYNC + sync + (sync + out) + image));
+    std::memset(ex->h_io, 0, IO_SYNC + sync);
+    ex->h_down = ex->h_io + IO_SYNC + sync;
+    ex->h_image = ex->h_down + sync + out;
+    ex->sync_cap = sync;
+    ex->out_cap = out;
+    ex->image_cap = image;
+    return ORBGPU_OK;
+}
+// Level 0 from the caller's image.  A pageable image goes through page-locked
+// memory in the plane's row pitch, one chunk copied on while the next is
+// staged: the runtime's own copy of a pageable 640x480 image holds the caller
+// for 31 us, the staging 10.
+static int upload_image(orbgpu_extractor* ex, uint8_t* dst, size_t pitch, const uint8_t* image, size_t step, int width,
+                        int height, int image_mem, cudaStream_t st) {
+    bool stage = false;
+    if (image_mem != ORBGPU_MEM_DEVICE) {
+        cudaPointerAttributes at;
+        if (cudaPointerGetAttributes(&at, image) == cudaSuccess) stage = at.type == cudaMemoryTypeUnregistered;
+        else cudaGetLastError();
+    }
+    if (!stage) {
+        ORBGPU_CUDA_TRY(cudaMemcpy2DAsync(dst, pitch, image, step, width, height,
+                                          image_mem == ORBGPU_MEM_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, st));
+        return ORBGPU_OK;
+    }
+    const int chunk = std::max(1, (int)((256 << 10) / pitch));
+    for (int y0 = 0; y0 < height; y0 += chunk) {
+        const int y1 = std::min(height, y0 + chunk);
+        uint8_t* h = ex->h_image + (size_t)y0 * pitch;
+        if (step == pitch && (size_t)width == pitch) std::memcpy(h, image + (size_t)y0 * step, (size_t)(y1 - y0) * pitch);
+        else
+            for (int y = y0; y < y1; y++) std::memcpy(ex->h_image + (size_t)y * pitch, image + (size_t)y * step, width);
+        ORBGPU_CUDA_TRY(cudaMemcpyAsync(dst + (size_t)y0 * pitch, h, (size_t)(y1 - y0 - 1) * pitch + width,
+                                        cudaMemcpyHostToDevice, st));
+    }
     return ORBGPU_OK;
 }
 
@@ -760,13 +805,6 @@ extern "C" int orbgpu_extractor_create(int nfeatures, float scale_factor, int nl
         orbgpu_extractor_destroy(ex);
         return ORBGPU_ERR_CUDA;
     }
-    cudaError_t e1 = cudaMalloc(&ex->d_descs, sizeof(LevelDesc) * ORBGPU_MAX_LEVELS);
-    cudaError_t e3 = cudaMallocHost(&ex->h_pinned, sizeof(int) * 32);
-    if (e1 != cudaSuccess || e3 != cudaSuccess) {
-        orbgpu_set_last_error("device allocation failed", __FILE__, __LINE__);
-        orbgpu_extractor_destroy(ex);
-        return ORBGPU_ERR_OOM;
-    }
     rc = ensure_constants();
     if (rc != ORBGPU_OK) {
         orbgpu_extractor_destroy(ex);
@@ -774,6 +812,9 @@ extern "C" int orbgpu_extractor_create(int nfeatures, float scale_factor, int nl
     }
     if (max_width > 0 && max_height > 0) {
         rc = setup_geometry(ex, max_width, max_height);
+        if (rc == ORBGPU_OK)
+            rc = ensure_io(ex, ex->cur->sync_bytes, host_out_bytes(ex->cur->max_total),
+                           ex->cur->geom[0].pitch * (size_t)max_height);
         if (rc != ORBGPU_OK) {
             orbgpu_extractor_destroy(ex);
             return rc;
@@ -793,10 +834,8 @@ extern "C" int orbgpu_extractor_destroy(orbgpu_extractor* ex) {
     if (ex->side) cudaStreamDestroy(ex->side);
     for (SizePlan* p : ex->plans) free_plan(p);
     ex->plans.clear();
-    cudaFree(ex->d_descs);
-    cudaFree(ex->d_kps);
-    cudaFree(ex->d_desc);
-    cudaFreeHost(ex->h_pinned);
+    cudaFree(ex->d_io);
+    cudaFreeHost(ex->h_io);
     if (ex->own_stream) cudaStreamDestroy(ex->stream);
     delete ex;
     return ORBGPU_OK;
@@ -823,45 +862,43 @@ extern "C" int orbgpu_extract(orbgpu_extractor* ex, const uint8_t* image, int wi
     const SizePlan& P = *ex->cur;
     const std::vector<LevelGeom>& g = P.geom;
     const int nl = (int)g.size();
-    // descriptors of this call (outputs go to the caller's device arrays or
-    // to the staging buffers)
-    orbgpu_keypoint* okps;
-    uint8_t* odesc;
-    if (out_mem == ORBGPU_MEM_DEVICE) {
-        okps = keypoints;
-        odesc = descriptors;
-    } else {
-        rc = ensure_out(ex, std::max(capacity, 1));
-        if (rc != ORBGPU_OK) return rc;
-        okps = ex->d_kps;
-        odesc = ex->d_desc;
-    }
-    LevelDesc hd[ORBGPU_MAX_LEVELS];
+    // outputs go to the caller's device arrays or through the call's block
+    const bool to_host = out_mem != ORBGPU_MEM_DEVICE;
+    const int staged = to_host ? std::min(capacity, P.max_total) : 0;
+    rc = ensure_io(ex, P.sync_bytes, host_out_bytes(staged), image_mem != ORBGPU_MEM_DEVICE ? g[0].pitch * (size_t)height : 0);
+    if (rc != ORBGPU_OK) return rc;
+    // the outputs follow the sync words
+    const size_t out_off = align256(P.sync_bytes), desc_off = out_off + align256(sizeof(orbgpu_keypoint) * staged);
+    uint8_t* const d_sync_bytes = ex->d_io + IO_SYNC;
+    int* const d_status = (int*)d_sync_bytes;
+    orbgpu_keypoint* const okps = to_host ? (orbgpu_keypoint*)(d_sync_bytes + out_off) : keypoints;
+    uint8_t* const odesc = to_host ? d_sync_bytes + desc_off : descriptors;
+    LevelDesc* const d_descs = (LevelDesc*)ex->d_io;
+    LevelDesc* const hd = (LevelDesc*)ex->h_io;
     fill_descs(g, ex->tables, P.layout, P.arena, 0, ex->ini_th, ex->min_th, 0, capacity, hd);
-    for (int l = 0; l < nl; l++) hd[l].done = P.d_sync + P.done_off[l];
-    int* const d_status = P.d_sync;
+    for (int l = 0; l < nl; l++) {
+        hd[l].done = d_status + P.done_off[l];
+        hd[l].frame_total = d_status + 1;
+    }
     cudaStream_t st = ex->stream;
-    ORBGPU_CUDA_TRY(cudaMemcpyAsync(ex->d_descs, hd, sizeof(LevelDesc) * nl, cudaMemcpyHostToDevice, st));
-    ORBGPU_CUDA_TRY(cudaMemsetAsync(P.d_sync, 0, P.sync_bytes, st));
+    ORBGPU_CUDA_TRY(cudaMemcpyAsync(ex->d_io, ex->h_io, IO_SYNC + P.sync_bytes, cudaMemcpyHostToDevice, st));
     // level 0 = the image
-    ORBGPU_CUDA_TRY(cudaMemcpy2DAsync(hd[0].dst, hd[0].pitch, image, step, width, height,
-                                      image_mem == ORBGPU_MEM_DEVICE ? cudaMemcpyDeviceToDevice
-                                                                     : cudaMemcpyHostToDevice,
-                                      st));
+    rc = upload_image(ex, hd[0].dst, hd[0].pitch, image, step, width, height, image_mem, st);
+    if (rc != ORBGPU_OK) return rc;
     if (P.fused) {
-        launch_pyramid(ex->d_descs, P.pyramid, nullptr, 1, nl, d_status + 4, d_status, st);
+        launch_pyramid(d_descs, P.pyramid, nullptr, 1, nl, d_status + 4, d_status, st);
     } else {
         // levels 1.. resized in a chain on the side stream while the strips of
         // the levels already resized run on the extractor's stream
         ORBGPU_CUDA_TRY(cudaEventRecord(ex->ev_fork, st));
         ORBGPU_CUDA_TRY(cudaStreamWaitEvent(ex->side, ex->ev_fork, 0));
         for (int l = 1; l < nl; l++) {
-            launch_level_resize(ex->d_descs, RangeMap{P.d_items + P.rb_first[l], 1, l, 0}, P.rb_count[l], P.rows, ex->side);
+            launch_level_resize(d_descs, RangeMap{P.d_items + P.rb_first[l], 1, l, 0}, P.rb_count[l], P.rows, ex->side);
             ORBGPU_CUDA_TRY(cudaEventRecord(ex->ev_level[l], ex->side));
         }
         for (int l = 0; l < nl; l++) {
             if (l > 0) ORBGPU_CUDA_TRY(cudaStreamWaitEvent(st, ex->ev_level[l], 0));
-            launch_level_strip(ex->d_descs, RangeMap{P.d_items + P.rb_first[l], 1, l, 0}, P.rb_count[l], P.rows, st);
+            launch_level_strip(d_descs, RangeMap{P.d_items + P.rb_first[l], 1, l, 0}, P.rb_count[l], P.rows, st);
         }
     }
     int mwc = 1, mhc = 1, mbox = 0;
@@ -870,16 +907,16 @@ extern "C" int orbgpu_extract(orbgpu_extractor* ex, const uint8_t* image, int wi
         mhc = std::max(mhc, L.hCell);
         if (L.ncells > 0) mbox = std::max(mbox, fast_cell_box_w(L.wCell) * (L.hCell + 6));
     }
-    launch_fast(ex->d_descs, RangeMap{P.d_items + P.fast_first, nl, 0, 1}, P.fast_count, d_status, mwc, mhc, mbox,
+    launch_fast(d_descs, RangeMap{P.d_items + P.fast_first, nl, 0, 1}, P.fast_count, d_status, mwc, mhc, mbox,
                 st);
-    launch_distribute(ex->d_descs, 1, nl, P.max_kept, d_status, st);
-    launch_describe(ex->d_descs, nl, P.features, okps, odesc, d_status, st);
+    launch_distribute(d_descs, 1, nl, P.max_kept, d_status, st);
+    launch_describe(d_descs, nl, P.features, okps, odesc, d_status, st);
     ORBGPU_CUDA_TRY(cudaGetLastError());
-    ORBGPU_CUDA_TRY(cudaMemcpyAsync(ex->h_pinned, d_status, sizeof(int), cudaMemcpyDeviceToHost, st));
-    ORBGPU_CUDA_TRY(cudaMemcpyAsync(ex->h_pinned + 4, hd[0].frame_total, sizeof(int), cudaMemcpyDeviceToHost, st));
+    const size_t down = to_host ? desc_off + 32 * (size_t)staged : 2 * sizeof(int);
+    ORBGPU_CUDA_TRY(cudaMemcpyAsync(ex->h_down, d_sync_bytes, down, cudaMemcpyDeviceToHost, st));
     ORBGPU_CUDA_TRY(cudaStreamSynchronize(st));
-    const int status = ex->h_pinned[0];
-    const int total = ex->h_pinned[4];
+    const int status = ((const int*)ex->h_down)[0];
+    const int total = ((const int*)ex->h_down)[1];
     *n_keypoints = total;
     if (status & ~16) {
         char msg[128];
@@ -891,10 +928,9 @@ extern "C" int orbgpu_extract(orbgpu_extractor* ex, const uint8_t* image, int wi
         orbgpu_set_last_error("output capacity too small", __FILE__, __LINE__);
         return ORBGPU_ERR_CAPACITY;
     }
-    if (out_mem != ORBGPU_MEM_DEVICE && total > 0) {
-        ORBGPU_CUDA_TRY(cudaMemcpyAsync(keypoints, okps, sizeof(orbgpu_keypoint) * total, cudaMemcpyDeviceToHost, st));
-        ORBGPU_CUDA_TRY(cudaMemcpyAsync(descriptors, odesc, 32 * (size_t)total, cudaMemcpyDeviceToHost, st));
-        ORBGPU_CUDA_TRY(cudaStreamSynchronize(st));
+    if (to_host && total > 0) {
+        std::memcpy(keypoints, ex->h_down + out_off, sizeof(orbgpu_keypoint) * total);
+        std::memcpy(descriptors, ex->h_down + desc_off, 32 * (size_t)total);
     }
     return ORBGPU_OK;
 }
