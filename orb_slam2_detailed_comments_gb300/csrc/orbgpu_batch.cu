@@ -439,7 +439,7 @@ static int plan_batch(orbgpu_batch* b, int nframes, const int* widths, const int
     b->features = 0;
     for (int f = 0; f < nframes; f++)
         for (auto& L : b->cur[f]->geom) {
-            if (L.ncells > 0) b->features += L.nfeat + 1;
+            if (L.ncells > 0) b->features += L.nfeat + 3;
             b->max_kept = std::max(b->max_kept, L.node_cap);
         }
     b->nframes = nframes;

@@ -664,7 +664,7 @@ static int build_plan(orbgpu_extractor* ex, int w, int h, SizePlan** out) {
     P->max_kept = 0;
     for (auto& L : g) {
         if (L.ncells > 0) {
-            P->features += L.nfeat + 1;
+            P->features += L.nfeat + 3;
             P->max_total += L.node_cap;
         }
         P->max_kept = std::max(P->max_kept, L.node_cap);

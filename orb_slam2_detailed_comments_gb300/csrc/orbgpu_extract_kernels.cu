@@ -10,7 +10,7 @@ namespace orbgpu {
 
 __constant__ int c_gauss_taps[7];
 __constant__ int c_umax[ORBGPU_HALF_PATCH + 1];
-__constant__ signed char c_pattern[256 * 4];
+__device__ signed char g_pattern[256 * 4];
 
 // Exception table of the descriptor rotation: sorted float bit patterns x for
 // which the host C library's cosf(x)/sinf(x) differ from the rounded
@@ -1382,19 +1382,22 @@ __global__ void __launch_bounds__(DIST_T, 3) k_distribute(const LevelDesc* descs
 }
 
 // ---------------------------------------------------------------- describe
-// The host library's value for input bits xb if the table lists xb, else v.
-// The bucket of xb bounds the search to a handful of entries.
-__device__ __forceinline__ float lookup_exception(const uint32_t* keys, const float* vals, const int* bucket,
-                                                  const uint16_t* sub, uint32_t xb, float v) {
+// The entries of a table of n exceptions that input bits xb may be among: its
+// bucket bounds them to a handful.
+__device__ __forceinline__ int2 exception_range(int n, const int* bucket, const uint16_t* sub, uint32_t xb) {
     const uint32_t b = xb >> ORBGPU_EXC_SHIFT;
-    if (bucket == nullptr || sub == nullptr || b >= (uint32_t)g_exc_nbuckets) return v;
+    if (n <= 0 || bucket == nullptr || sub == nullptr || b >= (uint32_t)g_exc_nbuckets) return {0, 0};
     constexpr uint32_t NS = 1u << ORBGPU_EXC_SUB_BITS;
     const uint32_t s = (xb >> (ORBGPU_EXC_SHIFT - ORBGPU_EXC_SUB_BITS)) & (NS - 1);
-    // the four loads are independent: one round trip for the entry range
+    // the loads are independent: one round trip
     const int base = bucket[b];
     const int lo = base + sub[b * NS + s];
     const int hi = s + 1 < NS ? base + sub[b * NS + s + 1] : bucket[b + 1];
-    for (int i = lo; i < hi; i++)
+    return {lo, hi};
+}
+// The host library's value for input bits xb if the table lists xb, else v.
+__device__ __forceinline__ float lookup_exception(const uint32_t* keys, const float* vals, int2 range, uint32_t xb, float v) {
+    for (int i = range.x; i < range.y; i++)
         if (keys[i] == xb) return vals[i];
     return v;
 }
@@ -1411,9 +1414,8 @@ __device__ __forceinline__ float lookup_exception(const uint32_t* keys, const fl
 // rounds are in flight while one is computed:
 //   pass A   the IC_Angle disc of each keypoint from the level plane
 //            (DESC_LBOX_*): moments with one lane per patch column;
-//   pass B   fastAtan2 and the double-precision rotation of all 32 keypoints
-//            at once, one per lane (the FP64 pipe is narrow on this GPU: a
-//            full warp per instruction);
+//   pass B   fastAtan2 and the rotation (two-float arithmetic) of all 32
+//            keypoints at once, one per lane;
 //   pass C   the rBRIEF disc from the blurred plane (DESC_BBOX_*): one
 //            descriptor byte per lane, two keypoints at a time, the pattern
 //            read from shared memory.
@@ -1422,7 +1424,11 @@ __device__ __forceinline__ float lookup_exception(const uint32_t* keys, const fl
 // frame is a difference of two prefix entries); keypoint g of the flattened
 // list finds its level by binary search.  R (1 / 2 / 4 keypoints per round)
 // and D (rounds in flight, 2 / 4; WPB = 24 / (R D) warps per block) are
-// chosen by the autotuner.  A copy
+// chosen by the autotuner.  Where a task is one keypoint (a frame or two), the
+// launch is the latency of one keypoint, and a third of that was the acquire of
+// the two tensor maps and the copies behind it (7,000 of 21,000 cycles): the
+// warp then copies both boxes at once in 16-byte pieces by cp.async
+// (one 1280x720 frame 16.1 -> 12.3 us).  A copy
 // that does not complete within the bounded wait sets status bit 128 and
 // ends the warp once the copies in flight are drained.
 static_assert(ORBGPU_EDGE_THRESHOLD >= DESC_BBOX_R && ORBGPU_EDGE_THRESHOLD >= ORBGPU_HALF_PATCH,
@@ -1452,8 +1458,9 @@ __global__ void __launch_bounds__(32 * WPB) k_describe(const LevelDesc* descs, i
         mbar_init_fence();
     }
     for (int i = threadIdx.x; i < 512; i += blockDim.x) {
-        const int l = i >> 4, p = i & 15;
-        s_pat[p][l] = make_float2((float)c_pattern[2 * i], (float)c_pattern[2 * i + 1]);
+        const int l = i & 31, p = i >> 5;
+        const char2 pt = __ldg(reinterpret_cast<const char2*>(g_pattern) + 16 * l + p);
+        s_pat[p][l] = make_float2((float)pt.x, (float)pt.y);
     }
     int base = 0;
     for (int e0 = 0; e0 < ndescs; e0 += blockDim.x) {
@@ -1483,6 +1490,7 @@ __global__ void __launch_bounds__(32 * WPB) k_describe(const LevelDesc* descs, i
     const int grid_warps = gridDim.x * WPB;
     const int TS = task ? task : min(32, max(1, (total + grid_warps - 1) / grid_warps));
     const int ntasks = (total + TS - 1) / TS;
+    const bool lone = TS == 1;
     // consecutive tasks on different blocks: the last, partial pass is spread over the SMs
     for (int t = warp * gridDim.x + blockIdx.x; t < ntasks; t += grid_warps) {
         // this lane's keypoint: level, position, output row, validity
@@ -1524,7 +1532,24 @@ __global__ void __launch_bounds__(32 * WPB) k_describe(const LevelDesc* descs, i
         const int nr = (nv + R - 1) / R;                         // rounds
         const void* tm_l = nullptr;
         const void* tm_b = nullptr;
-        if (valid) {
+        if (lone) {
+            // both boxes in 16-byte pieces by the whole warp, as far as the
+            // plane's rows reach; level in buffer 0, blurred in buffer 1
+            const int src = __ffs(vmask) - 1;
+            const LevelDesc& d = descs[__shfl_sync(FULL, e, src)];
+            const int kx = __shfl_sync(FULL, x, src), ky = __shfl_sync(FULL, y, src), pitch = d.pitch;
+            const uint8_t *level = d.dst, *blur = d.blur;
+            auto stage = [&](uint8_t* dst, const uint8_t* plane, int r, int w16, int h) {
+                const int x0 = (kx - r) & ~15;
+                for (int c = lane; c < w16 * h; c += 32) {
+                    const int row = c / w16, col = x0 + 16 * (c - row * w16);
+                    if (col < pitch) cp_async16(dst + 16 * c, plane + (size_t)(ky - r + row) * pitch + col);
+                }
+                cp_async_commit();
+            };
+            stage(wbuf, level, ORBGPU_HALF_PATCH, DESC_LBOX_W / 16, DESC_LBOX_H);
+            stage(wbuf + R * DESC_SLOT, blur, DESC_BBOX_R, DESC_BBOX_W / 16, DESC_BBOX_H);
+        } else if (valid) {
             tm_l = descs[e].tm_level;
             tm_b = descs[e].tm_blur;
             tensormap_acquire(tm_l);
@@ -1533,6 +1558,7 @@ __global__ void __launch_bounds__(32 * WPB) k_describe(const LevelDesc* descs, i
         // round i of a pass: the valid lanes of ranks [i R, i R + R) copy
         // their box into slot rank - i R of buffer i mod D
         auto issue = [&](int i, bool blurred) {
+            if (lone) return;
             const int b = i % D;
             if (lane == 0)
                 mbar_expect_tx(&bar[b], (uint32_t)min(R, nv - i * R) *
@@ -1546,7 +1572,13 @@ __global__ void __launch_bounds__(32 * WPB) k_describe(const LevelDesc* descs, i
         };
         // bounded wait for round i; on a timeout the rounds still in flight
         // (i .. i + D - 1) get one more bounded wait each before the warp leaves
-        auto wait = [&](int i) -> bool {
+        auto wait = [&](int i, bool blurred) -> bool {
+            if (lone) {
+                if (blurred) cp_async_wait<0>();
+                else cp_async_wait<1>();
+                __syncwarp();
+                return true;
+            }
             const int b = i % D;
             if (__all_sync(FULL, mbar_wait(&bar[b], (par >> b) & 1u))) {
                 par ^= 1u << b;
@@ -1563,7 +1595,7 @@ __global__ void __launch_bounds__(32 * WPB) k_describe(const LevelDesc* descs, i
         for (int i = 0; i < min(nr, D); i++) issue(i, false);
         unsigned rest = vmask;
         for (int i = 0; i < nr; i++) {
-            if (!wait(i)) return;
+            if (!wait(i, false)) return;
             const uint8_t* buf = wbuf + (i % D) * R * DESC_SLOT;
             for (int j = 0; j < R && rest; j++) {
                 const int k = __ffs(rest) - 1;
@@ -1598,13 +1630,12 @@ __global__ void __launch_bounds__(32 * WPB) k_describe(const LevelDesc* descs, i
             // computeOrbDescriptor on the blurred level (src/ORBextractor.cc:153-204)
             const float factorPI = (float)(3.1415926535897932384626433832795 / 180.f);
             const float ar = __fmul_rn(angle, factorPI);
-            double sd, cd;
-            sincos_taylor(ar, &sd, &cd);
-            ca = __double2float_rn(cd);
-            sb = __double2float_rn(sd);
             const uint32_t xb = __float_as_uint(ar);
-            if (g_cos_exc_n > 0) ca = lookup_exception(g_cos_exc_key, g_cos_exc_val, g_cos_exc_bucket, g_cos_exc_sub, xb, ca);
-            if (g_sin_exc_n > 0) sb = lookup_exception(g_sin_exc_key, g_sin_exc_val, g_sin_exc_bucket, g_sin_exc_sub, xb, sb);
+            const int2 xc = exception_range(g_cos_exc_n, g_cos_exc_bucket, g_cos_exc_sub, xb);
+            const int2 xs = exception_range(g_sin_exc_n, g_sin_exc_bucket, g_sin_exc_sub, xb);
+            sincos_float(ar, sb, ca);
+            ca = lookup_exception(g_cos_exc_key, g_cos_exc_val, xc, xb, ca);
+            sb = lookup_exception(g_sin_exc_key, g_sin_exc_val, xs, xb, sb);
             const LevelDesc& d = descs[e];
             orbgpu_keypoint kp;
             const float sc = d.scale;
@@ -1621,8 +1652,8 @@ __global__ void __launch_bounds__(32 * WPB) k_describe(const LevelDesc* descs, i
         // per lane, two keypoints at a time
         rest = vmask;
         for (int i = 0; i < nr; i++) {
-            if (!wait(i)) return;
-            const uint8_t* buf = wbuf + (i % D) * R * DESC_SLOT;
+            if (!wait(i, true)) return;
+            const uint8_t* buf = wbuf + (lone ? 1 : i % D) * R * DESC_SLOT;
 #pragma unroll
             for (int j = 0; j < R; j += 2) {
                 if (!rest) break;
@@ -1675,7 +1706,7 @@ __global__ void __launch_bounds__(32 * WPB) k_describe(const LevelDesc* descs, i
 void upload_constants(cudaStream_t st, const int* taps, const int* umax) {
     cudaMemcpyToSymbolAsync(c_gauss_taps, taps, 7 * sizeof(int), 0, cudaMemcpyHostToDevice, st);
     cudaMemcpyToSymbolAsync(c_umax, umax, (ORBGPU_HALF_PATCH + 1) * sizeof(int), 0, cudaMemcpyHostToDevice, st);
-    cudaMemcpyToSymbolAsync(c_pattern, kBriefPattern, sizeof(kBriefPattern), 0, cudaMemcpyHostToDevice, st);
+    cudaMemcpyToSymbolAsync(g_pattern, kBriefPattern, sizeof(kBriefPattern), 0, cudaMemcpyHostToDevice, st);
 }
 
 void set_sincos_exceptions(const uint32_t* ck, const float* cv, int cn, const uint32_t* sk, const float* sv, int sn,
@@ -1883,12 +1914,11 @@ namespace orbgpu {
 __global__ void k_sincos_probe(const float* x, int n, float* c, float* s) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    double sd, cd;
-    sincos_taylor(x[i], &sd, &cd);
-    float a = __double2float_rn(cd), b = __double2float_rn(sd);
+    float a, b;
+    sincos_float(x[i], b, a);
     const uint32_t xb = __float_as_uint(x[i]);
-    if (g_cos_exc_n > 0) a = lookup_exception(g_cos_exc_key, g_cos_exc_val, g_cos_exc_bucket, g_cos_exc_sub, xb, a);
-    if (g_sin_exc_n > 0) b = lookup_exception(g_sin_exc_key, g_sin_exc_val, g_sin_exc_bucket, g_sin_exc_sub, xb, b);
+    a = lookup_exception(g_cos_exc_key, g_cos_exc_val, exception_range(g_cos_exc_n, g_cos_exc_bucket, g_cos_exc_sub, xb), xb, a);
+    b = lookup_exception(g_sin_exc_key, g_sin_exc_val, exception_range(g_sin_exc_n, g_sin_exc_bucket, g_sin_exc_sub, xb), xb, b);
     c[i] = a;
     s[i] = b;
 }

@@ -318,3 +318,22 @@ def test_distribute_limits(torch, oracle, w, h, nf, nlevels, noise):
     ref = oracle.extract(img, nfeatures=nf, nlevels=nlevels, want_pyramid=False)
     assert_kps_equal(kps, ref.keypoints, f"{w}x{h} {nf}")
     assert np.array_equal(desc, ref.descriptors)
+
+
+def test_descriptor_rotation_around_the_axes(torch, oracle):
+    """Every float within 2^19 steps of a multiple of pi/4, where the reduced
+    angle cancels and the quadrant changes, equals the host library."""
+    import ctypes as C
+    from orb_slam2_detailed_comments_gb300._lib import lib, ptr
+    steps = np.arange(-(1 << 19), 1 << 19, dtype=np.int64)
+    hi = int(np.float32(np.float32(360.0) * np.float32(np.pi / 180.0)).view(np.uint32))
+    x = np.concatenate([int(np.float32(k * np.pi / 4).view(np.uint32)) + steps for k in range(1, 9)])
+    x = np.ascontiguousarray(x[x <= hi].astype(np.uint32).view(np.float32))
+    xd = torch.from_numpy(x).cuda()
+    c, s = torch.empty_like(xd), torch.empty_like(xd)
+    assert lib().orbgpu_descriptor_sincos(ptr(xd), len(x), ptr(c), ptr(s)) == 0
+    hc, hs = np.zeros_like(x), np.zeros_like(x)
+    oracle.lib.orc_sincos_table(x.ctypes.data_as(C.c_void_p), len(x), hc.ctypes.data_as(C.c_void_p),
+                                hs.ctypes.data_as(C.c_void_p))
+    assert np.array_equal(c.cpu().numpy().view(np.uint32), hc.view(np.uint32))
+    assert np.array_equal(s.cpu().numpy().view(np.uint32), hs.view(np.uint32))
