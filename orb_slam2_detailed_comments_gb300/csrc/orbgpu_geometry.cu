@@ -87,6 +87,81 @@ __global__ void __launch_bounds__(FR_THREADS) k_undistort_keypoints(const float*
     }
 }
 
+// The frustum test's double expressions in two-float arithmetic.  Each result
+// is a float rounded from a double; the pair (h, l) below holds the exact value
+// to within 'err', a bound that also covers the double's own roundings, and
+// where both ends of that interval round to the same float, the double does
+// too.  Elsewhere (a few results in a million; zeros, tiny, huge and
+// non-finite values always) the doubles are evaluated.  With the doubles for
+// every point the kernel was bound by the FP64 pipe (77 % busy): 64 frames of
+// 5,000 points 50 -> 14.5 us a call.
+struct TwoFloat {
+    float h, l, err;
+};
+__device__ __forceinline__ float two_sum(float a, float b, float& lo) {  // Knuth: a + b = sum + lo
+    const float s = __fadd_rn(a, b), bb = __fsub_rn(s, a);
+    lo = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
+    return s;
+}
+// The products and their errors are exact; of the errors' sum (at most 2^-22 of
+// the products' magnitude) four roundings of 2^-24 are lost, of the doubles' sum
+// two of 2^-53: 2^-42 of the magnitude covers both four times.
+__device__ __forceinline__ TwoFloat dot3_two_float(float a0, float b0, float a1, float b1, float a2, float b2) {
+    const float p0 = __fmul_rn(a0, b0), p1 = __fmul_rn(a1, b1), p2 = __fmul_rn(a2, b2);
+    float t1, t2, l;
+    const float s = two_sum(two_sum(p0, p1, t1), p2, t2);
+    const float e = __fadd_rn(__fadd_rn(__fmaf_rn(a0, b0, -p0), __fmaf_rn(a1, b1, -p1)), __fmaf_rn(a2, b2, -p2));
+    const float h = two_sum(s, __fadd_rn(__fadd_rn(t1, t2), e), l);
+    return {h, l, __fmul_rn(__fadd_rn(__fadd_rn(fabsf(p0), fabsf(p1)), fabsf(p2)), 0x1p-42f)};
+}
+// Whether the double behind v rounds to the float r (false for NaN).
+__device__ __forceinline__ bool rounds_to(const TwoFloat& v, float& r) {
+    r = __fadd_rn(v.h, __fsub_rn(v.l, v.err));
+    return r == __fadd_rn(v.h, __fadd_rn(v.l, v.err)) && fabsf(v.h) > 0x1p-60f && fabsf(v.h) < 0x1p+100f;
+}
+// The doubles, out of line: inlined, the compiler evaluated them for every
+// point and selected.
+__device__ __forceinline__ double dot3_double(float a0, float b0, float a1, float b1, float a2, float b2) {
+    const double s = __dadd_rn(__dmul_rn((double)a0, (double)b0), __dmul_rn((double)a1, (double)b1));
+    return __dadd_rn(s, __dmul_rn((double)a2, (double)b2));
+}
+__device__ __noinline__ float dot3_slow(float a0, float b0, float a1, float b1, float a2, float b2) {
+    return (float)dot3_double(a0, b0, a1, b1, a2, b2);
+}
+__device__ __noinline__ float norm3_slow(float a, float b, float c) { return (float)__dsqrt_rn(dot3_double(a, a, b, b, c, c)); }
+__device__ __noinline__ float dot3_over_slow(float a0, float b0, float a1, float b1, float a2, float b2, float d) {
+    return (float)__ddiv_rn(dot3_double(a0, b0, a1, b1, a2, b2), (double)d);
+}
+__device__ __forceinline__ float dot3_float(float a0, float b0, float a1, float b1, float a2, float b2) {
+    float r;
+    if (!rounds_to(dot3_two_float(a0, b0, a1, b1, a2, b2), r)) r = dot3_slow(a0, b0, a1, b1, a2, b2);
+    return r;
+}
+// The float of a vector's double norm: one Newton step from the float root
+// leaves the square of its error.
+__device__ __forceinline__ float norm3_float(float a, float b, float c) {
+    const TwoFloat s = dot3_two_float(a, a, b, b, c, c);
+    float r;
+    if (s.h > 0x1p-60f && s.h < 0x1p+100f) {
+        const float q = __fsqrt_rn(s.h), q2 = __fmul_rn(q, q);
+        const float rest = __fadd_rn(__fsub_rn(__fsub_rn(s.h, q2), __fmaf_rn(q, q, -q2)), s.l);
+        if (rounds_to({q, __fmul_rn(rest, __fdividef(0.5f, q)), __fmul_rn(q, 0x1p-41f)}, r)) return r;
+    }
+    return norm3_slow(a, b, c);
+}
+// The float of the double quotient a . b / d.
+__device__ __forceinline__ float dot3_over(float a0, float b0, float a1, float b1, float a2, float b2, float d) {
+    float r;
+    if (d > 0x1p-60f && d < 0x1p+60f) {
+        const TwoFloat p = dot3_two_float(a0, b0, a1, b1, a2, b2);
+        const float inv = __fdividef(1.0f, d), q = __fmul_rn(p.h, inv);
+        const float rest = __fadd_rn(__fmaf_rn(-q, d, p.h), p.l);
+        const float err = __fadd_rn(__fmul_rn(p.err, __fmul_rn(inv, 1.25f)), __fmul_rn(fabsf(q), 0x1p-42f));
+        if (rounds_to({q, __fmul_rn(rest, inv), err}, r)) return r;
+    }
+    return dot3_over_slow(a0, b0, a1, b1, a2, b2, d);
+}
+
 __global__ void __launch_bounds__(FR_THREADS) k_is_in_frustum(const orbgpu_frustum_frame* frames,
                                                               int nframes, const int* offsets,
                                                               const orbgpu_mappoint_geometry* __restrict__ mps,
@@ -108,6 +183,7 @@ __global__ void __launch_bounds__(FR_THREADS) k_is_in_frustum(const orbgpu_frust
     }
     const int first = offsets[0], last = offsets[nframes];
     if (first < 0) return;
+    const bool aligned = ((reinterpret_cast<uintptr_t>(mps) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
     const int lane = threadIdx.x & 31;
     const int stride = gridDim.x * FR_THREADS;
     // every lane runs the same number of iterations (warp-wide counting below)
@@ -126,17 +202,17 @@ __global__ void __launch_bounds__(FR_THREADS) k_is_in_frustum(const orbgpu_frust
             }
             f = lo;
             const orbgpu_frustum_frame& F = frames[f];
-            const orbgpu_mappoint_geometry g = mps[i];
             orbgpu_mappoint& o = out[i];
-            const double px = g.x, py = g.y, pz = g.z;
+            orbgpu_mappoint_geometry g;
+            static_assert(sizeof(g) == 32 && sizeof(o) == 32, "two 16-byte accesses each");
+            if (aligned) {
+                reinterpret_cast<float4*>(&g)[0] = __ldg(reinterpret_cast<const float4*>(mps + i));
+                reinterpret_cast<float4*>(&g)[1] = __ldg(reinterpret_cast<const float4*>(mps + i) + 1);
+            } else g = mps[i];
             float pc[3];
 #pragma unroll
-            for (int r = 0; r < 3; r++) {
-                double s = __dmul_rn((double)F.Rcw[3 * r], px);
-                s = __dadd_rn(s, __dmul_rn((double)F.Rcw[3 * r + 1], py));
-                s = __dadd_rn(s, __dmul_rn((double)F.Rcw[3 * r + 2], pz));
-                pc[r] = __fadd_rn((float)s, F.tcw[r]);
-            }
+            for (int r = 0; r < 3; r++)
+                pc[r] = __fadd_rn(dot3_float(F.Rcw[3 * r], g.x, F.Rcw[3 * r + 1], g.y, F.Rcw[3 * r + 2], g.z), F.tcw[r]);
             do {
                 if (pc[2] < 0.0f) break;
                 const float invz = __fdiv_rn(1.0f, pc[2]);
@@ -148,28 +224,29 @@ __global__ void __launch_bounds__(FR_THREADS) k_is_in_frustum(const orbgpu_frust
                 const float min_d = __fmul_rn(0.8f, g.min_distance);
                 const float po0 = __fsub_rn(g.x, F.Ow[0]), po1 = __fsub_rn(g.y, F.Ow[1]),
                             po2 = __fsub_rn(g.z, F.Ow[2]);
-                double ss = __dmul_rn((double)po0, (double)po0);
-                ss = __dadd_rn(ss, __dmul_rn((double)po1, (double)po1));
-                ss = __dadd_rn(ss, __dmul_rn((double)po2, (double)po2));
-                const float dist = (float)__dsqrt_rn(ss);
+                const float dist = norm3_float(po0, po1, po2);
                 if (dist < min_d || dist > max_d) break;
-                double dp = __dmul_rn((double)po0, (double)g.nx);
-                dp = __dadd_rn(dp, __dmul_rn((double)po1, (double)g.ny));
-                dp = __dadd_rn(dp, __dmul_rn((double)po2, (double)g.nz));
-                const float view_cos = (float)__ddiv_rn(dp, (double)dist);
+                const float view_cos = dot3_over(po0, g.nx, po1, g.ny, po2, g.nz, dist);
                 if (view_cos < cos_limit) break;
                 const float ratio = __fdiv_rn(g.max_distance, dist);
                 int level = 0;
                 const int nl = min(F.nlevels, 16);
                 for (int n = 0; n < nl - 1; n++) level += ratio > F.level_above[n] ? 1 : 0;
-                o.proj_x = u;
-                o.proj_y = v;
-                o.proj_xr = __fsub_rn(u, __fmul_rn(F.bf, invz));
-                o.view_cos = view_cos;
-                o.track_scale_level = level;
+                const float xr = __fsub_rn(u, __fmul_rn(F.bf, invz));
+                if (aligned) {
+                    *reinterpret_cast<float4*>(&o) = make_float4(u, v, xr, view_cos);
+                    *reinterpret_cast<int2*>(&o.track_scale_level) = make_int2(level, 1);
+                } else {
+                    o.proj_x = u;
+                    o.proj_y = v;
+                    o.proj_xr = xr;
+                    o.view_cos = view_cos;
+                    o.track_scale_level = level;
+                    o.track_in_view = 1;
+                }
                 inview = true;
             } while (false);
-            o.track_in_view = inview ? 1 : 0;
+            if (!inview) o.track_in_view = 0;
         }
         if (in_view) {
             // one atomic per frame present in the warp

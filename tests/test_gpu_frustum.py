@@ -80,6 +80,45 @@ def test_batch_of_frames_vs_oracle(torch, oracle, pinned):
         assert iv[f] == refs[f][1], f
 
 
+@pytest.mark.parametrize("scale", [-100, -62, -58, -20, 0, 20, 50, 60])
+def test_rounding_limits_vs_oracle(torch, oracle, scale):
+    """Worlds scaled by powers of two past the two-float range at both ends,
+    with sums that cancel (points at the camera centre and on its axes, normals
+    across the viewing ray) and signed zeros; records at a 4-byte offset too."""
+    from orb_slam2_detailed_comments_gb300 import synthetic as syn
+    from orb_slam2_detailed_comments_gb300 import FRUSTUM_FRAME_DTYPE, is_in_frustum
+    w, h, fx, sf, nl, m = 640, 480, 500.0, 1.2, 8, 4000
+    rng = np.random.default_rng(scale + 200)
+    Tcw, g = syn.frustum_case(m, 77, w, h, fx, sf, nl)
+    Tcw, g = np.array(Tcw, np.float32), np.array(g, np.float32)
+    R, t = Tcw[:3, :3].astype(np.float64), Tcw[:3, 3].astype(np.float64)
+    centre = -R.T @ t
+    ray = g[:, :3].astype(np.float64) - centre
+    across = np.cross(ray, rng.normal(size=(m, 3)))
+    g[:1000, 3:6] = (across / np.linalg.norm(across, axis=1, keepdims=True))[:1000]  # view_cos near 0
+    g[1000:1300, :3] = centre + np.outer(rng.uniform(0.5, 9, 300), R[2])  # on the optical axis
+    g[1300:1310, :3] = centre
+    g[1310:1400, :3] = np.where(rng.random((90, 3)) < 0.5, -0.0, 0.0)
+    k = np.float32(2.0) ** scale
+    g[:, :3] *= k
+    g[:, 6:8] *= k
+    Tcw[:3, 3] *= k
+    camera = np.array([fx, fx, w / 2, h / 2, 40.0, w, h, sf, nl, -0.5], np.float32)
+    init = np.zeros(m, pyoracle.MP_DTYPE)
+    cam = pyoracle.make_frustum_camera(Tcw, fx, fx, w / 2, h / 2, 40.0, 0.0, w, 0.0, h, sf, nl)
+    ref = oracle.is_in_frustum(cam, np.ascontiguousarray(g).view(pyoracle.GEOM_DTYPE).reshape(-1), -0.5, init)
+    (out,), iv = run(torch, [frame_record(Tcw, camera)], [g], [init], -0.5)
+    assert out.tobytes() == ref[0].tobytes()
+    assert iv[0] == ref[1]
+    # the same records and geometry one float past a 16-byte boundary
+    room = torch.zeros(2, 8 * m + 4, dtype=torch.float32, device="cuda")
+    G, M = room[0, 1:8 * m + 1].view(m, 8), room[1, 1:8 * m + 1]
+    G.copy_(torch.from_numpy(g))
+    F = torch.from_numpy(np.array([frame_record(Tcw, camera)], FRUSTUM_FRAME_DTYPE).view(np.uint8)).cuda()
+    is_in_frustum(F, torch.tensor([0, m], dtype=torch.int32, device="cuda"), G, M.view(torch.uint8), -0.5, None)
+    assert M.cpu().numpy().view(pyoracle.MP_DTYPE).tobytes() == ref[0].tobytes()
+
+
 def test_chained_into_search_by_projection(torch, oracle):
     """isInFrustum then SearchByProjection(Frame&, vector<MapPoint*>, th) with
     the records staying on the device, against the oracle doing the same."""
