@@ -1487,70 +1487,28 @@ struct StereoPair {
     float bf, fx;
 };
 
-__global__ void k_bstereo_rows_count(const orbgpu_keypoint* kps, const int* counts, int cap, const StereoPair* pairs,
-                                     int rows_stride, int* row_count) {
-    const StereoPair& P = pairs[blockIdx.y];
-    const int nR = min(counts[P.right], cap);
-    int* rc = row_count + (size_t)blockIdx.y * rows_stride;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nR; i += gridDim.x * blockDim.x) {
-        int lo, hi;
-        if (!stereo_rows_of(kps[(size_t)P.right * cap + i], P.lv, P.nRows, lo, hi)) continue;
-        for (int yi = lo; yi <= hi; yi++) atomicAdd(&rc[yi], 1);
-    }
-}
-
-// One block per pair: row_start = exclusive prefix of the row counts
-// (nRows + 1 entries), cursor = its copy.
-__global__ void k_bstereo_scan(const int* row_count, const StereoPair* pairs, int rows_stride, int* row_start,
-                               int* cursor) {
-    __shared__ int s_scan[32];
-    const int n = pairs[blockIdx.x].nRows + 1;
-    const size_t o = (size_t)blockIdx.x * rows_stride;
-    int carry = 0;
-    for (int b0 = 0; b0 < n; b0 += blockDim.x) {
-        const int i = b0 + threadIdx.x;
-        const int v = i < n ? row_count[o + i] : 0;
-        int tot;
-        const int ex = block_exclusive_scan(v, s_scan, &tot);
-        if (i < n) {
-            row_start[o + i] = carry + ex;
-            cursor[o + i] = carry + ex;
-        }
-        carry += tot;
-    }
-}
-
-__global__ void k_bstereo_rows_fill(const orbgpu_keypoint* kps, const int* counts, int cap, const StereoPair* pairs,
-                                    int rows_stride, int* cursor, int* row_keys, size_t key_stride) {
-    const StereoPair& P = pairs[blockIdx.y];
-    const int nR = min(counts[P.right], cap);
-    int* cur = cursor + (size_t)blockIdx.y * rows_stride;
-    int* keys = row_keys + blockIdx.y * key_stride;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nR; i += gridDim.x * blockDim.x) {
-        int lo, hi;
-        if (!stereo_rows_of(kps[(size_t)P.right * cap + i], P.lv, P.nRows, lo, hi)) continue;
-        for (int yi = lo; yi <= hi; yi++) keys[atomicAdd(&cur[yi], 1)] = i;
-    }
-}
-
-__global__ void k_bstereo_match(const orbgpu_keypoint* kps, const uint8_t* desc, const int* counts, int cap,
-                                const StereoPair* pairs, int rows_stride, const int* row_start, const int* row_keys,
-                                size_t key_stride, float* uright, float* depth, int* sad, int* status) {
-    const StereoPair& P = pairs[blockIdx.y];
-    const int iL = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (iL >= min(counts[P.left], cap)) return;
-    const size_t p = blockIdx.y, l0 = (size_t)P.left * cap, r0 = (size_t)P.right * cap;
-    stereo_match_warp(iL, kps + l0, desc + 32 * l0, kps + r0, desc + 32 * r0, P.lv, P.nRows,
-                      row_start + p * rows_stride, row_keys + p * key_stride, P.bf, P.fx, uright + p * cap,
-                      depth + p * cap, sad + p * cap, status);
-}
-
-__global__ void k_bstereo_median(const int* counts, int cap, const StereoPair* pairs, const int* sad, float* uright,
-                                 float* depth, int* sort_buf, int sort_cap) {
+__global__ void __launch_bounds__(STEREO_INDEX_THREADS) k_bstereo_index(const orbgpu_keypoint* kps, const int* counts,
+                                                                        int cap, const StereoPair* pairs, int* start,
+                                                                        uint4* recs, int* done, int* status) {
     const StereoPair& P = pairs[blockIdx.x];
     const size_t p = blockIdx.x;
-    stereo_median_block(min(counts[P.left], cap), sad + p * cap, uright + p * cap, depth + p * cap,
-                        sort_buf + p * sort_cap, sort_cap, nullptr);
+    if (threadIdx.x == 0) {
+        done[p] = 0;
+        if (p == 0) *status = 0;
+    }
+    stereo_index_block(kps + (size_t)P.right * cap, min(counts[P.right], cap), P.lv.nlevels, P.nRows,
+                       start + p * (ORBGPU_MAX_DIM + 1), recs + p * cap);
+}
+
+__global__ void __launch_bounds__(32 * STEREO_WARPS) k_bstereo_match(const orbgpu_keypoint* kps, const uint8_t* desc,
+                                                                     const int* counts, int cap, const StereoPair* pairs,
+                                                                     const int* start, const uint4* recs, float* uright,
+                                                                     float* depth, int* sad, int* done, int* status) {
+    const StereoPair& P = pairs[blockIdx.y];
+    const size_t p = blockIdx.y, l0 = (size_t)P.left * cap, r0 = (size_t)P.right * cap;
+    stereo_match_block(blockIdx.x * STEREO_WARPS, min(counts[P.left], cap), kps + l0, desc + 32 * l0, desc + 32 * r0,
+                       P.lv, P.nRows, start + p * (ORBGPU_MAX_DIM + 1), recs + p * cap, P.bf, P.fx, uright + p * cap,
+                       depth + p * cap, sad + p * cap, done + p, status);
 }
 
 }  // namespace orbgpu
@@ -1567,8 +1525,6 @@ extern "C" int orbgpu_batch_compute_stereo_matches(orbgpu_batch* b, const orbgpu
     if (npairs == 0) return ORBGPU_OK;
     const int cap = b->frame_cap, nl = b->nlevels;
     std::vector<StereoPair> hp(npairs);
-    int max_rows = 1;
-    float maxscale = 1.0f;
     for (int p = 0; p < npairs; p++) {
         const int lf = left_frame[p], rf = right_frame[p];
         if (lf < 0 || rf < 0 || lf >= b->nframes || rf >= b->nframes || !(bf[p] > 0.f) || !(fx[p] > 0.f)) {
@@ -1591,7 +1547,6 @@ extern "C" int orbgpu_batch_compute_stereo_matches(orbgpu_batch* b, const orbgpu
             P.lv.pitch[l] = L->geom[l].pitch;
             P.lv.scale[l] = L->tables.scale[l];
             P.lv.inv_scale[l] = 1.0f / L->tables.scale[l];
-            maxscale = std::max(maxscale, P.lv.scale[l]);
         }
         P.lv.nlevels = nl;
         P.left = lf;
@@ -1599,17 +1554,10 @@ extern "C" int orbgpu_batch_compute_stereo_matches(orbgpu_batch* b, const orbgpu
         P.nRows = L->geom[0].h;
         P.bf = bf[p];
         P.fx = fx[p];
-        max_rows = std::max(max_rows, P.nRows);
     }
-    const int rows_stride = max_rows + 2;
-    const int rows_per_key = 2 * (int)std::ceil(2.0f * maxscale) + 4;
-    const size_t key_stride = (size_t)cap * rows_per_key;
-    int sort_cap = 1;
-    while (sort_cap < cap) sort_cap <<= 1;
     cudaStream_t st = b->stream;
-    const size_t need = sizeof(StereoPair) * npairs + 3 * sizeof(int) * (size_t)npairs * rows_stride +
-                        sizeof(int) * npairs * key_stride + sizeof(int) * (size_t)npairs * (cap + sort_cap) +
-                        16 * 256;
+    const size_t need = sizeof(StereoPair) * npairs + sizeof(int) * (size_t)npairs * (ORBGPU_MAX_DIM + 2 + cap) +
+                        sizeof(uint4) * (size_t)npairs * cap + 16 * 256;
     if (need > b->st_bytes) {
         ORBGPU_CUDA_TRY(cudaStreamSynchronize(st));
         if (b->st_scratch) cudaFree(b->st_scratch);
@@ -1627,24 +1575,15 @@ extern "C" int orbgpu_batch_compute_stereo_matches(orbgpu_batch* b, const orbgpu
         return q;
     };
     StereoPair* d_pairs = (StereoPair*)take(sizeof(StereoPair) * npairs);
-    int* row_count = (int*)take(sizeof(int) * (size_t)npairs * rows_stride);
-    int* row_start = (int*)take(sizeof(int) * (size_t)npairs * rows_stride);
-    int* cursor = (int*)take(sizeof(int) * (size_t)npairs * rows_stride);
-    int* row_keys = (int*)take(sizeof(int) * npairs * key_stride);
+    int* start = (int*)take(sizeof(int) * (size_t)npairs * (ORBGPU_MAX_DIM + 1));
+    uint4* recs = (uint4*)take(sizeof(uint4) * (size_t)npairs * cap);
     int* sad = (int*)take(sizeof(int) * (size_t)npairs * cap);
-    int* sort_buf = (int*)take(sizeof(int) * (size_t)npairs * sort_cap);
+    int* done = (int*)take(sizeof(int) * (size_t)npairs);
     int* status = (int*)take(sizeof(int) * 4);
     ORBGPU_CUDA_TRY(cudaMemcpyAsync(d_pairs, hp.data(), sizeof(StereoPair) * npairs, cudaMemcpyHostToDevice, st));
-    ORBGPU_CUDA_TRY(cudaMemsetAsync(row_count, 0, sizeof(int) * (size_t)npairs * rows_stride, st));
-    ORBGPU_CUDA_TRY(cudaMemsetAsync(status, 0, sizeof(int) * 4, st));
-    const dim3 gk((cap + 255) / 256, npairs);
-    k_bstereo_rows_count<<<gk, 256, 0, st>>>(kps, counts, cap, d_pairs, rows_stride, row_count);
-    k_bstereo_scan<<<npairs, 1024, 0, st>>>(row_count, d_pairs, rows_stride, row_start, cursor);
-    k_bstereo_rows_fill<<<gk, 256, 0, st>>>(kps, counts, cap, d_pairs, rows_stride, cursor, row_keys, key_stride);
-    const int wpb = 8;
-    k_bstereo_match<<<dim3((cap + wpb - 1) / wpb, npairs), 32 * wpb, 0, st>>>(
-        kps, desc, counts, cap, d_pairs, rows_stride, row_start, row_keys, key_stride, uright, depth, sad, status);
-    k_bstereo_median<<<npairs, 1024, 0, st>>>(counts, cap, d_pairs, sad, uright, depth, sort_buf, sort_cap);
+    k_bstereo_index<<<npairs, STEREO_INDEX_THREADS, 0, st>>>(kps, counts, cap, d_pairs, start, recs, done, status);
+    k_bstereo_match<<<dim3((cap + STEREO_WARPS - 1) / STEREO_WARPS, npairs), 32 * STEREO_WARPS, 0, st>>>(
+        kps, desc, counts, cap, d_pairs, start, recs, uright, depth, sad, done, status);
     ORBGPU_CUDA_TRY(cudaGetLastError());
     ORBGPU_CUDA_TRY(cudaMemcpyAsync(b->st_pinned, status, sizeof(int), cudaMemcpyDeviceToHost, st));
     ORBGPU_CUDA_TRY(cudaStreamSynchronize(st));

@@ -874,36 +874,21 @@ __global__ void __launch_bounds__(1024) k_pf_finish(int n, int m, const int* res
 
 // ----------------------------------------------------------------- stereo
 // (the device functions are in orbgpu_stereo.cuh)
-__global__ void k_stereo_rows_count(const orbgpu_keypoint* kpsR, int nR, StereoLevels lv, int nRows, int* row_count) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    int lo, hi;
-    if (i >= nR || !stereo_rows_of(kpsR[i], lv, nRows, lo, hi)) return;
-    for (int yi = lo; yi <= hi; yi++) atomicAdd(&row_count[yi], 1);
+__global__ void __launch_bounds__(STEREO_INDEX_THREADS) k_stereo_index(const orbgpu_keypoint* kpsR, int nR, int nlevels,
+                                                                       int nRows, int* start, uint4* recs,
+                                                                       int* status_done) {
+    if (threadIdx.x < 2) status_done[threadIdx.x] = 0;
+    stereo_index_block(kpsR, nR, nlevels, nRows, start, recs);
 }
 
-__global__ void k_stereo_rows_fill(const orbgpu_keypoint* kpsR, int nR, StereoLevels lv, int nRows, int* cursor,
-                                   int* row_keys) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    int lo, hi;
-    if (i >= nR || !stereo_rows_of(kpsR[i], lv, nRows, lo, hi)) return;
-    for (int yi = lo; yi <= hi; yi++) row_keys[atomicAdd(&cursor[yi], 1)] = i;
-}
-
-// Frame::ComputeStereoMatches per left keypoint (src/Frame.cc:884-1064), one warp each.
-__global__ void k_stereo_match(const orbgpu_keypoint* kpsL, const uint8_t* descL, int nL, const orbgpu_keypoint* kpsR,
-                               const uint8_t* descR, StereoLevels lv, int nRows, const int* row_start,
-                               const int* row_keys, float bf, float fx, float* uright, float* depth, int* sad_out,
-                               int* status) {
-    const int iL = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (iL >= nL) return;
-    stereo_match_warp(iL, kpsL, descL, kpsR, descR, lv, nRows, row_start, row_keys, bf, fx, uright, depth, sad_out,
-                      status);
-}
-
-// Median cut (src/Frame.cc:1069-1081): one block.
-__global__ void k_stereo_median(int nL, const int* sad, float* uright, float* depth, int* sort_buf, int cap,
-                                int* n_valid) {
-    stereo_median_block(nL, sad, uright, depth, sort_buf, cap, n_valid);
+__global__ void __launch_bounds__(32 * STEREO_WARPS) k_stereo_match(const orbgpu_keypoint* kpsL, const uint8_t* descL,
+                                                                    int nL, const uint8_t* descR,
+                                                                    const __grid_constant__ StereoLevels lv, int nRows,
+                                                                    const int* start, const uint4* recs, float bf,
+                                                                    float fx, float* uright, float* depth, int* sad,
+                                                                    int* status_done) {
+    stereo_match_block(blockIdx.x * STEREO_WARPS, nL, kpsL, descL, descR, lv, nRows, start, recs, bf, fx, uright, depth,
+                       sad, status_done + 1, status_done);
 }
 
 // ----------------------------------------------------------------- distance batch
@@ -1847,24 +1832,15 @@ extern "C" int orbgpu_compute_stereo_matches(orbgpu_matcher* m, const orbgpu_ext
     }
     lv.nlevels = nlev;
     const int nRows = lv.h[0];
-    float maxscale = 1.0f;
-    for (int l = 0; l < nlev; l++) maxscale = std::max(maxscale, lv.scale[l]);
-    const int rows_per_key = 2 * (int)std::ceil(2.0f * maxscale) + 4;
-    int sort_cap = 1;
-    while (sort_cap < nL) sort_cap <<= 1;
-    const size_t est = frame_stage_bytes(fl) + frame_stage_bytes(fr) + (size_t)(2 * nRows + 8) * sizeof(int) +
-                       (size_t)nR * rows_per_key * sizeof(int) + (size_t)nL * 3 * sizeof(float) + sort_cap * sizeof(int) +
-                       64 * 1024;
+    const size_t est = frame_stage_bytes(fl) + frame_stage_bytes(fr) + (ORBGPU_MAX_DIM + 1) * sizeof(int) +
+                       (size_t)nR * sizeof(uint4) + (size_t)nL * 3 * sizeof(float) + 64 * 1024;
     int rc = ensure_scratch(m, est);
     if (rc) return rc;
     Bump b{(uint8_t*)m->scratch, 0, m->scratch_bytes};
     Staged sl, sr;
     if ((rc = stage_frame(m, fl, b, sl)) || (rc = stage_frame(m, fr, b, sr))) return rc;
-    int* row_count = b.take<int>(nRows + 1);
-    int* row_start = b.take<int>(nRows + 1);
-    int* cursor = b.take<int>(nRows + 1);
-    int* row_keys = b.take<int>((size_t)std::max(1, nR) * rows_per_key);
-    int* d_total = b.take<int>(1);
+    int* row_start = b.take<int>(ORBGPU_MAX_DIM + 1);
+    uint4* recs = b.take<uint4>(std::max(1, nR));
     float* d_ur = uright;
     float* d_dp = depth;
     if (mem != ORBGPU_MEM_DEVICE) {
@@ -1872,18 +1848,10 @@ extern "C" int orbgpu_compute_stereo_matches(orbgpu_matcher* m, const orbgpu_ext
         d_dp = b.take<float>(nL);
     }
     int* sad = b.take<int>(nL);
-    int* sort_buf = b.take<int>(sort_cap);
-    int* status = b.take<int>(2);
-    ORBGPU_CUDA_TRY(cudaMemsetAsync(row_count, 0, sizeof(int) * (nRows + 1), m->stream));
-    ORBGPU_CUDA_TRY(cudaMemsetAsync(status, 0, sizeof(int) * 2, m->stream));
-    if (nR > 0) k_stereo_rows_count<<<(nR + 255) / 256, 256, 0, m->stream>>>(sr.kps, nR, lv, nRows, row_count);
-    k_exclusive_scan<<<1, 1024, 0, m->stream>>>(row_count, nRows + 1, row_start, d_total);
-    ORBGPU_CUDA_TRY(cudaMemcpyAsync(cursor, row_start, sizeof(int) * (nRows + 1), cudaMemcpyDeviceToDevice, m->stream));
-    if (nR > 0) k_stereo_rows_fill<<<(nR + 255) / 256, 256, 0, m->stream>>>(sr.kps, nR, lv, nRows, cursor, row_keys);
-    const int wpb = 8;
-    k_stereo_match<<<(nL + wpb - 1) / wpb, 32 * wpb, 0, m->stream>>>(sl.kps, sl.desc, nL, sr.kps, sr.desc, lv, nRows,
-                                                                   row_start, row_keys, bf, fx, d_ur, d_dp, sad, status);
-    k_stereo_median<<<1, 1024, 0, m->stream>>>(nL, sad, d_ur, d_dp, sort_buf, sort_cap, status + 1);
+    int* status = b.take<int>(2);  // status, blocks done
+    k_stereo_index<<<1, STEREO_INDEX_THREADS, 0, m->stream>>>(sr.kps, nR, nlev, nRows, row_start, recs, status);
+    k_stereo_match<<<(nL + STEREO_WARPS - 1) / STEREO_WARPS, 32 * STEREO_WARPS, 0, m->stream>>>(
+        sl.kps, sl.desc, nL, sr.desc, lv, nRows, row_start, recs, bf, fx, d_ur, d_dp, sad, status);
     ORBGPU_CUDA_TRY(cudaGetLastError());
     if (mem != ORBGPU_MEM_DEVICE) {
         ORBGPU_CUDA_TRY(cudaMemcpyAsync(uright, d_ur, sizeof(float) * nL, cudaMemcpyDeviceToHost, m->stream));

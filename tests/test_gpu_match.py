@@ -616,3 +616,28 @@ def test_search_by_sim3_vs_oracle(torch, oracle, seed, th):
     assert nf == ref_nf
     assert np.array_equal(m12, ref)
     assert ref_nf > 100 and (pre12 >= 0).sum() > 20
+
+
+@pytest.mark.parametrize("w,h,nf", [(320, 240, 40), (751, 481, 1201), (2301, 4096, 3000)])
+def test_stereo_row_index(torch, oracle, w, h, nf):
+    """The row index at few keypoints, odd sizes and the tallest image: the
+    same matches from the per-frame and the batched call, within 1e-4 of the
+    oracle's."""
+    from orb_slam2_detailed_comments_gb300 import ORBextractor, ORBmatcher, compute_stereo_matches
+    from orb_slam2_detailed_comments_gb300 import synthetic as syn
+    from orb_slam2_detailed_comments_gb300.batch import BatchExtractor, BatchStereo
+    left, right, _ = syn.stereo_pair(w, h, 11)
+    L, R = oracle.extract(left, nfeatures=nf), oracle.extract(right, nfeatures=nf)
+    u1, d1 = oracle.compute_stereo_matches(L.keypoints, L.descriptors, R.keypoints, R.descriptors, L.pyramid, R.pyramid,
+                                           w, h, 386.1, 718.856)
+    exL, exR = ORBextractor(nf, 1.2, 8, 20, 7), ORBextractor(nf, 1.2, 8, 20, 7)
+    kL, dL = exL(left)
+    kR, dR = exR(right)
+    u2, d2 = compute_stereo_matches(ORBmatcher(0.75, True), exL, exR, frame(kL, dL, w, h), frame(kR, dR, w, h), 386.1,
+                                    718.856)
+    np.testing.assert_allclose(u2, u1, atol=1e-4, rtol=0)
+    np.testing.assert_allclose(d2, d1, atol=1e-4, rtol=1e-6)
+    b = BatchExtractor(2, w, h, nf)
+    b.extract([torch.from_numpy(i).cuda() for i in (left, right)], [nf] * 2)
+    ur, dp = BatchStereo(b).compute([(0, 1)], 386.1, 718.856)
+    assert np.array_equal(ur[0, :len(u2)].cpu().numpy(), u2) and np.array_equal(dp[0, :len(d2)].cpu().numpy(), d2)
