@@ -78,24 +78,98 @@ __global__ void __launch_bounds__(BOW_THREADS) k_bow_descend(const uint4* __rest
     }
 }
 
-// Ascending bitonic sort of n2 (a power of two) 64-bit keys in shared memory.
+// Ascending bitonic sort of n2 (a power of two, at least 32) 64-bit keys in
+// shared memory.  Strides below 32 stay in a warp's registers: 21 of the 66
+// steps of 2,048 keys go through shared memory and a barrier.
 __device__ void bow_block_sort(unsigned long long* keys, int n2) {
-    for (int k = 2; k <= n2; k <<= 1) {
-        for (int j = k >> 1; j > 0; j >>= 1) {
-            for (int i = threadIdx.x; i < n2; i += blockDim.x) {
-                const int l = i ^ j;
-                if (l > i) {
-                    const unsigned long long a = keys[i], b = keys[l];
-                    const bool up = (i & k) == 0;
-                    if ((a > b) == up) {
-                        keys[i] = b;
-                        keys[l] = a;
-                    }
+    const int lane = threadIdx.x & 31;
+    // the strides from 'from' (at most 16) down of the merges of sizes k0 .. k1
+    const auto in_warp = [&](int k0, int k1, int from) {
+        for (int b = threadIdx.x - lane; b < n2; b += blockDim.x) {
+            const int i = b + lane;
+            unsigned long long key = keys[i];
+            for (int k = k0; k <= k1; k <<= 1)
+                for (int j = min(k >> 1, from); j > 0; j >>= 1) {
+                    const unsigned long long other = __shfl_xor_sync(0xffffffffu, key, j);
+                    const bool low = ((i & j) == 0) == ((i & k) == 0);
+                    key = (other < key) == low ? other : key;
+                }
+            keys[i] = key;
+        }
+        __syncthreads();
+    };
+    in_warp(2, 32, 16);
+    for (int k = 64; k <= n2; k <<= 1) {
+        for (int j = k >> 1; j >= 32; j >>= 1) {
+            for (int t = threadIdx.x; t < n2 / 2; t += blockDim.x) {
+                const int i = 2 * t - (t & (j - 1)), l = i + j;
+                const unsigned long long a = keys[i], b = keys[l];
+                if ((a > b) == ((i & k) == 0)) {
+                    keys[i] = b;
+                    keys[l] = a;
                 }
             }
             __syncthreads();
         }
+        in_warp(k, k, 16);
     }
+}
+
+// The sum of n terms (not negative) in ascending order, each addition rounded,
+// as a loop over doubles gives it, by one warp.  While the sum s stays within
+// one power of two, adding x adds x rounded to s's unit in the last place: an
+// integer that does not depend on s except where x lies halfway.  So 32 terms
+// become integers, a warp scan sums them, and only a term that is halfway, is
+// larger than s's power of two, carries s past it or is not a normal number is
+// added as a double (about two per power of two of the sum).  The loop over
+// doubles waits some 50 cycles a term for the FP64 pipe: 64 frames of 2,000
+// features took 104 us to assemble and take 51.
+template <bool SQUARES>
+__device__ double bow_sequential_sum(const double* v, int n) {
+    const int lane = threadIdx.x & 31;
+    const unsigned long long one = 1ull << 52, frac = one - 1;
+    const auto load = [&](int i) {
+        if (i >= n) return 0.0;
+        const double x = v[i];
+        return SQUARES ? __dmul_rn(x, x) : fabs(x);
+    };
+    double s = 0.0, next = load(lane);
+    for (int base = 0; base < n; base += 32) {
+        const double x = next;
+        next = load(base + 32 + lane);
+        const unsigned long long xb = __double_as_longlong(x);
+        const int ex = (int)(xb >> 52) & 0x7ff;
+        const unsigned long long mx = (xb & frac) | one;
+        unsigned todo = __ballot_sync(0xffffffffu, x != 0.0);  // a zero changes nothing
+        while (todo) {
+            const unsigned long long sb = __double_as_longlong(s);
+            const int es = (int)(sb >> 52) & 0x7ff;
+            const unsigned long long ms = (sb & frac) | one;
+            const bool mine = (todo >> lane) & 1u;
+            const int d = es - ex;
+            bool alone = ex == 0 || ex == 0x7ff || es == 0 || es == 0x7ff || d < 0;
+            unsigned long long q = 0;
+            if (mine && !alone && d <= 53) {
+                const unsigned long long rest = mx & ((1ull << d) - 1), half = (1ull << d) >> 1;
+                q = (mx >> d) + (rest > half ? 1 : 0);
+                alone = d > 0 && rest == half;
+            }
+            unsigned long long incl = q;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const unsigned long long y = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += y;
+            }
+            const unsigned event = __ballot_sync(0xffffffffu, mine && (alone || ms + incl >= 2 * one));
+            const int f = event ? __ffs(event) - 1 : 31;
+            const unsigned long long add = __shfl_sync(0xffffffffu, event ? incl - q : incl, f);
+            if (add) s = __longlong_as_double((long long)(((unsigned long long)es << 52) | ((ms + add) & frac)));
+            if (!event) break;
+            s = __dadd_rn(s, __shfl_sync(0xffffffffu, x, f));
+            todo &= ~((2u << f) - 1u);
+        }
+    }
+    return s;
 }
 
 // Two blocks per frame (block 2f builds frame f's BowVector, block 2f + 1 its
@@ -107,7 +181,7 @@ __global__ void __launch_bounds__(BOW_ASM_THREADS) k_bow_assemble(
     int* __restrict__ fv_nodes, int* __restrict__ fv_starts, int* __restrict__ fv_sizes,
     int* __restrict__ fv_features) {
     extern __shared__ unsigned long long keys[];
-    __shared__ int s_nkept, s_nruns;
+    __shared__ int s_nkept;
     __shared__ double s_norm;
     // two blocks per frame: pass 0 the BowVector (keys word << 32 | feature),
     // pass 1 the FeatureVector (node << 32 | feature)
@@ -118,7 +192,7 @@ __global__ void __launch_bounds__(BOW_ASM_THREADS) k_bow_assemble(
         if (threadIdx.x == 0) (pass == 0 ? bow_counts : fv_counts)[f] = -1;
         return;
     }
-    int n2 = 1;
+    int n2 = 32;
     while (n2 < n) n2 <<= 1;
     const unsigned long long pad = ~0ull;
     {
@@ -130,10 +204,7 @@ __global__ void __launch_bounds__(BOW_ASM_THREADS) k_bow_assemble(
             }
             keys[i] = key;
         }
-        if (threadIdx.x == 0) {
-            s_nkept = 0;
-            s_nruns = 0;
-        }
+        if (threadIdx.x == 0) s_nkept = 0;
         __syncthreads();
         bow_block_sort(keys, n2);
         // kept features sort first; runs of equal high words are the entries
@@ -144,26 +215,15 @@ __global__ void __launch_bounds__(BOW_ASM_THREADS) k_bow_assemble(
         __syncthreads();
         const int nk = s_nkept;
         // run starts in ascending order: a block-wide exclusive scan of the flags
-        __shared__ int s_warp[BOW_ASM_THREADS / 32];
+        __shared__ int s_scan[BOW_ASM_THREADS / 32];
+        int nruns = 0;
         for (int base = 0; base < nk; base += blockDim.x) {
             const int i = base + threadIdx.x;
             const bool start = i < nk && (i == 0 || (keys[i] >> 32) != (keys[i - 1] >> 32));
-            const unsigned bal = __ballot_sync(0xffffffffu, start);
-            const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-            if (lane == 0) s_warp[w] = __popc(bal);
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                int acc = s_nruns;
-                for (int q = 0; q < (int)(blockDim.x >> 5); q++) {
-                    const int c = s_warp[q];
-                    s_warp[q] = acc;
-                    acc += c;
-                }
-                s_nruns = acc;
-            }
-            __syncthreads();
+            int tot;
+            const int r = nruns + block_exclusive_scan(start ? 1 : 0, s_scan, &tot);
+            nruns += tot;
             if (start) {
-                const int r = s_warp[w] + __popc(bal & ((1u << lane) - 1u));
                 int end = i + 1;
                 while (end < nk && (keys[end] >> 32) == (keys[i] >> 32)) end++;
                 const unsigned hi = (unsigned)(keys[i] >> 32);
@@ -180,9 +240,7 @@ __global__ void __launch_bounds__(BOW_ASM_THREADS) k_bow_assemble(
                     fv_sizes[o0 + r] = end - i;
                 }
             }
-            __syncthreads();
         }
-        const int nruns = s_nruns;
         if (pass == 1) {
             // the features of every node, in feature order (the sort's low words)
             for (int i = threadIdx.x; i < nk; i += blockDim.x) fv_features[o0 + i] = (int)(keys[i] & 0xffffffffull);
@@ -192,18 +250,20 @@ __global__ void __launch_bounds__(BOW_ASM_THREADS) k_bow_assemble(
         // normalisation (ScoringObject.h:84-89: L1 for L1 / chi-square / KL /
         // Bhattacharyya, L2 for L2, none for the dot product, where TF divides
         // by the number of words instead)
-        if (threadIdx.x == 0) {
+        __syncthreads();
+        if (threadIdx.x < 32) {
             double norm = 0.0;
             if (scoring == 5) {
                 norm = (weighting == 0 || weighting == 1) && nruns > 0 ? (double)nruns : 0.0;
             } else if (scoring == 1) {
-                for (int r = 0; r < nruns; r++) norm = __dadd_rn(norm, __dmul_rn(bow_values[o0 + r], bow_values[o0 + r]));
-                norm = __dsqrt_rn(norm);
+                norm = __dsqrt_rn(bow_sequential_sum<true>(bow_values + o0, nruns));
             } else {
-                for (int r = 0; r < nruns; r++) norm = __dadd_rn(norm, fabs(bow_values[o0 + r]));
+                norm = bow_sequential_sum<false>(bow_values + o0, nruns);
             }
-            s_norm = norm;
-            bow_counts[f] = nruns;
+            if (threadIdx.x == 0) {
+                s_norm = norm;
+                bow_counts[f] = nruns;
+            }
         }
         __syncthreads();
         const double norm = s_norm;

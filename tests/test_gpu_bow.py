@@ -273,3 +273,36 @@ def test_search_for_triangulation_vs_oracle(torch, oracle, only_stereo, check_or
         assert np.array_equal(matches[p].cpu().numpy(), ref), p
         total += ref_nm
     assert total > 30
+
+
+@pytest.mark.parametrize("kind", ["random", "integers", "halfway", "spread", "subnormal", "overflow"])
+@pytest.mark.parametrize("n,scoring", [(1, 0), (31, 0), (33, 1), (1025, 0), (8192, 1)])
+def test_bow_values_of_any_weights(torch, kind, n, scoring):
+    """The normalisation is the loop's sum, bit for bit: ties, weights beyond
+    the sum's precision on either side, subnormal and overflowing ones."""
+    from orb_slam2_detailed_comments_gb300 import Vocabulary
+    from orb_slam2_detailed_comments_gb300 import synthetic as syn
+    rng = np.random.default_rng(n + scoring)
+    voc = syn.vocabulary(10, 3, 77)
+    nn = len(voc["weights"])
+    weights = {"random": rng.uniform(0.1, 10, nn),
+               "integers": rng.integers(1, 100, nn).astype(np.float64),
+               "halfway": rng.integers(1, 8, nn) * 2.0 ** rng.integers(-53, -48, nn) + (rng.random(nn) < 0.3),
+               "spread": 2.0 ** rng.uniform(-60, 60, nn),
+               "subnormal": rng.integers(1, 2 ** 52, nn) * 2.0 ** -1074 * 2.0 ** rng.integers(0, 4, nn),
+               "overflow": rng.uniform(0.5, 1, nn) * 2.0 ** rng.integers(1000, 1024, nn)}[kind]
+    V = Vocabulary.from_arrays(10, 3, scoring, 0, voc["parents"], voc["is_leaf"], voc["descriptors"], weights)
+    desc = torch.from_numpy(rng.integers(0, 256, (n, 32), dtype=np.uint8)).cuda()
+    r = {k: v.cpu().numpy() for k, v in V.transform(desc, torch.tensor([0, n], dtype=torch.int32).cuda(), 1).items()}
+    with np.errstate(all="ignore"):
+        values, norm = {}, np.float64(0)
+        for w, x in zip(r["word"], r["weight"]):
+            values[w] = values.get(w, np.float64(0)) + x
+        for w in sorted(values):
+            norm = norm + (values[w] * values[w] if scoring == 1 else values[w])
+        norm = np.sqrt(norm) if scoring == 1 else norm
+        want = np.array([values[w] / norm if norm > 0 else values[w] for w in sorted(values)])
+    m = int(r["bow_counts"][0])
+    assert np.array_equal(r["bow_words"][:m], sorted(values))
+    assert np.array_equal(r["bow_values"][:m].view(np.int64)[~np.isnan(want)], want.view(np.int64)[~np.isnan(want)])
+    assert np.array_equal(np.isnan(r["bow_values"][:m]), np.isnan(want))
