@@ -127,8 +127,8 @@ def search_by_bow(keypoints, descriptors, offsets, bow, kf_mappoints, pairs, nnr
     out_off = np.zeros(len(pr) + 1, np.int32)
     out_off[1:] = np.cumsum(sizes)
     dev = torch.device("cuda")
-    P = torch.from_numpy(pr.reshape(-1).copy()).to(dev)
-    OO = torch.from_numpy(out_off[:-1].copy()).to(dev)
+    both = torch.from_numpy(np.concatenate((pr.reshape(-1), out_off[:-1]))).to(dev)  # one copy
+    P, OO = both[:2 * len(pr)], both[2 * len(pr):]
     match = torch.empty(max(int(out_off[-1]), 1), dtype=torch.int32, device=dev)
     nm = torch.empty(max(len(pr), 1), dtype=torch.int32, device=dev)
     st = torch.cuda.current_stream().cuda_stream if stream is None else int(stream)

@@ -17,6 +17,8 @@
 // times sums its weight c times in sequence (the reference adds them in
 // feature order, and they are equal), and the norm is one sequential sum in
 // ascending word order, as std::map iterates.
+#include <cooperative_groups.h>
+
 #include <algorithm>
 #include <cstdio>
 #include <cstring>
@@ -274,19 +276,30 @@ __global__ void __launch_bounds__(BOW_ASM_THREADS) k_bow_assemble(
 }
 
 // ORBmatcher::SearchByBoW(KeyFrame* pKF, Frame& F, vpMapPointMatches),
-// src/ORBmatcher.cc:247-380, one block per (keyframe, frame) pair.  A frame
-// feature belongs to one FeatureVector node and so does a keyframe feature:
-// the nodes both vectors hold are independent, and one warp takes one node
-// (found by binary search in the keyframe's sorted node list).  Inside a node
-// the keyframe features run in list order, as in the reference: each takes,
-// among the node's frame features not matched yet (a shared bitmap), the
-// first at the least distance, with the second-best over the rest; kept when
-// best <= TH_LOW and best < nnratio * second.  Then the rotation histogram,
-// ComputeThreeMaxima (src/ORBmatcher.cc:2035-2077) and the resets.  With
-// 'keyframes' it is SearchByBoW(KeyFrame* pKF1, KeyFrame* pKF2, vpMatches12)
-// (src/ORBmatcher.cc:729-880): candidates need a map point that is not bad,
-// TH_LOW is exclusive, and the result is per pKF1 feature.
-#define SBB_THREADS 1024
+// src/ORBmatcher.cc:247-380, one cluster of 8 blocks per (keyframe, frame)
+// pair.  A frame feature belongs to one FeatureVector node and so does a
+// keyframe feature: the nodes both vectors hold are independent, and one warp
+// takes one node (found by a 32-way search in the keyframe's sorted node list).
+// Inside a node the keyframe features run in list order, as in the reference:
+// each takes, among the node's frame features not matched yet, the first at
+// the least distance, with the second-best over the rest; kept when
+// best <= TH_LOW and best < nnratio * second.  Then the rotation histogram
+// (block 0's shared memory), ComputeThreeMaxima (src/ORBmatcher.cc:2035-2077)
+// and the resets.  MODE 1 is SearchByBoW(KeyFrame* pKF1, KeyFrame* pKF2,
+// vpMatches12) (src/ORBmatcher.cc:729-880): candidates need a map point that
+// is not bad, TH_LOW is exclusive, and the result is per pKF1 feature.
+// MODE 2: SearchForTriangulation.
+//
+// Bound by latency: a node's features are taken one after the other.  A lane
+// holds two frame features' descriptors (nodes of more than 64 read theirs
+// again for every keyframe feature) and one keyframe feature's, passed round
+// by shuffles, so a turn waits for no memory; a pair's nodes are spread over 8
+// SMs.  32 pairs of 2,000 features: 98 us with a block per pair that read both
+// features from memory every turn, 48 with one frame feature a lane (nodes of
+// more than 32 then set the time), 38 with two.
+#define SBB_THREADS 256
+#define SBB_CLUSTER 8
+#define SBB_HELD 64  // frame features of a node in a warp's registers
 #define SBB_TH_LOW 50
 
 // SearchForTriangulation's per-call constants: pKF2's scale tables (read at
@@ -297,40 +310,47 @@ struct TriangulationDev {
     int only_stereo;
 };
 
+template <int MODE>
 __global__ void __launch_bounds__(SBB_THREADS) k_search_by_bow(
     const orbgpu_keypoint* __restrict__ kps, const uint4* __restrict__ desc, const int* __restrict__ offsets,
     const int* __restrict__ fv_counts, const int* __restrict__ fv_nodes, const int* __restrict__ fv_starts,
     const int* __restrict__ fv_sizes, const int* __restrict__ fv_features, const uint8_t* __restrict__ kf_mp,
-    const int* __restrict__ pairs, float nnratio, int check_ori, int keyframes, const float* __restrict__ pair_params,
-    const float* __restrict__ uright, TriangulationDev tri, const int* __restrict__ out_offsets,
-    int* __restrict__ match_out, int* __restrict__ nmatches) {
-    __shared__ unsigned s_taken[BOW_MAX_FEATURES / 32];
-    __shared__ unsigned char s_bin[BOW_MAX_FEATURES];
-    __shared__ int hist[ORBGPU_HISTO_LENGTH];
+    const int* __restrict__ pairs, float nnratio, int check_ori, const float* __restrict__ pair_params,
+    const float* __restrict__ uright, const __grid_constant__ TriangulationDev tri, const int* __restrict__ out_offsets,
+    int* match_out, int* __restrict__ nmatches) {
+    constexpr bool TRIANG = MODE == 2;
+    __shared__ unsigned s_taken[BOW_MAX_FEATURES / 32];  // of nodes with more than SBB_HELD frame features
+    __shared__ unsigned char s_bin[BOW_MAX_FEATURES];    // block 0's: every match's bin
+    __shared__ int s_hist[32];                           // block 0's
+    __shared__ int s_total[32];
     __shared__ int s_ind[3], s_nm;
-    const int p = blockIdx.x;
+    cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+    const int rank = (int)cluster.block_rank();
+    const int p = blockIdx.x / SBB_CLUSTER;
     const int kf = pairs[2 * p], fr = pairs[2 * p + 1];
     const int ok0 = offsets[kf], of0 = offsets[fr];
     const int kn = offsets[kf + 1] - ok0, frn = offsets[fr + 1] - of0;
     // the output (and bins) are per frame feature, or per first-keyframe
     // feature for two keyframes (vpMatches12)
-    const int fn = keyframes ? kn : frn;
+    const int fn = MODE ? kn : frn;
     const int ckf = fv_counts[kf], cf = fv_counts[fr];
     int* out = match_out + out_offsets[p];
     if (kn < 0 || kn > BOW_MAX_FEATURES || frn < 0 || frn > BOW_MAX_FEATURES || ckf < 0 || cf < 0) {
-        if (threadIdx.x == 0) nmatches[p] = -1;
+        if (rank == 0 && threadIdx.x == 0) nmatches[p] = -1;
         return;
     }
-    for (int i = threadIdx.x; i < fn; i += blockDim.x) out[i] = -1;
-    for (int i = threadIdx.x; i < BOW_MAX_FEATURES / 32; i += blockDim.x) s_taken[i] = 0;
-    if (threadIdx.x < ORBGPU_HISTO_LENGTH) hist[threadIdx.x] = 0;
+    const int first = rank * SBB_THREADS + threadIdx.x;
+    for (int i = first; i < fn; i += SBB_CLUSTER * SBB_THREADS) out[i] = -1;
+    for (int i = threadIdx.x; i < BOW_MAX_FEATURES / 32; i += SBB_THREADS) s_taken[i] = 0;
+    if (threadIdx.x < 32) s_hist[threadIdx.x] = 0;
     if (threadIdx.x == 0) s_nm = 0;
-    __syncthreads();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-    // mode 2: SearchForTriangulation -- F12 (row-major) and the epipole in pKF2
-    const bool triang = keyframes == 2;
+    unsigned char* bins = cluster.map_shared_rank(s_bin, 0);
+    int* hist = cluster.map_shared_rank(s_hist, 0);
+    cluster.sync();
+    const int lane = threadIdx.x & 31;
+    // F12 (row-major) and the epipole in pKF2
     float F[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0}, ex = 0.f, ey = 0.f;
-    if (triang) {
+    if (TRIANG) {
 #pragma unroll
         for (int q = 0; q < 9; q++) F[q] = pair_params[11 * p + q];
         ex = pair_params[11 * p + 9];
@@ -338,109 +358,165 @@ __global__ void __launch_bounds__(SBB_THREADS) k_search_by_bow(
     }
     const float factor = __fdiv_rn((float)ORBGPU_HISTO_LENGTH, 360.0f);
     const unsigned INF = 0x7fffffffu;
-    for (int j = warp; j < cf; j += nwarps) {
+    // neighbouring nodes, which are of like size, go to different SMs
+    for (int j = (threadIdx.x >> 5) * SBB_CLUSTER + rank; j < cf; j += SBB_CLUSTER * SBB_THREADS / 32) {
         const int node = fv_nodes[of0 + j];
-        int lo = 0, hi = ckf - 1, jk = -1;
-        while (lo <= hi) {
-            const int mid = (lo + hi) >> 1;
-            const int v = fv_nodes[ok0 + mid];
-            if (v == node) {
-                jk = mid;
+        int lo = 0, len = ckf, jk = -1;
+        while (len > 0) {
+            const int step = (len + 31) >> 5, at = lane * step;
+            const int v = at < len ? fv_nodes[ok0 + lo + at] : 0x7fffffff;
+            const unsigned same = __ballot_sync(0xffffffffu, at < len && v == node);
+            const int below = __popc(__ballot_sync(0xffffffffu, at < len && v < node));
+            if (same) {
+                jk = lo + (__ffs(same) - 1) * step;
                 break;
             }
-            if (v < node) lo = mid + 1;
-            else hi = mid - 1;
+            if (below == 0) break;
+            const int skip = (below - 1) * step + 1;
+            lo += skip;
+            len = min(step - 1, len - skip);
         }
         if (jk < 0) continue;
         const int* flist = fv_features + fv_starts[of0 + j];
         const int fcount = fv_sizes[of0 + j];
         const int* klist = fv_features + fv_starts[ok0 + jk];
         const int kcount = fv_sizes[ok0 + jk];
-        for (int t = 0; t < kcount; t++) {
-            const int ikf = klist[t];
-            bool st1 = false;
-            float x1 = 0.f, y1 = 0.f, la = 0.f, lb = 0.f, lc = 0.f;
-            if (triang) {
-                // features without a map point (bad or not), stereo ones only with bOnlyStereo
-                if (kf_mp[ok0 + ikf] != 0) continue;
-                st1 = uright[ok0 + ikf] >= 0.0f;
-                if (tri.only_stereo && !st1) continue;
-                x1 = kps[ok0 + ikf].x;
-                y1 = kps[ok0 + ikf].y;
-                // CheckDistEpipolarLine (src/ORBmatcher.cc:205-232): the line of kp1 in pKF2
-                la = __fadd_rn(__fadd_rn(__fmul_rn(x1, F[0]), __fmul_rn(y1, F[3])), F[6]);
-                lb = __fadd_rn(__fadd_rn(__fmul_rn(x1, F[1]), __fmul_rn(y1, F[4])), F[7]);
-                lc = __fadd_rn(__fadd_rn(__fmul_rn(x1, F[2]), __fmul_rn(y1, F[5])), F[8]);
-            } else if (kf_mp[ok0 + ikf] != 1) {
-                continue;
+        // the lane's frame features c + lane and c + 32 + lane
+        int jf[2] = {0, 0};
+        uint4 f0[2], f1[2];
+        bool open[2], st2[2] = {false, false};
+        float x2[2], y2[2], angle2[2] = {0.f, 0.f};
+        int octave2[2];
+        const auto load = [&](int c) {
+#pragma unroll
+            for (int u = 0; u < 2; u++) {
+                open[u] = false;
+                if (c + 32 * u + lane >= fcount) continue;
+                const int i = flist[c + 32 * u + lane];
+                jf[u] = i;
+                if (MODE == 1 && kf_mp[of0 + i] != 1) continue;
+                if (TRIANG) {
+                    st2[u] = uright[of0 + i] >= 0.0f;
+                    if (kf_mp[of0 + i] != 0 || (tri.only_stereo && !st2[u])) continue;
+                    x2[u] = kps[of0 + i].x;
+                    y2[u] = kps[of0 + i].y;
+                    octave2[u] = kps[of0 + i].octave;
+                }
+                open[u] = fcount <= SBB_HELD || !((s_taken[i >> 5] >> (i & 31)) & 1u);
+                f0[u] = __ldg(desc + 2 * (size_t)(of0 + i));
+                f1[u] = __ldg(desc + 2 * (size_t)(of0 + i) + 1);
+                if (check_ori) angle2[u] = kps[of0 + i].angle;
             }
-            const uint4 a0 = desc[2 * (size_t)(ok0 + ikf)], a1 = desc[2 * (size_t)(ok0 + ikf) + 1];
-            unsigned b1 = INF;
-            int b2 = 256;
-            for (int c = 0; c < fcount; c += 32) {
-                unsigned key = INF;
-                int d = 256;
-                if (c + lane < fcount) {
-                    const int jf = flist[c + lane];
-                    const bool free2 = !((s_taken[jf >> 5] >> (jf & 31)) & 1u);
-                    if (triang) {
-                        const bool st2 = uright[of0 + jf] >= 0.0f;
-                        if (free2 && kf_mp[of0 + jf] == 0 && (!tri.only_stereo || st2)) {
-                            const int dd = hamming256(a0, a1, desc[2 * (size_t)(of0 + jf)],
-                                                      desc[2 * (size_t)(of0 + jf) + 1]);
-                            const orbgpu_keypoint k2 = kps[of0 + jf];
-                            bool ok = dd <= SBB_TH_LOW && k2.octave >= 0 && k2.octave < 16;
-                            if (ok && !st1 && !st2) {
-                                const float dx = __fsub_rn(ex, k2.x), dy = __fsub_rn(ey, k2.y);
+        };
+        if (fcount <= SBB_HELD) load(0);
+        for (int t0 = 0; t0 < kcount; t0 += 32) {
+            // the lane's keyframe feature
+            int ik = 0;
+            uint4 k0 = make_uint4(0, 0, 0, 0), k1 = k0;
+            bool use = false, stereo1 = false;
+            float angle1 = 0.f, px = 0.f, py = 0.f;
+            if (t0 + lane < kcount) {
+                ik = klist[t0 + lane];
+                use = kf_mp[ok0 + ik] == (TRIANG ? 0 : 1);
+                if (TRIANG) {
+                    // features without a map point (bad or not), stereo ones only with bOnlyStereo
+                    stereo1 = uright[ok0 + ik] >= 0.0f;
+                    use = use && (!tri.only_stereo || stereo1);
+                    px = kps[ok0 + ik].x;
+                    py = kps[ok0 + ik].y;
+                }
+                if (use) {
+                    k0 = __ldg(desc + 2 * (size_t)(ok0 + ik));
+                    k1 = __ldg(desc + 2 * (size_t)(ok0 + ik) + 1);
+                    if (check_ori) angle1 = kps[ok0 + ik].angle;
+                }
+            }
+            unsigned todo = __ballot_sync(0xffffffffu, use);
+            while (todo) {
+                const int t = __ffs(todo) - 1;
+                todo &= todo - 1;
+                const auto from = [&](unsigned v) { return __shfl_sync(0xffffffffu, v, t); };
+                const uint4 a0 = make_uint4(from(k0.x), from(k0.y), from(k0.z), from(k0.w));
+                const uint4 a1 = make_uint4(from(k1.x), from(k1.y), from(k1.z), from(k1.w));
+                bool st1 = false;
+                float la = 0.f, lb = 0.f, lc = 0.f;
+                if (TRIANG) {
+                    st1 = __shfl_sync(0xffffffffu, (int)stereo1, t) != 0;
+                    const float x1 = __shfl_sync(0xffffffffu, px, t), y1 = __shfl_sync(0xffffffffu, py, t);
+                    // CheckDistEpipolarLine (src/ORBmatcher.cc:205-232): the line of kp1 in pKF2
+                    la = __fadd_rn(__fadd_rn(__fmul_rn(x1, F[0]), __fmul_rn(y1, F[3])), F[6]);
+                    lb = __fadd_rn(__fadd_rn(__fmul_rn(x1, F[1]), __fmul_rn(y1, F[4])), F[7]);
+                    lc = __fadd_rn(__fadd_rn(__fmul_rn(x1, F[2]), __fmul_rn(y1, F[5])), F[8]);
+                }
+                unsigned b1 = INF;
+                int b2 = 256;
+                for (int c = 0; c < fcount; c += SBB_HELD) {
+                    if (fcount > SBB_HELD) load(c);
+                    unsigned key[2] = {INF, INF};
+#pragma unroll
+                    for (int u = 0; u < 2; u++) {
+                        if (!open[u]) continue;
+                        const int dd = hamming256(a0, a1, f0[u], f1[u]);
+                        bool ok = true;
+                        if (TRIANG) {
+                            ok = dd <= SBB_TH_LOW && octave2[u] >= 0 && octave2[u] < 16;
+                            if (ok && !st1 && !st2[u]) {
+                                const float dx = __fsub_rn(ex, x2[u]), dy = __fsub_rn(ey, y2[u]);
                                 if (__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)) <
-                                    __fmul_rn(100.0f, tri.scale[k2.octave]))
+                                    __fmul_rn(100.0f, tri.scale[octave2[u]]))
                                     ok = false;
                             }
                             if (ok) {
-                                const float num = __fadd_rn(__fadd_rn(__fmul_rn(la, k2.x), __fmul_rn(lb, k2.y)), lc);
+                                const float num = __fadd_rn(__fadd_rn(__fmul_rn(la, x2[u]), __fmul_rn(lb, y2[u])), lc);
                                 const float den = __fadd_rn(__fmul_rn(la, la), __fmul_rn(lb, lb));
-                                ok = den != 0.0f &&
-                                     (double)__fdiv_rn(__fmul_rn(num, num), den) <
-                                         __dmul_rn(3.84, (double)tri.sigma2[k2.octave]);
-                            }
-                            if (ok) {
-                                // the last candidate at the least distance wins ("dist > bestDist" skips)
-                                d = dd;
-                                key = ((unsigned)dd << 13) | (unsigned)(8191 - (c + lane));
+                                ok = den != 0.0f && (double)__fdiv_rn(__fmul_rn(num, num), den) <
+                                                        __dmul_rn(3.84, (double)tri.sigma2[octave2[u]]);
                             }
                         }
-                    } else if (free2 && (!keyframes || kf_mp[of0 + jf] == 1)) {
-                        d = hamming256(a0, a1, desc[2 * (size_t)(of0 + jf)], desc[2 * (size_t)(of0 + jf) + 1]);
-                        key = ((unsigned)d << 13) | (unsigned)(c + lane);
+                        // triangulation: the last candidate at the least distance wins ("dist > bestDist" skips)
+                        const int i = c + 32 * u + lane;
+                        if (ok) key[u] = ((unsigned)dd << 13) | (unsigned)(TRIANG ? 8191 - i : i);
+                    }
+                    const unsigned c1 = __reduce_min_sync(0xffffffffu, min(key[0], key[1]));
+                    // a lone group beyond TH_LOW is not taken whatever its second
+                    if (TRIANG || (fcount <= SBB_HELD && c1 >> 13 > SBB_TH_LOW)) {
+                        b1 = min(b1, c1);
+                        continue;
+                    }
+                    const unsigned other = key[0] == c1 ? key[1] : key[1] == c1 ? key[0] : min(key[0], key[1]);
+                    const int c2 = (int)min(__reduce_min_sync(0xffffffffu, other) >> 13, 256u);
+                    if (c1 < b1) {
+                        b2 = min(b1 == INF ? 256 : (int)(b1 >> 13), c2);
+                        b1 = c1;
+                    } else {
+                        b2 = min(b2, c1 == INF ? 256 : (int)(c1 >> 13));
                     }
                 }
-                const unsigned c1 = __reduce_min_sync(0xffffffffu, key);
-                const int c2 = (int)__reduce_min_sync(0xffffffffu, (unsigned)(key == c1 ? 256 : d));
-                if (c1 < b1) {
-                    b2 = min(b1 == INF ? 256 : (int)(b1 >> 13), c2);
-                    b1 = c1;
-                } else {
-                    b2 = min(b2, c1 == INF ? 256 : (int)(c1 >> 13));
-                }
-            }
-            const int best1 = b1 == INF ? 256 : (int)(b1 >> 13);
-            // TH_LOW inclusive for (keyframe, frame), exclusive for two
-            // keyframes; triangulation: any candidate left (no ratio test)
-            const bool take = triang ? b1 != INF
-                                     : (keyframes ? best1 < SBB_TH_LOW : best1 <= SBB_TH_LOW) &&
-                                           (float)best1 < __fmul_rn(nnratio, (float)b2);
-            if (take) {
-                if (lane == 0) {
-                    const int jf = flist[triang ? 8191u - (b1 & 8191u) : (b1 & 8191u)];
-                    atomicOr(&s_taken[jf >> 5], 1u << (jf & 31));
-                    const int slot = keyframes ? ikf : jf;
-                    out[slot] = keyframes ? jf : ikf;  // modes 1 and 2 report per first-keyframe feature
+                const int best1 = b1 == INF ? 256 : (int)(b1 >> 13);
+                // TH_LOW inclusive for (keyframe, frame), exclusive for two
+                // keyframes; triangulation: any candidate left (no ratio test)
+                const bool take = TRIANG ? b1 != INF
+                                         : (MODE ? best1 < SBB_TH_LOW : best1 <= SBB_TH_LOW) &&
+                                               (float)best1 < __fmul_rn(nnratio, (float)b2);
+                if (!take) continue;
+                const int at = (int)(TRIANG ? 8191u - (b1 & 8191u) : b1 & 8191u);
+                const int ikf = __shfl_sync(0xffffffffu, ik, t);
+                const float a = __shfl_sync(0xffffffffu, angle1, t);
+                if (fcount > SBB_HELD) load(at & ~(SBB_HELD - 1));
+                if (lane == (at & 31)) {
+                    const bool second = (at & 32) != 0;
+                    const int i = second ? jf[1] : jf[0];
+                    if (second) open[1] = false;
+                    else open[0] = false;
+                    if (fcount > SBB_HELD) atomicOr(&s_taken[i >> 5], 1u << (i & 31));
+                    const int slot = MODE ? ikf : i;
+                    out[slot] = MODE ? i : ikf;  // modes 1 and 2 report per first-keyframe feature
                     if (check_ori) {
-                        float rot = __fsub_rn(kps[ok0 + ikf].angle, kps[of0 + jf].angle);
+                        float rot = __fsub_rn(a, second ? angle2[1] : angle2[0]);
                         if (rot < 0.0f) rot = __fadd_rn(rot, 360.0f);
                         int bin = (int)roundf(__fmul_rn(rot, factor));
                         if (bin == ORBGPU_HISTO_LENGTH) bin = 0;
-                        s_bin[slot] = (unsigned char)bin;
+                        bins[slot] = (unsigned char)bin;
                         atomicAdd(&hist[bin], 1);
                     }
                 }
@@ -448,13 +524,15 @@ __global__ void __launch_bounds__(SBB_THREADS) k_search_by_bow(
             }
         }
     }
+    cluster.sync();
+    if (threadIdx.x < 32) s_total[threadIdx.x] = hist[threadIdx.x];
     __syncthreads();
     if (threadIdx.x == 0) {
         int ind1 = -1, ind2 = -1, ind3 = -1;
         if (check_ori) {
             int max1 = 0, max2 = 0, max3 = 0;
             for (int b = 0; b < ORBGPU_HISTO_LENGTH; b++) {  // ComputeThreeMaxima, src/ORBmatcher.cc:2035-2077
-                const int sz = hist[b];
+                const int sz = s_total[b];
                 if (sz > max1) {
                     max3 = max2; max2 = max1; max1 = sz;
                     ind3 = ind2; ind2 = ind1; ind1 = b;
@@ -479,10 +557,10 @@ __global__ void __launch_bounds__(SBB_THREADS) k_search_by_bow(
     }
     __syncthreads();
     int kept = 0;
-    for (int i = threadIdx.x; i < fn; i += blockDim.x) {
-        if (out[i] < 0) continue;
+    for (int i = first; i < fn; i += SBB_CLUSTER * SBB_THREADS) {
+        if (__ldcg(out + i) < 0) continue;
         if (check_ori) {
-            const int b = s_bin[i];
+            const int b = bins[i];
             if (b != s_ind[0] && b != s_ind[1] && b != s_ind[2]) {
                 out[i] = -1;
                 continue;
@@ -491,9 +569,9 @@ __global__ void __launch_bounds__(SBB_THREADS) k_search_by_bow(
         kept++;
     }
     kept = __reduce_add_sync(0xffffffffu, kept);
-    if (lane == 0 && kept) atomicAdd(&s_nm, kept);
-    __syncthreads();
-    if (threadIdx.x == 0) nmatches[p] = s_nm;
+    if (lane == 0 && kept) atomicAdd(cluster.map_shared_rank(&s_nm, 0), kept);
+    cluster.sync();
+    if (rank == 0 && threadIdx.x == 0) nmatches[p] = s_nm;
 }
 
 }  // namespace orbgpu
@@ -514,10 +592,21 @@ static int search_by_bow(const orbgpu_keypoint* kps, const uint8_t* desc, const 
         return ORBGPU_ERR_BAD_ARG;
     }
     if (npairs == 0) return ORBGPU_OK;
-    k_search_by_bow<<<npairs, SBB_THREADS, 0, (cudaStream_t)stream>>>(
-        kps, reinterpret_cast<const uint4*>(desc), offsets, fv_counts, fv_nodes, fv_starts, fv_sizes, fv_features,
-        kf_mappoints, pairs, nnratio, check_ori, keyframes, pair_params, uright, tri ? *tri : TriangulationDev{},
-        out_offsets, match_out, nmatches);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)npairs * SBB_CLUSTER);
+    cfg.blockDim = dim3(SBB_THREADS);
+    cfg.stream = (cudaStream_t)stream;
+    cudaLaunchAttribute attr = {};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = SBB_CLUSTER;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    const auto kernel = keyframes == 0 ? k_search_by_bow<0> : keyframes == 1 ? k_search_by_bow<1> : k_search_by_bow<2>;
+    ORBGPU_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, kps, reinterpret_cast<const uint4*>(desc), offsets, fv_counts, fv_nodes,
+                                       fv_starts, fv_sizes, fv_features, kf_mappoints, pairs, nnratio, check_ori,
+                                       pair_params, uright, tri ? *tri : TriangulationDev{}, out_offsets, match_out,
+                                       nmatches));
     ORBGPU_CUDA_TRY(cudaGetLastError());
     return ORBGPU_OK;
 }

@@ -306,3 +306,31 @@ def test_bow_values_of_any_weights(torch, kind, n, scoring):
     assert np.array_equal(r["bow_words"][:m], sorted(values))
     assert np.array_equal(r["bow_values"][:m].view(np.int64)[~np.isnan(want)], want.view(np.int64)[~np.isnan(want)])
     assert np.array_equal(np.isnan(r["bow_values"][:m]), np.isnan(want))
+
+
+@pytest.mark.parametrize("levelsup,nf", [(1, 1500), (3, 1500), (4, 700), (3, 9)])
+@pytest.mark.parametrize("keyframes", [False, True])
+def test_search_by_bow_node_sizes(torch, oracle, levelsup, nf, keyframes):
+    """Nodes from one feature to a whole frame: those of up to 64 frame
+    features stay in a warp's registers, larger ones are read group by group."""
+    from orb_slam2_detailed_comments_gb300 import Vocabulary, search_by_bow
+    from orb_slam2_detailed_comments_gb300 import synthetic as syn
+    voc = syn.vocabulary(10, 4, 5)
+    oracle.vocabulary_from_arrays("sbbn", voc)
+    V = Vocabulary.from_arrays(10, 4, 0, 0, voc["parents"], voc["is_leaf"], voc["descriptors"], voc["weights"])
+    ents = [oracle.extract(f, nfeatures=nf) for f in syn.frame_pair(640, 480, 61)[:2]]
+    ents = [(e.keypoints[:nf], e.descriptors[:nf]) for e in ents]
+    offs = np.array([0, len(ents[0][0]), len(ents[0][0]) + len(ents[1][0])], np.int32)
+    kps, desc = (np.concatenate([e[i] for e in ents]) for i in range(2))
+    mp = np.random.default_rng(6).choice([0, 1, 1, 1, 2], len(kps)).astype(np.uint8)
+    K, D = torch.from_numpy(kps.view(np.float32).reshape(-1, 7).copy()).cuda(), torch.from_numpy(desc).cuda()
+    O = torch.from_numpy(offs).cuda()
+    nm, matches = search_by_bow(K, D, O, V.transform(D, O, levelsup), torch.from_numpy(mp).cuda(), [(0, 1)], 0.9,
+                                keyframes=keyframes)
+    (ka, da), (kb, db) = ents
+    fa, fb = ([r["fv_nodes"], r["fv_offsets"], r["fv_features"]]
+              for r in (oracle.bow_transform("sbbn", d, levelsup) for d in (da, db)))
+    ma, mb = mp[:offs[1]], mp[offs[1]:]
+    ref_nm, ref = (oracle.search_by_bow_kf(ka, da, ma, tuple(fa), kb, db, mb, tuple(fb), 0.9, True) if keyframes else
+                   oracle.search_by_bow(ka, da, ma, tuple(fa), kb, db, tuple(fb), 0.9, True))
+    assert int(nm[0]) == ref_nm and np.array_equal(matches[0].cpu().numpy(), ref)
