@@ -5,10 +5,10 @@
 // The vocabulary tree lives in HBM with every node's children contiguous
 // (grouped by parent in node-id order, the order loadFromTextFile appends
 // them), so one descent level reads the k child descriptors of one node as
-// consecutive 32-byte rows.  k_bow_descend: one thread per feature walks the
+// consecutive 32-byte rows.  k_bow_descend: 8 lanes per feature walk the
 // tree (TemplatedVocabulary.h:1240-1290: at every level the first child with
 // the least Hamming distance, strict <; the node of level L - levelsup kept
-// for the feature vector; stop at a node without children) and writes the
+// for the feature vector; stop at a node without children) and write the
 // word, its weight and that node.  k_bow_assemble: two blocks per frame sort
 // the kept features (weight > 0) by word and by node in shared memory and
 // writes BowVector (BowVector::addWeight / addIfNotExist, then normalize,
@@ -32,10 +32,9 @@
 struct orbgpu_vocabulary {
     int k, L, scoring, weighting, nnodes, nwords;
     uint4* child_desc;   // one 32-byte row per non-root node, grouped by parent
-    int* child_start;    // nnodes + 1: children of node p at positions [child_start[p], child_start[p + 1])
-    int* pos_node;       // node id at each position
-    int* node_word;      // word id of every node (0 where none, as DBoW2's Node default)
+    int4* child_info;    // per position: node id, its children's positions [y, z), word id (0 where none, as DBoW2's Node)
     double* node_weight;
+    int root_end;        // the root's children are positions [0, root_end)
 };
 
 namespace orbgpu {
@@ -44,39 +43,57 @@ namespace orbgpu {
 #define BOW_ASM_THREADS 1024
 #define BOW_MAX_FEATURES 8192  // per frame (the assembly sorts a frame in shared memory)
 
+// Bound by the latency of the levels (two dependent loads each) and by POPC.
+// A lane takes half a child's row, so the 8 lanes of a feature read 4
+// children's 128 bytes at once; a thread per feature touched 32 lines with
+// every load, and asked three arrays for a node where child_info is one load
+// (128,000 features in ten children and six levels: 48 -> 40 us).
 __global__ void __launch_bounds__(BOW_THREADS) k_bow_descend(const uint4* __restrict__ desc, const int* __restrict__ offsets,
                                                              int nframes, const uint4* __restrict__ child_desc,
-                                                             const int* __restrict__ child_start,
-                                                             const int* __restrict__ pos_node,
-                                                             const int* __restrict__ node_word,
+                                                             const int4* __restrict__ child_info, int root_end,
                                                              const double* __restrict__ node_weight, int nid_level,
                                                              int* __restrict__ word_out, double* __restrict__ weight_out,
                                                              int* __restrict__ node_out) {
     const int first = __ldg(offsets), last = __ldg(offsets + nframes);
     if (first < 0) return;
-    for (int i = first + blockIdx.x * BOW_THREADS + threadIdx.x; i < last; i += gridDim.x * BOW_THREADS) {
-        const uint4 f0 = __ldg(desc + 2 * (size_t)i), f1 = __ldg(desc + 2 * (size_t)i + 1);
-        int node = 0, level = 0, nid = 0;
-        int s = __ldg(child_start), e = __ldg(child_start + 1);
-        while (s < e) {
+    const int l = threadIdx.x & 7;
+    const unsigned group = 0xffu << (threadIdx.x & 24);
+    for (int i = first + (blockIdx.x * BOW_THREADS + threadIdx.x) / 8; i < last; i += gridDim.x * (BOW_THREADS / 8)) {
+        const uint4 f = __ldg(desc + 2 * (size_t)i + (l & 1));
+        int4 at = make_int4(0, 0, root_end, 0);  // the root
+        int level = 0, nid = 0;
+        while (at.y < at.z) {
             ++level;
-            int best = s;
-            int best_d = hamming256(f0, f1, __ldg(child_desc + 2 * (size_t)s), __ldg(child_desc + 2 * (size_t)s + 1));
-            for (int p = s + 1; p < e; p++) {
-                const int d = hamming256(f0, f1, __ldg(child_desc + 2 * (size_t)p), __ldg(child_desc + 2 * (size_t)p + 1));
-                if (d < best_d) {
+            int best_d = 512, best = 0;
+            for (int c0 = at.y; c0 < at.z; c0 += 4) {
+                const int c = c0 + (l >> 1);
+                int d = 0;
+                if (c < at.z) {
+                    const uint4 r = __ldg(child_desc + 2 * (size_t)c + (l & 1));
+                    d = __popc(f.x ^ r.x) + __popc(f.y ^ r.y) + __popc(f.z ^ r.z) + __popc(f.w ^ r.w);
+                }
+                d += __shfl_xor_sync(group, d, 1);
+                if (c < at.z && d < best_d) {
                     best_d = d;
-                    best = p;
+                    best = c;
                 }
             }
-            node = __ldg(pos_node + best);
-            if (level == nid_level) nid = node;
-            s = __ldg(child_start + node);
-            e = __ldg(child_start + node + 1);
+#pragma unroll
+            for (int o = 2; o <= 4; o <<= 1) {
+                const int d = __shfl_xor_sync(group, best_d, o), c = __shfl_xor_sync(group, best, o);
+                if (d < best_d || (d == best_d && c < best)) {
+                    best_d = d;
+                    best = c;
+                }
+            }
+            at = __ldg(child_info + best);
+            if (level == nid_level) nid = at.x;
         }
-        word_out[i] = __ldg(node_word + node);
-        weight_out[i] = __ldg(node_weight + node);
-        node_out[i] = nid;
+        if (l == 0) {
+            word_out[i] = at.w;
+            weight_out[i] = __ldg(node_weight + at.x);
+            node_out[i] = nid;
+        }
     }
 }
 
@@ -651,18 +668,19 @@ extern "C" int orbgpu_vocabulary_create(int k, int L, int scoring, int weighting
     }
     std::vector<int> start(nnodes + 1, 0);
     for (int p = 0; p < nnodes; p++) start[p + 1] = start[p] + count[p + 1];
-    std::vector<int> fill(start.begin(), start.end() - 1), pos_node(std::max(nc, 1));
+    std::vector<int> fill(start.begin(), start.end() - 1), word(nnodes, 0);
+    std::vector<int4> info(std::max(nc, 1));
     std::vector<uint8_t> cdesc((size_t)std::max(nc, 1) * 32);
-    std::vector<int> word(nnodes, 0);
     std::vector<double> w(nnodes, 0.0);
     int nwords = 0;
     for (int i = 0; i < nc; i++) {
         const int node = i + 1, pos = fill[parents[i]]++;
-        pos_node[pos] = node;
+        info[pos] = make_int4(node, start[node], start[node + 1], 0);
         std::memcpy(&cdesc[(size_t)pos * 32], descriptors + (size_t)i * 32, 32);
         w[node] = weights[i];
         if (is_leaf[i]) word[node] = nwords++;
     }
+    for (int4& c : info) c.w = word[c.x];
     orbgpu_vocabulary* v = new orbgpu_vocabulary();
     v->k = k;
     v->L = L;
@@ -671,17 +689,14 @@ extern "C" int orbgpu_vocabulary_create(int k, int L, int scoring, int weighting
     v->nnodes = nnodes;
     v->nwords = nwords;
     v->child_desc = nullptr;
-    v->child_start = v->pos_node = v->node_word = nullptr;
+    v->child_info = nullptr;
+    v->root_end = start[1];
     v->node_weight = nullptr;
     cudaError_t e = cudaMalloc(&v->child_desc, cdesc.size());
-    if (e == cudaSuccess) e = cudaMalloc(&v->child_start, sizeof(int) * (nnodes + 1));
-    if (e == cudaSuccess) e = cudaMalloc(&v->pos_node, sizeof(int) * pos_node.size());
-    if (e == cudaSuccess) e = cudaMalloc(&v->node_word, sizeof(int) * nnodes);
+    if (e == cudaSuccess) e = cudaMalloc(&v->child_info, sizeof(int4) * info.size());
     if (e == cudaSuccess) e = cudaMalloc(&v->node_weight, sizeof(double) * nnodes);
     if (e == cudaSuccess) e = cudaMemcpy(v->child_desc, cdesc.data(), cdesc.size(), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(v->child_start, start.data(), sizeof(int) * (nnodes + 1), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(v->pos_node, pos_node.data(), sizeof(int) * pos_node.size(), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(v->node_word, word.data(), sizeof(int) * nnodes, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemcpy(v->child_info, info.data(), sizeof(int4) * info.size(), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(v->node_weight, w.data(), sizeof(double) * nnodes, cudaMemcpyHostToDevice);
     if (e != cudaSuccess) {
         orbgpu_vocabulary_destroy(v);
@@ -742,9 +757,7 @@ extern "C" int orbgpu_vocabulary_destroy(orbgpu_vocabulary* v) {
     // tree is freed
     cudaDeviceSynchronize();
     cudaFree(v->child_desc);
-    cudaFree(v->child_start);
-    cudaFree(v->pos_node);
-    cudaFree(v->node_word);
+    cudaFree(v->child_info);
     cudaFree(v->node_weight);
     delete v;
     return ORBGPU_OK;
@@ -779,8 +792,8 @@ extern "C" int orbgpu_bow_transform(const orbgpu_vocabulary* v, const uint8_t* d
     ORBGPU_CUDA_TRY(allow_max_dynamic_smem(k_bow_assemble));
     const int blocks = nsm_of_current_device() * 8;
     k_bow_descend<<<blocks, BOW_THREADS, 0, st>>>(reinterpret_cast<const uint4*>(desc), offsets, nframes,
-                                                  v->child_desc, v->child_start, v->pos_node, v->node_word,
-                                                  v->node_weight, v->L - levelsup, word_ids, weights, node_ids);
+                                                  v->child_desc, v->child_info, v->root_end, v->node_weight,
+                                                  v->L - levelsup, word_ids, weights, node_ids);
     ORBGPU_CUDA_TRY(cudaGetLastError());
     k_bow_assemble<<<2 * nframes, BOW_ASM_THREADS, BOW_MAX_FEATURES * 8, st>>>(
         offsets, word_ids, weights, node_ids, v->weighting, v->scoring, bow_counts, bow_words, bow_values, fv_counts,
