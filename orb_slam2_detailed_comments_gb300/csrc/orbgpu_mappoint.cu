@@ -10,20 +10,28 @@
 // obs_rows, each entry a row of a descriptor pool (the keyframes' descriptor
 // matrices, resident in HBM), -1 for an observation of a bad keyframe.
 //
-// One warp takes 4 consecutive map points.  A map point with at most 8, 16 or
-// 32 observations goes to a lane group of that width (4, 2 or 1 map points per
-// pass), each lane holding one observation's descriptor; the group's
-// descriptors sit in shared memory.  In groups of 8 and 16 every lane computes
-// the distances to the next G/2 lanes of its group (cyclically) and receives
-// the other half from the lanes before it (distances are symmetric), then
-// sorts its row with a bitonic network and reads element k.  In a group of 32
-// every lane computes its whole row (up to the list length, in chunks of 8)
-// as 16-bit pairs and finds element k by binary lifting over the distance
-// range 0..256.  The
-// group's minimum of (median, lane) is the reference's first least median.
+// One warp takes 4 to 32 consecutive map points, a lane each for their list's
+// bounds.  Lists of one or two need no distances: every median is the own 0,
+// so the lane keeps its first valid observation.  The others go to lane groups
+// of 4, 8, 16 or 32, the smallest that holds the list, each lane holding one
+// observation's descriptor; the lists of a group's width are numbered over
+// the warp's map points, so that a pass takes 8, 4, 2 or 1 of them and only
+// the last is not full.  The group's descriptors sit in shared memory.  In
+// groups up to 16 every lane computes the distances to the next G/2 lanes of
+// its group (cyclically) and receives the other half from the lanes before it
+// (distances are symmetric), then sorts its row with Batcher's odd-even
+// network and reads element k.  In a group of 32 the cycle is the list's own
+// length, and element k is found by binary lifting over the distance range
+// 0..256 on 16-bit pairs.  The group's minimum of (median, lane) is the
+// reference's first least median.
 // Longer lists (more than 32 observations) run one map point per warp: rows
 // in chunks of 32 lanes, each row's median from two histogram passes (d >> 4,
 // then d & 15 inside the coarse bin) in lane-private shared-memory columns.
+//
+// Bound by issue: the distances are a tenth of the instructions, the rest is
+// lanes without an observation, sorts and bookkeeping (fixed groups of 4
+// map points, without the width of 4, took 261 instructions a map point).  A
+// million map points of 6 observations 463 -> 343 us, of 3 187 -> 89.
 #include <algorithm>
 
 #include "orbgpu_host.h"
@@ -31,7 +39,6 @@
 namespace orbgpu {
 
 #define DD_WARPS 8          // warps per block
-#define DD_MPW 4            // map points a warp takes per iteration
 #ifndef DD_BLOCKS_PER_SM
 #define DD_BLOCKS_PER_SM 4  // resident blocks per SM (64 registers x 256 threads)
 #endif
@@ -43,24 +50,26 @@ struct DDArgs {
     const int* rows;     // n_obs
     int n_obs;
     int m;
+    int per_warp;  // map points a warp takes per iteration (4 to 32)
     int* best;   // m
     uint4* out;  // m x 32 bytes, or null
 };
 
 struct DDShared {
     uint4 desc[DD_WARPS][2][32];  // one warp's staged descriptors (low, high halves)
+    unsigned char order[DD_WARPS][32];  // lanes of the lists of one width, in order
     int hist[DD_WARPS][17][32];   // lane-private histogram columns (long lists)
 };
 
 #define DD_FULL 0xffffffffu
 
-// Element k of a row of 32 distances held as 16-bit pairs (p[i] = d[2i] |
-// d[2i+1] << 16): the smallest v in 0..256 with #{j : d[j] <= v} > k, by
-// binary lifting.  Per pair, (0x8000 + v) - d stays within its half (d <= 512,
-// v <= 511) and has bit 15 set exactly when d <= v; dp2a adds the two flags.
-// Entries of absent or skipped observations hold 512 and never count; the
-// pairs of chunks past jmax are all such entries.
-__device__ __forceinline__ int dd_row_rank32(const unsigned (&p)[16], int k, int jmax) {
+// Element k of a row whose distances, the own 0 apart, are held as 16-bit
+// pairs: the smallest v in 0..256 with 1 + #{d <= v} > k, by binary lifting.
+// Per pair, (0x8000 + v) - d stays within its half (d <= 512, v <= 511) and
+// has bit 15 set exactly when d <= v; dp2a adds the two flags.  Entries of
+// absent or skipped observations hold 512 and never count; the pairs from
+// 'pairs' on are all such entries.
+__device__ __forceinline__ int dd_row_rank(const unsigned (&p)[16], int k, int pairs) {
     int lo = 0;
 #pragma unroll 1
     for (int step = 256; step >= 1; step >>= 1) {
@@ -69,33 +78,29 @@ __device__ __forceinline__ int dd_row_rank32(const unsigned (&p)[16], int k, int
         unsigned acc = 0;
 #pragma unroll
         for (int ic = 0; ic < 16; ic += 4) {
-            if (2 * ic >= jmax) break;
+            if (ic >= pairs) break;
 #pragma unroll
             for (int i = ic; i < ic + 4; i++) acc = __dp2a_lo((v2 - p[i]) & 0x80008000u, 0x0101u, acc);
         }
-        if ((int)(acc >> 15) <= k) lo += step;
+        if ((int)(acc >> 15) < k) lo += step;
     }
     return lo;
 }
 
-// Ascending bitonic sorting network over G registers.
-template <int G>
+// Ascending sort of G registers: Batcher's odd-even merge sort (5, 19 and 63
+// exchanges for 4, 8 and 16; a bitonic network has 6, 24 and 80).
+template <int G, int P = 1, int K = 1>
 __device__ __forceinline__ void dd_sort(int (&d)[G]) {
 #pragma unroll
-    for (int k = 2; k <= G; k <<= 1) {
-#pragma unroll
-        for (int j = k >> 1; j > 0; j >>= 1) {
-#pragma unroll
-            for (int i = 0; i < G; i++) {
-                const int l = i ^ j;
-                if (l > i) {
-                    const int lo = min(d[i], d[l]), hi = max(d[i], d[l]);
-                    d[i] = (i & k) == 0 ? lo : hi;
-                    d[l] = (i & k) == 0 ? hi : lo;
-                }
-            }
+    for (int x = K % P; x + K < G; x++) {
+        if ((x - K % P) % (2 * K) < K && x / (2 * P) == (x + K) / (2 * P)) {
+            const int lo = min(d[x], d[x + K]), hi = max(d[x], d[x + K]);
+            d[x] = lo;
+            d[x + K] = hi;
         }
     }
+    if constexpr (K > 1) dd_sort<G, P, K / 2>(d);
+    else if constexpr (2 * P < G) dd_sort<G, 2 * P, 2 * P>(d);
 }
 
 __device__ __forceinline__ void dd_store(const DDArgs& a, int mp, int row, uint4 d0, uint4 d1) {
@@ -106,27 +111,24 @@ __device__ __forceinline__ void dd_store(const DDArgs& a, int mp, int row, uint4
     }
 }
 
-// The map points of 'mask' (bit g = map point base + g, every list 1..G long)
-// in lane groups of width G.  off: lane g (g <= 4) holds obs_offsets[base + g].
+// The lists of the lanes of 'mask' (all of 1..G observations from o0) in lane
+// groups of width G; lane g's map point is base + g.
 template <int G>
-__device__ __forceinline__ void dd_group_pass(const DDArgs& a, uint4 (*sd)[32], int lane, int base, int off, unsigned mask) {
+__device__ __forceinline__ void dd_group_pass(const DDArgs& a, uint4 (*sd)[32], unsigned char* order, int lane, int base,
+                                              int o0_own, int n_own, unsigned mask) {
     constexpr int NG = 32 / G;
     const int grp = lane / G, l = lane % G;
     const unsigned gmask = G == 32 ? DD_FULL : ((1u << G) - 1u);
-    while (mask) {
-        // group k takes the k-th map point left in the mask
-        int g = -1;
-        unsigned mm = mask;
-#pragma unroll
-        for (int k = 0; k < NG; k++) {
-            if (k == grp && mm) g = __ffs(mm) - 1;
-            if (mm) mm &= mm - 1;
-        }
-        mask = mm;
+    const int count = __popc(mask);
+    __syncwarp();
+    if ((mask >> lane) & 1u) order[__popc(mask & ((1u << lane) - 1u))] = (unsigned char)lane;
+    __syncwarp();
+    for (int q = 0; q < count; q += NG) {
+        const int g = q + grp < count ? order[q + grp] : -1;
         const int gs = g < 0 ? 0 : g;
-        const int o0 = __shfl_sync(DD_FULL, off, gs);
-        const int o1 = __shfl_sync(DD_FULL, off, gs + 1);
-        const int n = g < 0 ? 0 : o1 - o0;
+        const int o0 = __shfl_sync(DD_FULL, o0_own, gs);
+        const int n_of = __shfl_sync(DD_FULL, n_own, gs);
+        const int n = g < 0 ? 0 : n_of;
         int r = -1;
         if (l < n) r = __ldg(a.rows + o0 + l);
         const bool valid = r >= 0 && r < a.pool_rows;
@@ -167,24 +169,27 @@ __device__ __forceinline__ void dd_group_pass(const DDArgs& a, uint4 (*sd)[32], 
 #pragma unroll
             for (int i = 1; i < G / 2; i++) median = i == k ? d[i] : median;
         } else {
-            const int jmax = __reduce_max_sync(DD_FULL, n);
+            // step t + 1: the distances to the lanes t + 1 after and before, cyclically over the list
+            const int pairs = n >> 1;
             unsigned p[16];
 #pragma unroll
-            for (int jc = 0; jc < 32; jc += 8) {
+            for (int tc = 0; tc < 16; tc += 4) {
 #pragma unroll
-                for (int i = jc / 2; i < jc / 2 + 4; i++) p[i] = 512u * 0x10001u;
-                if (jc < jmax) {
+                for (int t = tc; t < tc + 4; t++) p[t] = 512u * 0x10001u;
+                if (tc < pairs) {
 #pragma unroll
-                    for (int j = jc; j < jc + 8; j += 2) {
-                        const int h0 = hamming256(d0, d1, sd[0][j], sd[1][j]);
-                        const int h1 = hamming256(d0, d1, sd[0][j + 1], sd[1][j + 1]);
-                        const unsigned e0 = (gv >> j) & 1u ? (unsigned)h0 : 512u;
-                        const unsigned e1 = (gv >> (j + 1)) & 1u ? (unsigned)h1 : 512u;
-                        p[j / 2] = e0 | (e1 << 16);
+                    for (int t = tc; t < tc + 4; t++) {
+                        const int up = l + t + 1 - (l + t + 1 >= n ? n : 0), down = l - t - 1 + (l - t - 1 < 0 ? n : 0);
+                        const int h = hamming256(d0, d1, sd[0][up & 31], sd[1][up & 31]);
+                        const int hd = __shfl_sync(DD_FULL, h, down & 31);
+                        const bool in = 2 * (t + 1) <= n;  // at 2 (t + 1) = n both are the same lane
+                        const unsigned e0 = in && ((gv >> (up & 31)) & 1u) ? (unsigned)h : 512u;
+                        const unsigned e1 = in && 2 * (t + 1) < n && ((gv >> (down & 31)) & 1u) ? (unsigned)hd : 512u;
+                        p[t] = e0 | (e1 << 16);
                     }
                 }
             }
-            median = dd_row_rank32(p, k, jmax);
+            median = dd_row_rank(p, k, pairs);
         }
         int key = valid ? (median << 5) | l : 0x7fffffff;
 #pragma unroll
@@ -289,38 +294,38 @@ __device__ __forceinline__ void dd_long_list(const DDArgs& a, uint4 (*sd)[32], i
 __global__ void __launch_bounds__(DD_WARPS * 32, DD_BLOCKS_PER_SM) k_distinctive_descriptors(const __grid_constant__ DDArgs a) {
     __shared__ DDShared sh;
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int stride = gridDim.x * DD_WARPS * DD_MPW;
-    for (int base = (blockIdx.x * DD_WARPS + w) * DD_MPW; base < a.m; base += stride) {
-        int off = 0;
-        if (lane <= DD_MPW && base + lane <= a.m) off = __ldg(a.offsets + base + lane);
-        unsigned c8 = 0, c16 = 0, c32 = 0, clong = 0;
-#pragma unroll
-        for (int g = 0; g < DD_MPW; g++) {
-            const int o0 = __shfl_sync(DD_FULL, off, g), o1 = __shfl_sync(DD_FULL, off, g + 1);
-            if (base + g >= a.m) continue;
-            const int n = o1 - o0;
+    const int per = a.per_warp, stride = gridDim.x * DD_WARPS * per;
+    for (int base = (blockIdx.x * DD_WARPS + w) * per; base < a.m; base += stride) {
+        const bool mine = lane < per && base + lane < a.m;
+        int o0 = 0, n = 0;
+        if (mine) {
+            o0 = __ldg(a.offsets + base + lane);
+            const int o1 = __ldg(a.offsets + base + lane + 1);
+            n = o1 - o0;
             if (o0 < 0 || n < 0 || o1 > a.n_obs) {
-                if (lane == 0) a.best[base + g] = -2;
-            } else if (n == 0) {
-                if (lane == 0) a.best[base + g] = -1;
-            } else if (n <= 8) {
-                c8 |= 1u << g;
-            } else if (n <= 16) {
-                c16 |= 1u << g;
-            } else if (n <= 32) {
-                c32 |= 1u << g;
-            } else {
-                clong |= 1u << g;
+                a.best[base + lane] = -2;
+                n = 0;
+            } else if (n <= 2) {
+                const int r0 = n > 0 ? __ldg(a.rows + o0) : -1, r1 = n > 1 ? __ldg(a.rows + o0 + 1) : -1;
+                const int r = r0 >= 0 ? r0 : r1;
+                if (r0 < -1 || r0 >= a.pool_rows || r1 < -1 || r1 >= a.pool_rows) a.best[base + lane] = -2;
+                else if (r < 0) a.best[base + lane] = -1;
+                else dd_store(a, base + lane, r, __ldg(a.pool + 2 * (size_t)r), __ldg(a.pool + 2 * (size_t)r + 1));
             }
         }
-        if (c8) dd_group_pass<8>(a, sh.desc[w], lane, base, off, c8);
-        if (c16) dd_group_pass<16>(a, sh.desc[w], lane, base, off, c16);
-        if (c32) dd_group_pass<32>(a, sh.desc[w], lane, base, off, c32);
+        __syncwarp();
+        const unsigned c4 = __ballot_sync(DD_FULL, n > 2 && n <= 4), c8 = __ballot_sync(DD_FULL, n > 4 && n <= 8);
+        const unsigned c16 = __ballot_sync(DD_FULL, n > 8 && n <= 16), c32 = __ballot_sync(DD_FULL, n > 16 && n <= 32);
+        unsigned clong = __ballot_sync(DD_FULL, n > 32);
+        if (c4) dd_group_pass<4>(a, sh.desc[w], sh.order[w], lane, base, o0, n, c4);
+        if (c8) dd_group_pass<8>(a, sh.desc[w], sh.order[w], lane, base, o0, n, c8);
+        if (c16) dd_group_pass<16>(a, sh.desc[w], sh.order[w], lane, base, o0, n, c16);
+        if (c32) dd_group_pass<32>(a, sh.desc[w], sh.order[w], lane, base, o0, n, c32);
         while (clong) {
             const int g = __ffs(clong) - 1;
             clong &= clong - 1;
-            const int o0 = __shfl_sync(DD_FULL, off, g), o1 = __shfl_sync(DD_FULL, off, g + 1);
-            dd_long_list(a, sh.desc[w], sh.hist[w], lane, base + g, o0, o1 - o0);
+            const int of = __shfl_sync(DD_FULL, o0, g), nf = __shfl_sync(DD_FULL, n, g);
+            dd_long_list(a, sh.desc[w], sh.hist[w], lane, base + g, of, nf);
         }
     }
 }
@@ -352,9 +357,12 @@ extern "C" int orbgpu_distinctive_descriptors(const uint8_t* pool, int pool_rows
     a.m = m;
     a.best = best_rows;
     a.out = reinterpret_cast<uint4*>(descriptors);
-    const long long per_block = DD_WARPS * DD_MPW;
-    const long long want = (m + per_block - 1) / per_block;
-    const int blocks = (int)std::min<long long>(want, (long long)nsm_of_current_device() * DD_BLOCKS_PER_SM);
+    // as many map points per warp (fuller groups) as leave every resident warp some
+    const int resident = nsm_of_current_device() * DD_BLOCKS_PER_SM;
+    a.per_warp = 4;
+    while (a.per_warp < 32 && (long long)a.per_warp * 2 * resident * DD_WARPS <= m) a.per_warp *= 2;
+    const long long per_block = (long long)DD_WARPS * a.per_warp;
+    const int blocks = (int)std::min<long long>((m + per_block - 1) / per_block, resident);
     k_distinctive_descriptors<<<blocks, DD_WARPS * 32, 0, (cudaStream_t)stream>>>(a);
     ORBGPU_CUDA_TRY(cudaGetLastError());
     return ORBGPU_OK;

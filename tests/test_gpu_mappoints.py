@@ -114,3 +114,18 @@ def test_full_size_sampled_against_oracle(torch, oracle):
     sub_rows = np.concatenate([rows[offsets[i]:offsets[i + 1]] for i in idx]).astype(np.int32)
     ob, _ = oracle.distinctive_descriptors(pool, sub_off, sub_rows)
     assert np.array_equal(best[idx], ob)
+
+
+@pytest.mark.parametrize("copies", [140, 290, 580, 1130, 4520])
+def test_lists_per_warp(torch, oracle, copies):
+    """Lengths 0..34 mixed, at every number of map points a warp takes (4 to 32 on 152 SMs)."""
+    rng = np.random.default_rng(copies)
+    lens = rng.permutation(np.repeat(np.arange(35), copies))
+    offsets = np.zeros(len(lens) + 1, np.int32)
+    offsets[1:] = np.cumsum(lens)
+    pool = rng.integers(0, 256, (500, 32), dtype=np.uint8) & np.uint8(0x13)
+    rows = rng.integers(-1, 500, int(offsets[-1])).astype(np.int32)
+    init = rng.integers(0, 256, (len(lens), 32), dtype=np.uint8)
+    best, desc = run(torch, pool, offsets, rows, init)
+    ob, od = oracle.distinctive_descriptors(pool, offsets, rows, init)
+    assert np.array_equal(best, ob) and np.array_equal(desc, od)
