@@ -250,13 +250,14 @@ __device__ __forceinline__ void dd_long_list(const DDArgs& a, uint4 (*sd)[32], i
                 sd[1][lane] = b1;
                 __syncwarp();
                 if (vi) {
-                    unsigned todo = vj;
-                    while (todo) {
-                        const int jj = __ffs(todo) - 1;
-                        todo &= todo - 1;
+                    const int jn = min(32, n - jc);
+#pragma unroll 2
+                    for (int jj = 0; jj < jn; jj++) {
+                        if (!((vj >> jj) & 1u)) continue;
                         const int d = hamming256(m0, m1, sd[0][jj], sd[1][jj]);
-                        if (pass == 0) hist[d >> 4][lane]++;
-                        else if ((d >> 4) == coarse) hist[d & 15][lane]++;
+                        // an atomic without a result: the next distance does not wait for the count
+                        if (pass == 0) atomicAdd(&hist[d >> 4][lane], 1);
+                        else if ((d >> 4) == coarse) atomicAdd(&hist[d & 15][lane], 1);
                     }
                 }
             }
