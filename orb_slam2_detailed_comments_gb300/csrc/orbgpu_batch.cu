@@ -1489,13 +1489,10 @@ struct StereoPair {
 
 __global__ void __launch_bounds__(STEREO_INDEX_THREADS) k_bstereo_index(const orbgpu_keypoint* kps, const int* counts,
                                                                         int cap, const StereoPair* pairs, int* start,
-                                                                        uint4* recs, int* done, int* status) {
+                                                                        uint4* recs, int* status) {
     const StereoPair& P = pairs[blockIdx.x];
     const size_t p = blockIdx.x;
-    if (threadIdx.x == 0) {
-        done[p] = 0;
-        if (p == 0) *status = 0;
-    }
+    if (p == 0 && threadIdx.x == 0) *status = 0;
     stereo_index_block(kps + (size_t)P.right * cap, min(counts[P.right], cap), P.lv.nlevels, P.nRows,
                        start + p * (ORBGPU_MAX_DIM + 1), recs + p * cap);
 }
@@ -1503,12 +1500,19 @@ __global__ void __launch_bounds__(STEREO_INDEX_THREADS) k_bstereo_index(const or
 __global__ void __launch_bounds__(32 * STEREO_WARPS) k_bstereo_match(const orbgpu_keypoint* kps, const uint8_t* desc,
                                                                      const int* counts, int cap, const StereoPair* pairs,
                                                                      const int* start, const uint4* recs, float* uright,
-                                                                     float* depth, int* sad, int* done, int* status) {
+                                                                     float* depth, int* sad, int* status) {
     const StereoPair& P = pairs[blockIdx.y];
+    const int iL = blockIdx.x * STEREO_WARPS + (threadIdx.x >> 5);
+    if (iL >= min(counts[P.left], cap)) return;
     const size_t p = blockIdx.y, l0 = (size_t)P.left * cap, r0 = (size_t)P.right * cap;
-    stereo_match_block(blockIdx.x * STEREO_WARPS, min(counts[P.left], cap), kps + l0, desc + 32 * l0, desc + 32 * r0,
-                       P.lv, P.nRows, start + p * (ORBGPU_MAX_DIM + 1), recs + p * cap, P.bf, P.fx, uright + p * cap,
-                       depth + p * cap, sad + p * cap, done + p, status);
+    stereo_match_warp(iL, kps + l0, desc + 32 * l0, desc + 32 * r0, P.lv, P.nRows, start + p * (ORBGPU_MAX_DIM + 1),
+                      recs + p * cap, P.bf, P.fx, uright + p * cap, depth + p * cap, sad + p * cap, status);
+}
+
+__global__ void __launch_bounds__(STEREO_INDEX_THREADS) k_bstereo_median(const int* counts, int cap, const StereoPair* pairs,
+                                                                         const int* sad, float* uright, float* depth) {
+    const size_t p = blockIdx.x;
+    stereo_median_block(min(counts[pairs[p].left], cap), sad + p * cap, uright + p * cap, depth + p * cap);
 }
 
 }  // namespace orbgpu
@@ -1556,7 +1560,7 @@ extern "C" int orbgpu_batch_compute_stereo_matches(orbgpu_batch* b, const orbgpu
         P.fx = fx[p];
     }
     cudaStream_t st = b->stream;
-    const size_t need = sizeof(StereoPair) * npairs + sizeof(int) * (size_t)npairs * (ORBGPU_MAX_DIM + 2 + cap) +
+    const size_t need = sizeof(StereoPair) * npairs + sizeof(int) * (size_t)npairs * (ORBGPU_MAX_DIM + 1 + cap) +
                         sizeof(uint4) * (size_t)npairs * cap + 16 * 256;
     if (need > b->st_bytes) {
         ORBGPU_CUDA_TRY(cudaStreamSynchronize(st));
@@ -1578,12 +1582,12 @@ extern "C" int orbgpu_batch_compute_stereo_matches(orbgpu_batch* b, const orbgpu
     int* start = (int*)take(sizeof(int) * (size_t)npairs * (ORBGPU_MAX_DIM + 1));
     uint4* recs = (uint4*)take(sizeof(uint4) * (size_t)npairs * cap);
     int* sad = (int*)take(sizeof(int) * (size_t)npairs * cap);
-    int* done = (int*)take(sizeof(int) * (size_t)npairs);
     int* status = (int*)take(sizeof(int) * 4);
     ORBGPU_CUDA_TRY(cudaMemcpyAsync(d_pairs, hp.data(), sizeof(StereoPair) * npairs, cudaMemcpyHostToDevice, st));
-    k_bstereo_index<<<npairs, STEREO_INDEX_THREADS, 0, st>>>(kps, counts, cap, d_pairs, start, recs, done, status);
+    k_bstereo_index<<<npairs, STEREO_INDEX_THREADS, 0, st>>>(kps, counts, cap, d_pairs, start, recs, status);
     k_bstereo_match<<<dim3((cap + STEREO_WARPS - 1) / STEREO_WARPS, npairs), 32 * STEREO_WARPS, 0, st>>>(
-        kps, desc, counts, cap, d_pairs, start, recs, uright, depth, sad, done, status);
+        kps, desc, counts, cap, d_pairs, start, recs, uright, depth, sad, status);
+    k_bstereo_median<<<npairs, STEREO_INDEX_THREADS, 0, st>>>(counts, cap, d_pairs, sad, uright, depth);
     ORBGPU_CUDA_TRY(cudaGetLastError());
     ORBGPU_CUDA_TRY(cudaMemcpyAsync(b->st_pinned, status, sizeof(int), cudaMemcpyDeviceToHost, st));
     ORBGPU_CUDA_TRY(cudaStreamSynchronize(st));

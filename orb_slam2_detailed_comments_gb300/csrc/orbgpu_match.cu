@@ -876,8 +876,8 @@ __global__ void __launch_bounds__(1024) k_pf_finish(int n, int m, const int* res
 // (the device functions are in orbgpu_stereo.cuh)
 __global__ void __launch_bounds__(STEREO_INDEX_THREADS) k_stereo_index(const orbgpu_keypoint* kpsR, int nR, int nlevels,
                                                                        int nRows, int* start, uint4* recs,
-                                                                       int* status_done) {
-    if (threadIdx.x < 2) status_done[threadIdx.x] = 0;
+                                                                       int* status) {
+    if (threadIdx.x == 0) *status = 0;
     stereo_index_block(kpsR, nR, nlevels, nRows, start, recs);
 }
 
@@ -886,9 +886,14 @@ __global__ void __launch_bounds__(32 * STEREO_WARPS) k_stereo_match(const orbgpu
                                                                     const __grid_constant__ StereoLevels lv, int nRows,
                                                                     const int* start, const uint4* recs, float bf,
                                                                     float fx, float* uright, float* depth, int* sad,
-                                                                    int* status_done) {
-    stereo_match_block(blockIdx.x * STEREO_WARPS, nL, kpsL, descL, descR, lv, nRows, start, recs, bf, fx, uright, depth,
-                       sad, status_done + 1, status_done);
+                                                                    int* status) {
+    const int iL = blockIdx.x * STEREO_WARPS + (threadIdx.x >> 5);
+    if (iL < nL)
+        stereo_match_warp(iL, kpsL, descL, descR, lv, nRows, start, recs, bf, fx, uright, depth, sad, status);
+}
+
+__global__ void __launch_bounds__(STEREO_INDEX_THREADS) k_stereo_median(int nL, const int* sad, float* uright, float* depth) {
+    stereo_median_block(nL, sad, uright, depth);
 }
 
 // ----------------------------------------------------------------- distance batch
@@ -1848,10 +1853,11 @@ extern "C" int orbgpu_compute_stereo_matches(orbgpu_matcher* m, const orbgpu_ext
         d_dp = b.take<float>(nL);
     }
     int* sad = b.take<int>(nL);
-    int* status = b.take<int>(2);  // status, blocks done
+    int* status = b.take<int>(1);
     k_stereo_index<<<1, STEREO_INDEX_THREADS, 0, m->stream>>>(sr.kps, nR, nlev, nRows, row_start, recs, status);
     k_stereo_match<<<(nL + STEREO_WARPS - 1) / STEREO_WARPS, 32 * STEREO_WARPS, 0, m->stream>>>(
         sl.kps, sl.desc, nL, sr.desc, lv, nRows, row_start, recs, bf, fx, d_ur, d_dp, sad, status);
+    k_stereo_median<<<1, STEREO_INDEX_THREADS, 0, m->stream>>>(nL, sad, d_ur, d_dp);
     ORBGPU_CUDA_TRY(cudaGetLastError());
     if (mem != ORBGPU_MEM_DEVICE) {
         ORBGPU_CUDA_TRY(cudaMemcpyAsync(uright, d_ur, sizeof(float) * nL, cudaMemcpyDeviceToHost, m->stream));

@@ -13,8 +13,8 @@
 //                (22 lanes: each offset's rows in two halves), the first
 //                minimum, the parabola, disparity and depth
 //                (src/Frame.cc:884-1064)
-//   median cut   the pair's last block: SADs of the accepted matches at or
-//                above 1.5 * 1.4 * median discarded (src/Frame.cc:1069-1081)
+//   median cut   one block per pair: SADs of the accepted matches at or above
+//                1.5 * 1.4 * median discarded (src/Frame.cc:1069-1081)
 //
 // Bound by latency: a chain of loads per left keypoint.  Listing a keypoint
 // once instead of under every row of its band (9 to 30 of them) makes the
@@ -25,6 +25,9 @@
 // median is selected by two histograms of a byte of the SAD (at most 61,710,
 // 16 bits); a bitonic sort in global memory took 66 barriers at 2,000 matches.
 // A 1241x376 pair with its extractions 452 -> 416 us, 32 pairs 866 -> 843.
+// The cut by the last block of the match, one launch less, made every warp of
+// the match wait for its stores and its block: the call of 32 pairs 209 us
+// against 187 with a launch of its own, of one pair the same.
 #pragma once
 
 #include "orbgpu_common.cuh"
@@ -262,8 +265,7 @@ __device__ __forceinline__ int stereo_select_bin(const int* hist, int& k) {
     return __shfl_sync(0xffffffffu, bin, src);
 }
 
-// The median cut of one pair's nL left keypoints by the calling block; the
-// SADs are read past the L1 (other blocks wrote them).
+// The median cut of one pair's nL left keypoints by the calling block.
 __device__ __forceinline__ void stereo_median_block(int nL, const int* sad, float* uright, float* depth) {
     __shared__ int s_hist[2][256];
     __shared__ int s_at[2];
@@ -273,7 +275,7 @@ __device__ __forceinline__ void stereo_median_block(int nL, const int* sad, floa
     __syncthreads();
     int cnt = 0;
     for (int i = threadIdx.x; i < nL; i += blockDim.x) {
-        const int v = __ldcg(sad + i);
+        const int v = sad[i];
         if (v >= 0) {
             cnt++;
             atomicAdd(&s_hist[0][v >> 8], 1);
@@ -290,7 +292,7 @@ __device__ __forceinline__ void stereo_median_block(int nL, const int* sad, floa
     __syncthreads();
     const int high = s_at[0];
     for (int i = threadIdx.x; i < nL; i += blockDim.x) {
-        const int v = __ldcg(sad + i);
+        const int v = sad[i];
         if (v >= 0 && (v >> 8) == high) atomicAdd(&s_hist[1][v & 255], 1);
     }
     __syncthreads();
@@ -302,34 +304,12 @@ __device__ __forceinline__ void stereo_median_block(int nL, const int* sad, floa
     const float median = (float)(high << 8 | s_at[1]);
     const float thDist = __fmul_rn(1.5f * 1.4f, median);
     for (int i = threadIdx.x; i < nL; i += blockDim.x) {
-        const int v = __ldcg(sad + i);
+        const int v = sad[i];
         if (v >= 0 && !((float)v < thDist)) {
             uright[i] = -1.0f;
             depth[i] = -1.0f;
         }
     }
-}
-
-// STEREO_WARPS left keypoints of one pair from 'first' by the calling block;
-// the pair's last block (done: a zeroed counter) makes the median cut.
-__device__ __forceinline__ void stereo_match_block(int first, int nL, const orbgpu_keypoint* kpsL, const uint8_t* descL,
-                                                   const uint8_t* descR, const StereoLevels& lv, int nRows,
-                                                   const int* start, const uint4* recs, float bf, float fx,
-                                                   float* uright, float* depth, int* sad, int* done, int* status) {
-    __shared__ bool s_last;
-    if (first >= nL) return;
-    const int iL = first + (threadIdx.x >> 5);
-    if (iL < nL) {
-        stereo_match_warp(iL, kpsL, descL, descR, lv, nRows, start, recs, bf, fx, uright, depth, sad, status);
-        if ((threadIdx.x & 31) == 0) __threadfence();
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        s_last = atomicAdd(done, 1) == (nL + STEREO_WARPS - 1) / STEREO_WARPS - 1;
-        __threadfence();
-    }
-    __syncthreads();
-    if (s_last) stereo_median_block(nL, sad, uright, depth);
 }
 
 }  // namespace orbgpu
