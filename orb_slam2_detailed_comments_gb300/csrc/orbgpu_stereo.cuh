@@ -30,6 +30,8 @@
 // against 187 with a launch of its own, of one pair the same.
 #pragma once
 
+#include <cuda_fp16.h>
+
 #include "orbgpu_common.cuh"
 #include "orbgpu_ext.h"
 
@@ -95,6 +97,14 @@ __device__ __forceinline__ void stereo_row11(const uint8_t* row, int x0, unsigne
     w[0] = __funnelshift_r(a, b, 8 * o);
     w[1] = __funnelshift_r(b, c, 8 * o);
     w[2] = __funnelshift_r(c, d, 8 * o);
+}
+
+// Bytes 2h and 2h + 1 of a word as 1024 + byte in halves (0x6400 is 1024, its
+// last place 1).
+template <int H>
+__device__ __forceinline__ __half2 stereo_halves(unsigned w) {
+    const unsigned v = __byte_perm(w, 0x64646464u, H ? 0x4342 : 0x4140);
+    return *reinterpret_cast<const __half2*>(&v);
 }
 
 // The match of left keypoint iL, by the calling warp.  Writes uright[iL],
@@ -187,12 +197,16 @@ __device__ __forceinline__ void stereo_match_warp(int iL, const orbgpu_keypoint*
         const uint8_t* left = lv.left[levelL] + (size_t)ly0 * lp;
         const uint8_t* right = lv.right[levelL] + (size_t)ly0 * lp;
         // offset t = incR + L on lanes t and t + 11: rows 0-5 and rows 6-10
-        int part = 0;
+        // In halves: l - r - c is at most 510, four of them sum to at most 2,040,
+        // and integers up to 2,048 are exact.  In integers a pixel took 5
+        // instructions of the ALU pipe: the call of 32 pairs 187 us against 169.
+        float part = 0.f;
         if (lane < 2 * (2 * L + 1)) {
             const bool upper = lane < 2 * L + 1;
             const int t = upper ? lane : lane - (2 * L + 1);
             const int rx0 = (int)(scaleduR0 + (t - L) - W);
             const int c = (int)left[(size_t)W * lp + lx0 + W] - (int)right[(size_t)W * lp + rx0 + W];
+            const __half2 c2 = __half2half2(__int2half_rn(c));
             const uint8_t* lr = left + (upper ? 0 : (size_t)(W + 1) * lp);
             const uint8_t* rr = right + (upper ? 0 : (size_t)(W + 1) * lp);
 #pragma unroll
@@ -201,16 +215,20 @@ __device__ __forceinline__ void stereo_match_warp(int iL, const orbgpu_keypoint*
                 unsigned a[3], b[3];
                 stereo_row11(lr + (size_t)yy * lp, lx0, a);
                 stereo_row11(rr + (size_t)yy * lp, rx0, b);
-#pragma unroll
-                for (int xx = 0; xx < 2 * W + 1; xx++) {
-                    const int l = (a[xx >> 2] >> (8 * (xx & 3))) & 255, r = (b[xx >> 2] >> (8 * (xx & 3))) & 255;
-                    part += abs(l - r - c);
-                }
+                const auto diff = [&](__half2 l, __half2 r) { return __habs2(__hsub2(__hsub2(l, r), c2)); };
+                const __half2 s8 = __hadd2(__hadd2(diff(stereo_halves<0>(a[0]), stereo_halves<0>(b[0])),
+                                                   diff(stereo_halves<1>(a[0]), stereo_halves<1>(b[0]))),
+                                           __hadd2(diff(stereo_halves<0>(a[1]), stereo_halves<0>(b[1])),
+                                                   diff(stereo_halves<1>(a[1]), stereo_halves<1>(b[1]))));
+                const __half2 s2 = diff(stereo_halves<0>(a[2]), stereo_halves<0>(b[2]));
+                const __half2 s1 = diff(stereo_halves<1>(a[2]), stereo_halves<1>(b[2]));  // column 10, and one past it
+                const float2 f8 = __half22float2(s8), f3 = __half22float2(__hadd2(s2, __halves2half2(__low2half(s1), __ushort_as_half(0))));
+                part += f8.x + f8.y + f3.x + f3.y;
             }
         }
-        const int other = __shfl_down_sync(0xffffffffu, part, 2 * L + 1);
+        const float other = __shfl_down_sync(0xffffffffu, part, 2 * L + 1);
         // first minimum over incR = -L..L: SAD (16 bits), then the offset
-        const unsigned key = lane < 2 * L + 1 ? (unsigned)(part + other) << 4 | (unsigned)lane : ~0u;
+        const unsigned key = lane < 2 * L + 1 ? (unsigned)(int)(part + other) << 4 | (unsigned)lane : ~0u;
         const unsigned least = __reduce_min_sync(0xffffffffu, key);
         const int t = (int)(least & 15), bestinc = t - L;
         if (bestinc == -L || bestinc == L) return;
