@@ -31,16 +31,16 @@
 // Bound by issue: the distances are a tenth of the instructions, the rest is
 // lanes without an observation, sorts and bookkeeping (fixed groups of 4
 // map points, without the width of 4, took 261 instructions a map point).  A
-// million map points of 6 observations 463 -> 343 us, of 3 187 -> 89.
+// million map points of 6 observations 463 -> 285 us, of 3 187 -> 87.
 #include <algorithm>
 
 #include "orbgpu_host.h"
 
 namespace orbgpu {
 
-#define DD_WARPS 8          // warps per block
+#define DD_WARPS 4          // warps per block
 #ifndef DD_BLOCKS_PER_SM
-#define DD_BLOCKS_PER_SM 4  // resident blocks per SM (64 registers x 256 threads)
+#define DD_BLOCKS_PER_SM 8  // resident blocks per SM (64 registers x 128 threads)
 #endif
 
 struct DDArgs {
@@ -50,7 +50,7 @@ struct DDArgs {
     const int* rows;     // n_obs
     int n_obs;
     int m;
-    int per_warp;  // map points a warp takes per iteration (4 to 32)
+    int per_warp;  // map points a warp takes (4 to 32)
     int* best;   // m
     uint4* out;  // m x 32 bytes, or null
 };
@@ -295,39 +295,39 @@ __device__ __forceinline__ void dd_long_list(const DDArgs& a, uint4 (*sd)[32], i
 __global__ void __launch_bounds__(DD_WARPS * 32, DD_BLOCKS_PER_SM) k_distinctive_descriptors(const __grid_constant__ DDArgs a) {
     __shared__ DDShared sh;
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int per = a.per_warp, stride = gridDim.x * DD_WARPS * per;
-    for (int base = (blockIdx.x * DD_WARPS + w) * per; base < a.m; base += stride) {
-        const bool mine = lane < per && base + lane < a.m;
-        int o0 = 0, n = 0;
-        if (mine) {
-            o0 = __ldg(a.offsets + base + lane);
-            const int o1 = __ldg(a.offsets + base + lane + 1);
-            n = o1 - o0;
-            if (o0 < 0 || n < 0 || o1 > a.n_obs) {
-                a.best[base + lane] = -2;
-                n = 0;
-            } else if (n <= 2) {
-                const int r0 = n > 0 ? __ldg(a.rows + o0) : -1, r1 = n > 1 ? __ldg(a.rows + o0 + 1) : -1;
-                const int r = r0 >= 0 ? r0 : r1;
-                if (r0 < -1 || r0 >= a.pool_rows || r1 < -1 || r1 >= a.pool_rows) a.best[base + lane] = -2;
-                else if (r < 0) a.best[base + lane] = -1;
-                else dd_store(a, base + lane, r, __ldg(a.pool + 2 * (size_t)r), __ldg(a.pool + 2 * (size_t)r + 1));
-            }
+    const unsigned at = (blockIdx.x * DD_WARPS + w) * (unsigned)a.per_warp;
+    if (at >= (unsigned)a.m) return;
+    const int base = (int)at;
+    const bool mine = lane < a.per_warp && lane < a.m - base;
+    int o0 = 0, n = 0;
+    if (mine) {
+        o0 = __ldg(a.offsets + base + lane);
+        const int o1 = __ldg(a.offsets + base + lane + 1);
+        n = o1 - o0;
+        if (o0 < 0 || n < 0 || o1 > a.n_obs) {
+            a.best[base + lane] = -2;
+            n = 0;
+        } else if (n <= 2) {
+            const int r0 = n > 0 ? __ldg(a.rows + o0) : -1, r1 = n > 1 ? __ldg(a.rows + o0 + 1) : -1;
+            const int r = r0 >= 0 ? r0 : r1;
+            if (r0 < -1 || r0 >= a.pool_rows || r1 < -1 || r1 >= a.pool_rows) a.best[base + lane] = -2;
+            else if (r < 0) a.best[base + lane] = -1;
+            else dd_store(a, base + lane, r, __ldg(a.pool + 2 * (size_t)r), __ldg(a.pool + 2 * (size_t)r + 1));
         }
-        __syncwarp();
-        const unsigned c4 = __ballot_sync(DD_FULL, n > 2 && n <= 4), c8 = __ballot_sync(DD_FULL, n > 4 && n <= 8);
-        const unsigned c16 = __ballot_sync(DD_FULL, n > 8 && n <= 16), c32 = __ballot_sync(DD_FULL, n > 16 && n <= 32);
-        unsigned clong = __ballot_sync(DD_FULL, n > 32);
-        if (c4) dd_group_pass<4>(a, sh.desc[w], sh.order[w], lane, base, o0, n, c4);
-        if (c8) dd_group_pass<8>(a, sh.desc[w], sh.order[w], lane, base, o0, n, c8);
-        if (c16) dd_group_pass<16>(a, sh.desc[w], sh.order[w], lane, base, o0, n, c16);
-        if (c32) dd_group_pass<32>(a, sh.desc[w], sh.order[w], lane, base, o0, n, c32);
-        while (clong) {
-            const int g = __ffs(clong) - 1;
-            clong &= clong - 1;
-            const int of = __shfl_sync(DD_FULL, o0, g), nf = __shfl_sync(DD_FULL, n, g);
-            dd_long_list(a, sh.desc[w], sh.hist[w], lane, base + g, of, nf);
-        }
+    }
+    __syncwarp();
+    const unsigned c4 = __ballot_sync(DD_FULL, n > 2 && n <= 4), c8 = __ballot_sync(DD_FULL, n > 4 && n <= 8);
+    const unsigned c16 = __ballot_sync(DD_FULL, n > 8 && n <= 16), c32 = __ballot_sync(DD_FULL, n > 16 && n <= 32);
+    unsigned clong = __ballot_sync(DD_FULL, n > 32);
+    if (c4) dd_group_pass<4>(a, sh.desc[w], sh.order[w], lane, base, o0, n, c4);
+    if (c8) dd_group_pass<8>(a, sh.desc[w], sh.order[w], lane, base, o0, n, c8);
+    if (c16) dd_group_pass<16>(a, sh.desc[w], sh.order[w], lane, base, o0, n, c16);
+    if (c32) dd_group_pass<32>(a, sh.desc[w], sh.order[w], lane, base, o0, n, c32);
+    while (clong) {
+        const int g = __ffs(clong) - 1;
+        clong &= clong - 1;
+        const int of = __shfl_sync(DD_FULL, o0, g), nf = __shfl_sync(DD_FULL, n, g);
+        dd_long_list(a, sh.desc[w], sh.hist[w], lane, base + g, of, nf);
     }
 }
 
@@ -358,12 +358,13 @@ extern "C" int orbgpu_distinctive_descriptors(const uint8_t* pool, int pool_rows
     a.m = m;
     a.best = best_rows;
     a.out = reinterpret_cast<uint4*>(descriptors);
-    // as many map points per warp (fuller groups) as leave every resident warp some
-    const int resident = nsm_of_current_device() * DD_BLOCKS_PER_SM;
-    a.per_warp = 4;
-    while (a.per_warp < 32 && (long long)a.per_warp * 2 * resident * DD_WARPS <= m) a.per_warp *= 2;
-    const long long per_block = (long long)DD_WARPS * a.per_warp;
-    const int blocks = (int)std::min<long long>((m + per_block - 1) / per_block, resident);
+    // a block takes its map points once and ends, so that the device evens out
+    // long and short lists (a million map points in rounds over resident
+    // blocks: 346 us against 285); as many per warp (fuller groups) as leave
+    // every resident warp some
+    const long long warps = (long long)nsm_of_current_device() * DD_BLOCKS_PER_SM * DD_WARPS;
+    a.per_warp = (int)std::min(32LL, std::max(4LL, (m + warps - 1) / warps));
+    const int per_block = DD_WARPS * a.per_warp, blocks = (int)(((long long)m + per_block - 1) / per_block);
     k_distinctive_descriptors<<<blocks, DD_WARPS * 32, 0, (cudaStream_t)stream>>>(a);
     ORBGPU_CUDA_TRY(cudaGetLastError());
     return ORBGPU_OK;
