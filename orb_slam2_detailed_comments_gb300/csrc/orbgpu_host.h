@@ -88,6 +88,36 @@ inline cudaError_t allow_max_dynamic_smem(K* kernel) {
     return allow_max_dynamic_smem(reinterpret_cast<const void*>(kernel));
 }
 
+// The workspace of one orbgpu_knn2 call.  A matcher keeps those of its calls
+// for the next ones (allocating and releasing them cost ten times the kernels
+// of a 2,000 x 2,000 call, 0.4 ms at 50,000 x 200,000); a call holds its own
+// until it returns, so that host threads may search with one matcher at once.
+struct KnnBuffers {
+    uint8_t* data = nullptr;
+    size_t bytes = 0;
+    int* pinned = nullptr;  // 64 page-locked bytes
+    KnnBuffers* next = nullptr;
+    void drop() {
+        cudaFree(data);
+        data = nullptr;
+        bytes = 0;
+    }
+};
+class KnnWorkspace {
+public:
+    explicit KnnWorkspace(orbgpu_matcher* matcher) : m(matcher) {}
+    ~KnnWorkspace();  // back to the matcher
+    KnnWorkspace(const KnnWorkspace&) = delete;
+    KnnWorkspace& operator=(const KnnWorkspace&) = delete;
+    int take(size_t need);
+    uint8_t* data() const { return b->data; }
+    int* pinned() const { return b->pinned; }
+
+private:
+    orbgpu_matcher* m;
+    KnnBuffers* b = nullptr;
+};
+
 // SM count of the current device, cached per device ordinal.
 inline int nsm_of_current_device() {
     static int cache[64] = {};

@@ -12,8 +12,6 @@
 #include "orbgpu_host.h"
 
 cudaStream_t orbgpu_matcher_stream_internal(orbgpu_matcher* m);
-int orbgpu_matcher_scratch_internal(orbgpu_matcher* m, size_t bytes, void** scratch, int** pinned);
-void orbgpu_matcher_trim_internal(orbgpu_matcher* m);
 
 namespace orbgpu {
 
@@ -184,19 +182,15 @@ extern "C" int orbgpu_knn2(orbgpu_matcher* m, const uint8_t* query, int nq, cons
     cudaStream_t st = orbgpu_matcher_stream_internal(m);
     int slice, nslices;
     knn_slices(nq, nt, 0x7fffffff, &slice, &nslices);
-    // the slices' results live in the matcher's scratch: allocating and
-    // releasing them cost ten times the kernels of a 2,000 x 2,000 call
-    void* scratch = nullptr;
-    int* pinned = nullptr;
-    const int rc = orbgpu_matcher_scratch_internal(m, sizeof(int4) * (size_t)nq * nslices, &scratch, &pinned);
+    KnnWorkspace work(m);
+    const int rc = work.take(sizeof(int4) * (size_t)nq * nslices);
     if (rc != ORBGPU_OK) return rc;
-    int4* partial = (int4*)scratch;
+    int4* partial = (int4*)work.data();
     dim3 grid((nq + KNN_Q - 1) / KNN_Q, nslices);
     k_knn_popc<<<grid, 32 * KNN_WARPS, 0, st>>>((const uint4*)query, nq, (const uint4*)train, nt, slice, partial);
     k_knn_merge<<<(nq + 255) / 256, 256, 0, st>>>(partial, nq, nslices, idx1, d1, idx2, d2);
     ORBGPU_CUDA_TRY(cudaGetLastError());
     ORBGPU_CUDA_TRY(cudaStreamSynchronize(st));
-    orbgpu_matcher_trim_internal(m);
     return ORBGPU_OK;
 }
 

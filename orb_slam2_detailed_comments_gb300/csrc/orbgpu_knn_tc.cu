@@ -39,8 +39,6 @@
 #include "orbgpu_host.h"
 
 cudaStream_t orbgpu_matcher_stream_internal(orbgpu_matcher* m);
-int orbgpu_matcher_scratch_internal(orbgpu_matcher* m, size_t bytes, void** scratch, int** pinned);
-void orbgpu_matcher_trim_internal(orbgpu_matcher* m);
 
 namespace orbgpu {
 
@@ -631,9 +629,7 @@ extern "C" int orbgpu_debug_tc_probe(const uint8_t* q128, const uint8_t* t256, f
     return ORBGPU_OK;
 }
 
-// The tensor-core kNN (algo 1 of orbgpu_knn2); see orbgpu.h.  The expansions
-// and the segments' results live in the matcher's scratch (allocating and
-// releasing them on every call cost 0.4 ms at 50,000 x 200,000).
+// The tensor-core kNN (algo 1 of orbgpu_knn2); see orbgpu.h.
 int orbgpu_knn2_tc(orbgpu_matcher* m, const uint8_t* query, int nq, const uint8_t* train, int nt, int* idx1, int* d1,
                    int* idx2, int* d2) {
     if (nq <= 0 || nt <= 0) return ORBGPU_ERR_BAD_ARG;  // the caller answers empty sets
@@ -646,11 +642,10 @@ int orbgpu_knn2_tc(orbgpu_matcher* m, const uint8_t* query, int nq, const uint8_
     const int slots = (tt + run - 1) / run + 1;  // segments of one query pair, at most
     const size_t q_bytes = (size_t)pairs * TC_QPAIR_BYTES, t_bytes = (size_t)tt * TC_TTILE_BYTES,
                  p_bytes = (sizeof(uint2) * (size_t)nq * slots + 255) & ~(size_t)255;
-    void* scratch = nullptr;
-    int* pinned = nullptr;
-    int rc = orbgpu_matcher_scratch_internal(m, q_bytes + t_bytes + p_bytes + 256, &scratch, &pinned);
+    KnnWorkspace work(m);
+    const int rc = work.take(q_bytes + t_bytes + p_bytes + 256);
     if (rc != ORBGPU_OK) return rc;
-    uint8_t* eq = (uint8_t*)scratch;
+    uint8_t* eq = work.data();
     uint8_t* et = eq + q_bytes;
     uint2* partial = (uint2*)(et + t_bytes);
     int* status = (int*)(et + t_bytes + p_bytes);
@@ -661,10 +656,9 @@ int orbgpu_knn2_tc(orbgpu_matcher* m, const uint8_t* query, int nq, const uint8_
     k_knn_tc<<<ctas, TC_THREADS, smem, st>>>(eq, et, nq, nt, items, tt, run, partial, status);
     k_knn_tc_finish<<<(nq + 7) / 8, 256, 0, st>>>(partial, query, train, nq, nt, tt, run, idx1, d1, idx2, d2);
     ORBGPU_CUDA_TRY(cudaGetLastError());
-    ORBGPU_CUDA_TRY(cudaMemcpyAsync(pinned, status, sizeof(int), cudaMemcpyDeviceToHost, st));
+    ORBGPU_CUDA_TRY(cudaMemcpyAsync(work.pinned(), status, sizeof(int), cudaMemcpyDeviceToHost, st));
     ORBGPU_CUDA_TRY(cudaStreamSynchronize(st));
-    const int hstatus = pinned[0];
-    orbgpu_matcher_trim_internal(m);
+    const int hstatus = work.pinned()[0];
     if (hstatus) {
         char msg[96];
         std::snprintf(msg, sizeof(msg), "tensor-core kNN wait timed out (status 0x%x)", hstatus);

@@ -16,6 +16,8 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
+#include <new>
 #include <vector>
 
 #include "orbgpu_grid.cuh"
@@ -916,6 +918,10 @@ struct orbgpu_matcher {
     void* scratch = nullptr;
     size_t scratch_bytes = 0;
     int* h_pinned = nullptr;
+    // kNN workspaces that no call holds (KnnWorkspace)
+    std::mutex knn_mutex;
+    orbgpu::KnnBuffers* knn_work = nullptr;
+    size_t knn_kept = 0;  // their bytes
 };
 
 namespace {
@@ -1017,22 +1023,45 @@ bool frame_ok(const orbgpu_frame* f) {
 
 }  // namespace
 
-// The matcher's scratch, grown to 'bytes', and its 64 page-locked bytes, for
-// the kNN (every call on a matcher is complete when it returns, so the
-// scratch is free between calls).
-int orbgpu_matcher_scratch_internal(orbgpu_matcher* m, size_t bytes, void** scratch, int** pinned) {
-    const int rc = ensure_scratch(m, bytes);
-    *scratch = m->scratch;
-    *pinned = m->h_pinned;
-    return rc;
+// A matcher keeps the workspaces of its kNN calls up to this many bytes.
+#define KNN_KEEP_BYTES ((size_t)512 << 20)
+
+KnnWorkspace::~KnnWorkspace() {
+    if (!b) return;
+    std::lock_guard<std::mutex> lock(m->knn_mutex);
+    if (m->knn_kept + b->bytes > KNN_KEEP_BYTES) b->drop();
+    m->knn_kept += b->bytes;
+    b->next = m->knn_work;
+    m->knn_work = b;
 }
-// Gives back a scratch that one very large call grew beyond what a matcher
-// keeps between calls.
-void orbgpu_matcher_trim_internal(orbgpu_matcher* m) {
-    if (m->scratch_bytes <= (size_t)512 << 20) return;
-    cudaFree(m->scratch);
-    m->scratch = nullptr;
-    m->scratch_bytes = 0;
+int KnnWorkspace::take(size_t need) {
+    {
+        std::lock_guard<std::mutex> lock(m->knn_mutex);
+        // the smallest that is large enough, else the largest
+        KnnBuffers** best = &m->knn_work;
+        for (KnnBuffers** p = best; *p; p = &(*p)->next)
+            if ((*best)->bytes < need ? (*p)->bytes > (*best)->bytes : (*p)->bytes >= need && (*p)->bytes < (*best)->bytes)
+                best = p;
+        b = *best;
+        if (b) {
+            *best = b->next;
+            m->knn_kept -= b->bytes;
+        }
+    }
+    if (!b) {
+        KnnBuffers* fresh = new (std::nothrow) KnnBuffers();
+        if (!fresh || cudaMallocHost(&fresh->pinned, 64) != cudaSuccess) {
+            delete fresh;
+            orbgpu_set_last_error("page-locked allocation failed", __FILE__, __LINE__);
+            return ORBGPU_ERR_OOM;
+        }
+        b = fresh;
+    }
+    if (b->bytes >= need) return ORBGPU_OK;
+    b->drop();
+    ORBGPU_CUDA_TRY(cudaMalloc(&b->data, need));
+    b->bytes = need;
+    return ORBGPU_OK;
 }
 
 extern "C" int orbgpu_matcher_create(float nnratio, int check_orientation, void* stream, orbgpu_matcher** out) {
@@ -1063,6 +1092,12 @@ extern "C" int orbgpu_matcher_destroy(orbgpu_matcher* m) {
     if (m->stream) cudaStreamSynchronize(m->stream);
     cudaFree(m->scratch);
     cudaFreeHost(m->h_pinned);
+    while (KnnBuffers* w = m->knn_work) {
+        m->knn_work = w->next;
+        w->drop();
+        cudaFreeHost(w->pinned);
+        delete w;
+    }
     if (m->own_stream) cudaStreamDestroy(m->stream);
     delete m;
     return ORBGPU_OK;

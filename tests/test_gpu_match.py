@@ -328,6 +328,48 @@ def test_knn_tile_edges(torch, oracle, nq, nt):
             assert np.array_equal(a.cpu().numpy(), b), (algo, shift, name)
 
 
+def test_knn_threads_share_a_matcher(torch, oracle):
+    """Four host threads search with one matcher at once, with both kernels, at
+    sizes that grow the kept workspaces, beside a thread in another search of
+    the same matcher."""
+    import threading
+    from orb_slam2_detailed_comments_gb300 import FrameView, ORBmatcher
+    from orb_slam2_detailed_comments_gb300 import synthetic as syn
+    from oracle import pyoracle
+    m = ORBmatcher(0.9, True)
+    jobs = []
+    for i, (nq, nt) in enumerate([(1, 40), (300, 500), (257, 3000), (900, 700), (64, 9000), (1500, 2000)]):
+        q, t = syn.random_descriptors(nq, 50 + i), syn.random_descriptors(nt, 60 + i)
+        jobs.append((torch.from_numpy(q).cuda(), torch.from_numpy(t).cuda(), oracle.knn2(q, t)))
+    k, d = random_frame(900, 640, 480, 3, 2)
+    prev = np.ascontiguousarray(np.stack([k["x"], k["y"]], 1))
+    s, _ = pyoracle.scale_tables(8, 1.2)
+    view = FrameView(k, d, 640, 480, s)
+    init = oracle.search_for_initialization(k.view(pyoracle.KP_DTYPE), d, k.view(pyoracle.KP_DTYPE), d, 640, 480,
+                                            prev_xy=prev, window=40, nnratio=0.9, check_ori=True)
+    torch.cuda.synchronize()
+    bad = []
+
+    def knn(thread):
+        for r in range(30):
+            q, t, ref = jobs[(r * (thread + 1) + thread) % len(jobs)]
+            out = m.knn2(q, t, algo=(r + thread) & 1)
+            if any(not np.array_equal(a.cpu().numpy(), b) for a, b in zip(out, ref)):
+                bad.append(("knn", thread, r))
+
+    def windows():
+        for r in range(30):
+            nm, m12, _ = m.SearchForInitialization(view, view, prev.copy(), 40)
+            if nm != init[0] or not np.array_equal(m12, init[1]):
+                bad.append(("init", r))
+    threads = [threading.Thread(target=knn, args=(i,)) for i in range(4)] + [threading.Thread(target=windows)]
+    for th in threads:
+        th.start()
+    for th in threads:
+        th.join()
+    assert not bad, bad
+
+
 def test_knn_tensor_cores_golden_and_ties(torch, golden):
     """Golden vectors, then clustered descriptors (many equal distances) against
     the popcount kernel at a size with many slices."""
