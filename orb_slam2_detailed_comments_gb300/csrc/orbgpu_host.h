@@ -97,8 +97,9 @@ struct KnnBuffers {
     size_t bytes = 0;
     int* pinned = nullptr;  // 64 page-locked bytes
     KnnBuffers* next = nullptr;
-    void drop() {
-        cudaFree(data);
+    // in stream order: a call too large to keep stops no other stream
+    void drop(cudaStream_t st) {
+        if (data) cudaFreeAsync(data, st);
         data = nullptr;
         bytes = 0;
     }

@@ -1029,7 +1029,7 @@ bool frame_ok(const orbgpu_frame* f) {
 KnnWorkspace::~KnnWorkspace() {
     if (!b) return;
     std::lock_guard<std::mutex> lock(m->knn_mutex);
-    if (m->knn_kept + b->bytes > KNN_KEEP_BYTES) b->drop();
+    if (m->knn_kept + b->bytes > KNN_KEEP_BYTES) b->drop(m->stream);
     m->knn_kept += b->bytes;
     b->next = m->knn_work;
     m->knn_work = b;
@@ -1058,8 +1058,8 @@ int KnnWorkspace::take(size_t need) {
         b = fresh;
     }
     if (b->bytes >= need) return ORBGPU_OK;
-    b->drop();
-    ORBGPU_CUDA_TRY(cudaMalloc(&b->data, need));
+    b->drop(m->stream);
+    ORBGPU_CUDA_TRY(cudaMallocAsync((void**)&b->data, need, m->stream));
     b->bytes = need;
     return ORBGPU_OK;
 }
@@ -1094,7 +1094,7 @@ extern "C" int orbgpu_matcher_destroy(orbgpu_matcher* m) {
     cudaFreeHost(m->h_pinned);
     while (KnnBuffers* w = m->knn_work) {
         m->knn_work = w->next;
-        w->drop();
+        w->drop(m->stream);
         cudaFreeHost(w->pinned);
         delete w;
     }

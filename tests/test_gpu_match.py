@@ -370,6 +370,28 @@ def test_knn_threads_share_a_matcher(torch, oracle):
     assert not bad, bad
 
 
+def test_knn_beyond_the_kept_workspace_stops_no_other_stream(torch):
+    """A search whose workspace is too large to keep returns while a kernel of
+    another stream still runs."""
+    from orb_slam2_detailed_comments_gb300 import ORBmatcher
+    m = ORBmatcher()
+    t = torch.randint(0, 256, (4_300_000, 32), dtype=torch.uint8, device="cuda")  # 550 MB of operands
+    q = t[::43000][:100].clone()
+    side, done = torch.cuda.Stream(), torch.cuda.Event()
+    ref = m.knn2(q, t, algo=0)
+    m.knn2(q, t, algo=1)
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side):
+        torch.cuda._sleep(1_000_000_000)  # about half a second
+        done.record()
+    out = m.knn2(q, t, algo=1)
+    running = not done.query()
+    torch.cuda.synchronize()
+    assert running
+    for a, b, name in zip(out, ref, ("idx1", "d1", "idx2", "d2")):
+        assert torch.equal(a, b), name
+
+
 def test_knn_tensor_cores_golden_and_ties(torch, golden):
     """Golden vectors, then clustered descriptors (many equal distances) against
     the popcount kernel at a size with many slices."""
