@@ -485,7 +485,9 @@ __host__ __device__ inline PyrEntry pyr_entry(int stage, int n) {
     return {stage - (n - 1), false};  // the last two strips
 }
 
-// Waits until the bands [b0, b1] of d are written.
+// Waits until the bands [b0, b1] of d are written.  (A tile also loads the rows
+// that its loop runs ahead to, past its last output row; nothing waits for
+// those, as nothing uses their values.)
 __device__ __forceinline__ bool bands_ready(const LevelDesc& d, int b0, int b1) {
     const int lane = threadIdx.x & 31;
     const int need = (d.w + RS_COLS - 1) / RS_COLS;
@@ -506,6 +508,9 @@ __device__ __forceinline__ bool bands_ready(const LevelDesc& d, int b0, int b1) 
             }
         }
     }
+    // the polling lanes' acquires before every lane's reads of the rows (a vote
+    // orders no memory)
+    __syncwarp();
     return __all_sync(0xffffffffu, ok);
 }
 

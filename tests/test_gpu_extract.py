@@ -299,6 +299,47 @@ def test_pyramid_launches(torch, oracle, w, h, scale, nlevels):
         autotune.apply({k: v for k, v in before.items() if k != "knn_tc_min_pairs"})
 
 
+def test_pyramid_on_several_streams(torch, oracle):
+    """The one-launch pyramid from four extractors and two batches at once, each
+    on its own stream and host thread."""
+    import threading
+    from orb_slam2_detailed_comments_gb300 import synthetic as syn
+    from orb_slam2_detailed_comments_gb300._lib import KEYPOINT_DTYPE
+    from orb_slam2_detailed_comments_gb300.batch import BatchExtractor
+    sizes = [(640, 480), (1241, 376), (321, 243), (1280, 720)]
+    imgs = [syn.scene(w, h, 70 + i) for i, (w, h) in enumerate(sizes)]
+    refs = [oracle.extract(i, nfeatures=700) for i in imgs]
+    dev = [torch.from_numpy(i).cuda() for i in imgs]
+    torch.cuda.synchronize()
+    bad = []
+
+    def frames(first):
+        ex = extractor(700)
+        for r in range(12):
+            i = (first + r) % len(imgs)
+            kps, desc = ex(imgs[i])
+            if kps.tobytes() != refs[i].keypoints.tobytes() or not np.array_equal(desc, refs[i].descriptors):
+                bad.append(("frame", first, r))
+
+    def batch(n):
+        b = BatchExtractor(n, 1280, 720, 700)
+        for r in range(12):
+            k, d, c = b.extract(dev[:n], [700] * n)
+            k = k.cpu().numpy().view(KEYPOINT_DTYPE).reshape(n, -1)
+            d, c = d.cpu().numpy().reshape(n, -1, 32), c.cpu().numpy()
+            for f in range(n):
+                if (k[f, :c[f]].tobytes() != refs[f].keypoints.tobytes()
+                        or not np.array_equal(d[f, :c[f]], refs[f].descriptors)):
+                    bad.append(("batch", n, r, f))
+    threads = [threading.Thread(target=frames, args=(i,)) for i in range(4)]
+    threads += [threading.Thread(target=batch, args=(n,)) for n in (2, 4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad, bad
+
+
 # DistributeOctTree: one key, lists of a few and of thousands of nodes (counted
 # and sorted places in the final phase, node and key arrays in shared and in
 # global memory), one and many initial nodes, more cells than threads.
