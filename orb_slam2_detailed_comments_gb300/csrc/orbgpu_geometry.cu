@@ -149,7 +149,8 @@ __device__ __forceinline__ float norm3_float(float a, float b, float c) {
     }
     return norm3_slow(a, b, c);
 }
-// The float of the double quotient a . b / d.
+// The float of the double quotient a . b / d.  The numerator has a bound of its
+// own: near 2^-120 the products' errors underflow.
 __device__ __forceinline__ float dot3_over(float a0, float b0, float a1, float b1, float a2, float b2, float d) {
     float r;
     if (d > 0x1p-60f && d < 0x1p+60f) {
@@ -157,7 +158,7 @@ __device__ __forceinline__ float dot3_over(float a0, float b0, float a1, float b
         const float inv = __fdividef(1.0f, d), q = __fmul_rn(p.h, inv);
         const float rest = __fadd_rn(__fmaf_rn(-q, d, p.h), p.l);
         const float err = __fadd_rn(__fmul_rn(p.err, __fmul_rn(inv, 1.25f)), __fmul_rn(fabsf(q), 0x1p-42f));
-        if (rounds_to({q, __fmul_rn(rest, inv), err}, r)) return r;
+        if (fabsf(p.h) > 0x1p-60f && rounds_to({q, __fmul_rn(rest, inv), err}, r)) return r;
     }
     return dot3_over_slow(a0, b0, a1, b1, a2, b2, d);
 }

@@ -119,6 +119,29 @@ def test_rounding_limits_vs_oracle(torch, oracle, scale):
     assert M.cpu().numpy().view(pyoracle.MP_DTYPE).tobytes() == ref[0].tobytes()
 
 
+@pytest.mark.parametrize("normals", [-66, -60, -58])
+def test_tiny_normals_vs_oracle(torch, oracle, normals):
+    """Worlds and normals near 2^-58: the view cosine's quotient and divisor are
+    inside the two-float range, its numerator's products are not."""
+    from orb_slam2_detailed_comments_gb300 import synthetic as syn
+    w, h, fx, sf, nl, m = 640, 480, 500.0, 1.2, 8, 60000
+    Tcw, g = syn.frustum_case(m, 78, w, h, fx, sf, nl)
+    Tcw, g = np.array(Tcw, np.float32), np.array(g, np.float32)
+    k = np.float32(2.0) ** -61  # most distances from 2^-60 to 2^-56
+    g[:, :3] *= k
+    g[:, 6:8] *= k
+    Tcw[:3, 3] *= k
+    g[:, 3:6] *= np.float32(2.0) ** normals
+    camera = np.array([fx, fx, w / 2, h / 2, 40.0, w, h, sf, nl, -0.5], np.float32)
+    init = np.zeros(m, pyoracle.MP_DTYPE)
+    cam = pyoracle.make_frustum_camera(Tcw, fx, fx, w / 2, h / 2, 40.0, 0.0, w, 0.0, h, sf, nl)
+    ref = oracle.is_in_frustum(cam, np.ascontiguousarray(g).view(pyoracle.GEOM_DTYPE).reshape(-1), -0.5, init)
+    assert ref[1] > m // 4
+    (out,), iv = run(torch, [frame_record(Tcw, camera)], [g], [init], -0.5)
+    assert out.tobytes() == ref[0].tobytes()
+    assert iv[0] == ref[1]
+
+
 def test_chained_into_search_by_projection(torch, oracle):
     """isInFrustum then SearchByProjection(Frame&, vector<MapPoint*>, th) with
     the records staying on the device, against the oracle doing the same."""
