@@ -118,6 +118,8 @@ int orbgpu_serving_retry_select(int* match, int* nmatches, const int* match2, co
 int orbgpu_batch_stage_times(orbgpu_batch* b, float* ms, int n);
 /* Kernel launches of one orbgpu_batch_extract of the last frame list. */
 int orbgpu_batch_launch_count(const orbgpu_batch* b);
+/* Whether the batch holds a captured graph (of the frame list it replays). */
+int orbgpu_debug_batch_has_graph(const orbgpu_batch* b);
 /* The batch's CUDA stream (cudaStream_t). */
 void* orbgpu_batch_stream(const orbgpu_batch* b);
 

@@ -351,8 +351,10 @@ static int plan_batch(orbgpu_batch* b, int nframes, const int* widths, const int
     const int ndesc = nframes * nlevels;
     if ((size_t)ndesc > b->descs_cap) {
         ORBGPU_CUDA_TRY(cudaStreamSynchronize(st));
-        if (b->d_descs) cudaFree(b->d_descs);
+        destroy_graph(b);  // its kernels hold the address
+        cudaFree(b->d_descs);
         b->d_descs = nullptr;
+        b->descs_cap = 0;
         ORBGPU_CUDA_TRY(dev_malloc(&b->d_descs, sizeof(LevelDesc) * b->max_frames * nlevels));
         b->descs_cap = (size_t)b->max_frames * nlevels;
     }
@@ -427,8 +429,10 @@ static int plan_batch(orbgpu_batch* b, int nframes, const int* widths, const int
     pre.insert(pre.end(), b->pyramid.prefix.begin(), b->pyramid.prefix.end());
     if (pre.size() > b->prefix_cap) {
         ORBGPU_CUDA_TRY(cudaStreamSynchronize(st));
-        if (b->d_prefix) cudaFree(b->d_prefix);
+        destroy_graph(b);  // its kernels hold the address
+        cudaFree(b->d_prefix);
         b->d_prefix = nullptr;
+        b->prefix_cap = 0;
         const size_t cap = (size_t)(b->max_frames + 1) * nlevels + (size_t)b->max_frames * nlevels + 1 +
                            (size_t)(2 * nlevels - 1) * b->max_frames;
         ORBGPU_CUDA_TRY(dev_malloc(&b->d_prefix, sizeof(int) * std::max(cap, pre.size())));
@@ -622,6 +626,7 @@ extern "C" int orbgpu_batch_stage_times(orbgpu_batch* b, float* ms, int n) {
 
 // Kernels launched by one orbgpu_batch_extract call.
 extern "C" int orbgpu_batch_launch_count(const orbgpu_batch* b) { return b ? b->launches_per_run : 0; }
+extern "C" int orbgpu_debug_batch_has_graph(const orbgpu_batch* b) { return b && b->graph ? 1 : 0; }
 extern "C" void* orbgpu_batch_stream(const orbgpu_batch* b) { return b ? (void*)b->stream : nullptr; }
 
 // ---------------------------------------------------------------- batched SearchByProjection

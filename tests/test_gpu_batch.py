@@ -286,3 +286,37 @@ def test_batch_frame_projection_vs_oracle(torch, oracle, dz, mono, ori):
         assert nm[f] == refs[f][0], f"frame {f}"
         assert np.array_equal(match[f, :n], refs[f][1]), f"frame {f}"
         assert (match[f, n:] == -3).all()
+
+
+def check_batch(b, torch, imgs, nfs, refs):
+    """One extraction of 'imgs' against the per-frame oracle."""
+    from orb_slam2_detailed_comments_gb300._lib import KEYPOINT_DTYPE
+    k, d, c = b.extract([torch.from_numpy(i).cuda() for i in imgs], nfs)
+    k = k.cpu().numpy().view(KEYPOINT_DTYPE).reshape(len(imgs), -1)
+    d, c = d.cpu().numpy().reshape(len(imgs), -1, 32), c.cpu().numpy()
+    for f, ref in enumerate(refs):
+        assert_kps_equal(k[f, :c[f]], ref.keypoints, f"frame {f}")
+        assert np.array_equal(d[f, :c[f]], ref.descriptors)
+
+
+def test_graph_is_dropped_when_its_buffers_move(torch, oracle):
+    """A captured list, then one of more levels on smaller images (the
+    descriptors and block ranges grow, the arena does not): the graph goes with
+    the buffers, and the first list is extracted anew."""
+    from orb_slam2_detailed_comments_gb300 import synthetic as syn
+    from orb_slam2_detailed_comments_gb300._lib import lib
+    from orb_slam2_detailed_comments_gb300.batch import BatchExtractor
+    b = BatchExtractor(2, 1280, 720, 500, nlevels=4)
+    large = [syn.scene(1280, 720, 80), syn.scene(1241, 376, 81)]
+    small = [syn.scene(320, 240, 82), syn.scene(400, 300, 83)]
+    ref4 = [oracle.extract(i, nfeatures=500, nlevels=4, want_pyramid=False) for i in large]
+    ref8 = [oracle.extract(i, nfeatures=500, nlevels=8, want_pyramid=False) for i in small]
+    for _ in range(3):
+        check_batch(b, torch, large, [500, 500], ref4)
+    assert lib().orbgpu_debug_batch_has_graph(b.handle) == 1
+    b.nlevels = 8
+    check_batch(b, torch, small, [500, 500], ref8)
+    assert lib().orbgpu_debug_batch_has_graph(b.handle) == 0
+    b.nlevels = 4
+    for _ in range(3):
+        check_batch(b, torch, large, [500, 500], ref4)
