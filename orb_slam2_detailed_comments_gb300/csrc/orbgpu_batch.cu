@@ -14,6 +14,7 @@
 #include <algorithm>
 #include <cstdio>
 #include <cstring>
+#include <memory>
 #include <vector>
 
 #include "orbgpu_grid.cuh"
@@ -241,26 +242,34 @@ extern "C" int orbgpu_batch_destroy(orbgpu_batch* b) {
     return ORBGPU_OK;
 }
 
-static int get_plan(orbgpu_batch* b, int w, int h, int nf, const FramePlan** out) {
-    for (FramePlan* p : b->plans)
-        if (p->w == w && p->h == h && p->nf == nf) {
+// A frame's configuration: one of 'known' or 'fresh', else made and added to
+// 'fresh'.
+static int get_plan(const std::vector<FramePlan*>& known, std::vector<std::unique_ptr<FramePlan>>& fresh,
+                    float scale_factor, int nlevels, int w, int h, int nf, const FramePlan** out) {
+    const auto same = [&](const FramePlan& p) { return p.w == w && p.h == h && p.nf == nf; };
+    for (const FramePlan* p : known)
+        if (same(*p)) {
             *out = p;
             return ORBGPU_OK;
         }
-    FramePlan* P = new FramePlan();
+    for (const auto& p : fresh)
+        if (same(*p)) {
+            *out = p.get();
+            return ORBGPU_OK;
+        }
+    std::unique_ptr<FramePlan> P(new FramePlan());
     P->w = w;
     P->h = h;
     P->nf = nf;
-    P->tables = make_tables(nf, b->scale_factor, b->nlevels);
+    P->tables = make_tables(nf, scale_factor, nlevels);
     int rc = level_geometry(P->tables, w, h, P->geom);
     if (rc != ORBGPU_OK) {
-        delete P;
         orbgpu_set_last_error("frame size not supported by the level geometry", __FILE__, __LINE__);
         return rc;
     }
     P->layout.plan(P->geom, 0);
-    P->table_blob.assign(b->nlevels, {});
-    for (int l = 0; l < b->nlevels; l++) {
+    P->table_blob.assign(nlevels, {});
+    for (int l = 0; l < nlevels; l++) {
         const LevelGeom& L = P->geom[l];
         if (l == 0) continue;
         const LevelOffsets& o = P->layout.lv[l];
@@ -269,14 +278,13 @@ static int get_plan(orbgpu_batch* b, int w, int h, int nf, const FramePlan** out
         blob.assign(hi - lo, 0);
         if (!resize_tables(P->geom[l - 1].w, P->geom[l - 1].h, L.w, L.h, (int*)&blob[o.xofs - lo],
                            (short*)&blob[o.xalpha - lo], (int*)&blob[o.yofs - lo], (short*)&blob[o.ybeta - lo])) {
-            delete P;
             orbgpu_set_last_error("resize weights out of range", __FILE__, __LINE__);
             return ORBGPU_ERR_BAD_ARG;
         }
     }
     P->gen = tune_generation();
-    b->plans.push_back(P);
-    *out = P;
+    *out = P.get();
+    fresh.push_back(std::move(P));
     return ORBGPU_OK;
 }
 
@@ -299,28 +307,40 @@ static int plan_batch(orbgpu_batch* b, int nframes, const int* widths, const int
         b->same_sig_runs++;
         return ORBGPU_OK;
     }
+    // a list with a frame that is refused changes nothing: the last extraction
+    // stays what the searches read
+    const bool reshaped = nlevels != b->nlevels || scale_factor != b->scale_factor;
+    std::vector<std::unique_ptr<FramePlan>> fresh;
+    const std::vector<FramePlan*> none, &known = reshaped ? none : b->plans;
+    std::vector<const FramePlan*> cur(nframes);
+    size_t need = b->slot_bytes;
+    for (int f = 0; f < nframes; f++) {
+        const int rc =
+            get_plan(known, fresh, scale_factor, nlevels, widths[f], heights[f], nfeatures[f], &cur[f]);
+        if (rc != ORBGPU_OK) return rc;
+        need = std::max(need, (cur[f]->layout.bytes + 4095) & ~(size_t)4095);
+    }
+    cudaStream_t st = b->stream;
+    ORBGPU_CUDA_TRY(cudaStreamSynchronize(st));
+    // from here on the state changes: until the plan is complete there is no
+    // last extraction, and no signature that a later list could be taken for
+    b->sig.clear();
+    b->nframes = 0;
     b->same_sig_runs = 0;
     b->frame_w.assign(widths, widths + nframes);
     b->frame_h.assign(heights, heights + nframes);
     b->frame_cap = per_frame_cap;
-    if (nlevels != b->nlevels || scale_factor != b->scale_factor) {  // configuration cache is per pyramid shape
-        ORBGPU_CUDA_TRY(cudaStreamSynchronize(b->stream));
+    if (reshaped) {  // configuration cache is per pyramid shape
         for (FramePlan* p : b->plans) delete p;
         b->plans.clear();
         std::fill(b->slot_plan.begin(), b->slot_plan.end(), nullptr);
         b->nlevels = nlevels;
         b->scale_factor = scale_factor;
     }
+    for (auto& p : fresh) b->plans.push_back(p.release());
     b->ini_th = ini_th;
     b->min_th = min_th;
-    b->cur.assign(nframes, nullptr);
-    size_t need = b->slot_bytes;
-    for (int f = 0; f < nframes; f++) {
-        int rc = get_plan(b, widths[f], heights[f], nfeatures[f], &b->cur[f]);
-        if (rc != ORBGPU_OK) return rc;
-        need = std::max(need, (b->cur[f]->layout.bytes + 4095) & ~(size_t)4095);
-    }
-    cudaStream_t st = b->stream;
+    b->cur.swap(cur);
     if (need > b->slot_bytes || !b->arena) {
         ORBGPU_CUDA_TRY(cudaStreamSynchronize(st));
         destroy_graph(b);

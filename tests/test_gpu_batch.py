@@ -320,3 +320,45 @@ def test_graph_is_dropped_when_its_buffers_move(torch, oracle):
     b.nlevels = 4
     for _ in range(3):
         check_batch(b, torch, large, [500, 500], ref4)
+
+
+def test_refused_and_failed_lists_leave_a_usable_batch(torch, oracle):
+    """A list with a frame that is refused (a portrait image) changes nothing:
+    the searches still read the last extraction, also after a refused list of
+    other levels.  After a failed allocation there is no last extraction, and
+    the list before is planned anew."""
+    from orb_slam2_detailed_comments_gb300 import OrbGpuError
+    from orb_slam2_detailed_comments_gb300 import synthetic as syn
+    from orb_slam2_detailed_comments_gb300._lib import lib
+    from orb_slam2_detailed_comments_gb300.batch import BatchExtractor, BatchStereo
+    b = BatchExtractor(3, 1280, 1280, 500)
+    good = [syn.scene(640, 480, 90), np.roll(syn.scene(640, 480, 90), -9, axis=1)]
+    refs = [oracle.extract(i, nfeatures=500, want_pyramid=False) for i in good]
+    check_batch(b, torch, good, [500, 500], refs)
+    n = len(refs[0].keypoints)
+
+    def stereo():
+        return [x[0, :n].cpu().numpy().tobytes() for x in BatchStereo(b).compute([(0, 1)], 40.0, 500.0)]
+    before = stereo()
+    portrait = [torch.zeros(480, 640, dtype=torch.uint8, device="cuda"),
+                torch.zeros(1200, 100, dtype=torch.uint8, device="cuda")]
+    for nlevels in (8, 5):
+        b.nlevels = nlevels
+        with pytest.raises(OrbGpuError):
+            b.extract(portrait + portrait[:1], [500, 500, 500])
+        assert stereo() == before
+        b.nlevels = 8
+        for _ in range(3):
+            check_batch(b, torch, good, [500, 500], refs)
+    large = [torch.from_numpy(syn.scene(1280, 720, 91)).cuda()] * 3
+    for fail in (1, 2, 3):
+        lib().orbgpu_debug_fail_allocations(fail)
+        try:
+            with pytest.raises(OrbGpuError):
+                b.extract(large, [500] * 3)
+        finally:
+            lib().orbgpu_debug_fail_allocations(0)
+        with pytest.raises(OrbGpuError):
+            stereo()
+        check_batch(b, torch, good, [500, 500], refs)
+        assert stereo() == before
