@@ -145,6 +145,9 @@ int orbgpu_descriptor_sincos(const float* x, int n, float* c, float* s);
  * host 128 x 256 floats. */
 int orbgpu_debug_tc_probe(const uint8_t* q128, const uint8_t* t256, float* dots, int* status_out, int lbo, int sbo);
 
+/* The kernel orbgpu_knn2(algo -1) takes: 0 popcount, 1 tensor cores. */
+int orbgpu_debug_knn_algo(int nq, int nt);
+
 /* ------------------------------------------------------------ autotuner parameters */
 /* Launch shapes the autotuner chooses (orb_slam2_detailed_comments_gb300.autotune):
  *   "resize_rows"          strip rows of the resize and blur / FAST pre-test kernels: 8, 22, 36, 64
@@ -153,6 +156,7 @@ int orbgpu_debug_tc_probe(const uint8_t* q128, const uint8_t* t256, float* dots,
  *   "describe_depth"       staging rounds in flight per warp of the descriptor kernel: 2, 4
  *                          (with describe_group 4, 2 is used)
  *   "knn_tc_min_pairs"     query x train size from which orbgpu_knn2(algo -1) uses tcgen05
+ *                          (with more than 256 train rows; under 128 queries, up to 2^22 of them)
  * and three policies for launches too small to fill the device (one frame, a
  * few frames), which the autotuner leaves alone:
  *   "describe_task"        keypoints per descriptor warp task: 0 (by the launch's keypoint

@@ -92,6 +92,7 @@ inline cudaError_t allow_max_dynamic_smem(K* kernel) {
 // for the next ones (allocating and releasing them cost ten times the kernels
 // of a 2,000 x 2,000 call, 0.4 ms at 50,000 x 200,000); a call holds its own
 // until it returns, so that host threads may search with one matcher at once.
+#define KNN_KEEP_BYTES ((size_t)512 << 20)  // kept per matcher, at most
 struct KnnBuffers {
     uint8_t* data = nullptr;
     size_t bytes = 0;

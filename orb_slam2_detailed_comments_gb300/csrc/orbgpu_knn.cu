@@ -169,15 +169,29 @@ extern "C" int orbgpu_knn2_accept(const int* d1, const int* d2, int n, float rat
 int orbgpu_knn2_tc(orbgpu_matcher* m, const uint8_t* query, int nq, const uint8_t* train, int nt, int* idx1, int* d1,
                    int* idx2, int* d2);
 
+// The automatic choice: the tensor cores from the tuned number of pairs on, but
+// not where their operands (128 bytes a row, of a query pair and a train tile
+// at least) cost more than the pairs.  A call in microseconds, popcount against
+// tensor cores:
+// * up to 256 train rows: 1,000,000 x 16 119 / 339, x 128 242 / 365, x 256 394 /
+//   372; 64,000 x 256 72 / 77, x 512 93 / 81;
+// * under 128 queries, a train set whose operands a matcher does not keep:
+//   8 x 8,000,000 722 / 1,382, 64 898 / 1,384, 128 1,457 / 1,381; kept, 8 x
+//   4,000,000 488 / 281.
+extern "C" int orbgpu_debug_knn_algo(int nq, int nt) {
+    if (nt >= (1 << 23)) return 0;  // the tensor-core epilogue packs train indices in 23 bits
+    if ((long long)nq * nt < tunables().knn_tc_min_pairs || nt <= 256) return 0;
+    return nq >= 128 || (size_t)nt * 128 <= KNN_KEEP_BYTES;
+}
+
 extern "C" int orbgpu_knn2(orbgpu_matcher* m, const uint8_t* query, int nq, const uint8_t* train, int nt, int* idx1,
                            int* d1, int* idx2, int* d2, int algo) {
     if (!m || nq < 0 || nt < 0 || (nq > 0 && (!query || !idx1 || !d1 || !idx2 || !d2)) || (nt > 0 && !train) ||
         (algo != 0 && algo != 1 && algo != -1))
         return ORBGPU_ERR_BAD_ARG;
     if (nq == 0) return ORBGPU_OK;
-    if (algo == -1)  // automatic: the tensor cores from the tuned problem size on
-        algo = (long long)nq * nt >= tunables().knn_tc_min_pairs ? 1 : 0;
-    if (nt >= (1 << 23)) algo = 0;  // the tensor-core epilogue packs train indices in 23 bits
+    if (algo == -1) algo = orbgpu_debug_knn_algo(nq, nt);
+    if (nt >= (1 << 23)) algo = 0;
     if (algo == 1 && nt > 0) return orbgpu_knn2_tc(m, query, nq, train, nt, idx1, d1, idx2, d2);
     cudaStream_t st = orbgpu_matcher_stream_internal(m);
     int slice, nslices;

@@ -1023,9 +1023,6 @@ bool frame_ok(const orbgpu_frame* f) {
 
 }  // namespace
 
-// A matcher keeps the workspaces of its kNN calls up to this many bytes.
-#define KNN_KEEP_BYTES ((size_t)512 << 20)
-
 KnnWorkspace::~KnnWorkspace() {
     if (!b) return;
     std::lock_guard<std::mutex> lock(m->knn_mutex);

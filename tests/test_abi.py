@@ -90,3 +90,13 @@ def test_launch_policies_set_and_get_without_gpu(library):
         for bad in (-1, 3, 64):
             assert library.orbgpu_tune_set(name.encode(), C.c_longlong(bad)) != 0
         assert library.orbgpu_tune_set(name.encode(), C.c_longlong(old)) == 0
+
+
+@pytest.mark.parametrize("nq,nt,algo", [
+    (2000, 2000, 0), (2000, 4195, 1), (50000, 200000, 1), (0, 5000, 0), (5000, 0, 0),
+    # few train rows: their tiles of 160 and the queries' operands are mostly padding
+    (1000000, 16, 0), (2**31 - 1, 256, 0), (1000000, 256, 0), (1000000, 257, 1),
+    # few queries: up to the train rows whose operands a matcher keeps
+    (2, 2**22, 1), (2, 2**22 + 1, 0), (127, 2**23 - 1, 0), (128, 2**23 - 1, 1), (128, 2**23, 0), (50000, 2**23, 0)])
+def test_knn_automatic_choice_without_gpu(library, nq, nt, algo):
+    assert library.orbgpu_debug_knn_algo(nq, nt) == algo
