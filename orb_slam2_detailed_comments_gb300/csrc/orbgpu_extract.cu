@@ -735,18 +735,18 @@ static int ensure_io(orbgpu_extractor* ex, size_t sync, size_t out, size_t image
     ex->image_cap = image;
     return ORBGPU_OK;
 }
+static bool pageable(const void* p) {
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, p) == cudaSuccess) return at.type == cudaMemoryTypeUnregistered;
+    cudaGetLastError();
+    return false;
+}
 // Level 0 from the caller's image.  A pageable image goes through page-locked
-// memory in the plane's row pitch, one chunk copied on while the next is
-// staged: the runtime's own copy of a pageable 640x480 image holds the caller
-// for 31 us, the staging 10.
+// memory ('stage', h_image) in the plane's row pitch, one chunk copied on while
+// the next is staged: the runtime's own copy of a pageable 640x480 image holds
+// the caller for 31 us, the staging 10.
 static int upload_image(orbgpu_extractor* ex, uint8_t* dst, size_t pitch, const uint8_t* image, size_t step, int width,
-                        int height, int image_mem, cudaStream_t st) {
-    bool stage = false;
-    if (image_mem != ORBGPU_MEM_DEVICE) {
-        cudaPointerAttributes at;
-        if (cudaPointerGetAttributes(&at, image) == cudaSuccess) stage = at.type == cudaMemoryTypeUnregistered;
-        else cudaGetLastError();
-    }
+                        int height, int image_mem, bool stage, cudaStream_t st) {
     if (!stage) {
         ORBGPU_CUDA_TRY(cudaMemcpy2DAsync(dst, pitch, image, step, width, height,
                                           image_mem == ORBGPU_MEM_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, st));
@@ -865,7 +865,8 @@ extern "C" int orbgpu_extract(orbgpu_extractor* ex, const uint8_t* image, int wi
     // outputs go to the caller's device arrays or through the call's block
     const bool to_host = out_mem != ORBGPU_MEM_DEVICE;
     const int staged = to_host ? std::min(capacity, P.max_total) : 0;
-    rc = ensure_io(ex, P.sync_bytes, host_out_bytes(staged), image_mem != ORBGPU_MEM_DEVICE ? g[0].pitch * (size_t)height : 0);
+    const bool stage = image_mem != ORBGPU_MEM_DEVICE && pageable(image);
+    rc = ensure_io(ex, P.sync_bytes, host_out_bytes(staged), stage ? g[0].pitch * (size_t)height : 0);
     if (rc != ORBGPU_OK) return rc;
     // the outputs follow the sync words
     const size_t out_off = align256(P.sync_bytes), desc_off = out_off + align256(sizeof(orbgpu_keypoint) * staged);
@@ -883,7 +884,7 @@ extern "C" int orbgpu_extract(orbgpu_extractor* ex, const uint8_t* image, int wi
     cudaStream_t st = ex->stream;
     ORBGPU_CUDA_TRY(cudaMemcpyAsync(ex->d_io, ex->h_io, IO_SYNC + P.sync_bytes, cudaMemcpyHostToDevice, st));
     // level 0 = the image
-    rc = upload_image(ex, hd[0].dst, hd[0].pitch, image, step, width, height, image_mem, st);
+    rc = upload_image(ex, hd[0].dst, hd[0].pitch, image, step, width, height, image_mem, stage, st);
     if (rc != ORBGPU_OK) return rc;
     if (P.fused) {
         launch_pyramid(d_descs, P.pyramid, nullptr, 1, nl, d_status + 4, d_status, st);

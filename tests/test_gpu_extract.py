@@ -74,6 +74,28 @@ def test_device_in_device_out(torch, oracle):
     assert np.array_equal(desc.cpu().numpy(), ref.descriptors)
 
 
+def test_page_locked_images_reserve_no_staging(torch):
+    """A page-locked image after a device image of its size allocates nothing;
+    a pageable one then needs its staging, and works once there is memory."""
+    from orb_slam2_detailed_comments_gb300 import OrbGpuError
+    from orb_slam2_detailed_comments_gb300 import synthetic as syn
+    from orb_slam2_detailed_comments_gb300._lib import lib
+    img = syn.scene(640, 480, 19)
+    pinned = torch.from_numpy(img).pin_memory()
+    ex = extractor(500)
+    ref = ex(torch.from_numpy(img).cuda())
+    lib().orbgpu_debug_fail_allocations(1)
+    try:
+        out = ex(pinned.numpy())
+        with pytest.raises(OrbGpuError):
+            ex(img)
+    finally:
+        lib().orbgpu_debug_fail_allocations(0)
+    for got in (out, ex(img), ex(pinned.numpy())):
+        assert_kps_equal(got[0], ref[0])
+        assert np.array_equal(got[1], ref[1])
+
+
 def test_edge_cases(torch):
     from orb_slam2_detailed_comments_gb300 import OrbGpuError
     ex = extractor(1000)
