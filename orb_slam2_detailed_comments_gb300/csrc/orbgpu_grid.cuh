@@ -368,9 +368,12 @@ __device__ __forceinline__ int proj_resolve_block(const orbgpu_keypoint* kps, in
         second = best == PROJ_NOKEY ? s2 : b;
         best = best == PROJ_NOKEY ? b : best;
     };
-    // whether a key behind 'last' can change what (best, second) decide
+    // whether a key behind 'last' can change what (best, second) decide (with a
+    // negative ratio a farther one fails the test where a nearer one passes)
+    const bool falling = !(nnratio >= 0.0f);
     auto look_on = [&](uint32_t best, uint32_t second, uint32_t last) {
-        return second == PROJ_NOKEY && (best == PROJ_NOKEY ? dist_of(last) <= ORBGPU_TH_HIGH : ratio_fails(best, last));
+        return second == PROJ_NOKEY &&
+               (best == PROJ_NOKEY ? dist_of(last) <= ORBGPU_TH_HIGH : falling || ratio_fails(best, last));
     };
     auto full_scan = [&](int i, int c, uint32_t& best, uint32_t& second) {
         best = PROJ_NOKEY;

@@ -278,6 +278,27 @@ def test_projection_search_limits(torch, oracle, n, m, w, h, th, nnratio, entrop
     assert nm == ref[0] and np.array_equal(match, ref[1])
 
 
+@pytest.mark.parametrize("nnratio", [-1.0, -0.5, 0.0, 0.9])
+def test_projection_search_looks_behind_equal_keys(torch, oracle, nnratio):
+    """Map points whose first four (and eight) keys are at distance 0 and all but
+    one claimed: with a negative ratio the key behind them decides."""
+    from oracle import pyoracle
+    from orb_slam2_detailed_comments_gb300 import FrameView, ORBmatcher
+    from orb_slam2_detailed_comments_gb300._lib import KEYPOINT_DTYPE, MAPPOINT_DTYPE
+    w, h = 640, 480
+    k, d, mps = np.zeros(5 + 9, KEYPOINT_DTYPE), np.zeros((5 + 9, 32), np.uint8), np.zeros(4 + 8, MAPPOINT_DTYPE)
+    k["x"][:5], k["x"][5:], k["y"], k["class_id"] = 100, 400, 200, -1
+    d[[4, 13], 0] = 31  # five bits from the others
+    mps["proj_x"][:4], mps["proj_x"][4:], mps["proj_y"], mps["view_cos"] = 100, 400, 200, 1.0
+    mps["proj_xr"], mps["track_in_view"] = -1, 1
+    mpd = np.zeros((len(mps), 32), np.uint8)
+    s, _ = pyoracle.scale_tables(8, 1.2)
+    ref = oracle.search_by_projection(k.view(pyoracle.KP_DTYPE), d, w, h, mps.view(pyoracle.MP_DTYPE), mpd, th=1.0,
+                                      nnratio=nnratio, claimed=np.zeros(len(k), np.uint8))
+    nm, match = ORBmatcher(nnratio, True).SearchByProjection(FrameView(k, d, w, h, s), mps, mpd, 1.0)
+    assert nm == ref[0] and np.array_equal(match, ref[1])
+
+
 @pytest.mark.parametrize("n1,n2,window,nnratio,entropy", [
     (1, 1, 10, 0.9, 2), (300, 33, 60, 0.9, 1), (2049, 1500, 40, 0.9, 1), (3000, 3000, 30, 0.6, 2),
     (9000, 8200, 20, 0.9, 1), (1200, 1200, 100, 1.2, 1)])
