@@ -145,6 +145,12 @@ int orbgpu_descriptor_sincos(const float* x, int n, float* c, float* s);
  * host 128 x 256 floats. */
 int orbgpu_debug_tc_probe(const uint8_t* q128, const uint8_t* t256, float* dots, int* status_out, int lbo, int sbo);
 
+/* The tensor-core kNN's product of one query tile (nq <= 128 rows) and one
+ * train tile (nt <= 160 rows) of host descriptors, through its own expansion,
+ * operand layout and instruction: dots, host 128 x 160 floats (the last row of
+ * a set repeats), and maxima, host 128 x 5 floats (of every 32 train rows). */
+int orbgpu_debug_knn_tile(const uint8_t* query, int nq, const uint8_t* train, int nt, float* dots, float* maxima,
+                          int* status_out);
 /* The kernel orbgpu_knn2(algo -1) takes: 0 popcount, 1 tensor cores. */
 int orbgpu_debug_knn_algo(int nq, int nt);
 

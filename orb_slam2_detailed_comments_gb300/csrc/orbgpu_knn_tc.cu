@@ -42,7 +42,7 @@ cudaStream_t orbgpu_matcher_stream_internal(orbgpu_matcher* m);
 
 namespace orbgpu {
 
-// the layout self-test: one 128 x 256 tile of FP8 +-1 rows
+// the FP8 operand layout's test: one 128 x 256 tile of +-1 rows
 #define TCP_M 128
 #define TCP_N 256
 #define TCP_K 256                        // bytes (= FP8 elements) per row
@@ -218,6 +218,19 @@ __device__ __forceinline__ void tc_fill8(uint32_t taddr, uint32_t v) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%1,%1,%1,%1,%1,%1,%1};" ::"r"(taddr), "r"(v) : "memory");
 }
 
+// Block scales of 1 (UE8M0 0x7F) in the scale columns of this warp's 32 TMEM
+// lanes (ta: its first lane); every lane holds them, whichever an MMA reads.
+__device__ __forceinline__ void tc_fill_scales(uint32_t ta) {
+    for (int c = 0; c < 512 - TC_SCALE_COL; c += 8) tc_fill8(ta + TC_SCALE_COL + c, 0x7F7F7F7Fu);
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+// A tile's operand descriptor, and the MMAs of two tiles' whole rows.
+__device__ __forceinline__ uint64_t tc_operand(const void* tile) { return smem_desc(tile, 128, 8 * TC_ROW); }
+__device__ __forceinline__ void tc_tile_mma(uint32_t d, uint64_t ad, uint64_t bd, uint32_t idesc, uint32_t scales) {
+#pragma unroll
+    for (int ks = 0; ks < TC_ROW / 32; ks++) tc_mma_mxf4(d, ad + 16 * ks, bd + 16 * ks, idesc, scales, ks > 0);
+}
+
 // 32 consecutive FP32 columns of this warp's 32 TMEM lanes.
 __device__ __forceinline__ void tc_ld32(uint32_t taddr, float (&v)[32]) {
     uint32_t r[32];
@@ -298,6 +311,66 @@ __global__ void __launch_bounds__(128) k_tc_probe(const uint8_t* qa, const uint8
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 256;" ::"r"(tmem));
 }
 
+// One query tile against one train tile as k_knn_tc takes them (operand strides,
+// instruction descriptor, scale columns, the reduction of a group's columns):
+// the 128 x 160 dot products and every row's five group maxima.
+__global__ void __launch_bounds__(128) k_knn_tile_probe(const uint8_t* qa, const uint8_t* tb, float* dots, float* maxima,
+                                                        int* status) {
+    extern __shared__ __align__(1024) uint8_t tc_smem[];
+    uint8_t* sB = tc_smem + TC_QTILE_BYTES;
+    __shared__ __align__(8) uint64_t bar_load, bar_mma;
+    __shared__ uint32_t tmem_base;
+    const int warp = threadIdx.x >> 5;
+    if (threadIdx.x == 0) {
+        mbar_init(&bar_load, 1);
+        mbar_init(&bar_mma, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(&tmem_base)));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = tmem_base, ta = tmem + ((uint32_t)(warp * 32) << 16);
+    tc_fill_scales(ta);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    if (threadIdx.x == 0) {
+        mbar_expect_tx(&bar_load, TC_QTILE_BYTES + TC_TTILE_BYTES);
+        bulk_g2s(tc_smem, qa, TC_QTILE_BYTES, &bar_load);
+        bulk_g2s(sB, tb, TC_TTILE_BYTES, &bar_load);
+        if (mbar_wait(&bar_load, 0)) {
+            tc_fence_after();
+            tc_tile_mma(tmem, tc_operand(tc_smem), tc_operand(sB), idesc_mxf4(TC_M, TC_N), tmem + TC_SCALE_COL);
+            tc_commit(&bar_mma);
+        } else {
+            atomicOr(status, 1);
+            mbar_wait(&bar_load, 0);  // give the copies in flight one more bounded wait
+        }
+    }
+    __syncthreads();
+    if (!(*status & 1)) {
+        const bool done = __all_sync(0xffffffffu, mbar_wait(&bar_mma, 0));
+        if (!done) atomicOr(status, 2);
+        tc_fence_after();
+        for (int g = 0; done && g < TC_GROUPS; g++) {
+            float v[32];
+            uint32_t r[TC_GROUP];
+            tc_ld32(ta + (uint32_t)(g * TC_GROUP), v);
+            const float m = tc_max32(ta + (uint32_t)(g * TC_GROUP), r);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            for (int i = 0; i < TC_GROUP; i++) dots[(size_t)threadIdx.x * TC_N + g * TC_GROUP + i] = v[i];
+            maxima[threadIdx.x * TC_GROUPS + g] = m;
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem));
+}
+
 // mbar_wait_sleep by every lane of the warp, with one outcome.
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity) {
     return __all_sync(0xffffffffu, mbar_wait_sleep(bar, parity));
@@ -366,13 +439,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = tmem_base;
-    // every block scale is 1 (UE8M0 0x7F): the scale columns of all lanes hold
-    // it, whichever of them an MMA reads
-    if (warp < 4) {
-        for (int c = 0; c < 512 - TC_SCALE_COL; c += 8)
-            tc_fill8(tmem + ((uint32_t)(warp * 32) << 16) + TC_SCALE_COL + c, 0x7F7F7F7Fu);
-        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-    }
+    if (warp < 4) tc_fill_scales(tmem + ((uint32_t)(warp * 32) << 16));
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -416,7 +483,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
         const int u = warp - issuer;
         const bool one = tc_elect();
         const uint32_t idesc = idesc_mxf4(TC_M, TC_N), d = tmem + (uint32_t)(u * TC_N);
-        const uint64_t a0 = smem_desc(sA, 128, 8 * TC_ROW), b0 = smem_desc(sB, 128, 8 * TC_ROW);
+        const uint64_t a0 = tc_operand(sA), b0 = tc_operand(sB);
         bool ok = true;
         int segs = 0, last = -1;  // last query tile issued
         TcItem it = first;
@@ -438,9 +505,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
                 const uint64_t ad = a0 + (uint32_t)((((segs - 1) & 1) * TC_QPAIR + (j & 1)) * (TC_QTILE_BYTES >> 4)),
                                bd = b0 + (uint32_t)(s * (TC_TTILE_BYTES >> 4));
                 if (one) {
-#pragma unroll
-                    for (int ks = 0; ks < TC_ROW / 32; ks++)
-                        tc_mma_mxf4(d, ad + 16 * ks, bd + 16 * ks, idesc, tmem + TC_SCALE_COL, ks > 0);
+                    tc_tile_mma(d, ad, bd, idesc, tmem + TC_SCALE_COL);
                     tc_commit(&bar_empty[s]);  // the train buffer is free when both tiles' MMAs are done
                     tc_commit(&bar_acc[u]);    // and the accumulator ready
                 }
@@ -625,6 +690,43 @@ extern "C" int orbgpu_debug_tc_probe(const uint8_t* q128, const uint8_t* t256, f
     cudaFree(eq);
     cudaFree(et);
     cudaFree(dd);
+    cudaFree(st);
+    return ORBGPU_OK;
+}
+
+// The kNN kernel's tile product: nq <= 128 queries against nt <= 160 train rows
+// (host arrays), expanded as for a search; the last row of a set repeats in its
+// tile.
+extern "C" int orbgpu_debug_knn_tile(const uint8_t* query, int nq, const uint8_t* train, int nt, float* dots,
+                                     float* maxima, int* status_out) {
+    if (!query || !train || nq < 1 || nq > TC_M || nt < 1 || nt > TC_N || !dots || !maxima || !status_out)
+        return ORBGPU_ERR_BAD_ARG;
+    uint8_t *dq = nullptr, *dt = nullptr, *operands = nullptr;
+    float* out = nullptr;
+    int* st = nullptr;
+    const size_t nd = (size_t)TC_M * TC_N, nm = (size_t)TC_M * TC_GROUPS;
+    ORBGPU_CUDA_TRY(cudaMalloc(&dq, 32 * (size_t)nq));
+    ORBGPU_CUDA_TRY(cudaMalloc(&dt, 32 * (size_t)nt));
+    ORBGPU_CUDA_TRY(cudaMalloc(&operands, TC_QTILE_BYTES + TC_TTILE_BYTES));
+    ORBGPU_CUDA_TRY(cudaMalloc(&out, sizeof(float) * (nd + nm)));
+    ORBGPU_CUDA_TRY(cudaMalloc(&st, sizeof(int)));
+    ORBGPU_CUDA_TRY(cudaMemcpy(dq, query, 32 * (size_t)nq, cudaMemcpyHostToDevice));
+    ORBGPU_CUDA_TRY(cudaMemcpy(dt, train, 32 * (size_t)nt, cudaMemcpyHostToDevice));
+    ORBGPU_CUDA_TRY(cudaMemset(out, 0, sizeof(float) * (nd + nm)));
+    const long qth = TC_QTILE_BYTES / 16, tth = TC_TTILE_BYTES / 16;
+    k_expand_fp4<<<(unsigned)((qth + tth + 255) / 256), 256>>>(dq, nq, qth, operands, dt, nt, tth,
+                                                             operands + TC_QTILE_BYTES, st);
+    ORBGPU_CUDA_TRY(allow_max_dynamic_smem(k_knn_tile_probe));
+    k_knn_tile_probe<<<1, 128, TC_QTILE_BYTES + TC_TTILE_BYTES>>>(operands, operands + TC_QTILE_BYTES, out, out + nd, st);
+    ORBGPU_CUDA_TRY(cudaGetLastError());
+    ORBGPU_CUDA_TRY(cudaDeviceSynchronize());
+    ORBGPU_CUDA_TRY(cudaMemcpy(dots, out, sizeof(float) * nd, cudaMemcpyDeviceToHost));
+    ORBGPU_CUDA_TRY(cudaMemcpy(maxima, out + nd, sizeof(float) * nm, cudaMemcpyDeviceToHost));
+    ORBGPU_CUDA_TRY(cudaMemcpy(status_out, st, sizeof(int), cudaMemcpyDeviceToHost));
+    cudaFree(dq);
+    cudaFree(dt);
+    cudaFree(operands);
+    cudaFree(out);
     cudaFree(st);
     return ORBGPU_OK;
 }

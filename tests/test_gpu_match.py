@@ -226,6 +226,28 @@ def test_tc_operand_layout(torch):
     assert np.array_equal(dots, (bq @ bt.T).astype(np.float32))
 
 
+@pytest.mark.parametrize("nq,nt", [(128, 160), (127, 129), (1, 1)])
+def test_knn_tile_product(torch, nq, nt):
+    """Every dot product and group maximum of a tile as the tensor-core kNN forms
+    them equals the integer ones, those of the repeated last rows included."""
+    import ctypes as C
+    from orb_slam2_detailed_comments_gb300._lib import lib
+    from orb_slam2_detailed_comments_gb300 import synthetic as syn
+    q, t = syn.random_descriptors(nq, 21), syn.random_descriptors(nt, 22)
+    q[0], t[0] = 255, 255  # the extremes: 256 and, where there is a last row, -256
+    t[-1] = 255 if nt == 1 else 0
+    dots, maxima = np.zeros((128, 160), np.float32), np.zeros((128, 5), np.float32)
+    st = np.full(1, -1, np.int32)
+    rc = lib().orbgpu_debug_knn_tile(q.ctypes.data_as(C.c_void_p), nq, t.ctypes.data_as(C.c_void_p), nt,
+                                     dots.ctypes.data_as(C.c_void_p), maxima.ctypes.data_as(C.c_void_p),
+                                     st.ctypes.data_as(C.c_void_p))
+    assert rc == 0 and st[0] == 0
+    signs = [1 - 2 * np.unpackbits(a, axis=1).astype(np.int32) for a in (q, t)]
+    ref = signs[0][np.minimum(np.arange(128), nq - 1)] @ signs[1][np.minimum(np.arange(160), nt - 1)].T
+    assert np.array_equal(dots, ref.astype(np.float32))
+    assert np.array_equal(maxima, ref.reshape(128, 5, 32).max(2).astype(np.float32))
+
+
 @pytest.mark.parametrize("nq,nt", [(1, 1), (129, 257), (1000, 20000)])
 def test_knn_tensor_cores_oracle(torch, oracle, nq, nt):
     from orb_slam2_detailed_comments_gb300 import ORBmatcher
