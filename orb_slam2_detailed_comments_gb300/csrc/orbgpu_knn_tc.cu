@@ -67,6 +67,10 @@ namespace orbgpu {
 #define TC_GROUPS (TC_N / TC_GROUP)     // groups of a train tile
 #define TC_THREADS (32 * (TC_EPI_WARPS + 1 + TC_ACCS))  // + producer warp + MMA warps
 static_assert(TC_N % TC_GROUP == 0, "whole groups");
+// An issuer takes tiles of two items in three.  With the stages a multiple of
+// the accumulators it takes from a stage either at every fill or never, so it
+// sees every phase of the stage's barrier and a parity names one fill.
+static_assert(TC_STAGES % TC_ACCS == 0, "an issuer would skip fills of a stage");
 
 // ---------------------------------------------------------------- operand layout
 // Byte offset of byte k of row r inside a tile of 256-byte rows (the
