@@ -39,9 +39,7 @@
 namespace orbgpu {
 
 #define DD_WARPS 4          // warps per block
-#ifndef DD_BLOCKS_PER_SM
 #define DD_BLOCKS_PER_SM 8  // resident blocks per SM (64 registers x 128 threads)
-#endif
 
 struct DDArgs {
     const uint4* pool;  // pool_rows x 32 bytes
