@@ -1885,13 +1885,15 @@ void launch_describe(const LevelDesc* descs, int ndescs, long features, orbgpu_k
     const int nsm = nsm_of_current_device();
     const int R = tunables().describe_group, D = R * tunables().describe_depth > 8 ? 2 : tunables().describe_depth;
     // D buffers of R box slots per warp, 24 slots (60 KiB) per block: three
-    // blocks per SM.  A launch short of keypoints is bound by one warp's
-    // staging rounds, a long one by its tasks' double-precision passes (one per
-    // task, whatever its lanes): up to 8 keypoints per warp of the full device
-    // it takes as many blocks as keypoints give warps (one 640x480 frame 32 ->
-    // 19 us against 8 keypoints a task, five frames 43 -> 29), beyond that the
-    // blocks per SM that hold them in tasks of at most 32 (96,000 keypoints: 94
-    // us with two, 117 with three; 128,000: 136 with three, 159 with two)
+    // blocks per SM.  A launch short of keypoints is bound by one warp's staging
+    // rounds: up to 8 keypoints per warp of the full device it takes as many
+    // blocks as keypoints give warps (the describe stage of one 1280x720 frame
+    // 12.3 us, with 38 / 76 / 152 blocks 18.4 / 16.0 / 14.3; 10,000 keypoints
+    // 22.5, with 76 / 152 / 304 blocks 30.4 / 22.5 / 20.5).  A longer one takes
+    // the blocks per SM that hold its keypoints in tasks of at most 32, so that
+    // no warp has a second task (64,000 keypoints 121 us with one, 65 with two,
+    // 70 with three; 96,000 90 with two, 88 with three; 128,000 154 with two,
+    // 111 with three; at 48,000, where one suffices, 63 against 55 and 54).
     const int wpb = 24 / (R * D);
     const size_t smem = (size_t)D * R * wpb * DESC_SLOT + 128 + sizeof(int) * (ndescs + 1);
     const long full = (long)nsm * wpb;  // warps of one block per SM
