@@ -182,27 +182,80 @@ __global__ void k_exclusive_scan(const int* in, int n, int* out, int* total) {
 // over the keypoints: round r fixes the first r + 1).  The match of an F2
 // keypoint is then its last taker's, and the rotation histogram counts every
 // taker.  A warp walking the keypoints in order took 236 us at 640 x 480 /
-// 1000 features, this 9.  Arrays (shared memory when 'local', else global):
-// choice and its distance (n1 each), two sets of list heads (n2) and links (n1).
+// 1000 features, this 9.  Keypoints that depend on one another in a long chain
+// (a row of alike features, each with a second candidate that the one before
+// leaves it) settle one a round: after INIT_ROUNDS rounds, or where a list of
+// takers passes INIT_TAKERS, the warp's walk decides after all, so that the
+// time stays linear in the keypoints.  Arrays (shared memory when 'local', else
+// global): choice and its distance (n1 each), two sets of list heads (n2) and
+// links (n1).
+#define INIT_ROUNDS 64
+#define INIT_TAKERS 4096
+// (best, second): the least (distance, position) key and the least distance of
+// the others, with one more key.
+__device__ __forceinline__ void init_insert(uint64_t key, uint64_t& best, int& second) {
+    const uint64_t other = key < best ? best : key;
+    best = key < best ? key : best;
+    if (other != ~0ull) second = min(second, (int)(other >> 40));
+}
+__device__ __forceinline__ bool init_accepts(uint64_t best, int second, float nnratio) {
+    const int d = (int)(best >> 40);
+    return best != ~0ull && d <= ORBGPU_TH_LOW && (float)d < __fmul_rn((float)second, nnratio);
+}
+// The walk, by the calling warp: choice[n1]; least[n2] (the matched distances)
+// holds 0x7fffffff before.
+__device__ __forceinline__ void init_walk(int n1, int slot_cap, const int* slot_count, const uint64_t* slots, float nnratio,
+                                          int* choice, int* least) {
+    const int lane = threadIdx.x & 31;
+    for (int i0 = 0; i0 < n1; i0 += 32) {
+        const int mine = i0 + lane < n1 ? min(slot_count[i0 + lane], slot_cap) : 0;
+        if (i0 + lane < n1) choice[i0 + lane] = -1;
+        __syncwarp();
+        unsigned todo = __ballot_sync(0xffffffffu, mine > 0);
+        while (todo) {
+            const int t = __ffs(todo) - 1, cnt = __shfl_sync(0xffffffffu, mine, t);
+            todo &= todo - 1;
+            const uint64_t* row = slots + (size_t)(i0 + t) * slot_cap;
+            uint64_t best = ~0ull;
+            int second = 0x7fffffff;
+            for (int e = lane; e < cnt; e += 32) {
+                const uint64_t key = row[e];
+                if (least[key & 0xFFFFF] > (int)(key >> 40)) init_insert(key, best, second);
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                const uint64_t ob = __shfl_xor_sync(0xffffffffu, best, o);
+                const int os = __shfl_xor_sync(0xffffffffu, second, o);
+                second = min(second, os);
+                init_insert(ob, best, second);
+            }
+            if (lane == 0 && init_accepts(best, second, nnratio)) {
+                choice[i0 + t] = (int)(best & 0xFFFFF);
+                least[best & 0xFFFFF] = (int)(best >> 40);
+            }
+            __syncwarp();  // lane 0's update is seen by the next keypoint's filter
+        }
+    }
+}
 __host__ __device__ inline size_t init_resolve_bytes(int n1, int n2) { return 4 * (4 * (size_t)n1 + 2 * (size_t)n2); }
-__global__ void __launch_bounds__(1024)
+__global__ void __launch_bounds__(1024, 1)
     k_init_resolve(const orbgpu_keypoint* kps1, int n1, const orbgpu_keypoint* kps2, int n2, int slot_cap,
                    const int* slot_count, const uint64_t* slots, float nnratio, int check_ori, int local, int* work,
                    int* matches12, int* nmatches_out) {
     extern __shared__ int s_init[];
     __shared__ int hist[ORBGPU_HISTO_LENGTH];
-    __shared__ int s_flag[3], s_nm, s_ind[3];
+    __shared__ int s_flag[3], s_long, s_nm, s_ind[3];
     const int tid = threadIdx.x, nt = blockDim.x;
     int* const choice = local ? s_init : work;  // n1: F2 keypoint or -1
     int* const cdist = choice + n1;             // n1
     int *head_r = cdist + n1, *head_w = head_r + n2, *next_r = head_w + n2, *next_w = next_r + n1;
     if (tid < ORBGPU_HISTO_LENGTH) hist[tid] = 0;
     if (tid < 3) s_flag[tid] = 0;
-    if (tid == 0) s_nm = 0;
+    if (tid == 0) s_nm = s_long = 0;
     for (int j = tid; j < n2; j += nt) head_r[j] = head_w[j] = -1;
     for (int i = tid; i < n1; i += nt) choice[i] = -2;
     bool converged = false;
-    for (int round = 0; round <= n1 + 1 && !converged; round++) {
+    for (int round = 0; round < INIT_ROUNDS && !converged; round++) {
         if (tid == 0) s_flag[(round + 1) % 3] = 0;
         __syncthreads();
         // the choices' distances of the round before are read below, this
@@ -217,19 +270,14 @@ __global__ void __launch_bounds__(1024)
                 const uint64_t key = row[e];
                 const int dist = (int)(key >> 40), j = (int)(key & 0xFFFFF);
                 bool taken = false;
-                for (int k = head_r[j]; k >= 0 && !taken; k = next_r[k]) taken = k < i && cdist[k] <= dist;
+                int k = head_r[j], seen = 0;
+                for (; k >= 0 && !taken && seen < INIT_TAKERS; k = next_r[k], seen++) taken = k < i && cdist[k] <= dist;
                 if (taken) continue;
-                if (key < best) {
-                    if (best != ~0ull) second = min(second, (int)(best >> 40));
-                    best = key;
-                } else {
-                    second = min(second, dist);
-                }
+                if (k >= 0) s_long = 1;
+                init_insert(key, best, second);
             }
-            const int d = (int)(best >> 40);
-            const bool ok = best != ~0ull && d <= ORBGPU_TH_LOW && (float)d < __fmul_rn((float)second, nnratio);
-            r = ok ? (int)(best & 0xFFFFF) : -1;
-            rd = d;
+            r = init_accepts(best, second, nnratio) ? (int)(best & 0xFFFFF) : -1;
+            rd = (int)(best >> 40);
         };
         const bool few = n1 <= 2 * nt;  // results wait in registers, else in the links' spare array
         for (int i = tid; i < n1; i += nt, q++) {
@@ -262,6 +310,7 @@ __global__ void __launch_bounds__(1024)
             if (r >= 0) next_w[i] = atomicExch(&head_w[r], i);
         }
         __syncthreads();
+        if (s_long) break;
         converged = s_flag[round % 3] == 0;
         int* t = head_r;
         head_r = head_w;
@@ -272,9 +321,15 @@ __global__ void __launch_bounds__(1024)
         if (!converged)
             for (int j = tid; j < n2; j += nt) head_w[j] = -1;
     }
-    // the owner of each F2 keypoint: its last taker
     int* const owner = head_w;
     __syncthreads();
+    if (!converged) {
+        for (int j = tid; j < n2; j += nt) owner[j] = 0x7fffffff;
+        __syncthreads();
+        if (tid < 32) init_walk(n1, slot_cap, slot_count, slots, nnratio, choice, owner);
+        __syncthreads();
+    }
+    // the owner of each F2 keypoint: its last taker
     for (int j = tid; j < n2; j += nt) owner[j] = -1;
     __syncthreads();
     const float factor = __fdiv_rn((float)ORBGPU_HISTO_LENGTH, 360.0f);
@@ -332,7 +387,7 @@ __global__ void __launch_bounds__(1024)
     nm = warp_sum(nm);
     if ((tid & 31) == 0 && nm) atomicAdd(&s_nm, nm);
     __syncthreads();
-    if (tid == 0) *nmatches_out = converged ? s_nm : -1;
+    if (tid == 0) *nmatches_out = s_nm;
 }
 
 // ----------------------------------------------------------------- SearchByProjection(Frame, MapPoints)
@@ -1164,10 +1219,6 @@ extern "C" int orbgpu_search_for_initialization(orbgpu_matcher* m, const orbgpu_
         if (m->h_pinned[0] > slot_cap) {  // a window held more candidates than a row: widen and redo
             slot_cap = ((m->h_pinned[0] + 63) / 64) * 64;
             continue;
-        }
-        if (m->h_pinned[1] < 0) {
-            orbgpu_set_last_error("initialisation search: resolution failed", __FILE__, __LINE__);
-            return ORBGPU_ERR_CUDA;
         }
         *nmatches = m->h_pinned[1];
         // vbPrevMatched update (src/ORBmatcher.cc:712-714)

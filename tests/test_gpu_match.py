@@ -346,6 +346,48 @@ def test_initialization_search_limits(torch, oracle, n1, n2, window, nnratio, en
     assert nm == ref[0] and np.array_equal(m12, ref[1]) and np.array_equal(prev_out, ref[2])
 
 
+def plain_frame(x, y, bits):
+    """Keypoints of level 0 at (x, y) whose descriptors have 'bits' leading ones."""
+    from orb_slam2_detailed_comments_gb300._lib import KEYPOINT_DTYPE
+    k = np.zeros(len(x), KEYPOINT_DTYPE)
+    k["x"], k["y"], k["class_id"] = x, y, -1
+    return k, np.packbits(np.arange(256) < np.asarray(bits)[:, None], axis=1, bitorder="little")
+
+
+@pytest.mark.parametrize("kind,n", [("chain", 63), ("chain", 66), ("chain", 2000), ("chain", 30000),
+                                    ("takers", 4096), ("takers", 6000), ("takers", 20000)])
+def test_initialization_search_long_dependencies(torch, oracle, kind, n):
+    """Keypoints that each decide for the next one (a row of alike features, the
+    windows seeing two of them), and thousands that take one keypoint in turn:
+    the same matches, in time linear in the keypoints (a round of the resolution
+    for every link would grow with their square)."""
+    import time
+    from oracle import pyoracle
+    from orb_slam2_detailed_comments_gb300 import FrameView, ORBmatcher
+    i = np.arange(n)
+    if kind == "chain":
+        w, h, window = 5 * n, 480, 3
+        k1, d1 = plain_frame(4 * i + 2, 100, 0 * i)
+        k2, d2 = plain_frame(4 * np.arange(n + 1), 100, np.zeros(n + 1))
+        k1["x"][0] = 4  # sees the second one only
+    else:
+        w, h, window = 640, 480, 10
+        k1, d1 = plain_frame(100 + i % 7, 100, 49 - 50 * i // n)
+        k2, d2 = plain_frame([103], [100], [0])
+    prev = np.ascontiguousarray(np.stack([k1["x"], k1["y"]], 1))
+    s, _ = pyoracle.scale_tables(8, 1.2)
+    ref = oracle.search_for_initialization(k1.view(pyoracle.KP_DTYPE), d1, k2.view(pyoracle.KP_DTYPE), d2, w, h,
+                                           prev_xy=prev, window=window, nnratio=0.9, check_ori=True)
+    assert ref[0] == (n if kind == "chain" else 1)
+    m, views = ORBmatcher(0.9, True), (FrameView(k1, d1, w, h, s), FrameView(k2, d2, w, h, s))
+    for _ in range(2):
+        t0 = time.perf_counter()
+        nm, m12, _ = m.SearchForInitialization(*views, prev.copy(), window)
+        seconds = time.perf_counter() - t0
+        assert nm == ref[0] and np.array_equal(m12, ref[1])
+    assert seconds < 0.5
+
+
 # tile edges: query pairs of 256 rows, train tiles of 160 and groups of 32,
 # popcount tiles of 256 rows and shares of 32; several runs of one query pair
 @pytest.mark.parametrize("nq,nt", [(1, 31), (31, 32), (33, 33), (128, 159), (129, 160), (255, 161), (256, 255),
