@@ -116,6 +116,16 @@ __device__ __forceinline__ uint64_t cand_key(int dist, int cell, int idx) {
     return ((uint64_t)(uint32_t)dist << 40) | ((uint64_t)(uint32_t)cell << 20) | (uint64_t)(uint32_t)idx;
 }
 
+// A query's row of candidate keys: of slot_cap keys from slots on, one row
+// after the other, or from slots[start[i]] on where start is given (64-bit keys
+// only: rows of the queries' own lengths).
+template <typename Key>
+__device__ __forceinline__ Key* cand_row(Key* slots, int slot_cap, const long long* start, int i) {
+    if constexpr (sizeof(Key) > sizeof(uint32_t))
+        if (start) return slots + start[i];
+    return slots + (size_t)i * slot_cap;
+}
+
 // ----------------------------------------------------------------- SearchForInitialization
 // The candidates of every level-0 keypoint of F1 in the window around
 // prev[i1] (src/ORBmatcher.cc:603-640), one warp each, into rows of slot_cap
@@ -124,8 +134,8 @@ __device__ __forceinline__ uint64_t cand_key(int dist, int cell, int idx) {
 // <= TH_LOW < nnratio * dist): the lists leave it out, and with it all but a
 // few of a window's keypoints.
 __global__ void k_init_candidates(GridDev g2, const orbgpu_keypoint* kps1, const uint8_t* desc1, int n1,
-                                  const float* prev, float window, float nnratio, int slot_cap, uint64_t* slots,
-                                  int* slot_count, int* status) {
+                                  const float* prev, float window, float nnratio, int slot_cap, const long long* start,
+                                  uint64_t* slots, int* slot_count, int* status) {
     const bool drop_far = nnratio <= 1.0f;
     const int lane = threadIdx.x & 31;
     const int i1 = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -137,6 +147,7 @@ __global__ void k_init_candidates(GridDev g2, const orbgpu_keypoint* kps1, const
         const uint4* d1 = reinterpret_cast<const uint4*>(desc1 + (size_t)i1 * 32);
         const uint4 a0 = d1[0], a1 = d1[1];
         const float px = prev[2 * i1], py = prev[2 * i1 + 1];
+        uint64_t* row = cand_row(slots, slot_cap, start, i1);
         warp_window_recs(g2, x0, x1, y0, y1, [&](const GridRec& rec, bool valid) {
             bool ok = valid && in_area(rec, px, py, window, octave, octave);
             int dist = 256;
@@ -147,7 +158,7 @@ __global__ void k_init_candidates(GridDev g2, const orbgpu_keypoint* kps1, const
             }
             const unsigned m = __ballot_sync(0xffffffffu, ok);
             const int pos = total + __popc(m & ((1u << lane) - 1));
-            if (ok && pos < slot_cap) slots[(size_t)i1 * slot_cap + pos] = cand_key(dist, rec.cell(), (int)rec.idx);
+            if (ok && pos < slot_cap) row[pos] = cand_key(dist, rec.cell(), (int)rec.idx);
             total += __popc(m);
         });
     }
@@ -204,8 +215,8 @@ __device__ __forceinline__ bool init_accepts(uint64_t best, int second, float nn
 }
 // The walk, by the calling warp: choice[n1]; least[n2] (the matched distances)
 // holds 0x7fffffff before.
-__device__ __forceinline__ void init_walk(int n1, int slot_cap, const int* slot_count, const uint64_t* slots, float nnratio,
-                                          int* choice, int* least) {
+__device__ __forceinline__ void init_walk(int n1, int slot_cap, const long long* start, const int* slot_count,
+                                          const uint64_t* slots, float nnratio, int* choice, int* least) {
     const int lane = threadIdx.x & 31;
     for (int i0 = 0; i0 < n1; i0 += 32) {
         const int mine = i0 + lane < n1 ? min(slot_count[i0 + lane], slot_cap) : 0;
@@ -215,7 +226,7 @@ __device__ __forceinline__ void init_walk(int n1, int slot_cap, const int* slot_
         while (todo) {
             const int t = __ffs(todo) - 1, cnt = __shfl_sync(0xffffffffu, mine, t);
             todo &= todo - 1;
-            const uint64_t* row = slots + (size_t)(i0 + t) * slot_cap;
+            const uint64_t* row = cand_row(slots, slot_cap, start, i0 + t);
             uint64_t best = ~0ull;
             int second = 0x7fffffff;
             for (int e = lane; e < cnt; e += 32) {
@@ -240,8 +251,8 @@ __device__ __forceinline__ void init_walk(int n1, int slot_cap, const int* slot_
 __host__ __device__ inline size_t init_resolve_bytes(int n1, int n2) { return 4 * (4 * (size_t)n1 + 2 * (size_t)n2); }
 __global__ void __launch_bounds__(1024, 1)
     k_init_resolve(const orbgpu_keypoint* kps1, int n1, const orbgpu_keypoint* kps2, int n2, int slot_cap,
-                   const int* slot_count, const uint64_t* slots, float nnratio, int check_ori, int local, int* work,
-                   int* matches12, int* nmatches_out) {
+                   const long long* start, const int* slot_count, const uint64_t* slots, float nnratio, int check_ori,
+                   int local, int* work, int* matches12, int* nmatches_out) {
     extern __shared__ int s_init[];
     __shared__ int hist[ORBGPU_HISTO_LENGTH];
     __shared__ int s_flag[3], s_long, s_nm, s_ind[3];
@@ -263,7 +274,7 @@ __global__ void __launch_bounds__(1024, 1)
         int mine[2], mdist[2], q = 0;
         auto eval = [&](int i, int& r, int& rd) {
             const int cnt = min(slot_count[i], slot_cap);
-            const uint64_t* row = slots + (size_t)i * slot_cap;
+            const uint64_t* row = cand_row(slots, slot_cap, start, i);
             uint64_t best = ~0ull;
             int second = 0x7fffffff;
             for (int e = 0; e < cnt; e++) {
@@ -326,7 +337,7 @@ __global__ void __launch_bounds__(1024, 1)
     if (!converged) {
         for (int j = tid; j < n2; j += nt) owner[j] = 0x7fffffff;
         __syncthreads();
-        if (tid < 32) init_walk(n1, slot_cap, slot_count, slots, nnratio, choice, owner);
+        if (tid < 32) init_walk(n1, slot_cap, start, slot_count, slots, nnratio, choice, owner);
         __syncthreads();
     }
     // the owner of each F2 keypoint: its last taker
@@ -395,7 +406,8 @@ __global__ void __launch_bounds__(1024, 1)
 #define PROJ_SEG 16
 template <typename Key>
 __global__ void k_proj_candidates(GridDev g, const orbgpu_mappoint* mps, const uint8_t* mp_desc, int m, float th,
-                                  float nnratio, int slot_cap, Key* slots, int* slot_count, int* status) {
+                                  float nnratio, int slot_cap, const long long* start, Key* slots, int* slot_count,
+                                  int* status) {
     const int lane = threadIdx.x & 31;
     const int imp = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * (32 / PROJ_SEG) + lane / PROJ_SEG;
     const bool have = imp < m;
@@ -404,7 +416,7 @@ __global__ void k_proj_candidates(GridDev g, const orbgpu_mappoint* mps, const u
     if (have) mp = mps[imp];
     const ProjFrame F{g.cell_start, g.recs, g.desc, g.uright, g.minX, g.minY, g.invW, g.invH, g.scale};
     const int total = proj_candidates<PROJ_SEG, Key>(F, mp, have, mp_desc + (size_t)imp * 32, th, nnratio,
-                                                     slots + (size_t)imp * slot_cap, slot_cap);
+                                                     cand_row(slots, slot_cap, have ? start : nullptr, imp), slot_cap);
     if (have && (lane & (PROJ_SEG - 1)) == 0) {
         slot_count[imp] = total;
         if (total > slot_cap) atomicMax(status, total);
@@ -427,14 +439,14 @@ __global__ void __launch_bounds__(1024) k_proj_resolve_smem(const orbgpu_keypoin
 // global memory, one launch each, and a serial replay if none converged.
 // In-order resolution (src/ORBmatcher.cc:117-180) by one warp.
 // claimed[] starts with the caller's pre-claimed keypoints.
-__global__ void k_proj_resolve(GridDev g, int m, int slot_cap, const int* slot_count, const uint64_t* slots,
-                               float nnratio, int* match_out, int* nmatches_out, const int* converged_flags) {
+__global__ void k_proj_resolve(GridDev g, int m, int slot_cap, const long long* start, const int* slot_count,
+                               const uint64_t* slots, float nnratio, int* match_out, int* nmatches_out, const int* converged_flags) {
     if (converged_flags && converged_flags[PROJ_ROUNDS - 1] == 0) return;
     const int lane = threadIdx.x;
     int nmatches = 0;
     for (int imp = 0; imp < m; imp++) {
         const int cnt = min(slot_count[imp], slot_cap);
-        const uint64_t* row = slots + (size_t)imp * slot_cap;
+        const uint64_t* row = cand_row(slots, slot_cap, start, imp);
         if (cnt == 0) continue;
         uint64_t best = ~0ull, second = ~0ull;
         for (int b = 0; b < cnt; b += 32) {
@@ -482,8 +494,8 @@ __global__ void k_proj_resolve(GridDev g, int m, int slot_cap, const int* slot_c
 // claims of round r-1's results; when a round changes nothing the results
 // equal the sequential ones.  Pre-claimed keypoints (match_out == -2) are
 // always excluded.  k_proj_resolve replays serially if no round converged.
-__global__ void k_proj_round(GridDev g, int m, int slot_cap, const int* slot_count, const uint64_t* slots,
-                             float nnratio, int round, int* claims3, int* res, int* changed, const int* pre) {
+__global__ void k_proj_round(GridDev g, int m, int slot_cap, const long long* start, const int* slot_count,
+                             const uint64_t* slots, float nnratio, int round, int* claims3, int* res, int* changed, const int* pre) {
     const int lane = threadIdx.x & 31;
     const int local = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const int nwarps = gridDim.x * (blockDim.x >> 5);
@@ -495,7 +507,7 @@ __global__ void k_proj_round(GridDev g, int m, int slot_cap, const int* slot_cou
     for (int i = local * 32 + lane; i < n; i += nwarps * 32) claims_z[i] = PROJ_NONE;
     if (local >= m) return;
     const int cnt = min(slot_count[local], slot_cap);
-    const uint64_t* row = slots + (size_t)local * slot_cap;
+    const uint64_t* row = cand_row(slots, slot_cap, start, local);
     uint64_t best = ~0ull, second = ~0ull;
     for (int b = 0; b < cnt; b += 32) {
         uint64_t key = ~0ull;
@@ -1176,6 +1188,43 @@ static int candidate_lists(orbgpu_matcher* m, int nq, Bump& b, Launch launch, in
     return ORBGPU_OK;
 }
 
+// The candidate rows of a search's nq queries (cand_row): of 64 keys, widened
+// where a window holds more; rows of the queries' own lengths where a few
+// crowded windows would make wide rows take more than CAND_ROWS_BYTES.
+#define CAND_ROWS_BYTES ((size_t)1 << 30)
+struct CandRows {
+    int cap = 64;
+    std::vector<long long> start;  // empty: rows of 'cap' keys
+    size_t keys;                   // in all rows
+
+    explicit CandRows(int nq) : keys((size_t)64 * nq) {}
+    // after a call whose longest row was 'longest'; count: the queries' candidates (device)
+    int widen(orbgpu_matcher* m, int nq, int longest, const int* count, size_t key_bytes, bool own_lengths) {
+        cap = (longest + 63) / 64 * 64;
+        keys = (size_t)nq * cap;
+        if (!own_lengths || keys * key_bytes <= CAND_ROWS_BYTES) return ORBGPU_OK;
+        std::vector<int> n(nq);
+        ORBGPU_CUDA_TRY(cudaMemcpyAsync(n.data(), count, sizeof(int) * nq, cudaMemcpyDeviceToHost, m->stream));
+        ORBGPU_CUDA_TRY(cudaStreamSynchronize(m->stream));
+        start.resize(nq);
+        keys = 0;
+        for (int i = 0; i < nq; i++) {
+            start[i] = (long long)keys;
+            keys += n[i];
+        }
+        return ORBGPU_OK;
+    }
+    size_t bytes(size_t key_bytes) const { return key_bytes * std::max<size_t>(1, keys) + sizeof(long long) * start.size() + 512; }
+    int stage(orbgpu_matcher* m, Bump& b, const long long** d_start) const {
+        *d_start = nullptr;
+        if (start.empty()) return ORBGPU_OK;
+        long long* d = b.take<long long>(start.size());
+        ORBGPU_CUDA_TRY(cudaMemcpyAsync(d, start.data(), sizeof(long long) * start.size(), cudaMemcpyHostToDevice, m->stream));
+        *d_start = d;
+        return ORBGPU_OK;
+    }
+};
+
 extern "C" int orbgpu_search_for_initialization(orbgpu_matcher* m, const orbgpu_frame* f1, const orbgpu_frame* f2,
                                                 float* prev_matched, int* matches12, int window_size, int* nmatches) {
     if (!m || !frame_ok(f1) || !frame_ok(f2) || !prev_matched || !matches12 || !nmatches) return ORBGPU_ERR_BAD_ARG;
@@ -1183,10 +1232,10 @@ extern "C" int orbgpu_search_for_initialization(orbgpu_matcher* m, const orbgpu_
     *nmatches = 0;
     for (int i = 0; i < n1; i++) matches12[i] = -1;
     if (n1 == 0) return ORBGPU_OK;
-    int slot_cap = 64;
+    CandRows rows(n1);
     for (int attempt = 0; attempt < 2; attempt++) {
         const size_t est = frame_stage_bytes(f1) + frame_stage_bytes(f2) + grid_bytes(n2) + (size_t)n1 * 5 * sizeof(int) +
-                           init_resolve_bytes(n1, n2) + sizeof(uint64_t) * (size_t)n1 * slot_cap + 16 * 1024;
+                           init_resolve_bytes(n1, n2) + rows.bytes(sizeof(uint64_t)) + 16 * 1024;
         int rc = ensure_scratch(m, est);
         if (rc) return rc;
         Bump b{(uint8_t*)m->scratch, 0, m->scratch_bytes};
@@ -1200,24 +1249,26 @@ extern "C" int orbgpu_search_for_initialization(orbgpu_matcher* m, const orbgpu_
         int* m12 = b.take<int>(n1);
         int* d_status = b.take<int>(2);  // most candidates of a keypoint, matches
         int* work = b.take<int>(init_resolve_bytes(n1, n2) / sizeof(int));
-        uint64_t* slots = b.take<uint64_t>((size_t)n1 * slot_cap);
+        uint64_t* slots = b.take<uint64_t>(std::max<size_t>(1, rows.keys));
+        const long long* d_start;
+        if ((rc = rows.stage(m, b, &d_start))) return rc;
         ORBGPU_CUDA_TRY(cudaMemsetAsync(d_status, 0, 2 * sizeof(int), m->stream));
         const int wpb = 8;
         k_init_candidates<<<(n1 + wpb - 1) / wpb, 32 * wpb, 0, m->stream>>>(g2, s1.kps, s1.desc, n1, d_prev,
-                                                                         (float)window_size, m->nnratio, slot_cap, slots,
-                                                                         count, d_status);
+                                                                         (float)window_size, m->nnratio, rows.cap, d_start,
+                                                                         slots, count, d_status);
         // the resolution's arrays in shared memory up to 200 KiB (8,500
         // keypoints a frame), else in the scratch
         const int local = init_resolve_bytes(n1, n2) <= 200 * 1024;
         ORBGPU_CUDA_TRY(allow_max_dynamic_smem(k_init_resolve));
         k_init_resolve<<<1, 1024, local ? init_resolve_bytes(n1, n2) : 0, m->stream>>>(
-            s1.kps, n1, s2.kps, n2, slot_cap, count, slots, m->nnratio, m->check_ori, local, work, m12, d_status + 1);
+            s1.kps, n1, s2.kps, n2, rows.cap, d_start, count, slots, m->nnratio, m->check_ori, local, work, m12, d_status + 1);
         ORBGPU_CUDA_TRY(cudaGetLastError());
         ORBGPU_CUDA_TRY(cudaMemcpyAsync(m->h_pinned, d_status, 2 * sizeof(int), cudaMemcpyDeviceToHost, m->stream));
         ORBGPU_CUDA_TRY(cudaMemcpyAsync(matches12, m12, sizeof(int) * n1, cudaMemcpyDeviceToHost, m->stream));
         ORBGPU_CUDA_TRY(cudaStreamSynchronize(m->stream));
-        if (m->h_pinned[0] > slot_cap) {  // a window held more candidates than a row: widen and redo
-            slot_cap = ((m->h_pinned[0] + 63) / 64) * 64;
+        if (m->h_pinned[0] > rows.cap) {  // a window held more candidates than a row: widen and redo
+            if ((rc = rows.widen(m, n1, m->h_pinned[0], count, sizeof(uint64_t), true))) return rc;
             continue;
         }
         *nmatches = m->h_pinned[1];
@@ -1250,11 +1301,10 @@ extern "C" int orbgpu_search_by_projection(orbgpu_matcher* m, const orbgpu_frame
     // with 64-bit keys in global-memory rounds
     const bool smem = n < ORBGPU_KEY32_MAX_N && proj_resolve_smem(n, M) <= 200 * 1024;
     const size_t key_bytes = smem ? sizeof(uint32_t) : sizeof(uint64_t);
-    int slot_cap = 64;
+    CandRows rows(M);
     for (int attempt = 0; attempt < 2; attempt++) {
-        const size_t est = frame_stage_bytes(f) + grid_bytes(n) +
-                           (size_t)std::max(1, M) * (sizeof(orbgpu_mappoint) + 32 + 16 + key_bytes * slot_cap) +
-                           (size_t)std::max(1, n) * 24 + 64 * 1024;
+        const size_t est = frame_stage_bytes(f) + grid_bytes(n) + (size_t)std::max(1, M) * (sizeof(orbgpu_mappoint) + 32 + 16) +
+                           rows.bytes(key_bytes) + (size_t)std::max(1, n) * 24 + 64 * 1024;
         int rc = ensure_scratch(m, est);
         if (rc) return rc;
         Bump b{(uint8_t*)m->scratch, 0, m->scratch_bytes};
@@ -1284,20 +1334,22 @@ extern "C" int orbgpu_search_by_projection(orbgpu_matcher* m, const orbgpu_frame
         }
         int* d_status = b.take<int>(3);  // most candidates of a map point, not converged, matches
         int* count = b.take<int>(std::max(1, M));
-        void* slots = b.take<uint8_t>(key_bytes * (size_t)std::max(1, M) * slot_cap);
+        void* slots = b.take<uint8_t>(key_bytes * std::max<size_t>(1, rows.keys));
+        const long long* d_start;
+        if ((rc = rows.stage(m, b, &d_start))) return rc;
         ORBGPU_CUDA_TRY(cudaMemsetAsync(d_status, 0, 3 * sizeof(int), m->stream));
         const int wpb = 8, mpb = wpb * (32 / PROJ_SEG);
         if (smem) {
             if (M > 0)
                 k_proj_candidates<uint32_t><<<(M + mpb - 1) / mpb, 32 * wpb, 0, m->stream>>>(
-                    g, d_mps, d_mpd, M, th, m->nnratio, slot_cap, (uint32_t*)slots, count, d_status);
+                    g, d_mps, d_mpd, M, th, m->nnratio, rows.cap, d_start, (uint32_t*)slots, count, d_status);
             ORBGPU_CUDA_TRY(allow_max_dynamic_smem(k_proj_resolve_smem));
             k_proj_resolve_smem<<<1, 1024, proj_resolve_smem(n, M), m->stream>>>(
-                s.kps, n, M, (const uint32_t*)slots, slot_cap, count, m->nnratio, d_claimed, d_match, d_status + 2, d_status);
+                s.kps, n, M, (const uint32_t*)slots, rows.cap, count, m->nnratio, d_claimed, d_match, d_status + 2, d_status);
         } else {
             if (M > 0)
                 k_proj_candidates<uint64_t><<<(M + mpb - 1) / mpb, 32 * wpb, 0, m->stream>>>(
-                    g, d_mps, d_mpd, M, th, m->nnratio, slot_cap, (uint64_t*)slots, count, d_status);
+                    g, d_mps, d_mpd, M, th, m->nnratio, rows.cap, d_start, (uint64_t*)slots, count, d_status);
             if (n > 0) k_init_match_out<<<(n + 255) / 256, 256, 0, m->stream>>>(d_claimed, n, d_match);
             int* claims3 = b.take<int>((size_t)3 * std::max(1, n));
             int* res = b.take<int>(std::max(1, M));
@@ -1309,10 +1361,10 @@ extern "C" int orbgpu_search_by_projection(orbgpu_matcher* m, const orbgpu_frame
                 const int warps = std::max(M, (n + 31) / 32);
                 for (int r = 0; r < PROJ_ROUNDS; r++)
                     k_proj_round<<<(warps + wpb - 1) / wpb, 32 * wpb, 0, m->stream>>>(
-                        g, M, slot_cap, count, (const uint64_t*)slots, m->nnratio, r, claims3, res, changed, d_match);
+                        g, M, rows.cap, d_start, count, (const uint64_t*)slots, m->nnratio, r, claims3, res, changed, d_match);
                 k_proj_finish<<<1, 256, 0, m->stream>>>(M, changed, res, d_match, d_status + 2);
-                k_proj_resolve<<<1, 32, 0, m->stream>>>(g, M, slot_cap, count, (const uint64_t*)slots, m->nnratio, d_match,
-                                                        d_status + 2, changed);
+                k_proj_resolve<<<1, 32, 0, m->stream>>>(g, M, rows.cap, d_start, count, (const uint64_t*)slots, m->nnratio,
+                                                        d_match, d_status + 2, changed);
             }
         }
         ORBGPU_CUDA_TRY(cudaGetLastError());
@@ -1320,8 +1372,9 @@ extern "C" int orbgpu_search_by_projection(orbgpu_matcher* m, const orbgpu_frame
         if (mem != ORBGPU_MEM_DEVICE && n > 0)
             ORBGPU_CUDA_TRY(cudaMemcpyAsync(match_out, d_match, sizeof(int) * n, cudaMemcpyDeviceToHost, m->stream));
         ORBGPU_CUDA_TRY(cudaStreamSynchronize(m->stream));
-        if (m->h_pinned[0] > slot_cap) {  // a window held more candidates than a row: widen and redo
-            slot_cap = ((m->h_pinned[0] + 63) / 64) * 64;
+        if (m->h_pinned[0] > rows.cap) {  // a window held more candidates than a row: widen and redo
+            // (the one-block resolution reads rows of one length, of 4,095 keys at most)
+            if ((rc = rows.widen(m, M, m->h_pinned[0], count, key_bytes, !smem))) return rc;
             continue;
         }
         if (m->h_pinned[1]) {

@@ -388,6 +388,38 @@ def test_initialization_search_long_dependencies(torch, oracle, kind, n):
     assert seconds < 0.5
 
 
+@pytest.mark.parametrize("crowded", [1, 3000])
+def test_searches_with_a_crowded_window(torch, oracle, crowded):
+    """A million queries of which one has a window of 40,000 candidates (rows of
+    that many keys would be 320 GB), or 3,000 have one of 20,000: both searches'
+    rows take what the candidates take."""
+    from oracle import pyoracle
+    from orb_slam2_detailed_comments_gb300 import FrameView, ORBmatcher
+    from orb_slam2_detailed_comments_gb300._lib import KEYPOINT_DTYPE, MAPPOINT_DTYPE
+    n1, n2 = (1000000, 40000) if crowded == 1 else (20000, 20000)
+    rng = np.random.default_rng(n2)
+    k2, d2 = plain_frame(rng.uniform(99, 101, n2), rng.uniform(99, 101, n2), np.where(np.arange(n2), 1 + np.arange(n2) % 50, 0))
+    k1, d1 = np.zeros(n1, KEYPOINT_DTYPE), np.zeros((n1, 32), np.uint8)
+    k1["x"], k1["y"], k1["octave"] = 100, 100, 1  # not searched for, but:
+    at = rng.choice(n1, crowded, replace=False)
+    k1["octave"][at] = 0
+    d1[at[1:], 0] = rng.integers(0, 256, crowded - 1)
+    prev = np.ascontiguousarray(np.stack([k1["x"], k1["y"]], 1))
+    s, _ = pyoracle.scale_tables(8, 1.2)
+    ref = oracle.search_for_initialization(k1.view(pyoracle.KP_DTYPE), d1, k2.view(pyoracle.KP_DTYPE), d2, 640, 480,
+                                           prev_xy=prev, window=10, nnratio=0.9, check_ori=True)
+    view = FrameView(k2, d2, 640, 480, s)
+    nm, m12, _ = ORBmatcher(0.9, True).SearchForInitialization(FrameView(k1, d1, 640, 480, s), view, prev.copy(), 10)
+    assert nm == ref[0] > 0 and np.array_equal(m12, ref[1])
+    mps = np.zeros(n1, MAPPOINT_DTYPE)
+    mps["proj_x"], mps["proj_y"], mps["proj_xr"], mps["view_cos"] = 100, 100, -1, 1.0
+    mps["track_in_view"] = k1["octave"] == 0
+    ref = oracle.search_by_projection(k2.view(pyoracle.KP_DTYPE), d2, 640, 480, mps.view(pyoracle.MP_DTYPE), d1, th=2.0,
+                                      nnratio=0.9, claimed=np.zeros(n2, np.uint8))
+    nm, match = ORBmatcher(0.9, True).SearchByProjection(view, mps, d1, 2.0)
+    assert nm == ref[0] > 0 and np.array_equal(match, ref[1])
+
+
 # tile edges: query pairs of 256 rows, train tiles of 160 and groups of 32,
 # popcount tiles of 256 rows and shares of 32; several runs of one query pair
 @pytest.mark.parametrize("nq,nt", [(1, 31), (31, 32), (33, 33), (128, 159), (129, 160), (255, 161), (256, 255),
